@@ -78,14 +78,14 @@ int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, in
     const int tn = tile_width(policy, b.n);
     MDG_TRY(mdgi::encode_plane_map(g.tmA, b.dA, b.Kp, (long long)b.s * b.Mp, 128));
     MDG_TRY(mdgi::encode_plane_map(g.tmB, b.dB, b.Kp, (long long)b.s * b.Np, pair ? 128 : tn));
+    MDG_TRY(mdgi::encode_out_map(g.tmC, b.chunks, b.Np,
+                                 (long long)mdgi::total_chunks(b.s, b.D, b.Kp / 64) * b.Mp));
     g.s = b.s; g.D = b.D; g.Mp = b.Mp; g.Np = b.Np; g.KB = b.Kp / 64;
     g.tn = tn;
     g.mt = pair ? b.Mp / 256 : (b.m + 127) / 128;
     g.nt = (b.n + tn - 1) / tn;
     g.ktail = (b.k - (g.KB - 1) * 64 + 15) / 16;
     g.parts = 1;
-    g.out = b.chunks;
-    g.plane_c = b.plane_c;
     hg->push_back(g);
   }
   // work of one tile in k-steps of 128 x 128 output: digit pairs x k-blocks

@@ -40,7 +40,10 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr int TMEM_COLS = 512;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /* align */ + 256 /* barriers */;
+// per epilogue warp: a 32 x 32 int32 block on its way out
+constexpr int OUT_BYTES = 32 * 32 * 4;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * OUT_BYTES + 1024 /* align */ +
+                           256 /* barriers */;
 constexpr unsigned long long TIMEOUT_NS = 2000000000ull;
 
 // kind::f16 instruction descriptor: D F32 (bits 4-5 = 1), A BF16 (7-9 = 1),
@@ -208,6 +211,49 @@ __device__ __forceinline__ void drain128(uint32_t taddr, int (&acc)[128]) {
   add_exact(acc + 96, rb);
 }
 
+// Stores a warp's 32 rows x 128 columns of int32 sums (row = lane) at (x, y)
+// of the output planes and clears them.  Through shared memory and the TMA,
+// 32 columns at a time: a thread holds a row, so storing from registers
+// touches 32 lines per instruction and the L1 takes them one a cycle (8192
+// cycles for a CTA's 128 x 256 block, as long as a whole flush group, during
+// which the accumulators are not drained).  The staging block has the
+// 128-byte swizzle of the tensor map, so the 16-byte writes of eight rows
+// hit different banks.  Against stores from registers: double-double 64^3
+// 119 -> 106 us, a batch of 64 mixed problems 4.09 -> 3.84 ms a call.
+__device__ __forceinline__ void store_rows(uint32_t staging, int lane, int (&acc)[128],
+                                           const CUtensorMap *tm, int x, int y) {
+  const uint32_t line = staging + lane * 128;
+#pragma unroll
+  for (int cb = 0; cb < 4; ++cb) {
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      int *a = acc + 32 * cb + 4 * v;
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                       line + ((uint32_t)(v ^ (lane & 7)) << 4)),
+                   "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3])
+                   : "memory");
+      a[0] = a[1] = a[2] = a[3] = 0;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+      asm volatile(
+          "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+              reinterpret_cast<uint64_t>(tm)),
+          "r"(x + 32 * cb), "r"(y), "r"(staging)
+          : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+}
+
+// Waits until this thread's stores have been written.
+__device__ __forceinline__ void stores_done() {
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // Diagonals [d0, d1) of part `part` of a tile cut into `parts` ranges whose
 // digit-pair counts add up to about 1/parts of the tile's pairs each (empty
 // when parts exceeds what the pair counts allow).
@@ -236,23 +282,19 @@ __device__ __forceinline__ void part_diagonals(int s, int D, int part, int parts
 // rows); ktail: MMAs of K = 16 issued for the last k-block (1..4; the rest
 // of that block is the zero padding of k).
 struct TileJob {
-  const CUtensorMap *tmA, *tmB;
+  const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, row, col, tn, ktail, d0, d1;
-  int *out;
-  long long plane_c;
 };
 
 // A single problem cut into 128 x 256 tiles.
 struct SingleJobs {
-  const CUtensorMap *tmA, *tmB;
+  const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB;
-  int *out;
-  long long plane_c;
   __device__ int tiles() const { return (Mp / TM) * (Np / TN); }
   __device__ TileJob job(int t) const {
     const int MB = Mp / TM;
-    return TileJob{tmA, tmB, s, D, Mp, Np, KB, (t % MB) * TM, (t / MB) * TN, TN, TK / 16,
-                   0, D, out, plane_c};
+    return TileJob{tmA, tmB, tmC, s, D, Mp, Np, KB, (t % MB) * TM, (t / MB) * TN, TN, TK / 16,
+                   0, D};
   }
 };
 
@@ -261,7 +303,7 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES + EPI_WARPS * OUT_BYTES);
   // bars: [0,4) full, [4,8) empty, [8,10) accfull, [10,12) accempty, 12 mma drain
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + 16);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 17);
@@ -391,6 +433,7 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
   } else {
     // -------------------------------------------------------- epilogue --
     const int q = warp & 3, h = (warp - 2) >> 2;
+    const uint32_t staging = smem_base + STAGES * STAGE_BYTES + (warp - 2) * OUT_BYTES;
     int acc[128];
 #pragma unroll
     for (int j = 0; j < 128; ++j) acc[j] = 0;
@@ -402,7 +445,7 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
       // alone (128 columns each, as for a 256-column tile); the others only
       // release the accumulator
       const bool active = jb.tn == TN || h == 0;
-      const int row = jb.row + 32 * q + lane;
+      const int row = jb.row + 32 * q;
       const int col = jb.col + 128 * h;
       int chunk = 0;
       for (int d = 0; d < jb.d0; ++d) chunk += mdgi::diag_chunks(d, jb.s, jb.KB);
@@ -425,21 +468,14 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
           buf ^= 1;
           const int g1 = g0 + mdgi::GROUP_STEPS;
           if (g1 % mdgi::CHUNK_STEPS == 0 || g1 >= S) {
-            if (active) {
-              int4 *dst = reinterpret_cast<int4 *>(jb.out + (size_t)chunk * jb.plane_c +
-                                                   (size_t)row * jb.Np + col);
-#pragma unroll
-              for (int v = 0; v < 32; ++v) {
-                dst[v] = make_int4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
-                acc[4 * v] = acc[4 * v + 1] = acc[4 * v + 2] = acc[4 * v + 3] = 0;
-              }
-            }
+            if (active) store_rows(staging, lane, acc, jb.tmC, col, chunk * jb.Mp + row);
             ++chunk;
           }
         }
       }
     }
-  epi_done:;
+  epi_done:
+    if (lane == 0) stores_done();
   }
   __syncwarp();
   fence_before();
@@ -455,9 +491,10 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
 
 __global__ void __launch_bounds__(THREADS, 1)
     diag_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,
-                        const __grid_constant__ CUtensorMap tmB, int s, int D, int Mp, int Np,
-                        int KB, int *__restrict__ out, long long plane_c) {
-  tc1_body(SingleJobs{&tmA, &tmB, s, D, Mp, Np, KB, out, plane_c});
+                        const __grid_constant__ CUtensorMap tmB,
+                        const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
+                        int KB) {
+  tc1_body(SingleJobs{&tmA, &tmB, &tmC, s, D, Mp, Np, KB});
 }
 
 // Many problems: a table of GroupedProblem in global memory (tensor maps
@@ -485,9 +522,9 @@ struct GroupedJobs {
     int d0, d1;
     part_diagonals(g.s, g.D, part, g.parts, d0, d1);
     return TileJob{reinterpret_cast<const CUtensorMap *>(g.tmA),
-                   reinterpret_cast<const CUtensorMap *>(g.tmB), g.s, g.D, g.Mp, g.Np, g.KB,
-                   (tile % g.mt) * TM, (tile / g.mt) * g.tn, g.tn, g.ktail, d0, d1, g.out,
-                   g.plane_c};
+                   reinterpret_cast<const CUtensorMap *>(g.tmB),
+                   reinterpret_cast<const CUtensorMap *>(g.tmC), g.s, g.D, g.Mp, g.Np, g.KB,
+                   (tile % g.mt) * TM, (tile / g.mt) * g.tn, g.tn, g.ktail, d0, d1};
   }
 };
 
@@ -519,7 +556,7 @@ constexpr int STAGES2 = 6;
 constexpr int A2_BYTES = TM * TK * 2;  // 16 KiB
 constexpr int B2_BYTES = BH * TK * 2;  // 16 KiB
 constexpr int STAGE2_BYTES = A2_BYTES + B2_BYTES;
-constexpr int SMEM2_BYTES = STAGES2 * STAGE2_BYTES + 1024 + 256;
+constexpr int SMEM2_BYTES = STAGES2 * STAGE2_BYTES + EPI_WARPS * OUT_BYTES + 1024 + 256;
 constexpr uint32_t IDESC2 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN2 >> 3) << 17) |
                             ((uint32_t)(256 >> 4) << 24);
 
@@ -616,10 +653,8 @@ __device__ __forceinline__ uint32_t pace_load(int slot, int ncl, uint32_t epoch)
 // One unit of work of the pair kernel: a 256 x 256 tile of one problem
 // (rows row0.., columns col0..) and the diagonals [d0, d1) it computes.
 struct PairJob {
-  const CUtensorMap *tmA, *tmB;
+  const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, row0, col0, d0, d1;
-  int *out;
-  long long plane_c;
 };
 
 // A single problem: units are tiles, or parts of tiles (ranges of
@@ -629,10 +664,8 @@ struct PairJob {
 // the same time read few distinct A row blocks and B column blocks and share
 // them in L2 (raster = 1 walks each column block top to bottom).
 struct PairSingle {
-  const CUtensorMap *tmA, *tmB;
+  const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB;
-  int *out;
-  long long plane_c;
   int parts, raster;
   __device__ int units() const { return (Mp / 256) * (Np / TN2) * parts; }
   __device__ PairJob job(int u) const {
@@ -645,7 +678,7 @@ struct PairSingle {
     const int c0 = strip * raster;
     const int g = NB - c0 < raster ? NB - c0 : raster;
     const int rb = idx / g, cb = c0 + idx - rb * g;
-    return PairJob{tmA, tmB, s, D, Mp, Np, KB, rb * 256, cb * TN2, d0, d1, out, plane_c};
+    return PairJob{tmA, tmB, tmC, s, D, Mp, Np, KB, rb * 256, cb * TN2, d0, d1};
   }
 };
 
@@ -663,8 +696,9 @@ struct PairGrouped {
     int d0, d1;
     part_diagonals(g.s, g.D, part, g.parts, d0, d1);
     return PairJob{reinterpret_cast<const CUtensorMap *>(g.tmA),
-                   reinterpret_cast<const CUtensorMap *>(g.tmB), g.s, g.D, g.Mp, g.Np, g.KB,
-                   (tile % g.mt) * 256, (tile / g.mt) * TN2, d0, d1, g.out, g.plane_c};
+                   reinterpret_cast<const CUtensorMap *>(g.tmB),
+                   reinterpret_cast<const CUtensorMap *>(g.tmC), g.s, g.D, g.Mp, g.Np, g.KB,
+                   (tile % g.mt) * 256, (tile / g.mt) * TN2, d0, d1};
   }
 };
 
@@ -674,7 +708,8 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES2 * STAGE2_BYTES);
+  uint64_t *bars =
+      reinterpret_cast<uint64_t *>(smem + STAGES2 * STAGE2_BYTES + EPI_WARPS * OUT_BYTES);
   // bars: STAGES2 full, STAGES2 empty, 2 accfull, 2 accempty, 1 drain, then
   // the TMEM address and the abort flag
   static_assert(2 * STAGES2 + 9 <= 32, "barrier area holds 32 words of 8 bytes");
@@ -858,6 +893,7 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
   } else {
     // -------------------------------------------------------- epilogue --
     const int q = warp & 3, h = (warp - 2) >> 2;
+    const uint32_t staging = smem_base + STAGES2 * STAGE2_BYTES + (warp - 2) * OUT_BYTES;
     int acc[128];
 #pragma unroll
     for (int j = 0; j < 128; ++j) acc[j] = 0;
@@ -866,7 +902,7 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
     const uint32_t accempty0[2] = {map_to_rank0(accempty(0)), map_to_rank0(accempty(1))};
     for (int u = cid; u < units; u += ncl) {
       const PairJob jb = jobs.job(u);
-      const int row = jb.row0 + (int)rank * TM + 32 * q + lane;
+      const int row = jb.row0 + (int)rank * TM + 32 * q;
       const int col = jb.col0 + 128 * h;
       int chunk = 0;
       for (int d = 0; d < jb.d0; ++d) chunk += mdgi::diag_chunks(d, jb.s, jb.KB);
@@ -887,19 +923,14 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
           buf ^= 1;
           const int g1 = g0 + mdgi::GROUP_STEPS;
           if (g1 % mdgi::CHUNK_STEPS == 0 || g1 >= S) {
-            int4 *dst = reinterpret_cast<int4 *>(jb.out + (size_t)chunk * jb.plane_c +
-                                                 (size_t)row * jb.Np + col);
-#pragma unroll
-            for (int v = 0; v < 32; ++v) {
-              dst[v] = make_int4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
-              acc[4 * v] = acc[4 * v + 1] = acc[4 * v + 2] = acc[4 * v + 3] = 0;
-            }
+            store_rows(staging, lane, acc, jb.tmC, col, chunk * jb.Mp + row);
             ++chunk;
           }
         }
       }
     }
-  epi_done:;
+  epi_done:
+    if (lane == 0) stores_done();
   }
   __syncwarp();
   fence_before();
@@ -914,11 +945,10 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
     diag_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA,
-                         const __grid_constant__ CUtensorMap tmB, int s, int D, int Mp, int Np,
-                         int KB, int *__restrict__ out, long long plane_c, int parts,
-                         int raster, int pace, uint32_t epoch, int no_loads) {
-  tc2_body(PairSingle{&tmA, &tmB, s, D, Mp, Np, KB, out, plane_c, parts, raster}, pace, epoch,
-           no_loads);
+                         const __grid_constant__ CUtensorMap tmB,
+                         const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
+                         int KB, int parts, int raster, int pace, uint32_t epoch, int no_loads) {
+  tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, parts, raster}, pace, epoch, no_loads);
 }
 
 // The batched plan's grouped GEMM on CTA pairs (no pacing: the clusters work
@@ -959,6 +989,21 @@ int make_map(CUtensorMap *m, const void *base, int Kp, long long rows_total, int
   return r == CUDA_SUCCESS ? MDG_SUCCESS : MDG_ERROR_NOT_SUPPORTED;
 }
 
+// 2-D map over `planes` int32 output planes of rows x Np, box 32 x 32,
+// 128-byte swizzle (store_rows).
+int make_out_map(CUtensorMap *m, const void *base, int Np, long long rows_total) {
+  auto fn = encode_fn();
+  if (!fn) return MDG_ERROR_NOT_SUPPORTED;
+  cuuint64_t dims[2] = {(cuuint64_t)Np, (cuuint64_t)rows_total};
+  cuuint64_t strides[1] = {(cuuint64_t)Np * 4};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void *>(base), dims, strides, box,
+                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? MDG_SUCCESS : MDG_ERROR_NOT_SUPPORTED;
+}
+
 }  // namespace
 
 namespace mdgi {
@@ -973,7 +1018,9 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, co
     return MDG_ERROR_INVALID_SIZE;
   // the CTA-pair kernel needs 256-row tiles
   const bool pair = (Mp % 256 == 0) && !single;
-  CUtensorMap ma, mb;
+  if (plane_c != (long long)Mp * Np) return MDG_ERROR_INVALID_SIZE;
+  CUtensorMap ma, mb, mc;
+  MDG_TRY(make_out_map(&mc, chunks, Np, (long long)total_chunks(s, D, Kp / TK) * Mp));
   MDG_TRY(make_map(&ma, dA, Kp, (long long)s * Mp, TM));
   MDG_TRY(make_map(&mb, dB, Kp, (long long)s * Np, pair ? BH : TN));
   int dev = 0, sms = 0;
@@ -1038,12 +1085,11 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, co
     const char *nl = std::getenv("MDG_TC_SELFTEST_NO_LOADS");
     const int no_loads = (nl && *nl == '1') ? 1 : 0;
     diag_gemm_tc2_kernel<<<2 * clusters, THREADS2, SMEM2_BYTES, st>>>(
-        ma, mb, s, D, Mp, Np, Kp / TK, chunks, plane_c, parts, raster, pace, epoch, no_loads);
+        ma, mb, mc, s, D, Mp, Np, Kp / TK, parts, raster, pace, epoch, no_loads);
   } else {
     const int tiles = (Mp / TM) * (Np / TN);
     const int grid = tiles < sms ? tiles : sms;
-    diag_gemm_tc_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(ma, mb, s, D, Mp, Np, Kp / TK, chunks,
-                                                           plane_c);
+    diag_gemm_tc_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(ma, mb, mc, s, D, Mp, Np, Kp / TK);
   }
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
@@ -1051,6 +1097,10 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, co
 
 int encode_plane_map(void *map128, const void *base, int Kp, long long rows_total, int box_rows) {
   return make_map(reinterpret_cast<CUtensorMap *>(map128), base, Kp, rows_total, box_rows);
+}
+
+int encode_out_map(void *map128, const void *base, int Np, long long rows_total) {
+  return make_out_map(reinterpret_cast<CUtensorMap *>(map128), base, Np, rows_total);
 }
 
 int launch_diag_gemm_grouped(const GroupedProblem *dev_probs, int count, int total_units,

@@ -101,11 +101,11 @@ int launch_renorm(int p, int s, int D, int KB, int m, int n, const int *chunks,
 struct alignas(64) GroupedProblem {
   unsigned char tmA[128];  // CUtensorMap, A planes, box 64 x 128
   unsigned char tmB[128];  // CUtensorMap, B planes, box 64 x tn (pairs: 64 x 128)
+  unsigned char tmC[128];  // CUtensorMap, int32 output chunk planes, box 32 x 32
   int s, D, Mp, Np, KB, unit_begin, tn, mt, nt, ktail, parts;
-  int *out;
-  long long plane_c;
 };
 int encode_plane_map(void *map128, const void *base, int Kp, long long rows_total, int box_rows);
+int encode_out_map(void *map128, const void *base, int Np, long long rows_total);
 // The batched plan's entries in the tuning cache (plan.cu), under the
 // current device: the tile policy and split mode recorded for a batch key,
 // if any (left alone otherwise; a record without a split mode sets only the
