@@ -110,6 +110,12 @@ int mdg_default_fp64_digits(int p);
 size_t mdg_gemm_workspace_size(int form, int p, int m, int n, int k,
                                const mdg_options *opt);
 
+/* Bytes that mdg_gemm cannot do without (the BF16 form on large problems is
+ * faster with mdg_gemm_workspace_size bytes, in which it keeps sums of digit
+ * planes; with fewer, down to these, it returns the same bits). */
+size_t mdg_gemm_least_workspace_size(int form, int p, int m, int n, int k,
+                                     const mdg_options *opt);
+
 /* C = A * B, all device pointers, asynchronous on `stream`.
  * Replaces matmulTCnt (TCcuda.cu:248, form PLAIN) and the split GEMM of
  * TCtest.cu:48-114 (form FP64_SPLIT); any m, n, k >= 0. */

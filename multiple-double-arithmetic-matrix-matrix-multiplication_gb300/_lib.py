@@ -36,6 +36,7 @@ SIGNATURES = {
     "mdg_default_slices": (c_int, [c_int]),
     "mdg_default_fp64_digits": (c_int, [c_int]),
     "mdg_gemm_workspace_size": (c_size, [c_int] * 5 + [_P_OPT]),
+    "mdg_gemm_least_workspace_size": (c_size, [c_int] * 5 + [_P_OPT]),
     "mdg_gemm": (c_int, [c_int] * 5 + [c_vp, c_int, c_vp, c_int, c_vp, c_int, _P_OPT, c_vp, c_size,
                                         c_vp]),
     "mdg_gemm_host": (c_int, [c_int] * 5 + [c_vp, c_vp, c_vp, _P_OPT]),

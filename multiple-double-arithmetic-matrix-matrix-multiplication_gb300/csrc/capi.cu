@@ -226,6 +226,12 @@ static size_t workspace_bytes(int form, int p, int m, int n, int k, const Opts &
   if (form == MDG_FORM_PLAIN) return 0;
   if (form == MDG_FORM_FP64_SPLIT) return make_split_plan(p, o.split_kind, m, n, k).total;
   if (form == MDG_FORM_FP64_DIGITS) return make_digits64_plan(p, o.slices, o.diagonals, m, n, k).total;
+  return best_slice_plan(p, o.slices, o.diagonals, m, n, k).total;
+}
+
+// The same without sum planes: what mdg_gemm cannot do with less than.
+static size_t least_workspace_bytes(int form, int p, int m, int n, int k, const Opts &o) {
+  if (form != MDG_FORM_SLICE_BF16) return workspace_bytes(form, p, m, n, k, o);
   return make_slice_plan(p, o.slices, o.diagonals, m, n, k).total;
 }
 
@@ -378,6 +384,14 @@ size_t mdg_gemm_workspace_size(int form, int p, int m, int n, int k, const mdg_o
   return workspace_bytes(form, p, m, n, k, o);
 }
 
+size_t mdg_gemm_least_workspace_size(int form, int p, int m, int n, int k,
+                                     const mdg_options *opt) {
+  Opts o;
+  if (!valid_p(p) || m < 0 || n < 0 || k < 0) return 0;
+  if (resolve_opts(form, p, opt, &o) != MDG_SUCCESS) return 0;
+  return least_workspace_bytes(form, p, m, n, k, o);
+}
+
 int mdg_gemm(int form, int p, int m, int n, int k, const double *A, int lda, const double *B,
              int ldb, double *C, int ldc, const mdg_options *opt, void *workspace,
              size_t workspace_bytes_, void *stream) {
@@ -394,17 +408,24 @@ int mdg_gemm(int form, int p, int m, int n, int k, const double *A, int lda, con
     NvtxRange range("mdg plain");
     return launch_plain_gemm(p, m, n, k, A, lda, B, ldb, C, ldc, st);
   }
+  if (form == MDG_FORM_SLICE_BF16) {
+    // the sum-plane form where it pays, on CTA pairs, in a workspace that
+    // holds it; otherwise the digit pairs
+    const int engine = engine_choice(o.engine);
+    SlicePlan pl = best_slice_plan(p, o.slices, o.diagonals, m, n, k);
+    if (pl.sums && (engine == 0 || engine == 2 || workspace_bytes_ < pl.total))
+      pl = make_slice_plan(p, o.slices, o.diagonals, m, n, k);
+    if (!workspace || workspace_bytes_ < pl.total) return MDG_ERROR_WORKSPACE;
+    if (pl.Mp > 65535 || pl.Np > 65535) return MDG_ERROR_NOT_SUPPORTED;
+    return run_slice_gemm(pl, A, lda, B, ldb, C, ldc, workspace, engine, o.parts, o.raster, st,
+                          o.pace);
+  }
   const size_t need = workspace_bytes(form, p, m, n, k, o);
   if (!workspace || workspace_bytes_ < need) return MDG_ERROR_WORKSPACE;
   if (form == MDG_FORM_FP64_SPLIT)
     return run_split_gemm(p, o, m, n, k, A, lda, B, ldb, C, ldc, workspace, st);
-  if (form == MDG_FORM_FP64_DIGITS)
-    return run_digits64_gemm(make_digits64_plan(p, o.slices, o.diagonals, m, n, k), A, lda, B,
-                             ldb, C, ldc, workspace, st);
-  const SlicePlan pl = make_slice_plan(p, o.slices, o.diagonals, m, n, k);
-  if (pl.Mp > 65535 || pl.Np > 65535) return MDG_ERROR_NOT_SUPPORTED;
-  return run_slice_gemm(pl, A, lda, B, ldb, C, ldc, workspace, engine_choice(o.engine), o.parts,
-                        o.raster, st, o.pace);
+  return run_digits64_gemm(make_digits64_plan(p, o.slices, o.diagonals, m, n, k), A, lda, B, ldb,
+                           C, ldc, workspace, st);
 }
 
 int mdg_gemm_host(int form, int p, int m, int n, int k, const double *A, const double *B,
@@ -417,7 +438,7 @@ int mdg_gemm_host(int form, int p, int m, int n, int k, const double *A, const d
   const size_t sa = sizeof(double) * (size_t)m * k * p, sb = sizeof(double) * (size_t)k * n * p,
                sc = sizeof(double) * (size_t)m * n * p;
   if (alloc_over_limit(sa) || alloc_over_limit(sb) || alloc_over_limit(sc) ||
-      alloc_over_limit(workspace_bytes(form, p, m, n, k, o)))
+      alloc_over_limit(least_workspace_bytes(form, p, m, n, k, o)))
     return MDG_ERROR_ALLOCATION;
   std::lock_guard<std::mutex> lk(g_cache.mu);
   MDG_TRY(g_cache.bind_device());
@@ -427,8 +448,11 @@ int mdg_gemm_host(int form, int p, int m, int n, int k, const double *A, const d
   MDG_TRY(g_cache.get(2, sc, &dC));
   if (form == MDG_FORM_SLICE_BF16 && k > 0 && m >= 2048)
     return host_slice_panels(p, o, m, n, k, A, B, C, (double *)dA, (double *)dB, (double *)dC);
-  const size_t need = workspace_bytes(form, p, m, n, k, o);
-  if (need) MDG_TRY(g_cache.get(3, need, &ws));
+  size_t need = workspace_bytes(form, p, m, n, k, o);
+  if (need && g_cache.get(3, need, &ws) != MDG_SUCCESS) {
+    need = least_workspace_bytes(form, p, m, n, k, o);
+    MDG_TRY(g_cache.get(3, need, &ws));
+  }
   cudaStream_t st = 0;
   if (sa) MDG_TRY_CUDA(cudaMemcpyAsync(dA, A, sa, cudaMemcpyHostToDevice, st));
   if (sb) MDG_TRY_CUDA(cudaMemcpyAsync(dB, B, sb, cudaMemcpyHostToDevice, st));

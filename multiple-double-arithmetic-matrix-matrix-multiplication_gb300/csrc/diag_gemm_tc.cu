@@ -28,6 +28,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "cross_sums.cuh"
 #include "slice_tc.cuh"
 
 namespace {
@@ -650,11 +651,107 @@ __device__ __forceinline__ uint32_t pace_load(int slot, int ncl, uint32_t epoch)
   return (uint32_t)(v >> 32) == epoch ? (uint32_t)v : 0u;
 }
 
-// One unit of work of the pair kernel: a 256 x 256 tile of one problem
-// (rows row0.., columns col0..) and the diagonals [d0, d1) it computes.
+// A run of plane products that goes into one accumulation: product p takes
+// plane a0 + p of A and plane b0 + bstep p of B, KB k-steps each; its first
+// output plane is `chunk`.  cuts: flush groups per plane (sums form).
+struct Run {
+  int a0, b0, products, chunk, cuts;
+};
+
+// One unit of work of the pair kernel over digit planes: a 256 x 256 tile
+// of one problem (rows row0.., columns col0..) and the diagonals [d0, d1) it
+// computes, one run each.  FP32 flushes every GROUP_STEPS k-steps of a run
+// whatever plane they fall in, chunk stores every CHUNK_STEPS.
 struct PairJob {
+  static constexpr int bstep = -1;
   const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, row0, col0, d0, d1;
+
+  struct Runs {
+    int s, KB, d, d1, chunk;
+    __device__ bool next(Run &r) {
+      if (d >= d1) return false;
+      r.a0 = d - (s - 1) > 0 ? d - (s - 1) : 0;
+      r.b0 = d - r.a0;
+      r.products = mdgi::diag_pairs(d, s);
+      r.chunk = chunk;
+      chunk += mdgi::diag_chunks(d, s, KB);
+      ++d;
+      return true;
+    }
+  };
+  // the first chunk's number is wanted by the epilogue alone
+  __device__ Runs runs(bool chunks) const {
+    int chunk = 0;
+    if (chunks)
+      for (int d = 0; d < d0; ++d) chunk += mdgi::diag_chunks(d, s, KB);
+    return Runs{s, KB, d0, d1, chunk};
+  }
+  struct Groups {
+    int pos, steps;
+    __device__ Groups(const Run &r, int KB) : pos(0), steps(r.products * KB) {}
+    __device__ int next() {  // k-steps of the next flush group, 0 at the end
+      const int n = steps - pos < mdgi::GROUP_STEPS ? steps - pos : mdgi::GROUP_STEPS;
+      pos += n;
+      return n;
+    }
+    __device__ bool store() const { return pos % mdgi::CHUNK_STEPS == 0 || pos >= steps; }
+  };
+};
+
+// One unit of work over digit and sum planes (cross_sums.cuh): a tile and
+// `planes` consecutive products of its list, which is the squares [sq, nsq),
+// then the sums of the diagonals from d on, chunk by chunk.  The same plane
+// index on both sides; flush groups never span two planes, because their
+// exactness rests on the norms of windows of single sum planes.
+struct CrossJob {
+  static constexpr int bstep = 1;
+  const CUtensorMap *tmA, *tmB, *tmC;
+  int Mp, Np, KB, row0, col0;
+  int sq, nsq, d, i, chunk, planes;  // start of the unit's list
+  int plane0, ppc, cuts;             // plane of diagonal d's pair 0 is plane0 + cross_offset(d)
+
+  struct Runs {
+    int sq, nsq, d, i, chunk, planes, plane0, ppc, cuts1, cuts;
+    __device__ bool next(Run &r) {
+      if (planes <= 0) return false;
+      if (sq < nsq) {
+        r = Run{sq, sq, 1, sq, cuts1};
+        ++sq;
+      } else {
+        const int left = mdgi::cross_pairs(d) - i;
+        const int np = left < ppc ? left : ppc;
+        const int t = plane0 + mdgi::cross_offset(d) + i;
+        r = Run{t, t, np, chunk, cuts};
+        ++chunk;
+        i += np;
+        if (np == left) {
+          ++d;
+          i = 0;
+        }
+      }
+      planes -= r.products;
+      return true;
+    }
+  };
+  __device__ Runs runs(bool) const {
+    return Runs{sq, nsq, d, i, chunk, planes, plane0, ppc, mdgi::cross_groups(KB), cuts};
+  }
+  struct Groups {
+    int left, KB, cuts, j, at;
+    __device__ Groups(const Run &r, int KB_) : left(r.products), KB(KB_), cuts(r.cuts), j(0), at(0) {}
+    __device__ int next() {
+      if (left == 0) return 0;
+      const int to = ++j * KB / cuts, n = to - at;
+      at = to;
+      if (j == cuts) {
+        j = at = 0;
+        --left;
+      }
+      return n;
+    }
+    __device__ bool store() const { return left == 0; }
+  };
 };
 
 // A single problem: units are tiles, or parts of tiles (ranges of
@@ -699,6 +796,49 @@ struct PairGrouped {
                    reinterpret_cast<const CUtensorMap *>(g.tmB),
                    reinterpret_cast<const CUtensorMap *>(g.tmC), g.s, g.D, g.Mp, g.Np, g.KB,
                    (tile % g.mt) * 256, (tile / g.mt) * TN2, d0, d1};
+  }
+};
+
+// A single problem over digit and sum planes: units are tiles, or parts of
+// tiles whose lists hold about 1/parts of its products each (cut between
+// output planes), in the order of PairSingle's.
+struct PairCross {
+  const CUtensorMap *tmA, *tmB, *tmC;
+  int D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB;
+  int parts, raster;
+  const unsigned *norms;
+  __device__ int units() const { return (Mp / 256) * (Np / TN2) * parts; }
+  // Flush groups per sum plane.  |sum over a group| <= |a| |b| (Cauchy and
+  // Schwarz; every partial sum too) with |a|^2 <= 2 norms[0], |b|^2 <= 2
+  // norms[1] over a whole group (two windows), <= norms[0], norms[1] over
+  // half of one; a quarter holds at most 256 products of 2^16.  FP32 is
+  // exact up to 2^24, so whole groups where 4 norms[0] norms[1] <= 2^48.
+  __device__ int cuts() const {
+    const unsigned long long n2 = (unsigned long long)norms[0] * norms[1];
+    return mdgi::cross_groups(KB) * (4 * n2 <= 1ull << 48 ? 1 : n2 <= 1ull << 48 ? 2 : 4);
+  }
+  __device__ CrossJob job(int u) const {
+    const int MB = Mp / 256, NB = Np / TN2, tiles = MB * NB;
+    const int tile = u % tiles, part = u / tiles;
+    const int strip = tile / (MB * raster);
+    const int idx = tile - strip * MB * raster;
+    const int c0 = strip * raster;
+    const int g = NB - c0 < raster ? NB - c0 : raster;
+    const int rb = idx / g, cb = c0 + idx - rb * g;
+    const int total = nsq + mdgi::cross_offset(dhi) - mdgi::cross_offset(dlo);
+    const int lo = (int)((long long)total * part / parts);
+    const int hi = (int)((long long)total * (part + 1) / parts);
+    // the runs that start in [lo, hi)
+    CrossJob::Runs it{0, nsq, dlo, 0, D, total, plane0, ppc, 1, 1};
+    for (int d = 1; d < dlo; ++d) it.chunk += mdgi::cross_chunks(d, ppc);
+    Run r;
+    while (total - it.planes < lo && it.next(r)) {
+    }
+    const CrossJob::Runs first = it;
+    while (total - it.planes < hi && it.next(r)) {
+    }
+    return CrossJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2, first.sq, nsq, first.d, first.i,
+                    first.chunk, first.planes - it.planes, plane0, ppc, cuts()};
   }
 };
 
@@ -774,15 +914,16 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       // MMA thread's wait for data runs out, it raises the abort flag and
       // every role leaves with nothing in flight
       for (int u = no_loads ? units : cid; u < units; u += ncl) {
-        const PairJob jb = jobs.job(u);
-        const int s = jb.s, KB = jb.KB;
+        const auto jb = jobs.job(u);
+        const int KB = jb.KB;
         const int row = jb.row0 + (int)rank * TM;
         const int col = jb.col0 + (int)rank * BH;
-        for (int d = jb.d0; d < jb.d1; ++d) {
-          const int ilo = d - (s - 1) > 0 ? d - (s - 1) : 0;
-          const int S = mdgi::diag_pairs(d, s) * KB;
+        auto runs = jb.runs(false);
+        Run r;
+        while (runs.next(r)) {
+          const int S = r.products * KB;
           for (int t = 0; t < S; ++t) {
-            const int i = ilo + t / KB, kb = t - (t / KB) * KB, j = d - i;
+            const int q = t / KB, kb = t - q * KB, i = r.a0 + q, j = r.b0 + jb.bstep * q;
             if (pacing && steps > *pace_allowed) {
               const unsigned long long t0 = now_ns();
               while (steps > *pace_allowed) {
@@ -822,22 +963,23 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       uint32_t ph = 0, aph[2] = {0, 0};
       bool any = false;
       for (int u = cid; u < units; u += ncl) {
-        const PairJob jb = jobs.job(u);
-        for (int d = jb.d0; d < jb.d1; ++d) {
-          const int S = mdgi::diag_pairs(d, jb.s) * jb.KB;
-          for (int g0 = 0; g0 < S; g0 += mdgi::GROUP_STEPS) {
+        const auto jb = jobs.job(u);
+        auto runs = jb.runs(false);
+        Run r;
+        while (runs.next(r)) {
+          typename decltype(jb)::Groups groups(r, jb.KB);
+          for (int steps; (steps = groups.next()) > 0;) {
             if (!mbar_wait(accempty(buf), aph[buf] ^ 1, abort_flag)) goto mma_done;
             fence_after();
             const uint32_t dt = tmem_base + buf * TN2;
-            const int g1 = g0 + mdgi::GROUP_STEPS < S ? g0 + mdgi::GROUP_STEPS : S;
-            for (int t = g0; t < g1; ++t) {
+            for (int t = 0; t < steps; ++t) {
               if (!mbar_wait(full(st), ph, abort_flag)) goto mma_done;
               fence_after();
               const uint32_t a_addr = smem_base + st * STAGE2_BYTES;
               const uint64_t da = sw128_desc(a_addr), db = sw128_desc(a_addr + A2_BYTES);
 #pragma unroll
               for (int kk = 0; kk < TK / 16; ++kk)
-                mma_bf16_pair(dt, da + 2 * kk, db + 2 * kk, (t > g0 || kk > 0) ? 1u : 0u);
+                mma_bf16_pair(dt, da + 2 * kk, db + 2 * kk, (t > 0 || kk > 0) ? 1u : 0u);
               mma_commit_pair(empty(st));
               any = true;
               if (++st == STAGES2) {
@@ -901,14 +1043,15 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
     uint32_t aph[2] = {0, 0};
     const uint32_t accempty0[2] = {map_to_rank0(accempty(0)), map_to_rank0(accempty(1))};
     for (int u = cid; u < units; u += ncl) {
-      const PairJob jb = jobs.job(u);
+      const auto jb = jobs.job(u);
       const int row = jb.row0 + (int)rank * TM + 32 * q;
       const int col = jb.col0 + 128 * h;
-      int chunk = 0;
-      for (int d = 0; d < jb.d0; ++d) chunk += mdgi::diag_chunks(d, jb.s, jb.KB);
-      for (int d = jb.d0; d < jb.d1; ++d) {
-        const int S = mdgi::diag_pairs(d, jb.s) * jb.KB;
-        for (int g0 = 0; g0 < S; g0 += mdgi::GROUP_STEPS) {
+      auto runs = jb.runs(true);
+      Run r;
+      while (runs.next(r)) {
+        typename decltype(jb)::Groups groups(r, jb.KB);
+        int chunk = r.chunk;
+        while (groups.next() > 0) {
           int ok = 1;
           if (lane == 0) ok = mbar_wait(accfull(buf), aph[buf], abort_flag) ? 1 : 0;
           ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -921,8 +1064,7 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(accempty0[buf]);
           buf ^= 1;
-          const int g1 = g0 + mdgi::GROUP_STEPS;
-          if (g1 % mdgi::CHUNK_STEPS == 0 || g1 >= S) {
+          if (groups.store()) {
             store_rows(staging, lane, acc, jb.tmC, col, chunk * jb.Mp + row);
             ++chunk;
           }
@@ -949,6 +1091,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                          const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
                          int KB, int parts, int raster, int pace, uint32_t epoch, int no_loads) {
   tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, parts, raster}, pace, epoch, no_loads);
+}
+
+// The diagonal GEMM over digit and sum planes (cross_sums.cuh).  Bound by the
+// tensor cores as the kernel above, at 224 instead of 406 products of planes
+// for quad-double: qd 8192^3 146 instead of 268 ms (1684 TFLOP/s done), od
+// 2048^3 8.5 instead of 16.4 ms, qd 1024^3 353 instead of 607 us.  Flush
+// groups of 16, 8 and 4 k-steps (whole, halves, quarters) cost 17.0, 17.9
+// and 27.7 ms on the same quad-double 4096 x 4096 x 2048 digit pairs: reading
+// the accumulators back takes about 4000 cycles, 4 k-steps of products 2048.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
+    diag_gemm_cross_kernel(const __grid_constant__ CUtensorMap tmA,
+                           const __grid_constant__ CUtensorMap tmB,
+                           const __grid_constant__ CUtensorMap tmC, int D, int dlo, int dhi,
+                           int nsq, int plane0, int ppc, int Mp, int Np, int KB, int parts,
+                           int raster, const unsigned *__restrict__ norms, int pace,
+                           uint32_t epoch, int no_loads) {
+  tc2_body(PairCross{&tmA, &tmB, &tmC, D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB, parts, raster,
+                     norms},
+           pace, epoch, no_loads);
 }
 
 // The batched plan's grouped GEMM on CTA pairs (no pacing: the clusters work
@@ -1004,9 +1165,95 @@ int make_out_map(CUtensorMap *m, const void *base, int Np, long long rows_total)
   return r == CUDA_SUCCESS ? MDG_SUCCESS : MDG_ERROR_NOT_SUPPORTED;
 }
 
+// How one launch of a pair kernel runs: work units, tile order, pacing.
+struct PairSchedule {
+  int clusters, parts, raster, pace, no_loads;
+  uint32_t epoch;
+};
+
+// max_parts: runs of a tile that parts can separate (diagonals).
+PairSchedule pair_schedule(int Mp, int Np, int max_parts, int sms, int parts_opt, int raster_opt,
+                           int pace_opt) {
+  PairSchedule sc;
+  const int tiles = (Mp / 256) * (Np / TN2);
+  // split tiles into `parts` diagonal ranges when that shrinks the idle
+  // part of the last wave of clusters by more than it costs: each extra
+  // part makes the work about 4 % slower (fitted to quad-double 4096^3 and
+  // 8192^3: 1024 tiles on 76 clusters run best unsplit, 256 tiles best in
+  // two parts)
+  const int ncl = sms / 2;
+  sc.parts = 1;
+  double best = 0.0;
+  for (int u = 1; u <= 8 && u <= max_parts; ++u) {
+    const long long units = (long long)tiles * u;
+    const long long waves = (units + ncl - 1) / ncl;
+    const double cost = (double)waves / u * (1.0 + 0.04 * (u - 1));
+    if (u == 1 || cost < best) {
+      best = cost;
+      sc.parts = u;
+    }
+  }
+  if (parts_opt > 0) sc.parts = std::min(8, parts_opt);
+  // tile order: strips about sqrt(clusters) column blocks wide, so that
+  // the tiles in work at one time span few row and column blocks (the
+  // largest power of two not above sqrt(76) = 8.7 on 152 SMs)
+  const int NB = Np / TN2;
+  sc.raster = 1;
+  while ((sc.raster * 2) * (sc.raster * 2) <= ncl) sc.raster *= 2;
+  if (raster_opt > 0) sc.raster = raster_opt;
+  sc.raster = std::min(NB, sc.raster);
+  const long long units = (long long)tiles * sc.parts;
+  sc.clusters = units < ncl ? (int)units : ncl;
+  // pacing window in k-steps, 0 = off (MDG_TC_PACE overrides); every
+  // launch gets its own epoch so that slots left by earlier launches read
+  // as "not started"
+  // With no more units than clusters every tile is in work at once and
+  // the operands of the whole GEMM are read in one sweep: pacing has no
+  // drift to correct there and only costs (qd 1024^3: 7 % slower paced), so
+  // the default turns it off; an explicit window still applies.
+  sc.pace = units <= ncl ? 0 : kDefaultPace;
+  if (const char *e = std::getenv("MDG_TC_PACE")) sc.pace = std::max(0, std::atoi(e));
+  if (pace_opt > 0) sc.pace = pace_opt;
+  if (pace_opt < 0) sc.pace = 0;
+  static std::atomic<uint32_t> epochs{0};
+  sc.epoch = ++epochs;
+  if (sc.epoch == 0) sc.epoch = ++epochs;
+  // MDG_TC_SELFTEST_NO_LOADS=1: the producers issue no copies, the waits
+  // for data run out after their 2 s limit and mdg_device_status then
+  // reports MDG_ERROR_TIMEOUT (a test of the failure path; the result
+  // planes are not written)
+  const char *nl = std::getenv("MDG_TC_SELFTEST_NO_LOADS");
+  sc.no_loads = (nl && *nl == '1') ? 1 : 0;
+  return sc;
+}
+
 }  // namespace
 
 namespace mdgi {
+
+int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_planes, int Mp,
+                           int Np, int Kp, const void *dA, const void *dB, const unsigned *norms,
+                           int *out, int parts, int raster, int pace, cudaStream_t st) {
+  if (Mp % 256 || Np % TN2 || Kp % TK) return MDG_ERROR_INVALID_SIZE;
+  const int KB = Kp / TK;
+  if (KB < 1 || KB > CROSS_CHUNK_STEPS) return MDG_ERROR_INVALID_SIZE;
+  CUtensorMap ma, mb, mc;
+  MDG_TRY(make_map(&ma, dA, Kp, (long long)(s + sum_planes) * Mp, TM));
+  MDG_TRY(make_map(&mb, dB, Kp, (long long)(s + sum_planes) * Np, BH));
+  MDG_TRY(make_out_map(&mc, out, Np, (long long)cross_outputs(D, KB) * Mp));
+  int dev = 0, sms = 0;
+  MDG_TRY_CUDA(cudaGetDevice(&dev));
+  MDG_TRY_CUDA(cudaFuncSetAttribute(diag_gemm_cross_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
+  MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const PairSchedule sc =
+      pair_schedule(Mp, Np, squares + dhi - dlo, sms, parts, raster, pace);
+  diag_gemm_cross_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
+      ma, mb, mc, D, dlo, dhi, squares, s - cross_offset(dlo), cross_pairs_per_chunk(KB), Mp, Np, KB,
+      sc.parts, sc.raster, norms, sc.pace, sc.epoch, sc.no_loads);
+  MDG_TRY_LAUNCH();
+  return MDG_SUCCESS;
+}
 
 int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
                         int ld, long long plane_a, long long plane_b, int *chunks,
@@ -1035,57 +1282,9 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, co
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (pair) {
-    const int tiles = (Mp / 256) * (Np / TN2);
-    // split tiles into `parts` diagonal ranges when that shrinks the idle
-    // part of the last wave of clusters by more than it costs: each extra
-    // part makes the work about 4 % slower (fitted to quad-double 4096^3 and
-    // 8192^3: 1024 tiles on 76 clusters run best unsplit, 256 tiles best in
-    // two parts)
-    const int ncl = sms / 2;
-    int parts = 1;
-    double best = 0.0;
-    for (int u = 1; u <= 8 && u <= D; ++u) {
-      const long long units = (long long)tiles * u;
-      const long long waves = (units + ncl - 1) / ncl;
-      const double cost = (double)waves / u * (1.0 + 0.04 * (u - 1));
-      if (u == 1 || cost < best) {
-        best = cost;
-        parts = u;
-      }
-    }
-    if (parts_opt > 0) parts = std::min(8, parts_opt);
-    // tile order: strips about sqrt(clusters) column blocks wide, so that
-    // the tiles in work at one time span few row and column blocks (the
-    // largest power of two not above sqrt(76) = 8.7 on 152 SMs)
-    const int NB = Np / TN2;
-    int raster = 1;
-    while ((raster * 2) * (raster * 2) <= ncl) raster *= 2;
-    if (raster_opt > 0) raster = raster_opt;
-    raster = std::min(NB, raster);
-    const long long units = (long long)tiles * parts;
-    const int clusters = units < ncl ? (int)units : ncl;
-    // pacing window in k-steps, 0 = off (MDG_TC_PACE overrides); every
-    // launch gets its own epoch so that slots left by earlier launches read
-    // as "not started"
-    // With no more units than clusters every tile is in work at once and
-    // the operands of the whole GEMM are read in one sweep: pacing has no
-    // drift to correct there and only costs (qd 1024^3: 7 % slower paced), so
-    // the default turns it off; an explicit window still applies.
-    int pace = units <= ncl ? 0 : kDefaultPace;
-    if (const char *e = std::getenv("MDG_TC_PACE")) pace = std::max(0, std::atoi(e));
-    if (pace_opt > 0) pace = pace_opt;
-    if (pace_opt < 0) pace = 0;
-    static std::atomic<uint32_t> epochs{0};
-    uint32_t epoch = ++epochs;
-    if (epoch == 0) epoch = ++epochs;
-    // MDG_TC_SELFTEST_NO_LOADS=1: the producers issue no copies, the waits
-    // for data run out after their 2 s limit and mdg_device_status then
-    // reports MDG_ERROR_TIMEOUT (a test of the failure path; the result
-    // planes are not written)
-    const char *nl = std::getenv("MDG_TC_SELFTEST_NO_LOADS");
-    const int no_loads = (nl && *nl == '1') ? 1 : 0;
-    diag_gemm_tc2_kernel<<<2 * clusters, THREADS2, SMEM2_BYTES, st>>>(
-        ma, mb, mc, s, D, Mp, Np, Kp / TK, parts, raster, pace, epoch, no_loads);
+    const PairSchedule sc = pair_schedule(Mp, Np, D, sms, parts_opt, raster_opt, pace_opt);
+    diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
+        ma, mb, mc, s, D, Mp, Np, Kp / TK, sc.parts, sc.raster, sc.pace, sc.epoch, sc.no_loads);
   } else {
     const int tiles = (Mp / TM) * (Np / TN);
     const int grid = tiles < sms ? tiles : sms;

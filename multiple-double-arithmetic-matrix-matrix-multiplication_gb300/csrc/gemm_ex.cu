@@ -144,8 +144,10 @@ int mdg_gemm_ex(int form, int trans_a, int trans_b, int accumulate, int p, int m
                 const mdg_options *opt, void *workspace, size_t workspace_bytes,
                 void *stream) {
   MDG_TRY(check_ex(form, trans_a, trans_b, accumulate, p, m, n, k, lda, ldb, ldc));
-  const size_t inner = mdg_gemm_workspace_size(form, p, m, n, k, opt);
+  size_t inner = mdg_gemm_workspace_size(form, p, m, n, k, opt);
   if (form != MDG_FORM_PLAIN && inner == 0) return MDG_ERROR_INVALID_FORM;
+  if (ex_layout(inner, trans_a, trans_b, accumulate, p, m, n, k).total > workspace_bytes)
+    inner = mdg_gemm_least_workspace_size(form, p, m, n, k, opt);
   if (m == 0 || n == 0) return MDG_SUCCESS;  // nothing is read or written
   if (!C || (k > 0 && (!A || !B))) return MDG_ERROR_NULL_POINTER;
   cudaStream_t st = mdgi::as_stream(stream);

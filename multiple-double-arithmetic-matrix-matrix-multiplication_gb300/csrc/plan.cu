@@ -169,8 +169,10 @@ int mdg_plan_create(int form, int p, int m, int n, int k, const mdg_options *opt
   if (form < MDG_FORM_PLAIN || form > MDG_FORM_FP64_DIGITS) return MDG_ERROR_INVALID_FORM;
   if (!mdgi::valid_p(p)) return MDG_ERROR_INVALID_LIMBS;
   if (m < 0 || n < 0 || k < 0) return MDG_ERROR_INVALID_SIZE;
-  const size_t bytes = mdg_gemm_workspace_size(form, p, m, n, k, opt);
+  size_t bytes = mdg_gemm_workspace_size(form, p, m, n, k, opt);
   if (form != MDG_FORM_PLAIN && bytes == 0) return MDG_ERROR_INVALID_FORM;  // options rejected
+  const size_t least = mdg_gemm_least_workspace_size(form, p, m, n, k, opt);
+  if (mdgi::alloc_over_limit(bytes)) bytes = least;
   if (mdgi::alloc_over_limit(bytes)) return MDG_ERROR_ALLOCATION;
   auto *h = new mdg_plan_s();
   h->form = form;
@@ -196,6 +198,11 @@ int mdg_plan_create(int form, int p, int m, int n, int k, const mdg_options *opt
   }
   if (st == MDG_SUCCESS && bytes) {
     cudaError_t e = cudaMalloc(&h->ws, bytes);
+    if (e == cudaErrorMemoryAllocation && least < bytes) {
+      cudaGetLastError();  // handled: the smaller workspace gives the same bits
+      bytes = least;
+      e = cudaMalloc(&h->ws, bytes);
+    }
     if (e != cudaSuccess) {
       mdgi::set_cuda_error(e);
       st = MDG_ERROR_ALLOCATION;

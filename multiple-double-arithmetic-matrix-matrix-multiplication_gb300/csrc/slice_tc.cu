@@ -24,6 +24,7 @@
 // section 8 restates these steps on the CPU, and the GPU result equals it
 // bit for bit.
 #include "common.cuh"
+#include "cross_sums.cuh"
 #include "slice_common.cuh"
 #include "slice_tc.cuh"
 #include "slice_stages.cuh"
@@ -196,6 +197,27 @@ __global__ void __launch_bounds__(256)
 
 namespace mdgi {
 
+// kCrossSumBytes: sums of both operands held at once (beyond that the
+// diagonals are done in groups that reuse the buffer).  kCrossMaxBytes:
+// workspace beyond which the digit pairs are used, so that problems which
+// fill the device still fit.
+constexpr size_t kCrossSumBytes = 16ull << 30, kCrossMaxBytes = 160ull << 30;
+
+// Where sum planes beat digit pairs.  They save half the products (time as
+// Mp Np Kp) and cost the writing of the sums (as (Mp + Np) Kp) and a dearer
+// renormalisation (as Mp Np): so a least Mp Np / (Mp + Np) and a least k.
+// Measured whole calls, pairs against sums: qd 1024 x 768 x 1024 718 / 653
+// us, 1024 x 768 x 512 486 / 468, 1024 x 1024 x 256 421 / 517, 256 x 4096 x
+// 1024 1029 / 1073; dd 1024 x 768 x 1024 301 / 282, 512 x 2048 x 1024 347 /
+// 352.  Up to four 256 x 256 tiles leave most of the chip idle and the
+// length of a tile's work is what counts: qd 512 x 512 x 1024 571 / 431,
+// but x 512 370 / 332 and x 256 236 / 310.
+static bool cross_pays(int p, int Mp, int Np, int KB) {
+  const double tile = (double)Mp * Np / ((double)Mp + Np);
+  if (KB >= 16) return tile >= (p == 2 ? 500.0 : 384.0) || (p > 2 && Mp * (long long)Np <= 512 * 512);
+  return KB >= 8 && tile >= (p == 2 ? 1000.0 : 500.0);
+}
+
 int words_for(int s, int D) {
   // digits need S + 2 bits plus a word of headroom; W needs 8 (D - 1) + 64
   const int bits = std::max(7 + 8 * (s - 1) + 2, 8 * (D - 1) + 72);
@@ -207,7 +229,8 @@ int words_for(int s, int D) {
   return 0;
 }
 
-SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
+// sums: sum planes per operand (0: digit pairs alone)
+static SlicePlan layout_slice_plan(int p, int s, int D, int m, int n, int k, int sums) {
   SlicePlan pl{};
   pl.p = p;
   pl.s = s;
@@ -218,7 +241,8 @@ SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
   pl.Mp = (int)align_up(std::max(m, 1), 256);
   pl.Np = (int)align_up(std::max(n, 1), 256);
   pl.Kp = (int)align_up(std::max(k, 1), 64);
-  pl.chunks = total_chunks(s, D, pl.Kp / 64);
+  pl.sums = sums;
+  pl.chunks = sums ? cross_outputs(D, pl.Kp / 64) : total_chunks(s, D, pl.Kp / 64);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -229,14 +253,34 @@ SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
   pl.off_colbits = take(sizeof(unsigned long long) * pl.Np);
   pl.off_E = take(sizeof(int) * pl.Mp);
   pl.off_F = take(sizeof(int) * pl.Np);
+  pl.off_norms = sums ? take(2 * sizeof(unsigned)) : 0;
   pl.plane_a = (long long)pl.Mp * pl.Kp;
   pl.plane_b = (long long)pl.Np * pl.Kp;
   pl.plane_c = (long long)pl.Mp * pl.Np;
-  pl.off_dA = take(sizeof(__nv_bfloat16) * (size_t)s * pl.plane_a);
-  pl.off_dB = take(sizeof(__nv_bfloat16) * (size_t)s * pl.plane_b);
+  pl.off_dA = take(sizeof(__nv_bfloat16) * (size_t)(s + sums) * pl.plane_a);
+  pl.off_dB = take(sizeof(__nv_bfloat16) * (size_t)(s + sums) * pl.plane_b);
   pl.off_Cd = take(sizeof(int) * (size_t)pl.chunks * pl.plane_c);
   pl.total = off;
   return pl;
+}
+
+SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
+  return layout_slice_plan(p, s, D, m, n, k, 0);
+}
+
+SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k) {
+  const SlicePlan pairs = make_slice_plan(p, s, D, m, n, k);
+  const int KB = pairs.Kp / 64;
+  if (KB > CROSS_CHUNK_STEPS || !cross_pays(p, pairs.Mp, pairs.Np, KB) ||
+      !cross_renorm_supported(p, s, D))
+    return pairs;
+  const int all = cross_offset(D), least = cross_pairs(D - 1);
+  const double plane_bytes = 2.0 * ((double)pairs.plane_a + pairs.plane_b);
+  int sums = all;
+  if (all * plane_bytes > (double)kCrossSumBytes)
+    sums = std::max(least, (int)((double)kCrossSumBytes / plane_bytes));
+  const SlicePlan pl = layout_slice_plan(p, s, D, m, n, k, sums);
+  return pl.total <= kCrossMaxBytes && pl.total >= pairs.total ? pl : pairs;
 }
 
 int launch_scale_exponents(int p, int m, int n, int k, const double *A, int lda,
@@ -426,6 +470,20 @@ int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *
                           pl.Kp, st));
   }
   NvtxRange r2("diagonal GEMM and renormalisation");
+  if (pl.sums) {
+    auto *norms = reinterpret_cast<unsigned *>(base + pl.off_norms);
+    MDG_TRY_CUDA(cudaMemsetAsync(norms, 0, 2 * sizeof(unsigned), st));
+    for (int lo = 1, hi; lo < pl.D; lo = hi) {
+      hi = cross_group_end(lo, pl.D, pl.sums);
+      if (hi == lo) return MDG_ERROR_NOT_SUPPORTED;
+      MDG_TRY(launch_cross_sums(pl.s, lo, hi, pl.Kp, pl.m, pl.n, dA, dB, pl.plane_a, pl.plane_b,
+                                norms, st));
+      MDG_TRY(launch_diag_gemm_cross(pl.s, pl.D, lo, hi, lo == 1 ? pl.D : 0, pl.sums, pl.Mp,
+                                     pl.Np, pl.Kp, dA, dB, norms, Cd, parts, raster, pace, st));
+    }
+    return launch_cross_renorm(pl.p, pl.D, pl.Kp / 64, pl.m, pl.n, Cd, pl.plane_c, pl.Np, E, F, C,
+                               ldc, st);
+  }
   if (engine != 0) {
     MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, dA, dB, pl.Kp, pl.plane_a,
                                 pl.plane_b, Cd, pl.plane_c, engine == 2 ? 1 : 0, parts, raster, st,

@@ -40,10 +40,17 @@ struct SlicePlan {
   int Mp, Np, Kp;  // padded to 256, 256, 64
   int chunks;
   long long plane_a, plane_b, plane_c;  // elements between digit / chunk planes
-  size_t off_rowbits, off_colbits, off_E, off_F, off_dA, off_dB, off_Cd, total;
+  // sum planes behind each operand's digit planes (cross_sums.cuh); 0: the
+  // diagonal sums come from digit pairs alone.  off_norms: two unsigned.
+  int sums;
+  size_t off_rowbits, off_colbits, off_E, off_F, off_norms, off_dA, off_dB, off_Cd, total;
 };
 
+// The plan over digit pairs.
 SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k);
+// The plan over sum planes where that is faster, else make_slice_plan's;
+// never smaller than make_slice_plan's.
+SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k);
 int words_for(int s, int D);
 
 // The FP64-DMMA slice-digit form (digits64.cu): default digits per P
