@@ -9,7 +9,7 @@
 //   one launch: exponents of every row of every A and column of every B
 //   one launch: digits of every A and every B
 //   one launch: grouped tcgen05 diagonal GEMM over the tiles of all problems
-//   one launch per limb count present: renormalisation of its C
+//   one launch: renormalisation of every C
 // Each stage kernel finds its problem from its block index by binary search
 // over per-problem prefix counts, and branches on the problem's P to the
 // integer width that P needs (batched_stages.cuh).  The grouped GEMM's tiles
@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "renorm.cuh"
 #include "slice_stages.cuh"
 #include "slice_tc.cuh"
 
@@ -33,8 +34,7 @@
 struct mdg_batch_s {
   int count = 0, nwmax = 4, total_units = 0;
   int scale_units = 0, digit_units = 0, renorm_units = 0;
-  // per P = 2, 4, 8, 16: first output row, rows, widest n
-  int renorm_begin[4] = {0, 0, 0, 0}, renorm_count[4] = {0, 0, 0, 0}, renorm_n[4] = {0, 0, 0, 0};
+  int max_d = 1;  // most diagonals of any problem
   int tiles_policy = MDG_BATCH_TILES_256, split = 1;
   mdgi::BatchProblem *dprobs = nullptr;
   mdgi::GroupedProblem *dgroups = nullptr;
@@ -153,7 +153,6 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
   L->off_chunks.resize(count);
   int scale_u = 0, digit_u = 0, renorm_u = 0, offE = 0, offF = rows;
   h->nwmax = 4;
-  for (int i = 0; i < 4; ++i) h->renorm_begin[i] = h->renorm_count[i] = h->renorm_n[i] = 0;
   // the table is kept in order of P (stable): blocks of one P sit together
   // in every stage's launch
   std::vector<int> order(count);
@@ -180,7 +179,8 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
     // digits: valid rows and k-positions only (the padding is cleared once,
     // by mdg_batch_create)
     const int digit_a = q.m * kblocks, digit_b = q.n * kblocks;
-    const int out_u = q.m;  // renormalisation: one row of blocks per output row
+    const long long out_u = mdgi::ceil_div((long long)q.m * ((q.n + 1) / 2), mdgi::RENORM_THREADS);
+    if (renorm_u + out_u > (1LL << 30)) return MDG_ERROR_INVALID_SIZE;
     if (ws) {
       BatchProblem b{};
       b.p = q.p; b.s = s; b.D = D; b.m = q.m; b.n = q.n; b.k = q.k;
@@ -190,6 +190,8 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
       b.dA = reinterpret_cast<__nv_bfloat16 *>(ws + L->off_dA[i]);
       b.dB = reinterpret_cast<__nv_bfloat16 *>(ws + L->off_dB[i]);
       b.chunks = reinterpret_cast<int *>(ws + L->off_chunks[i]);
+      b.planes = nch;
+      b.wide = reinterpret_cast<uintptr_t>(q.C) % 16 == 0;
       b.plane_a = (long long)Mp * Kp;
       b.plane_b = (long long)Np * Kp;
       b.plane_c = (long long)Mp * Np;
@@ -198,13 +200,10 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
       b.out_begin = renorm_u;
       hp->push_back(b);
     }
-    const int pi = q.p == 2 ? 0 : q.p == 4 ? 1 : q.p == 8 ? 2 : 3;
-    if (h->renorm_count[pi] == 0) h->renorm_begin[pi] = renorm_u;
-    h->renorm_count[pi] += out_u;
-    h->renorm_n[pi] = std::max(h->renorm_n[pi], q.n);
+    h->max_d = std::max(h->max_d, D);
     scale_u += scale_a + scale_b;
     digit_u += digit_a + digit_b;
-    renorm_u += out_u;
+    renorm_u += (int)out_u;
     offE += std::max(q.m, 1);
     offF += std::max(q.n, 1);
   }
@@ -349,11 +348,7 @@ int mdg_batch_run(mdg_batch_s *h, void *stream) {
 #undef MDG_BATCH_STAGES
   MDG_TRY(mdgi::launch_diag_gemm_grouped(h->dgroups, h->count, h->total_units,
                                          h->tiles_policy == MDG_BATCH_TILES_PAIR, st));
-  const int *rb = h->renorm_begin, *rc = h->renorm_count, *rn = h->renorm_n;
-  MDG_TRY(mdgi::launch_batch_renorm<2>(h->dprobs, h->count, rb[0], rc[0], rn[0], h->exps, st));
-  MDG_TRY(mdgi::launch_batch_renorm<4>(h->dprobs, h->count, rb[1], rc[1], rn[1], h->exps, st));
-  MDG_TRY(mdgi::launch_batch_renorm<8>(h->dprobs, h->count, rb[2], rc[2], rn[2], h->exps, st));
-  MDG_TRY(mdgi::launch_batch_renorm<16>(h->dprobs, h->count, rb[3], rc[3], rn[3], h->exps, st));
+  MDG_TRY(mdgi::launch_batch_renorm(h->dprobs, h->count, h->renorm_units, h->max_d, h->exps, st));
   return MDG_SUCCESS;
 }
 

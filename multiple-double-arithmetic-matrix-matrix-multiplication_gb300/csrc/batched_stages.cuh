@@ -1,10 +1,9 @@
-// Exponent, digit and renormalisation kernels of the batched slice-digit
+// Exponent and digit kernels of the batched slice-digit
 // GEMM.  The exponent and digit kernels run once over every problem of the
 // batch, whatever its P: each block finds its problem in the table
 // (batched_table.cuh) and branches on the problem's P to the integer width
 // that P needs; the branches of wider integers than the batch holds are not
-// compiled into the instance that is launched (NWMAX).  The
-// renormalisation runs once per limb count present.  One translation unit
+// compiled into the instance that is launched (NWMAX).  One translation unit
 // per width (batched_w{4,6,10,16}.cu) so that the wide-integer code
 // compiles in parallel.
 #pragma once
@@ -90,21 +89,6 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// The renormalisation runs one launch per P (a kernel holding the bodies of
-// several widths measured 15 % slower): block (x, y) takes output row
-// row0 + x of the P group, columns 128 V y .. +128 V - 1.
-template <int P>
-__global__ void __launch_bounds__(128)
-    renorm_p(const BatchProblem *__restrict__ pr, int count, const int *__restrict__ exps,
-             int row0) {
-  constexpr int V = batch_cols_per_thread(P);
-  const int x = row0 + (int)blockIdx.x;
-  const BatchProblem &b = pr[find_problem<kRenormUnits>(pr, count, x)];
-  const int r = x - b.out_begin, c0 = ((int)blockIdx.y * 128 + (int)threadIdx.x) * V;
-  renorm_elems<P, batch_words(P), V>(b.s, b.D, b.Kp / 64, b.m, b.n, b.chunks, b.plane_c, b.Np,
-                                     exps + b.offE, exps + b.offF, b.C, b.ldc, r, c0);
-}
-
 template <int NWMAX>
 int launch_batch_scale(const BatchProblem *pr, int count, int units, int *exps, cudaStream_t st) {
   if (units == 0) return MDG_SUCCESS;
@@ -118,17 +102,6 @@ int launch_batch_digits(const BatchProblem *pr, int count, int units, const int 
                         cudaStream_t st) {
   if (units == 0) return MDG_SUCCESS;
   digits_all<NWMAX><<<units, 128, 0, st>>>(pr, count, exps);
-  MDG_TRY_LAUNCH();
-  return MDG_SUCCESS;
-}
-
-template <int P>
-int launch_batch_renorm(const BatchProblem *pr, int count, int row0, int rows, int max_n,
-                        const int *exps, cudaStream_t st) {
-  if (rows == 0 || max_n == 0) return MDG_SUCCESS;
-  constexpr int V = batch_cols_per_thread(P);
-  renorm_p<P><<<dim3(rows, ceil_div(ceil_div(max_n, V), 128)), 128, 0, st>>>(pr, count, exps,
-                                                                             row0);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }

@@ -15,19 +15,13 @@ __host__ __device__ constexpr int batch_words(int p) {
   return p == 2 ? 4 : p == 4 ? 6 : p == 8 ? 10 : 16;
 }
 
-// Columns per thread of the renormalisation for P limbs (vector loads of
-// the chunk planes; fewer for the wider integers to bound registers).
-__host__ __device__ constexpr int batch_cols_per_thread(int p) {
-  return p <= 4 ? 4 : p == 8 ? 2 : 1;
-}
-
 // Every stage kernel runs over a flat list of work units (thread blocks);
 // each problem owns a contiguous range of units in every list.
 //   scale:  ceil(m / 8) blocks of 8 rows of A, then ceil(n / 32) blocks of
 //           32 columns of B
 //   digits: Mp x ceil(Kp / 128) blocks of A's digit rows, then
 //           Np x ceil(Kp / 128) of B's
-//   renorm: one row of blocks per output row (m rows), per limb count
+//   renorm: blocks of RENORM_THREADS threads over C, two columns a thread
 struct BatchProblem {
   int p, s, D, m, n, k, Mp, Np, Kp;
   const double *A, *B;
@@ -36,10 +30,11 @@ struct BatchProblem {
   int offE, offF;  // exponents of A's rows at offE, of B's columns at offF
   __nv_bfloat16 *dA, *dB;
   int *chunks;
+  int planes, wide;  // chunk planes in all; C is 16-byte aligned
   long long plane_a, plane_b, plane_c;
   int scale_begin, scale_b_off;  // first scale unit; units of A's rows
   int dig_begin, dig_b_off;      // first digit unit; units of A's digit rows
-  int out_begin;                 // first output row among those of its P
+  int out_begin;                 // first renormalisation unit
 };
 
 enum { kScaleUnits = 0, kDigitUnits = 1, kRenormUnits = 2 };
@@ -62,15 +57,15 @@ __device__ __forceinline__ int find_problem(const BatchProblem *pr, int count, i
 // One launch each over every problem of the batch for the exponents and
 // the digits: NWMAX is the widest integer of the batch (4, 6, 10 or 16
 // words, the P of its widest problem); the kernels switch on each problem's
-// P.  The renormalisation: one launch per P over that P's output rows
-// [row0, row0 + rows), columns up to the widest n of the group.  (Instantiated in batched_w{4,6,10,16}.cu.)
+// P.  (Instantiated in batched_w{4,6,10,16}.cu.)
 template <int NWMAX>
 int launch_batch_scale(const BatchProblem *pr, int count, int units, int *exps, cudaStream_t st);
 template <int NWMAX>
 int launch_batch_digits(const BatchProblem *pr, int count, int units, const int *exps,
                         cudaStream_t st);
-template <int P>
-int launch_batch_renorm(const BatchProblem *pr, int count, int row0, int rows, int max_n,
-                        const int *exps, cudaStream_t st);
+// The renormalisation, whatever the limb counts (renorm.cu); max_d: the most
+// diagonals of any problem.
+int launch_batch_renorm(const BatchProblem *pr, int count, int units, int max_d, const int *exps,
+                        cudaStream_t st);
 
 }  // namespace mdgi

@@ -61,9 +61,7 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
                            int Np, int Kp, const void *dA, const void *dB, const unsigned *norms,
                            int *out, int parts, int raster, int pace, cudaStream_t st);
 
-// Renormalisation from the cross form's output planes (P = 2, 4, 8, 16 at
-// the integer width that the P's default digits need).
-bool cross_renorm_supported(int p, int s, int D);
+// Renormalisation from the cross form's output planes (renorm.cu).
 int launch_cross_renorm(int p, int D, int KB, int m, int n, const int *out, long long plane_c,
                         int ldcd, const int *E, const int *F, double *C, int ldc,
                         cudaStream_t st);

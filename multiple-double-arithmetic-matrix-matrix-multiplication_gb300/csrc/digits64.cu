@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "renorm.cuh"
 #include "slice_common.cuh"
 #include "slice_stages.cuh"
 #include "slice_tc.cuh"
@@ -152,11 +153,13 @@ __global__ void __launch_bounds__(128)
 
 // C[r][c] = RN_P(W * 2^(E[r] + F[c] - 2 (DB - 1) - DB (D - 1))), W built
 // from the top diagonal down: W = W 2^DB + C_d.
-template <int P, int NW>
+// W is built in registers and rounded from shared memory (emit_limbs_shared).
+template <int NW>
 __global__ void __launch_bounds__(128)
-    renorm64_kernel(int D, int m, int n, const long long *__restrict__ Cd,
+    renorm64_kernel(int P, int D, int m, int n, const long long *__restrict__ Cd,
                     const int *__restrict__ E, const int *__restrict__ F, double *__restrict__ C,
-                    int ldc) {
+                    int ldc, bool wide) {
+  __shared__ uint64_t words[(NW + 2) * 128];
   const int r = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
   if (c >= n || r >= m) return;
   uint64_t w[NW];
@@ -170,19 +173,25 @@ __global__ void __launch_bounds__(128)
     mdgi::wide_add_shifted<NW>(w, src[(size_t)d * m * n], 0);
   }
   const int scale = E[r] + F[c] - 2 * (DB - 1) - DB * (D - 1);
-  mdgi::emit_limbs<P, NW>(w, scale, C + ((size_t)r * ldc + c) * P);
+  uint64_t *out = words + threadIdx.x;
+  int lsb = 64 * NW;
+#pragma unroll
+  for (int i = NW - 1; i >= 0; --i) {
+    out[i * 128] = w[i];
+    if (w[i]) lsb = 64 * i + __ffsll((long long)w[i]) - 1;
+  }
+  const uint64_t sign = (uint64_t)((int64_t)w[NW - 1] >> 63);
+  out[NW * 128] = out[(NW + 1) * 128] = sign;
+  mdgi::emit_limbs_shared(P, out, 128, 64 * NW, lsb, sign, scale, C + ((size_t)r * ldc + c) * P,
+                          wide);
 }
 
 template <int NW>
 int launch_renorm64_w(int p, int D, int m, int n, const long long *Cd, const int *E,
                       const int *F, double *C, int ldc, cudaStream_t st) {
   const dim3 grid(mdgi::ceil_div(n, 128), m);
-  switch (p) {
-    case 2: renorm64_kernel<2, NW><<<grid, 128, 0, st>>>(D, m, n, Cd, E, F, C, ldc); break;
-    case 4: renorm64_kernel<4, NW><<<grid, 128, 0, st>>>(D, m, n, Cd, E, F, C, ldc); break;
-    case 8: renorm64_kernel<8, NW><<<grid, 128, 0, st>>>(D, m, n, Cd, E, F, C, ldc); break;
-    default: renorm64_kernel<16, NW><<<grid, 128, 0, st>>>(D, m, n, Cd, E, F, C, ldc); break;
-  }
+  renorm64_kernel<NW><<<grid, 128, 0, st>>>(p, D, m, n, Cd, E, F, C, ldc,
+                                            reinterpret_cast<uintptr_t>(C) % 16 == 0);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }

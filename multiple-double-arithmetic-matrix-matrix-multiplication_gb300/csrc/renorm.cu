@@ -1,0 +1,144 @@
+// Renormalisation kernels of one problem (renorm.cuh).
+#include <algorithm>
+
+#include "batched_table.cuh"
+#include "common.cuh"
+#include "renorm.cuh"
+
+namespace {
+
+using mdgi::RENORM_THREADS;
+
+// Two columns a thread halve the loads and the address work, one column
+// doubles the threads and leaves more blocks their shared memory.  Two / one:
+// dd 16001 x 96 58 / 68 us, qd 8192 x 8192 (cross form) 6.8 / 7.6 ms, qd 1024
+// x 1024 92 / 92 us; with the prefix sums of 55 and 110 diagonals od 2048 x
+// 2048 1275 / 833, hd 1024 x 1024 1120 / 630 us.
+constexpr long long kTwoColumnEntries = 1 << 19;
+constexpr int kTwoColumnDiagonals = 32;
+
+// Threads run over the rows' groups of V columns, row after row.
+template <int V>
+__global__ void __launch_bounds__(RENORM_THREADS)
+    renorm_kernel(int P, int s, int D, int KB, int planes, int m, int n,
+                  const int *__restrict__ chunks, long long plane_c, int ldcd,
+                  const int *__restrict__ E, const int *__restrict__ F, double *__restrict__ C,
+                  int ldc, bool wide) {
+  extern __shared__ uint4 smem[];
+  const int groups = (n + V - 1) / V;
+  const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
+  const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
+  if (r >= m) return;
+  mdgi::renorm_columns<V, false>(P, s, D, KB, planes, n, nullptr, chunks, plane_c, ldcd, E, F, C,
+                                 ldc, r, c0, wide, smem);
+}
+
+template <int V>
+__global__ void __launch_bounds__(RENORM_THREADS)
+    cross_renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::CrossChunks cross,
+                        int m, int n, const int *__restrict__ out, long long plane_c, int ldcd,
+                        const int *__restrict__ E, const int *__restrict__ F,
+                        double *__restrict__ C, int ldc, bool wide) {
+  extern __shared__ uint4 smem[];
+  const int groups = (n + V - 1) / V;
+  const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
+  const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
+  if (r >= m) return;
+  mdgi::renorm_columns<V, true>(P, 0, D, 0, planes, n, &cross, out, plane_c, ldcd, E, F, C, ldc,
+                                r, c0, wide, smem);
+}
+
+// Every problem of a batch: block x belongs to the problem whose units hold x.
+__global__ void __launch_bounds__(RENORM_THREADS)
+    batch_renorm_kernel(const mdgi::BatchProblem *__restrict__ pr, int count,
+                        const int *__restrict__ exps) {
+  extern __shared__ uint4 smem[];
+  const int x = blockIdx.x;
+  const mdgi::BatchProblem &b = pr[mdgi::find_problem<mdgi::kRenormUnits>(pr, count, x)];
+  const int groups = (b.n + 1) / 2;
+  const long long e = (x - b.out_begin) * (long long)RENORM_THREADS + threadIdx.x;
+  const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * 2;
+  if (r >= b.m) return;
+  mdgi::renorm_columns<2, false>(b.p, b.s, b.D, b.Kp / 64, b.planes, b.n, nullptr, b.chunks,
+                                 b.plane_c, b.Np, exps + b.offE, exps + b.offF, b.C, b.ldc, r, c0,
+                                 b.wide, smem);
+}
+
+bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+// The chip is filled anyway and the planes are aligned for 8-byte loads.
+bool two_columns(int m, int n, const int *chunks, long long plane_c, int ldcd) {
+  return (long long)m * n >= kTwoColumnEntries && ldcd % 2 == 0 && plane_c % 2 == 0 &&
+         reinterpret_cast<uintptr_t>(chunks) % 8 == 0;
+}
+
+unsigned blocks(int m, int n, int V) {
+  return mdgi::ceil_div((long long)m * ((n + V - 1) / V), RENORM_THREADS);
+}
+
+template <int V>
+int launch_direct(int p, int s, int D, int KB, int m, int n, const int *chunks, long long plane_c,
+                  int ldcd, const int *E, const int *F, double *C, int ldc, cudaStream_t st) {
+  const int smem = mdgi::renorm_smem(D, V, false);
+  MDG_TRY_CUDA(cudaFuncSetAttribute(renorm_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    smem));
+  renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
+      p, s, D, KB, mdgi::total_chunks(s, D, KB), m, n, chunks, plane_c, ldcd, E, F, C, ldc,
+      aligned16(C));
+  MDG_TRY_LAUNCH();
+  return MDG_SUCCESS;
+}
+
+template <int V>
+int launch_cross(int p, int D, int KB, int m, int n, const int *out, long long plane_c, int ldcd,
+                 const int *E, const int *F, double *C, int ldc, cudaStream_t st) {
+  mdgi::CrossChunks cross{};
+  cross.pairs_per_chunk = mdgi::cross_pairs_per_chunk(KB);
+  for (int d = 1; d < D; ++d)
+    cross.of[d] = (unsigned short)mdgi::cross_chunks(d, cross.pairs_per_chunk);
+  const int smem = mdgi::renorm_smem(D, V, true);
+  MDG_TRY_CUDA(cudaFuncSetAttribute(cross_renorm_kernel<V>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cross_renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
+      p, D, mdgi::cross_outputs(D, KB), cross, m, n, out, plane_c, ldcd, E, F, C, ldc,
+      aligned16(C));
+  MDG_TRY_LAUNCH();
+  return MDG_SUCCESS;
+}
+
+}  // namespace
+
+namespace mdgi {
+
+int launch_renorm(int p, int s, int D, int KB, int m, int n, const int *chunks,
+                  long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
+                  cudaStream_t st) {
+  if (m == 0 || n == 0) return MDG_SUCCESS;
+  if (!words_for(1, D)) return MDG_ERROR_NOT_SUPPORTED;
+  if (two_columns(m, n, chunks, plane_c, ldcd))
+    return launch_direct<2>(p, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
+  return launch_direct<1>(p, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
+}
+
+int launch_cross_renorm(int p, int D, int KB, int m, int n, const int *out, long long plane_c,
+                        int ldcd, const int *E, const int *F, double *C, int ldc,
+                        cudaStream_t st) {
+  if (m == 0 || n == 0) return MDG_SUCCESS;
+  if (!words_for(1, D) || KB > CROSS_CHUNK_STEPS) return MDG_ERROR_NOT_SUPPORTED;
+  if (D <= kTwoColumnDiagonals && two_columns(m, n, out, plane_c, ldcd))
+    return launch_cross<2>(p, D, KB, m, n, out, plane_c, ldcd, E, F, C, ldc, st);
+  return launch_cross<1>(p, D, KB, m, n, out, plane_c, ldcd, E, F, C, ldc, st);
+}
+
+int launch_batch_renorm(const BatchProblem *pr, int count, int units, int max_d, const int *exps,
+                        cudaStream_t st) {
+  if (units == 0) return MDG_SUCCESS;
+  const int smem = renorm_smem(max_d, 2, false);
+  MDG_TRY_CUDA(cudaFuncSetAttribute(batch_renorm_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  batch_renorm_kernel<<<units, RENORM_THREADS, smem, st>>>(pr, count, exps);
+  MDG_TRY_LAUNCH();
+  return MDG_SUCCESS;
+}
+
+}  // namespace mdgi

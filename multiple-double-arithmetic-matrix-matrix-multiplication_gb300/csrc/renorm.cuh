@@ -1,0 +1,340 @@
+// Renormalisation of diagonal sums to P limbs, shared by the single-problem
+// kernels (renorm.cu) and the batched one (batched_stages.cuh).
+//
+// W = sum_d C_d 256^(D-1-d), C_d the sum of diagonal d's chunk planes, is
+// built from the least significant diagonal up, eight diagonals (one 64-bit
+// word) per pass, and rounded to P limbs.  W lives in shared memory and the
+// passes are a loop: with W in registers every word position had to be
+// unrolled, and the code outgrew the instruction cache (registers / shared
+// memory: dd 64 x 64 29 / 8 us, qd 256 x 256 49 / 14 us, dd 16001 x 96 142 /
+// 58 us; the cross form of qd 8192 x 8192 16.3 / 6.8 ms).  It also makes the
+// limb count and the width run-time numbers, so one kernel serves every P
+// and one launch a whole batch (four launches before; 64 mixed problems of
+// 32 .. 512: 3.84 -> 3.42 ms a call).
+//
+// In the cross form (cross_sums.cuh) the planes are the squares P_i and the
+// chunks S of products of sums: a chunk holds the pairs i in [i0, i1) of
+// diagonal d, and
+//   sum over the chunk of A_i B_j + A_j B_i
+//     = S - sum_{i0 <= i < i1} P_i - sum_{d-i1 < j <= d-i0} P_j   (mod 2^32),
+// two differences of prefix sums Q_i = P_0 + .. + P_{i-1}; diagonal d has
+// its chunks, and P_{d/2} for even d.
+#pragma once
+
+#include <stdint.h>
+
+#include "cross_sums.cuh"
+#include "slice_tc.cuh"
+
+namespace mdgi {
+
+constexpr int RENORM_THREADS = 128;
+
+// Chunks of each diagonal in the cross form, by value to its kernel.
+struct CrossChunks {
+  unsigned short of[128];
+  int pairs_per_chunk;
+};
+
+// 64-bit words of W per column: the diagonals', the carry out of them, two
+// of sign (windows of emit_limbs_shared).
+__host__ __device__ inline int renorm_words(int D) { return (D + 7) / 8 + 3; }
+
+// Shared memory of a block: W, and in the cross form the prefix sums.
+__host__ __device__ inline int renorm_smem(int D, int V, bool cross) {
+  return RENORM_THREADS * V * (8 * renorm_words(D) + (cross ? 4 * (D + 1) : 0));
+}
+
+// V adjacent int32.
+template <int V>
+struct Ints;
+template <>
+struct Ints<1> {
+  using T = int;
+  static __device__ __forceinline__ int get(T t, int) { return t; }
+  static __device__ __forceinline__ T put(const int (&x)[1]) { return x[0]; }
+};
+template <>
+struct Ints<2> {
+  using T = int2;
+  static __device__ __forceinline__ int get(T t, int v) { return v ? t.y : t.x; }
+  static __device__ __forceinline__ T put(const int (&x)[2]) { return make_int2(x[0], x[1]); }
+};
+
+// The P limbs of W 2^scale from W's words (word i at w[i * stride]): limb l
+// is the residual R_l = W - (limbs 0..l-1), rounded to nearest-even to 53
+// bits.  W itself is never modified: after a limb rounded at bit sh, the
+// residual is W's bits below sh with every bit from sh up equal to f, where
+// f is all ones if that limb was rounded up and zero otherwise (rounding up
+// leaves a negative remainder, rounding down a non-negative one, and |R|
+// is below 2^sh either way).  So each limb needs: the highest bit of R
+// that differs from f (its magnitude), a 64-bit window of R at that bit,
+// and whether any bit of W lies below the rounding position (the sticky
+// bit, from W's lowest set bit lsb).  The search looks at a 128-bit window
+// of R ending at the current cut h and moves down 64 bits at a time while
+// the window's upper half carries nothing but f.  wide: out is 16-byte
+// aligned and limbs leave in pairs.
+__device__ __forceinline__ void emit_limbs_shared(int P, const uint64_t *w, int stride, int h,
+                                                  int lsb, uint64_t f, int scale, double *out,
+                                                  bool wide) {
+  double even = 0.0;
+#pragma unroll 1
+  for (int l = 0; l < P; ++l) {
+    double val = 0.0;
+    if (f != 0 || lsb < h) {  // else R = 0
+      int b0, t;
+      uint64_t lo, hi;
+      for (;;) {  // h drops by 64 per pass
+        b0 = h > 128 ? h - 128 : 0;
+        const uint64_t *p = w + (b0 >> 6) * stride;
+        const int r = b0 & 63;
+        const uint64_t w0 = p[0], w1 = p[stride], w2 = p[2 * stride];
+        lo = r ? ((w0 >> r) | (w1 << (64 - r))) : w0;
+        hi = r ? ((w1 >> r) | (w2 << (64 - r))) : w1;
+        const int cut = h - b0;  // 0..128: window bits from cut up are f
+        if (cut < 64) {
+          const uint64_t keep = cut ? ((1ull << cut) - 1) : 0ull;
+          lo = (lo & keep) | (f & ~keep);
+          hi = f;
+        } else if (cut < 128) {
+          const uint64_t keep = cut > 64 ? ((1ull << (cut - 64)) - 1) : 0ull;
+          hi = (hi & keep) | (f & ~keep);
+        }
+        const uint64_t xh = hi ^ f, xl = lo ^ f;
+        if (xh) {
+          t = b0 + 127 - __clzll((long long)xh);
+          break;
+        }
+        if (b0 == 0) {
+          t = xl ? 63 - __clzll((long long)xl) : -1;  // -1: R = -1
+          break;
+        }
+        h = b0 + 64;
+      }
+      // rounding position sh; x = bits [sh - 1, sh + 63) of R: the round bit,
+      // then m = floor(R / 2^sh), |m| <= 2^53 (sh = 0: R itself, b0 = 0)
+      const int sh = t > 52 ? t - 52 : 0;
+      uint64_t x;
+      if (sh == 0) {
+        x = lo << 1;
+      } else {
+        const int o = sh - 1 - b0;  // 0..127
+        if (o < 64)
+          x = o ? ((lo >> o) | (hi << (64 - o))) : lo;
+        else
+          x = o > 64 ? ((hi >> (o - 64)) | (f << (128 - o))) : hi;
+      }
+      const int64_t m = (int64_t)x >> 1;
+      const bool up = sh > 0 && (x & 1ull) && (lsb < sh - 1 || (m & 1));
+      const int64_t mr = up ? m + 1 : m;
+      f = up ? ~0ull : 0ull;
+      h = sh;
+      // mr 2^(sh + scale) as a double; with the top bit at 52 (or 53) and a
+      // normal exponent it is assembled from its fields by integer
+      // instructions, otherwise converted and scaled in FP64
+      const bool neg = mr < 0;
+      const uint64_t mm = neg ? (uint64_t)(-mr) : (uint64_t)mr;
+      const bool carry = mm >> 53;
+      const uint64_t frac = carry ? (mm >> 1) : mm;
+      const int be = sh + scale + 52 + (carry ? 1 : 0) + 1023;
+      if ((frac >> 52) == 1 && be >= 1 && be <= 2046)
+        val = __longlong_as_double((long long)(((uint64_t)be << 52) | (frac & ((1ull << 52) - 1))));
+      else
+        val = ldexp((double)mm, sh + scale);
+      if (neg) val = -val;
+    }
+    if (!wide)
+      out[l] = val;
+    else if (l & 1)
+      *reinterpret_cast<double2 *>(out + l - 1) = make_double2(even, val);
+    even = val;
+  }
+}
+
+// val += c 2^(8 j) for |c| < 2^54, what would pass 2^63 into `up`, whose
+// unit is 2^32.
+__device__ __forceinline__ void add_at(long long &val, long long &up, long long c, int j) {
+  if (j < 2) {
+    val += (c & 0xffffff) * (1ll << (8 * j)) + (c >> 24) * (1ll << (24 + 8 * j));
+  } else {
+    val += (c & 0xffffff) * (1ll << (8 * j));
+    up += (c >> 24) * (1ll << (8 * j - 8));
+  }
+}
+
+// One thread: row r, columns c0 .. c0 + V - 1 (c0 < n) of one problem.
+// planes: chunk planes in all.  The sums of a pass are loaded together, the
+// first two chunks of each of its eight diagonals, so that the DRAM latency
+// is paid once per eight to sixteen loads; in the cross form all D squares go
+// to shared memory first, where the thread turns its own columns into prefix
+// sums.
+template <int V, bool CROSS>
+__device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int planes, int n,
+                                               const CrossChunks *cross,
+                                               const int *__restrict__ chunks, long long plane_c,
+                                               int ldcd, const int *__restrict__ E,
+                                               const int *__restrict__ F, double *__restrict__ C,
+                                               int ldc, int r, int c0, bool wide, void *smem) {
+  using I = Ints<V>;
+  using Vec = typename I::T;
+  constexpr int T = RENORM_THREADS;
+  const int dwords = (D + 7) / 8;
+  // word i of column v at W[(i * V + v) * T]; Q_i at Q[i * T]
+  uint64_t *W = reinterpret_cast<uint64_t *>(smem) + threadIdx.x;
+  Vec *Q = reinterpret_cast<Vec *>(reinterpret_cast<uint64_t *>(smem) + (dwords + 3) * V * T) +
+           threadIdx.x;
+  const int *src = chunks + (size_t)r * ldcd + c0;
+  const int ppc = CROSS ? cross->pairs_per_chunk : 0;
+  if constexpr (CROSS) {
+    for (int i = 0; i < D; ++i) {
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Q + i * T);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst),
+                   "l"(src + (size_t)i * plane_c), "n"(4 * V)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    int run[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) run[v] = 0;
+#pragma unroll 4
+    for (int i = 0; i < D; ++i) {
+      const Vec x = Q[i * T];
+      Q[i * T] = I::put(run);
+#pragma unroll
+      for (int v = 0; v < V; ++v) run[v] = (int)((unsigned)run[v] + (unsigned)I::get(x, v));
+    }
+    Q[D * T] = I::put(run);
+  }
+
+  long long carry[V];
+  int lsb[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    carry[v] = 0;
+    lsb[v] = 1 << 20;
+  }
+  int q = planes;  // the chunk planes of the diagonals above the current one start here
+#pragma unroll 1
+  for (int wi = 0; wi < dwords; ++wi) {
+    Vec x0[8], x1[8];
+    int first[8], nc[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const int d = D - 1 - (wi * 8 + b);
+      nc[b] = d < 0 ? 0 : CROSS ? cross->of[d] : diag_chunks(d, s, KB);
+      q -= nc[b];
+      first[b] = q;
+      if (nc[b] > 0) x0[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)q * plane_c));
+      if (nc[b] > 1)
+        x1[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(q + 1) * plane_c));
+    }
+    uint64_t word[V];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      long long val[V], up[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        val[v] = carry[v];
+        up[v] = 0;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int b = 4 * half + j, d = D - 1 - (wi * 8 + b);
+        if (d < 0) continue;
+        const long long unit = 1ll << (8 * j);
+        if constexpr (CROSS) {
+          const bool even = !(d & 1);
+          int square[V];  // P_{d/2}
+          if (even) {
+            const Vec lo = Q[(d / 2) * T], hi = Q[(d / 2 + 1) * T];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              square[v] = (int)((unsigned)I::get(hi, v) - (unsigned)I::get(lo, v));
+              val[v] += square[v] * unit;
+            }
+          }
+          if (nc[b] == 1) {  // all pairs: every P_i, i <= d, but the middle one
+            const Vec all = Q[(d + 1) * T];
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+              val[v] += (int)((unsigned)I::get(x0[b], v) - (unsigned)I::get(all, v) +
+                              (even ? (unsigned)square[v] : 0u)) *
+                        unit;
+            continue;
+          }
+          const int pairs = cross_pairs(d);
+          for (int c = 0; c < nc[b]; ++c) {
+            const int i0 = c * ppc, i1 = min(pairs, i0 + ppc);
+            const Vec x = c == 0   ? x0[b]
+                          : c == 1 ? x1[b]
+                                   : __ldcs(reinterpret_cast<const Vec *>(
+                                         src + (size_t)(first[b] + c) * plane_c));
+            const Vec a0 = Q[i0 * T], a1 = Q[i1 * T];
+            const Vec b0 = Q[(d - i1 + 1) * T], b1 = Q[(d - i0 + 1) * T];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              const int t = (int)((unsigned)I::get(x, v) + (unsigned)I::get(a0, v) -
+                                  (unsigned)I::get(a1, v) + (unsigned)I::get(b0, v) -
+                                  (unsigned)I::get(b1, v));
+              if (c < 2)
+                val[v] += t * unit;
+              else
+                add_at(val[v], up[v], t, j);
+            }
+          }
+        } else {
+          // at most 2^31 2^24 each: the first two chunks of four diagonals
+          // stay below 2^58
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            val[v] += I::get(x0[b], v) * unit;
+            if (nc[b] > 1) val[v] += I::get(x1[b], v) * unit;
+          }
+          if (nc[b] > 2) {
+            long long rest[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) rest[v] = 0;
+            for (int c = 2; c < nc[b]; ++c) {
+              const Vec x =
+                  __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(first[b] + c) * plane_c));
+#pragma unroll
+              for (int v = 0; v < V; ++v) rest[v] += I::get(x, v);
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) add_at(val[v], up[v], rest[v], j);
+          }
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const uint64_t bits = (uint32_t)val[v];
+        word[v] = half ? (word[v] | bits << 32) : bits;
+        carry[v] = (val[v] >> 32) + up[v];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      W[(wi * V + v) * T] = word[v];
+      if (word[v] && lsb[v] == 1 << 20) lsb[v] = 64 * wi + __ffsll((long long)word[v]) - 1;
+    }
+  }
+  const int scale = E[r] - 14 - 8 * (D - 1);
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const uint64_t f = (uint64_t)(carry[v] >> 63);
+    W[(dwords * V + v) * T] = (uint64_t)carry[v];
+    W[((dwords + 1) * V + v) * T] = f;
+    W[((dwords + 2) * V + v) * T] = f;
+    if (carry[v] && lsb[v] == 1 << 20) lsb[v] = 64 * dwords + __ffsll(carry[v]) - 1;
+  }
+#pragma unroll 1
+  for (int v = 0; v < V; ++v) {
+    if (c0 + v >= n) break;
+    const int low = V == 2 && v ? lsb[V - 1] : lsb[0];
+    const long long top = V == 2 && v ? carry[V - 1] : carry[0];
+    emit_limbs_shared(P, W + v * T, V * T, 64 * (dwords + 1), low, (uint64_t)(top >> 63),
+                      scale + F[c0 + v], C + ((size_t)r * ldc + c0 + v) * P, wide);
+  }
+}
+
+}  // namespace mdgi

@@ -54,42 +54,6 @@ __device__ __forceinline__ uint64_t wide_bits64(const uint64_t (&w)[NW], int pos
   return r ? ((lo >> r) | (hi << (64 - r))) : lo;
 }
 
-// Bits [pos, pos + 128) of w (0 <= pos < 64 NW) as lo and hi; bits above the
-// top word read as the sign.  The same barrel shift as wide_bits64, over
-// one more word.
-template <int NW>
-__device__ __forceinline__ void wide_bits128(const uint64_t (&w)[NW], int pos, uint64_t &lo,
-                                             uint64_t &hi) {
-  const int qw = pos >> 6, r = pos & 63;
-  const uint64_t fill = (uint64_t)((int64_t)w[NW - 1] >> 63);
-  uint64_t t[NW + 2];
-#pragma unroll
-  for (int i = 0; i < NW; ++i) t[i] = w[i];
-  t[NW] = fill;
-  t[NW + 1] = fill;
-#pragma unroll
-  for (int bit = 1; bit <= NW; bit <<= 1) {
-    const bool on = (qw & bit) != 0;
-#pragma unroll
-    for (int i = 0; i <= NW + 1; ++i) {
-      const uint64_t src = (i + bit <= NW + 1) ? t[i + bit] : fill;
-      t[i] = on ? src : t[i];
-    }
-  }
-  lo = r ? ((t[0] >> r) | (t[1] << (64 - r))) : t[0];
-  hi = r ? ((t[1] >> r) | (t[2] << (64 - r))) : t[1];
-}
-
-// Index of the lowest set bit of w, 64 NW for zero.
-template <int NW>
-__device__ __forceinline__ int wide_lsb(const uint64_t (&w)[NW]) {
-  int b = 64 * NW;
-#pragma unroll
-  for (int i = NW - 1; i >= 0; --i)
-    if (w[i]) b = 64 * i + __ffsll((long long)w[i]) - 1;
-  return b;
-}
-
 // x = m 2^e2 with m an integer, |m| < 2^53 (0 for x = +-0), read from the
 // IEEE fields of a finite x with integer instructions only: the FP64 units
 // of this GPU are narrow, and frexp / ldexp / an FP64-to-int conversion per

@@ -271,8 +271,7 @@ SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
 SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k) {
   const SlicePlan pairs = make_slice_plan(p, s, D, m, n, k);
   const int KB = pairs.Kp / 64;
-  if (KB > CROSS_CHUNK_STEPS || !cross_pays(p, pairs.Mp, pairs.Np, KB) ||
-      !cross_renorm_supported(p, s, D))
+  if (D < 2 || D > s || KB > CROSS_CHUNK_STEPS || !cross_pays(p, pairs.Mp, pairs.Np, KB))
     return pairs;
   const int all = cross_offset(D), least = cross_pairs(D - 1);
   const double plane_bytes = 2.0 * ((double)pairs.plane_a + pairs.plane_b);
@@ -358,32 +357,6 @@ int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, co
                                      plane_b, chunks, plane_c, Np);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
-}
-
-int launch_renorm(int p, int s, int D, int KB, int m, int n, const int *chunks,
-                  long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
-                  cudaStream_t st) {
-  if (m == 0 || n == 0) return MDG_SUCCESS;
-  const int NW = words_for(1, D);
-  if (!NW) return MDG_ERROR_NOT_SUPPORTED;
-  // V adjacent columns per thread need V-aligned rows of chunk planes
-  const int Vmax = NW <= 6 ? 4 : NW <= 10 ? 2 : 1;
-  int V = Vmax;
-  while (V > 1 && ((ldcd % V) || (plane_c % V) ||
-                   (reinterpret_cast<uintptr_t>(chunks) % (4 * V))))
-    V >>= 1;
-  switch (p) {
-    case 2:
-      return launch_renorm_p<2>(NW, V, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
-    case 4:
-      return launch_renorm_p<4>(NW, V, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
-    case 8:
-      return launch_renorm_p<8>(NW, V, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
-    case 16:
-      return launch_renorm_p<16>(NW, V, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
-    default:
-      return MDG_ERROR_INVALID_LIMBS;
-  }
 }
 
 int slice_prepare_b(const SlicePlan &pl, const double *B, int ldb, void *ws, cudaStream_t st) {

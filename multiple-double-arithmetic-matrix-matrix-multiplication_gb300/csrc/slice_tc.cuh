@@ -86,12 +86,7 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, co
                         int ld, long long plane_a, long long plane_b, int *chunks,
                         long long plane_c, int single, int parts, int raster, cudaStream_t st,
                         int pace = 0);
-// Renormalisation for P limbs with NW-word integers, V columns per thread
-// (instantiated in renorm_p{2,4,8,16}.cu).
-template <int P>
-int launch_renorm_p(int NW, int V, int s, int D, int KB, int m, int n, const int *chunks,
-                    long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
-                    cudaStream_t st);
+// Renormalisation of chunk planes (renorm.cu).
 int launch_renorm(int p, int s, int D, int KB, int m, int n, const int *chunks,
                   long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
                   cudaStream_t st);
