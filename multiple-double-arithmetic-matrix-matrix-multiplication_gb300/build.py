@@ -24,11 +24,9 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler",
           "-fPIC,-ffp-contract=off", "-I", INCLUDE, "-I", CSRC,
           "--expt-relaxed-constexpr"] + ARCH
 
-# The batch's wide-integer stage kernels are spread over one unit per
-# integer width (batched_w*), so that ptxas works on them in parallel.
 SOURCES = ["capi.cu", "plain_gemm.cu", "floatybits.cu", "fp64split.cu", "slice_tc.cu",
            "diag_gemm_tc.cu", "cross_sums.cu", "renorm.cu", "dropin.cu", "noalloc.cu", "batched.cu", "generate.cu",
-           "gemm_ex.cu", "plan.cu", "digits64.cu", "batched_w4.cu", "batched_w6.cu", "batched_w10.cu", "batched_w16.cu"]
+           "gemm_ex.cu", "plan.cu", "digits64.cu", "batched_stages.cu"]
 
 
 def _compile(src):

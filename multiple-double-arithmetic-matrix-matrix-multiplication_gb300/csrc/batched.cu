@@ -11,8 +11,7 @@
 //   one launch: grouped tcgen05 diagonal GEMM over the tiles of all problems
 //   one launch: renormalisation of every C
 // Each stage kernel finds its problem from its block index by binary search
-// over per-problem prefix counts, and branches on the problem's P to the
-// integer width that P needs (batched_stages.cuh).  The grouped GEMM's tiles
+// over per-problem prefix counts (batched_stages.cu, renorm.cu).  The grouped GEMM's tiles
 // are 128 rows by 256 or 128 columns per problem, or 256 x 256 on CTA pairs
 // (a tile policy the plan can tune); heavy tiles can be cut into ranges of
 // diagonals (the split mode, tuned too).  Each problem's result equals the
@@ -32,9 +31,9 @@
 #include "batched_table.cuh"
 
 struct mdg_batch_s {
-  int count = 0, nwmax = 4, total_units = 0;
+  int count = 0, total_units = 0;
   int scale_units = 0, digit_units = 0, renorm_units = 0;
-  int max_d = 1;  // most diagonals of any problem
+  int max_d = 1;  // most digits (and diagonals) of any problem
   int tiles_policy = MDG_BATCH_TILES_256, split = 1;
   mdgi::BatchProblem *dprobs = nullptr;
   mdgi::GroupedProblem *dgroups = nullptr;
@@ -152,7 +151,6 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
   L->off_dB.resize(count);
   L->off_chunks.resize(count);
   int scale_u = 0, digit_u = 0, renorm_u = 0, offE = 0, offF = rows;
-  h->nwmax = 4;
   // the table is kept in order of P (stable): blocks of one P sit together
   // in every stage's launch
   std::vector<int> order(count);
@@ -171,14 +169,14 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
     L->off_dA[i] = take(sizeof(__nv_bfloat16) * (size_t)s * Mp * Kp);
     L->off_dB[i] = take(sizeof(__nv_bfloat16) * (size_t)s * Np * Kp);
     L->off_chunks[i] = take(sizeof(int) * (size_t)nch * Mp * Np);
-    const int nw = std::max(mdgi::words_for(s, 1), mdgi::words_for(1, D));
-    if (!nw || nw > mdgi::batch_words(q.p)) return MDG_ERROR_NOT_SUPPORTED;
-    h->nwmax = std::max(h->nwmax, mdgi::batch_words(q.p));
-    const int kblocks = (q.k + 127) / 128;
-    const int scale_a = (q.m + 7) / 8, scale_b = (q.n + 31) / 32;
+    const int scale_a = mdgi::ceil_div(q.m, mdgi::SCALE_ROWS);
+    const int scale_b = mdgi::ceil_div(q.n, mdgi::SCALE_COLS);
     // digits: valid rows and k-positions only (the padding is cleared once,
     // by mdg_batch_create)
-    const int digit_a = q.m * kblocks, digit_b = q.n * kblocks;
+    const long long kpairs = (q.k + 1) / 2;
+    const long long digit_a = mdgi::ceil_div(q.m * kpairs, mdgi::DIGIT_THREADS);
+    const long long digit_b = mdgi::ceil_div(q.n * kpairs, mdgi::DIGIT_THREADS);
+    if (digit_u + digit_a + digit_b > (1LL << 30)) return MDG_ERROR_INVALID_SIZE;
     const long long out_u = mdgi::ceil_div((long long)q.m * ((q.n + 1) / 2), mdgi::RENORM_THREADS);
     if (renorm_u + out_u > (1LL << 30)) return MDG_ERROR_INVALID_SIZE;
     if (ws) {
@@ -196,13 +194,13 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
       b.plane_b = (long long)Np * Kp;
       b.plane_c = (long long)Mp * Np;
       b.scale_begin = scale_u; b.scale_b_off = scale_a;
-      b.dig_begin = digit_u; b.dig_b_off = digit_a;
+      b.dig_begin = digit_u; b.dig_b_off = (int)digit_a;
       b.out_begin = renorm_u;
       hp->push_back(b);
     }
     h->max_d = std::max(h->max_d, D);
     scale_u += scale_a + scale_b;
-    digit_u += digit_a + digit_b;
+    digit_u += (int)(digit_a + digit_b);
     renorm_u += (int)out_u;
     offE += std::max(q.m, 1);
     offF += std::max(q.n, 1);
@@ -336,16 +334,8 @@ int mdg_batch_create(const mdg_problem *problems, int count, void *workspace,
 int mdg_batch_run(mdg_batch_s *h, void *stream) {
   if (!h) return MDG_ERROR_NULL_POINTER;
   cudaStream_t st = mdgi::as_stream(stream);
-#define MDG_BATCH_STAGES(W)                                                               \
-  MDG_TRY(mdgi::launch_batch_scale<W>(h->dprobs, h->count, h->scale_units, h->exps, st)); \
-  MDG_TRY(mdgi::launch_batch_digits<W>(h->dprobs, h->count, h->digit_units, h->exps, st))
-  switch (h->nwmax) {
-    case 4: MDG_BATCH_STAGES(4); break;
-    case 6: MDG_BATCH_STAGES(6); break;
-    case 10: MDG_BATCH_STAGES(10); break;
-    default: MDG_BATCH_STAGES(16); break;
-  }
-#undef MDG_BATCH_STAGES
+  MDG_TRY(mdgi::launch_batch_scale(h->dprobs, h->count, h->scale_units, h->exps, st));
+  MDG_TRY(mdgi::launch_batch_digits(h->dprobs, h->count, h->digit_units, h->max_d, h->exps, st));
   MDG_TRY(mdgi::launch_diag_gemm_grouped(h->dgroups, h->count, h->total_units,
                                          h->tiles_policy == MDG_BATCH_TILES_PAIR, st));
   MDG_TRY(mdgi::launch_batch_renorm(h->dprobs, h->count, h->renorm_units, h->max_d, h->exps, st));

@@ -1,6 +1,6 @@
 // The problem table of the batched slice-digit GEMM (batched.cu) and the
 // lookup of a block's problem, shared by the planning code and the stage
-// kernels of batched_w{4,6,10,16}.cu.
+// kernels (batched_stages.cu, renorm.cu).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -9,18 +9,11 @@
 
 namespace mdgi {
 
-// Integer words of the digit and renormalisation stages for P limbs at the
-// default digit count (words_for(s, 1) and words_for(1, D), s = D).
-__host__ __device__ constexpr int batch_words(int p) {
-  return p == 2 ? 4 : p == 4 ? 6 : p == 8 ? 10 : 16;
-}
-
 // Every stage kernel runs over a flat list of work units (thread blocks);
 // each problem owns a contiguous range of units in every list.
-//   scale:  ceil(m / 8) blocks of 8 rows of A, then ceil(n / 32) blocks of
-//           32 columns of B
-//   digits: Mp x ceil(Kp / 128) blocks of A's digit rows, then
-//           Np x ceil(Kp / 128) of B's
+//   scale:  blocks of SCALE_ROWS rows of A, then of SCALE_COLS columns of B
+//   digits: blocks of DIGIT_THREADS threads over A's digit rows, two
+//           k-positions a thread, then over B's
 //   renorm: blocks of RENORM_THREADS threads over C, two columns a thread
 struct BatchProblem {
   int p, s, D, m, n, k, Mp, Np, Kp;
@@ -54,14 +47,10 @@ __device__ __forceinline__ int find_problem(const BatchProblem *pr, int count, i
   return lo;
 }
 
-// One launch each over every problem of the batch for the exponents and
-// the digits: NWMAX is the widest integer of the batch (4, 6, 10 or 16
-// words, the P of its widest problem); the kernels switch on each problem's
-// P.  (Instantiated in batched_w{4,6,10,16}.cu.)
-template <int NWMAX>
+// One launch each over every problem of the batch (batched_stages.cu); max_s:
+// the most digits of any problem.
 int launch_batch_scale(const BatchProblem *pr, int count, int units, int *exps, cudaStream_t st);
-template <int NWMAX>
-int launch_batch_digits(const BatchProblem *pr, int count, int units, const int *exps,
+int launch_batch_digits(const BatchProblem *pr, int count, int units, int max_s, const int *exps,
                         cudaStream_t st);
 // The renormalisation, whatever the limb counts (renorm.cu); max_d: the most
 // diagonals of any problem.

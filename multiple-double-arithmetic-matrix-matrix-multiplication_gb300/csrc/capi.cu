@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "slice_stages.cuh"
 #include "slice_tc.cuh"
 
 namespace mdgi {
@@ -641,8 +642,7 @@ int mdg_scale_exponents(int p, int m, int n, int k, const double *A, int lda, co
   MDG_TRY(g_cache.get(3, sizeof(unsigned long long) * (size_t)(std::max(m, 1) + std::max(n, 1)),
                       &bits));
   auto *rb = reinterpret_cast<unsigned long long *>(bits);
-  return launch_scale_exponents(p, m, n, k, A, lda, B, ldb, rb, rb + std::max(m, 1), E, F,
-                                as_stream(stream));
+  return launch_scale_exponents(p, m, n, k, A, lda, B, ldb, rb, E, F, as_stream(stream));
 }
 
 int mdg_slice_digits(int p, int s, int rows, int cols, const double *X, int ldx, const int *E,
@@ -654,8 +654,11 @@ int mdg_slice_digits(int p, int s, int rows, int cols, const double *X, int ldx,
   if (trans ? (ldx < std::max(rows, 1)) : (ldx < std::max(cols, 1))) return MDG_ERROR_INVALID_SIZE;
   if (rows > 0 && cols > 0 && (!X || !E || !planes)) return MDG_ERROR_NULL_POINTER;
   if (rows > 65535) return MDG_ERROR_NOT_SUPPORTED;
-  return launch_digits(p, s, rows, cols, X, ldx, E, trans, planes, ld_out, plane_stride, rows,
-                       cols, as_stream(stream));
+  DigitSide x{X, E, reinterpret_cast<__nv_bfloat16 *>(planes), ldx, trans != 0, rows, cols, ld_out,
+              cols, plane_stride};
+  DigitSide none = x;
+  none.rows = 0;
+  return launch_digits(p, s, x, none, nullptr, as_stream(stream));
 }
 
 int mdg_slice_chunk_count(int s, int D, int k) {

@@ -236,8 +236,7 @@ Digits64Plan make_digits64_plan(int p, int s, int D, int m, int n, int k) {
     off = align_up(off + bytes, 256);
     return o;
   };
-  pl.off_rowbits = take(sizeof(unsigned long long) * std::max(m, 1));
-  pl.off_colbits = take(sizeof(unsigned long long) * std::max(n, 1));
+  pl.off_bits = take(sizeof(unsigned long long) * ((size_t)std::max(m, 1) + std::max(n, 1)));
   pl.off_E = take(sizeof(int) * std::max(m, 1));
   pl.off_F = take(sizeof(int) * std::max(n, 1));
   pl.off_dA = take(sizeof(double) * (size_t)s * m * k);
@@ -253,15 +252,14 @@ int run_digits64_gemm(const Digits64Plan &pl, const double *A, int lda, const do
   if (!NW) return MDG_ERROR_NOT_SUPPORTED;
   if (pl.m > 65535 || pl.n > 65535 || pl.D > 65535) return MDG_ERROR_NOT_SUPPORTED;
   char *base = reinterpret_cast<char *>(ws);
-  auto *rowbits = reinterpret_cast<unsigned long long *>(base + pl.off_rowbits);
-  auto *colbits = reinterpret_cast<unsigned long long *>(base + pl.off_colbits);
+  auto *bits = reinterpret_cast<unsigned long long *>(base + pl.off_bits);
   int *E = reinterpret_cast<int *>(base + pl.off_E);
   int *F = reinterpret_cast<int *>(base + pl.off_F);
   double *dA = reinterpret_cast<double *>(base + pl.off_dA);
   double *dB = reinterpret_cast<double *>(base + pl.off_dB);
   long long *Cd = reinterpret_cast<long long *>(base + pl.off_Cd);
   NvtxRange range("mdg fp64_digits");
-  MDG_TRY(launch_scale_exponents(pl.p, pl.m, pl.n, pl.k, A, lda, B, ldb, rowbits, colbits, E, F,
+  MDG_TRY(launch_scale_exponents(pl.p, pl.m, pl.n, pl.k, A, lda, B, ldb, bits, E, F,
                                  st));
   const long long pa = (long long)pl.m * pl.k, pb = (long long)pl.n * pl.k;
 #define MDG_DIGITS64(W)                                                                        \

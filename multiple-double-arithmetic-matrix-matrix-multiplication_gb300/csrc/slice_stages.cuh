@@ -1,6 +1,6 @@
-// Per-element / per-block bodies of the slice-digit stage kernels, shared
-// by the single-problem kernels (slice_tc.cu) and the batched kernels
-// (batched.cu).  See slice_tc.cu for what each stage computes.
+// Bodies of the scale and digit stages of the slice-digit form, shared by the
+// single-problem kernels (slice_tc.cu) and the batched kernels
+// (batched_stages.cu).  See slice_tc.cu for what each stage computes.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -12,6 +12,10 @@
 namespace mdgi {
 
 // ------------------------------------------------------------ exponents --
+__device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) {
+  return a > b ? a : b;
+}
+
 // sum_l |x_l| of one entry (FP64 additions in limb order), as its bit
 // pattern: maxima of non-negative doubles are taken as 64-bit unsigned
 // integers, which orders them like the doubles and keeps the reductions off
@@ -23,172 +27,182 @@ __device__ __forceinline__ unsigned long long abs_sum_bits(const double *x, int 
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   return b > 0x7ff0000000000000ull ? 0ull : b;
 }
-__device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) {
-  return a > b ? a : b;
+
+// The rows of A are taken a warp each, the columns of B 8 to a block, so
+// that a stage writes every maximum once: no atomics, nothing cleared first.
+constexpr int SCALE_THREADS = 256, SCALE_ROWS = SCALE_THREADS / 32, SCALE_COLS = 8;
+
+// Largest entry of row r over the columns [c0, c1), in every lane.
+__device__ __forceinline__ unsigned long long row_max(int P, const double *__restrict__ X, int ldx,
+                                                      int r, int c0, int c1) {
+  unsigned long long mx = 0;
+  const double *row = X + (size_t)r * ldx * P;
+#pragma unroll 4
+  for (int c = c0 + (int)(threadIdx.x & 31); c < c1; c += 32)
+    mx = umax64(mx, abs_sum_bits(row + (size_t)c * P, P));
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mx = umax64(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  return mx;
 }
 
-// Block 32 x 8 covers 32 columns x 256 rows; each warp walks 32 rows of
-// one 32-column strip.  Row maxima: warp reduction, one atomic per row per
-// warp.  Column maxima: one atomic per thread.
-__device__ __forceinline__ void absmax_block(int P, int R, int Cn, const double *__restrict__ X,
-                                             int ldx, unsigned long long *rowbits,
-                                             unsigned long long *colbits, int bx, int by) {
-  const int c = bx * 32 + threadIdx.x;
-  const int r0 = by * 256 + threadIdx.y * 32;
-  unsigned long long cm = 0;
-  for (int rr = 0; rr < 32; ++rr) {
-    const int r = r0 + rr;
-    if (r >= R) break;
-    const unsigned long long v = c < Cn ? abs_sum_bits(X + ((size_t)r * ldx + c) * P, P) : 0ull;
-    cm = umax64(cm, v);
-    if (rowbits) {
-      unsigned long long w = v;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) w = umax64(w, __shfl_xor_sync(0xffffffffu, w, o));
-      if (threadIdx.x == 0) atomicMax(rowbits + r, w);
-    }
+// Largest entry of column c0 + (thread % 8) over the rows [r0, r1), valid in
+// the block's first 8 threads.  A warp reads four rows of 8 adjacent entries.
+__device__ __forceinline__ unsigned long long col_max(int P, const double *__restrict__ X, int ldx,
+                                                      int c0, int cols, int r0, int r1) {
+  __shared__ unsigned long long part[SCALE_THREADS / 32][SCALE_COLS];
+  const int c = c0 + (int)(threadIdx.x & 7);
+  unsigned long long mx = 0;
+  if (c < cols) {
+#pragma unroll 4
+    for (int r = r0 + (int)(threadIdx.x >> 3); r < r1; r += SCALE_THREADS / 8)
+      mx = umax64(mx, abs_sum_bits(X + ((size_t)r * ldx + c) * P, P));
   }
-  if (colbits && c < Cn) atomicMax(colbits + c, cm);
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) mx = umax64(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) < SCALE_COLS) part[threadIdx.x >> 5][threadIdx.x & 7] = mx;
+  __syncthreads();
+  if (threadIdx.x < SCALE_COLS)
+#pragma unroll
+    for (int w = 1; w < SCALE_THREADS / 32; ++w) mx = umax64(mx, part[w][threadIdx.x]);
+  return mx;
 }
 
 // --------------------------------------------------------------- digits --
-// BF16 bits of an integer d in [-128, 127] without a conversion instruction
-// (conversions run at a fraction of the FP32 rate): 2^23 + 128 + d written
-// into the bit pattern of 2^23 is that integer as a float, and subtracting
-// 2^23 + 128 in FP32 leaves d exactly; a float with at most 8 significant
-// bits has its low 16 bits clear, so its top half is d in BF16.
-__device__ __forceinline__ uint32_t bf16_bits_of_digit(int d) {
-  const float f = __int_as_float(0x4B000000 + 128 + d) - 8388736.0f;
-  return __float_as_uint(f) >> 16;
+constexpr int DIGIT_THREADS = 128;
+
+// 32-bit words of an entry's integer V: the s - 1 low digits, then the 32
+// bits that the leading digit is read from.
+__host__ __device__ inline int digit_words(int s) { return (s - 1) / 4 + 2; }
+__host__ __device__ inline int digit_smem(int s, int V) {
+  return digit_words(s) * V * DIGIT_THREADS * 8;
 }
 
-// One thread per element of the padded plane (prow, pcol); pcol (the k
-// index) is the fastest, so plane stores are coalesced.  Outside the valid
-// region every digit is zero.
-template <int NW>
-__device__ __forceinline__ void digits_elem(int P, int s, int rows, int cols,
-                                            const double *__restrict__ X, int ldx,
-                                            const int *__restrict__ E, int trans,
-                                            __nv_bfloat16 *__restrict__ planes, int ld_out,
-                                            long long plane_stride, int rows_pad, int cols_pad,
-                                            int pr, int pc) {
-  if (pc >= cols_pad || pr >= rows_pad) return;
-  __nv_bfloat16 *out = planes + (size_t)pr * ld_out + pc;
-  if (pr >= rows || pc >= cols) {
-    for (int i = 0; i < s; ++i) out[i * plane_stride] = __float2bfloat16_rn(0.0f);
-    return;
-  }
-  const double *a = trans ? X + ((size_t)pc * ldx + pr) * P : X + ((size_t)pr * ldx + pc) * P;
-  const int S = 7 + 8 * (s - 1);
-  const int Er = E[pr];
-  uint64_t w[NW];
-#pragma unroll
-  for (int i = 0; i < NW; ++i) w[i] = 0;
-  for (int l = 0; l < P; ++l) {
-    int e2;
-    const int64_t m = mdgi::exact_significand(a[l], e2);
-    if (m == 0) continue;
-    const int q = e2 + S - Er;
-    if (q >= 0) {
-      mdgi::wide_add_shifted<NW>(w, m, q);
-    } else if (q > -64) {
-      mdgi::wide_add_shifted<NW>(w, m >> (-q), 0);
-    } else {
-      mdgi::wide_add_shifted<NW>(w, m < 0 ? -1 : 0, 0);
-    }
-  }
-  // balanced digits from the bottom: t = byte + carry, t >= 128 -> t - 256
-  int carry = 0;
-#pragma unroll
-  for (int wi = 0; wi < NW; ++wi) {
-    const uint64_t word = w[wi];
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int p = wi * 8 + b;
-      if (p < s - 1) {
-        const int t = (int)((word >> (8 * b)) & 255) + carry;
-        const int d = t >= 128 ? t - 256 : t;
-        carry = t >= 128 ? 1 : 0;
-        out[(s - 1 - p) * plane_stride] =
-            __ushort_as_bfloat16((unsigned short)bf16_bits_of_digit(d));
-      }
-    }
-  }
-  const int top = (int)(int64_t)mdgi::wide_bits64<NW>(w, 8 * (s - 1)) + carry;
-  out[0] = __float2bfloat16_rn((float)top);
-}
+// One operand: X rows x cols (trans: cols x rows), E its rows' exponents,
+// digit planes of rows x ld_out, of which cols_pad columns are written (the
+// ones from cols on with zeros).
+struct DigitSide {
+  const double *X;
+  const int *E;
+  __nv_bfloat16 *planes;
+  int ldx, trans, rows, cols, ld_out, cols_pad;
+  long long plane_stride;
+};
 
-// Four consecutive k-positions per thread: the same digits as digits_elem,
-// written as one 8-byte vector (4 BF16) per plane.  pc0 is a multiple of 4;
-// cols_pad, ld_out and plane_stride are multiples of 4.
-template <int NW>
-__device__ __forceinline__ void digits_elem4(int P, int s, int rows, int cols,
-                                             const double *__restrict__ X, int ldx,
-                                             const int *__restrict__ E, int trans,
-                                             __nv_bfloat16 *__restrict__ planes, int ld_out,
-                                             long long plane_stride, int rows_pad, int cols_pad,
-                                             int pr, int pc0) {
-  if (pc0 >= cols_pad || pr >= rows_pad) return;
-  uint2 *out = reinterpret_cast<uint2 *>(planes + (size_t)pr * ld_out + pc0);
-  const long long vstride = plane_stride / 4;
-  if (pr >= rows || pc0 >= cols) {
-    for (int i = 0; i < s; ++i) out[i * vstride] = make_uint2(0, 0);
-    return;
-  }
-  const int S = 7 + 8 * (s - 1);
-  const int Er = E[pr];
-  uint64_t w[4][NW];
+// One thread: the digits of V adjacent entries (row, pc0 ..) of one side.
+//
+// V = sum_l floor(a_l 2^(S-E)) is collected in 32-bit pieces, one signed
+// 64-bit sum per piece in shared memory: a limb touches the three pieces it
+// covers and needs no carry, whatever the width.  One pass from the bottom
+// then settles the carries.  Adding 128 at every digit but the leading one
+// turns the balanced digits d in [-128, 127] into plain bytes d + 128, so the
+// bytes of a piece need no carry among them either; byte b becomes BF16 by
+// writing it into the significand of 2^23 and subtracting 2^23 + 128, and
+// the top half of that float is d in BF16.
+//
+// Bound by the traffic, 8 P bytes in and 2 s out an entry.  With V's words in
+// registers (positions unrolled, per width) most of the time went to
+// instruction fetches and to 4 .. 16 carry steps a limb; both operands, so /
+// from shared memory: qd 8192^3 4.96 / 3.06 ms (11.8 GB, 3.9 TB/s), od 2048^3
+// 909 / 393 us, hd 1024 x 1024 x 512 880 / 116 us, dd 16001 x 96 x 3001 773 /
+// 515 us, qd 256^3 26 / 8 us.
+template <int V, int PL>
+__device__ __forceinline__ void digits_group(int P, int s, const DigitSide &d, int row, int pc0,
+                                             bool wide, void *smem) {
+  constexpr int T = DIGIT_THREADS;
+  const int words = digit_words(s);
+  // piece j of entry v at acc[(j * V + v) * T]
+  long long *acc = reinterpret_cast<long long *>(smem) + threadIdx.x;
+  for (int j = 0; j < words * V; ++j) acc[j * T] = 0;
+  const int base = 7 + 8 * (s - 1) - d.E[row];
+  const double *a[V];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
+  for (int v = 0; v < V; ++v)
+    a[v] = d.X + (d.trans ? (size_t)(pc0 + v) * d.ldx + row : (size_t)row * d.ldx + pc0 + v) * P;
+  for (int l0 = 0; l0 < P; l0 += PL) {
+    double x[V][PL];
 #pragma unroll
-    for (int i = 0; i < NW; ++i) w[e][i] = 0;
-  }
+    for (int v = 0; v < V; ++v) {
+      if (pc0 + v >= d.cols) {
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int pc = pc0 + e;
-    const double *a = trans ? X + ((size_t)pc * ldx + pr) * P : X + ((size_t)pr * ldx + pc) * P;
-    for (int l = 0; l < P; ++l) {
-      int e2;
-      const int64_t m = pc < cols ? mdgi::exact_significand(a[l], e2) : 0;
-      if (m == 0) continue;
-      const int q = e2 + S - Er;
-      if (q >= 0) {
-        mdgi::wide_add_shifted<NW>(w[e], m, q);
-      } else if (q > -64) {
-        mdgi::wide_add_shifted<NW>(w[e], m >> (-q), 0);
-      } else {
-        mdgi::wide_add_shifted<NW>(w[e], m < 0 ? -1 : 0, 0);
-      }
-    }
-  }
-  int carry[4] = {0, 0, 0, 0};
+        for (int l = 0; l < PL; ++l) x[v][l] = 0.0;
+      } else if (wide) {
 #pragma unroll
-  for (int wi = 0; wi < NW; ++wi) {
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int p = wi * 8 + b;
-      if (p < s - 1) {
-        uint32_t packed[2];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = (int)((w[e][wi] >> (8 * b)) & 255) + carry[e];
-          const int d = t >= 128 ? t - 256 : t;
-          carry[e] = t >= 128 ? 1 : 0;
-          const uint32_t bits = bf16_bits_of_digit(d);
-          if (e & 1) packed[e >> 1] |= bits << 16; else packed[e >> 1] = bits;
+        for (int l = 0; l < PL; l += 2) {
+          const double2 t = __ldg(reinterpret_cast<const double2 *>(a[v] + l0 + l));
+          x[v][l] = t.x;
+          x[v][l + 1] = t.y;
         }
-        out[(s - 1 - p) * vstride] = make_uint2(packed[0], packed[1]);
+      } else {
+#pragma unroll
+        for (int l = 0; l < PL; ++l) x[v][l] = __ldg(a[v] + l0 + l);
       }
     }
-  }
-  uint32_t packed[2];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int top = (int)(int64_t)mdgi::wide_bits64<NW>(w[e], 8 * (s - 1)) + carry[e];
-    const uint32_t bits = __bfloat16_as_ushort(__float2bfloat16_rn((float)top));
-    if (e & 1) packed[e >> 1] |= bits << 16; else packed[e >> 1] = bits;
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int l = 0; l < PL; ++l) {
+        int e2;
+        int64_t m = exact_significand(x[v][l], e2);
+        int q = e2 + base;
+        if (q < 0) {
+          m >>= q > -63 ? -q : 63;
+          q = 0;
+        }
+        if (m == 0) continue;
+        const int j = q >> 5, r = q & 31;
+        const uint64_t lo = (uint64_t)m << r;
+        const int64_t hi = r ? m >> (64 - r) : m >> 63;
+        // pieces above the leading digit's 32 bits do not count
+        long long *p = acc + (j * V + v) * T;
+        if (j < words) p[0] += (uint32_t)lo;
+        if (j + 1 < words) p[V * T] += (uint32_t)(lo >> 32);
+        if (j + 2 < words) p[2 * V * T] += hi;
+      }
   }
-  out[0] = make_uint2(packed[0], packed[1]);
+  __nv_bfloat16 *out = d.planes + (size_t)row * d.ld_out + pc0;
+  long long carry[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) carry[v] = 0;
+#pragma unroll 1
+  for (int j = 0;; ++j) {
+    const int low = min(s - 1 - 4 * j, 4);  // digits below the leading one in this piece
+    const uint32_t offset = low > 0 ? 0x80808080u >> (8 * (4 - low)) : 0u;
+    long long t[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      t[v] = acc[(j * V + v) * T] + carry[v] + offset;
+      carry[v] = t[v] >> 32;
+    }
+    __nv_bfloat16 *o = out + (s - 1 - 4 * j) * d.plane_stride;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      if (b >= low) continue;
+      uint32_t f[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        f[v] = __float_as_uint(
+            __int_as_float(__byte_perm((uint32_t)t[v], 0x4B000000u, 0x7440 | b)) - 8388736.0f);
+      if constexpr (V == 2)
+        *reinterpret_cast<uint32_t *>(o) = __byte_perm(f[0], f[1], 0x7632);
+      else
+        *reinterpret_cast<unsigned short *>(o) = (unsigned short)(f[0] >> 16);
+      o -= d.plane_stride;
+    }
+    if (low < 4) {
+      unsigned short top[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const uint64_t above = (uint64_t)acc[((j + 1) * V + v) * T] << (32 - 8 * low);
+        top[v] = __bfloat16_as_ushort(
+            __float2bfloat16_rn((float)(int)(uint32_t)((uint64_t)(t[v] >> (8 * low)) + above)));
+      }
+      if constexpr (V == 2)
+        *reinterpret_cast<uint32_t *>(out) = top[0] | (uint32_t)top[1] << 16;
+      else
+        *reinterpret_cast<unsigned short *>(out) = top[0];
+      return;
+    }
+  }
 }
 
 }  // namespace mdgi

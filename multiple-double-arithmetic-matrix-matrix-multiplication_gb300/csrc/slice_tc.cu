@@ -33,40 +33,73 @@
 
 namespace {
 
-using mdgi::wide_add_shifted;
+using mdgi::DIGIT_THREADS;
+using mdgi::DigitSide;
+using mdgi::SCALE_COLS;
+using mdgi::SCALE_ROWS;
+using mdgi::SCALE_THREADS;
 
 // ------------------------------------------------------------ exponents --
-__global__ void absmax_kernel(int P, int R, int Cn, const double *__restrict__ X, int ldx,
-                              unsigned long long *rowbits, unsigned long long *colbits) {
-  mdgi::absmax_block(P, R, Cn, X, ldx, rowbits, colbits, blockIdx.x, blockIdx.y);
+// Column blocks of B, then row blocks of A, each cut into `cuts` ranges of k.
+// One range: the exponents, at once.  More: maxima by atomics into bits (rows
+// then columns), and exps_kernel after.  Bound by reading A and B once; on
+// small problems one launch instead of two clears, two maxima and two
+// exponent launches (dd 64^3 56 -> 6 us, qd 256^3 64 -> 11 us, qd 8192^3 1.06
+// -> 1.10 ms, 3.9 TB/s).
+__global__ void __launch_bounds__(SCALE_THREADS)
+    scale_kernel(int P, int m, int n, int k, const double *__restrict__ A, int lda,
+                 const double *__restrict__ B, int ldb, int col_blocks, int cuts,
+                 int *__restrict__ E, int *__restrict__ F, unsigned long long *bits) {
+  const int blk = blockIdx.x / cuts, cut = blockIdx.x - blk * cuts;
+  const int k0 = (int)((long long)k * cut / cuts), k1 = (int)((long long)k * (cut + 1) / cuts);
+  if (blk < col_blocks) {
+    const int c = blk * SCALE_COLS + (int)threadIdx.x;
+    const unsigned long long mx = mdgi::col_max(P, B, ldb, blk * SCALE_COLS, n, k0, k1);
+    if (threadIdx.x >= SCALE_COLS || c >= n) return;
+    if (cuts == 1)
+      F[c] = mdgi::scale_exp(__longlong_as_double((long long)mx));
+    else
+      atomicMax(bits + m + c, mx);
+  } else {
+    const int r = (blk - col_blocks) * SCALE_ROWS + (int)(threadIdx.x >> 5);
+    if (r >= m) return;
+    const unsigned long long mx = mdgi::row_max(P, A, lda, r, k0, k1);
+    if (threadIdx.x & 31) return;
+    if (cuts == 1)
+      E[r] = mdgi::scale_exp(__longlong_as_double((long long)mx));
+    else
+      atomicMax(bits + r, mx);
+  }
 }
 
-__global__ void exps_kernel(int count, const unsigned long long *__restrict__ bits,
-                            int *__restrict__ E) {
+__global__ void exps_kernel(int m, int n, const unsigned long long *__restrict__ bits,
+                            int *__restrict__ E, int *__restrict__ F) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) E[i] = mdgi::scale_exp(__longlong_as_double((long long)bits[i]));
+  if (i >= m + n) return;
+  const int e = mdgi::scale_exp(__longlong_as_double((long long)bits[i]));
+  if (i < m)
+    E[i] = e;
+  else
+    F[i - m] = e;
 }
 
 // --------------------------------------------------------------- digits --
-template <int NW>
-__global__ void digits_kernel(int P, int s, int rows, int cols, const double *__restrict__ X,
-                              int ldx, const int *__restrict__ E, int trans,
-                              __nv_bfloat16 *__restrict__ planes, int ld_out,
-                              long long plane_stride, int rows_pad, int cols_pad) {
-  mdgi::digits_elem<NW>(P, s, rows, cols, X, ldx, E, trans, planes, ld_out, plane_stride,
-                        rows_pad, cols_pad, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// 4 k-positions per thread, consecutive threads on consecutive positions of
-// one plane row, so plane stores are coalesced for A and B alike.
-template <int NW>
-__global__ void __launch_bounds__(256)
-    digits4_kernel(int P, int s, int rows, int cols, const double *__restrict__ X, int ldx,
-                   const int *__restrict__ E, int trans, __nv_bfloat16 *__restrict__ planes,
-                   int ld_out, long long plane_stride, int rows_pad, int cols_pad) {
-  mdgi::digits_elem4<NW>(P, s, rows, cols, X, ldx, E, trans, planes, ld_out, plane_stride,
-                         rows_pad, cols_pad, blockIdx.y,
-                         (blockIdx.x * blockDim.x + threadIdx.x) * 4);
+// Both operands in one launch; threads run over the sides' groups of V
+// k-positions, row after row, so plane stores are coalesced for A and B
+// alike.  norms: two counters of a later stage, cleared on the way.
+template <int V, int PL>
+__global__ void __launch_bounds__(DIGIT_THREADS)
+    digits_kernel(int P, int s, const DigitSide a, const DigitSide b, bool wide, unsigned *norms) {
+  extern __shared__ uint4 smem[];
+  const long long e = blockIdx.x * (long long)DIGIT_THREADS + threadIdx.x;
+  if (norms && e < 2) norms[e] = 0;
+  const int groups = a.cols_pad / V;
+  const long long of_a = (long long)a.rows * groups;
+  const DigitSide &d = e < of_a ? a : b;
+  const long long i = e < of_a ? e : e - of_a;
+  const int row = (int)(i / groups);
+  if (row >= d.rows) return;
+  mdgi::digits_group<V, PL>(P, s, d, row, (int)(i - (long long)row * groups) * V, wide, smem);
 }
 
 // ---------------------------------------------------- diagonal GEMM v0 --
@@ -249,8 +282,7 @@ static SlicePlan layout_slice_plan(int p, int s, int D, int m, int n, int k, int
     off = align_up(off + bytes, 256);
     return o;
   };
-  pl.off_rowbits = take(sizeof(unsigned long long) * pl.Mp);
-  pl.off_colbits = take(sizeof(unsigned long long) * pl.Np);
+  pl.off_bits = take(sizeof(unsigned long long) * ((size_t)pl.Mp + pl.Np));
   pl.off_E = take(sizeof(int) * pl.Mp);
   pl.off_F = take(sizeof(int) * pl.Np);
   pl.off_norms = sums ? take(2 * sizeof(unsigned)) : 0;
@@ -283,68 +315,74 @@ SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k) {
 }
 
 int launch_scale_exponents(int p, int m, int n, int k, const double *A, int lda,
-                           const double *B, int ldb, unsigned long long *rowbits,
-                           unsigned long long *colbits, int *E, int *F, cudaStream_t st) {
-  MDG_TRY_CUDA(cudaMemsetAsync(rowbits, 0, sizeof(unsigned long long) * std::max(m, 1), st));
-  MDG_TRY_CUDA(cudaMemsetAsync(colbits, 0, sizeof(unsigned long long) * std::max(n, 1), st));
-  if (k > 0 && m > 0) {
-    dim3 grid(ceil_div(k, 32), ceil_div(m, 256));
-    absmax_kernel<<<grid, dim3(32, 8), 0, st>>>(p, m, k, A, lda, rowbits, nullptr);
-    MDG_TRY_LAUNCH();
-  }
-  if (k > 0 && n > 0) {
-    dim3 grid(ceil_div(n, 32), ceil_div(k, 256));
-    absmax_kernel<<<grid, dim3(32, 8), 0, st>>>(p, k, n, B, ldb, nullptr, colbits);
-    MDG_TRY_LAUNCH();
-  }
-  if (m > 0) {
-    exps_kernel<<<ceil_div(m, 256), 256, 0, st>>>(m, rowbits, E);
-    MDG_TRY_LAUNCH();
-  }
-  if (n > 0) {
-    exps_kernel<<<ceil_div(n, 256), 256, 0, st>>>(n, colbits, F);
+                           const double *B, int ldb, unsigned long long *bits, int *E, int *F,
+                           cudaStream_t st) {
+  if (m <= 0 && n <= 0) return MDG_SUCCESS;
+  const int col_blocks = ceil_div(std::max(n, 0), SCALE_COLS);
+  const long long blocks = (long long)col_blocks + ceil_div(std::max(m, 0), SCALE_ROWS);
+  // a thread takes k / 32 entries one after another: ranges of k where that
+  // is long and the blocks leave SMs idle (four 256-thread blocks fill one
+  // of 152)
+  const int cuts = (int)std::min<long long>(
+      std::max<long long>(1, 608 / std::max<long long>(blocks, 1)), std::max(1, k / 1024));
+  if (cuts > 1)
+    MDG_TRY_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned long long) * ((size_t)m + n), st));
+  scale_kernel<<<(unsigned)(blocks * cuts), SCALE_THREADS, 0, st>>>(p, m, n, k, A, lda, B, ldb,
+                                                                    col_blocks, cuts, E, F, bits);
+  MDG_TRY_LAUNCH();
+  if (cuts > 1) {
+    exps_kernel<<<ceil_div((long long)m + n, 256), 256, 0, st>>>(m, n, bits, E, F);
     MDG_TRY_LAUNCH();
   }
   return MDG_SUCCESS;
 }
 
-int launch_digits(int p, int s, int rows, int cols, const double *X, int ldx, const int *E,
-                  int trans, void *planes, int ld_out, long long plane_stride, int rows_pad,
-                  int cols_pad, cudaStream_t st) {
-  const int NW = words_for(s, 1);
-  if (!NW) return MDG_ERROR_NOT_SUPPORTED;
-  if (rows_pad == 0 || cols_pad == 0) return MDG_SUCCESS;
-  auto *pl = reinterpret_cast<__nv_bfloat16 *>(planes);
-  const bool vec = (cols_pad % 4 == 0) && (ld_out % 4 == 0) && (plane_stride % 4 == 0) &&
-                   (reinterpret_cast<uintptr_t>(planes) % 8 == 0);
-  if (vec) {
-    const dim3 grid(ceil_div(cols_pad / 4, 256), rows_pad);
-#define MDG_DIGITS8(W)                                                                      \
-  digits4_kernel<W><<<grid, 256, 0, st>>>(p, s, rows, cols, X, ldx, E, trans, pl, ld_out,   \
-                                           plane_stride, rows_pad, cols_pad)
-    switch (NW) {
-      case 4: MDG_DIGITS8(4); break;
-      case 6: MDG_DIGITS8(6); break;
-      case 10: MDG_DIGITS8(10); break;
-      default: MDG_DIGITS8(16); break;
-    }
-#undef MDG_DIGITS8
-    MDG_TRY_LAUNCH();
-    return MDG_SUCCESS;
-  }
-  dim3 grid(ceil_div(cols_pad, 128), rows_pad);
-#define MDG_DIGITS(W)                                                                    \
-  digits_kernel<W><<<grid, 128, 0, st>>>(p, s, rows, cols, X, ldx, E, trans, pl, ld_out, \
-                                          plane_stride, rows_pad, cols_pad)
-  switch (NW) {
-    case 4: MDG_DIGITS(4); break;
-    case 6: MDG_DIGITS(6); break;
-    case 10: MDG_DIGITS(10); break;
-    default: MDG_DIGITS(16); break;
-  }
-#undef MDG_DIGITS
+template <int V, int PL>
+static int launch_digits_v(int p, int s, const DigitSide &a, const DigitSide &b, bool wide,
+                           unsigned *norms, cudaStream_t st) {
+  const int smem = digit_smem(s, V);
+  MDG_TRY_CUDA(cudaFuncSetAttribute(digits_kernel<V, PL>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const long long groups = (long long)(a.rows + b.rows) * (a.cols_pad / V);
+  digits_kernel<V, PL>
+      <<<ceil_div(groups, DIGIT_THREADS), DIGIT_THREADS, smem, st>>>(p, s, a, b, wide, norms);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
+}
+
+int launch_digits(int p, int s, const DigitSide &a, const DigitSide &b, unsigned *norms,
+                  cudaStream_t st) {
+  if (!words_for(s, 1)) return MDG_ERROR_NOT_SUPPORTED;
+  if (b.rows && b.cols_pad != a.cols_pad) return MDG_ERROR_INVALID_SIZE;
+  if (a.rows + b.rows == 0 || a.cols_pad == 0) return MDG_SUCCESS;
+  auto addr = [](const void *x) { return reinterpret_cast<uintptr_t>(x); };
+  const bool wide = (addr(a.X) | addr(b.X)) % 16 == 0;
+  // two k-positions a thread where planes take 4-byte stores
+  auto even = [&](const DigitSide &d) {
+    return d.rows == 0 || (d.cols_pad % 2 == 0 && d.ld_out % 2 == 0 && d.plane_stride % 2 == 0 &&
+                           addr(d.planes) % 4 == 0);
+  };
+  if (even(a) && even(b))
+    return p == 2 ? launch_digits_v<2, 2>(p, s, a, b, wide, norms, st)
+                  : launch_digits_v<2, 4>(p, s, a, b, wide, norms, st);
+  return p == 2 ? launch_digits_v<1, 2>(p, s, a, b, wide, norms, st)
+                : launch_digits_v<1, 4>(p, s, a, b, wide, norms, st);
+}
+
+static unsigned long long *plan_bits(const SlicePlan &pl, void *ws) {
+  return reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(ws) + pl.off_bits);
+}
+
+static DigitSide side_a(const SlicePlan &pl, int rows, const double *A, int lda, const int *E,
+                        void *planes) {
+  return DigitSide{A, E, reinterpret_cast<__nv_bfloat16 *>(planes), lda, 0, rows, pl.k, pl.Kp,
+                   pl.Kp, pl.plane_a};
+}
+
+static DigitSide side_b(const SlicePlan &pl, const double *B, int ldb, const int *F,
+                        void *planes) {
+  return DigitSide{B, F, reinterpret_cast<__nv_bfloat16 *>(planes), ldb, 1, pl.n, pl.k, pl.Kp,
+                   pl.Kp, pl.plane_b};
 }
 
 int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
@@ -361,14 +399,13 @@ int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, co
 
 int slice_prepare_b(const SlicePlan &pl, const double *B, int ldb, void *ws, cudaStream_t st) {
   char *base = reinterpret_cast<char *>(ws);
-  auto *rowbits = reinterpret_cast<unsigned long long *>(base + pl.off_rowbits);
-  auto *colbits = reinterpret_cast<unsigned long long *>(base + pl.off_colbits);
-  int *E = reinterpret_cast<int *>(base + pl.off_E);
   int *F = reinterpret_cast<int *>(base + pl.off_F);
-  MDG_TRY(launch_scale_exponents(pl.p, 0, pl.n, pl.k, nullptr, 1, B, ldb, rowbits, colbits, E, F,
-                                 st));
-  return launch_digits(pl.p, pl.s, pl.n, pl.k, B, ldb, F, 1, base + pl.off_dB, pl.Kp,
-                       pl.plane_b, pl.Np, pl.Kp, st);
+  MDG_TRY(launch_scale_exponents(pl.p, 0, pl.n, pl.k, nullptr, 1, B, ldb, plan_bits(pl, ws),
+                                 nullptr, F, st));
+  const DigitSide b = side_b(pl, B, ldb, F, base + pl.off_dB);
+  DigitSide none = b;
+  none.rows = 0;
+  return launch_digits(pl.p, pl.s, none, b, nullptr, st);
 }
 
 int slice_panel_a(const SlicePlan &pl, int rows, const double *A, int lda, void *ws,
@@ -376,16 +413,13 @@ int slice_panel_a(const SlicePlan &pl, int rows, const double *A, int lda, void 
   if (rows <= 0) return MDG_SUCCESS;
   if (rows > pl.m) return MDG_ERROR_INVALID_SIZE;
   char *base = reinterpret_cast<char *>(ws);
-  auto *rowbits = reinterpret_cast<unsigned long long *>(base + pl.off_rowbits);
-  auto *colbits = reinterpret_cast<unsigned long long *>(base + pl.off_colbits);
   int *E = reinterpret_cast<int *>(base + pl.off_E);
-  int *F = reinterpret_cast<int *>(base + pl.off_F);
-  // E only (n = 0 leaves F, computed by slice_prepare_b, alone)
-  MDG_TRY(launch_scale_exponents(pl.p, rows, 0, pl.k, A, lda, nullptr, 1, rowbits, colbits, E,
-                                 F, st));
-  // rows beyond `rows` up to the plan's padded Mp get zero digits
-  return launch_digits(pl.p, pl.s, rows, pl.k, A, lda, E, 0, base + pl.off_dA, pl.Kp,
-                       pl.plane_a, pl.Mp, pl.Kp, st);
+  MDG_TRY(launch_scale_exponents(pl.p, rows, 0, pl.k, A, lda, nullptr, 1, plan_bits(pl, ws), E,
+                                 nullptr, st));
+  const DigitSide a = side_a(pl, rows, A, lda, E, base + pl.off_dA);
+  DigitSide none = a;
+  none.rows = 0;
+  return launch_digits(pl.p, pl.s, a, none, nullptr, st);
 }
 
 int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, void *wsb, int rows,
@@ -425,27 +459,22 @@ int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *
                    double *C, int ldc, void *ws, int engine, int parts, int raster,
                    cudaStream_t st, int pace) {
   char *base = reinterpret_cast<char *>(ws);
-  auto *rowbits = reinterpret_cast<unsigned long long *>(base + pl.off_rowbits);
-  auto *colbits = reinterpret_cast<unsigned long long *>(base + pl.off_colbits);
   int *E = reinterpret_cast<int *>(base + pl.off_E);
   int *F = reinterpret_cast<int *>(base + pl.off_F);
   void *dA = base + pl.off_dA;
   void *dB = base + pl.off_dB;
   auto *Cd = reinterpret_cast<int *>(base + pl.off_Cd);
+  unsigned *norms = pl.sums ? reinterpret_cast<unsigned *>(base + pl.off_norms) : nullptr;
   NvtxRange range("mdg slice_bf16");
   {
     NvtxRange r("split: scale exponents and digits");
-    MDG_TRY(launch_scale_exponents(pl.p, pl.m, pl.n, pl.k, A, lda, B, ldb, rowbits, colbits, E,
+    MDG_TRY(launch_scale_exponents(pl.p, pl.m, pl.n, pl.k, A, lda, B, ldb, plan_bits(pl, ws), E,
                                    F, st));
-    MDG_TRY(launch_digits(pl.p, pl.s, pl.m, pl.k, A, lda, E, 0, dA, pl.Kp, pl.plane_a, pl.Mp,
-                          pl.Kp, st));
-    MDG_TRY(launch_digits(pl.p, pl.s, pl.n, pl.k, B, ldb, F, 1, dB, pl.Kp, pl.plane_b, pl.Np,
-                          pl.Kp, st));
+    MDG_TRY(launch_digits(pl.p, pl.s, side_a(pl, pl.m, A, lda, E, dA), side_b(pl, B, ldb, F, dB),
+                          norms, st));
   }
   NvtxRange r2("diagonal GEMM and renormalisation");
   if (pl.sums) {
-    auto *norms = reinterpret_cast<unsigned *>(base + pl.off_norms);
-    MDG_TRY_CUDA(cudaMemsetAsync(norms, 0, 2 * sizeof(unsigned), st));
     for (int lo = 1, hi; lo < pl.D; lo = hi) {
       hi = cross_group_end(lo, pl.D, pl.sums);
       if (hi == lo) return MDG_ERROR_NOT_SUPPORTED;

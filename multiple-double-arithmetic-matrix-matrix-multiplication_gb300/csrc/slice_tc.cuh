@@ -43,7 +43,7 @@ struct SlicePlan {
   // sum planes behind each operand's digit planes (cross_sums.cuh); 0: the
   // diagonal sums come from digit pairs alone.  off_norms: two unsigned.
   int sums;
-  size_t off_rowbits, off_colbits, off_E, off_F, off_norms, off_dA, off_dB, off_Cd, total;
+  size_t off_bits, off_E, off_F, off_norms, off_dA, off_dB, off_Cd, total;
 };
 
 // The plan over digit pairs.
@@ -57,7 +57,7 @@ int words_for(int s, int D);
 // (19-bit), integer words, workspace layout and the whole GEMM.
 struct Digits64Plan {
   int p, s, D, m, n, k;
-  size_t off_rowbits, off_colbits, off_E, off_F, off_dA, off_dB, off_Cd, total;
+  size_t off_bits, off_E, off_F, off_dA, off_dB, off_Cd, total;
 };
 int digits64_default(int p);
 int words64_for(int s, int D);
@@ -65,12 +65,16 @@ Digits64Plan make_digits64_plan(int p, int s, int D, int m, int n, int k);
 int run_digits64_gemm(const Digits64Plan &pl, const double *A, int lda, const double *B, int ldb,
                       double *C, int ldc, void *ws, cudaStream_t st);
 
+// Scale exponents of A's rows (m of them) and B's columns (n); bits: m + n
+// words of scratch.
 int launch_scale_exponents(int p, int m, int n, int k, const double *A, int lda,
-                           const double *B, int ldb, unsigned long long *rowbits,
-                           unsigned long long *colbits, int *E, int *F, cudaStream_t st);
-int launch_digits(int p, int s, int rows, int cols, const double *X, int ldx, const int *E,
-                  int trans, void *planes, int ld_out, long long plane_stride, int rows_pad,
-                  int cols_pad, cudaStream_t st);
+                           const double *B, int ldb, unsigned long long *bits, int *E, int *F,
+                           cudaStream_t st);
+// Digit planes of two operands (slice_stages.cuh; rows = 0: none), and zeros
+// into norms[0], norms[1] where given.
+struct DigitSide;
+int launch_digits(int p, int s, const DigitSide &a, const DigitSide &b, unsigned *norms,
+                  cudaStream_t st);
 // Engines write chunk planes of Mp x Np int32 (row stride Np).
 // mma.sync engine (Mp % 128, Np % 64, Kp % 64)
 int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
