@@ -678,10 +678,10 @@ int mdg_slice_diagonals(int s, int D, int m, int n, int k, const void *dA, const
   const long long plane_c = (long long)m * n;
   const int eng = engine_choice(0);
   if (eng != 0 && ld == k)
-    return launch_diag_gemm_tc(s, D, m, n, k, dA, dB, ld, plane_a, plane_b, chunks, plane_c,
-                               eng == 2 ? 1 : 0, 0, 0, as_stream(stream));
+    return launch_diag_gemm_tc(s, D, m, n, k, m, n, dA, dB, ld, plane_a, plane_b, chunks, plane_c,
+                               CHUNK_STEPS, eng, 0, 0, as_stream(stream));
   return launch_diag_gemm_v0(s, D, m, n, k, dA, dB, ld, plane_a, plane_b, chunks, plane_c,
-                             as_stream(stream));
+                             CHUNK_STEPS, as_stream(stream));
 }
 
 int mdg_renorm_diagonals(int p, int s, int D, int k, int m, int n, const int *chunks,
@@ -696,7 +696,7 @@ int mdg_renorm_diagonals(int p, int s, int D, int k, int m, int n, const int *ch
   if (!chunks || !E || !F || !C) return MDG_ERROR_NULL_POINTER;
   if (m > 65535) return MDG_ERROR_NOT_SUPPORTED;
   const int KB = (int)(align_up(std::max(k, 1), 64) / 64);
-  return launch_renorm(p, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, as_stream(stream));
+  return launch_renorm(p, s, D, KB, CHUNK_STEPS, m, n, chunks, plane_c, ldcd, E, F, C, ldc, as_stream(stream));
 }
 
 int mdg_device_status(void) { return tc_device_status(); }

@@ -255,47 +255,94 @@ __device__ __forceinline__ void stores_done() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Diagonals [d0, d1) of part `part` of a tile cut into `parts` ranges whose
-// digit-pair counts add up to about 1/parts of the tile's pairs each (empty
-// when parts exceeds what the pair counts allow).
-__device__ __forceinline__ void part_diagonals(int s, int D, int part, int parts, int &d0,
-                                               int &d1) {
-  int total = 0;
-  for (int d = 0; d < D; ++d) total += mdgi::diag_pairs(d, s);
-  const long long lo = (long long)total * part / parts, hi = (long long)total * (part + 1) / parts;
-  int cum = 0;
-  d0 = D;
-  d1 = D;
-  for (int d = 0; d < D; ++d) {
-    if (cum >= lo && d0 == D) d0 = d;
-    if (cum >= hi) {
-      d1 = d;
-      break;
+// A run of plane products that goes into one output plane: `steps` k-steps
+// from step t0 of the products of planes (a0 + p, b0 + bstep p), KB k-steps
+// each, p = 0, 1, ..  cuts: flush groups per plane (sums form).
+struct Run {
+  int a0, b0, t0, steps, chunk, cuts;
+};
+
+// Runs over digit planes: the chunks (cs k-steps) of the diagonals.
+struct DigitRuns {
+  static constexpr int bstep = -1;
+  int s, D, KB, cs, d, c, chunk, left;
+  __device__ bool next(Run &r) {
+    if (left <= 0 || d >= D) return false;
+    const int S = mdgi::diag_pairs(d, s) * KB;
+    r.a0 = d - (s - 1) > 0 ? d - (s - 1) : 0;
+    r.b0 = d - r.a0;
+    r.t0 = c * cs;
+    r.steps = S - r.t0 < cs ? S - r.t0 : cs;
+    r.chunk = chunk++;
+    --left;
+    if (r.t0 + cs < S) {
+      ++c;
+    } else {
+      ++d;
+      c = 0;
     }
-    cum += mdgi::diag_pairs(d, s);
+    return true;
   }
-  if (d0 > d1) d0 = d1;
+  // FP32 flushes every GROUP_STEPS k-steps, whatever plane they fall in
+  struct Groups {
+    int left;
+    __device__ Groups(const Run &r, int) : left(r.steps) {}
+    __device__ int next() {  // k-steps of the next flush group, 0 at the end
+      const int n = left < mdgi::GROUP_STEPS ? left : mdgi::GROUP_STEPS;
+      left -= n;
+      return n;
+    }
+    __device__ bool last() const { return left == 0; }
+  };
+};
+
+// Part `part` of a tile's runs: run `part` itself where there are as many
+// parts as runs, else the runs that start in the part's 1/parts of the
+// tile's k-steps (none when parts exceeds what the runs allow).
+__device__ __forceinline__ DigitRuns part_runs(int s, int D, int KB, int cs, int part, int parts) {
+  DigitRuns all{s, D, KB, cs, 0, 0, 0, 1 << 30};
+  if (parts == 1) return all;
+  long long steps = 0;
+  int runs = 0;
+  for (int d = 0; d < D; ++d) {
+    steps += mdgi::diag_pairs(d, s) * KB;
+    runs += mdgi::diag_chunks(d, s, KB, cs);
+  }
+  const bool one = parts == runs;
+  const long long lo = one ? part : steps * part / parts;
+  const long long hi = one ? part + 1 : steps * (part + 1) / parts;
+  Run r;
+  long long at = 0;
+  while (at < lo && all.next(r)) at += one ? 1 : r.steps;
+  DigitRuns first = all;
+  first.left = 0;
+  while (at < hi && all.next(r)) {
+    at += one ? 1 : r.steps;
+    ++first.left;
+  }
+  return first;
 }
 
 // One unit of work: where its operands and output live, which of its
-// problem's rows / columns it covers and which diagonals [d0, d1) it
-// computes.  tn: tile width, 256 or 128 columns (the B box of tmB is tn
-// rows); ktail: MMAs of K = 16 issued for the last k-block (1..4; the rest
-// of that block is the zero padding of k).
+// problem's rows / columns it covers and which runs it computes.  tn: tile
+// width, 256 or 128 columns (the B box of tmB is tn rows); ktail: MMAs of
+// K = 16 issued for the last k-block (1..4; the rest of that block is the
+// zero padding of k).
 struct TileJob {
   const CUtensorMap *tmA, *tmB, *tmC;
-  int s, D, Mp, Np, KB, row, col, tn, ktail, d0, d1;
+  int Mp, Np, KB, row, col, tn, ktail;
+  DigitRuns runs;
 };
 
-// A single problem cut into 128 x 256 tiles.
+// A single problem cut into mt x nt tiles of 128 x tn, each into parts.
 struct SingleJobs {
   const CUtensorMap *tmA, *tmB, *tmC;
-  int s, D, Mp, Np, KB;
-  __device__ int tiles() const { return (Mp / TM) * (Np / TN); }
-  __device__ TileJob job(int t) const {
-    const int MB = Mp / TM;
-    return TileJob{tmA, tmB, tmC, s, D, Mp, Np, KB, (t % MB) * TM, (t / MB) * TN, TN, TK / 16,
-                   0, D};
+  int s, D, Mp, Np, KB, cs, tn, mt, nt, parts;
+  __device__ int units() const { return mt * nt * parts; }
+  __device__ TileJob job(int u) const {
+    const int tiles = mt * nt, tile = u % tiles;
+    return TileJob{tmA, tmB, tmC, Mp, Np, KB, (tile % mt) * TM, (tile / mt) * tn, tn, TK / 16,
+                   part_runs(s, D, KB, cs, u / tiles, parts)};
   }
 };
 
@@ -342,7 +389,7 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
   fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  const int tiles = jobs.tiles();
+  const int tiles = jobs.units();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -353,13 +400,12 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
       // (bit of `last_par`); bit masks so that they stay in registers
       uint32_t issued = 0, last_par = 0;
       for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const TileJob jb = jobs.job(tile);
-        const int s = jb.s, KB = jb.KB;
-        for (int d = jb.d0; d < jb.d1; ++d) {
-          const int ilo = d - (s - 1) > 0 ? d - (s - 1) : 0;
-          const int S = mdgi::diag_pairs(d, s) * KB;
-          for (int t = 0; t < S; ++t) {
-            const int i = ilo + t / KB, kb = t - (t / KB) * KB, j = d - i;
+        TileJob jb = jobs.job(tile);
+        const int KB = jb.KB;
+        Run r;
+        while (jb.runs.next(r)) {
+          for (int t = r.t0; t < r.t0 + r.steps; ++t) {
+            const int q = t / KB, kb = t - q * KB, i = r.a0 + q, j = r.b0 + DigitRuns::bstep * q;
             if (!mbar_wait(empty(st), ph ^ 1, abort_flag)) goto producer_done;
             mbar_expect_tx(full(st), A_BYTES + jb.tn * TK * 2);
             const uint32_t a_dst = smem_base + st * STAGE_BYTES;
@@ -386,17 +432,17 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
       uint32_t ph = 0, aph[2] = {0, 0};
       bool any = false;
       for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const TileJob jb = jobs.job(tile);
+        TileJob jb = jobs.job(tile);
         const uint32_t idesc = (IDESC & ~(0x3Fu << 17)) | ((uint32_t)(jb.tn >> 3) << 17);
-        for (int d = jb.d0; d < jb.d1; ++d) {
-          const int S = mdgi::diag_pairs(d, jb.s) * jb.KB;
-          int kb = 0;  // k-block of step t within its digit pair
-          for (int g0 = 0; g0 < S; g0 += mdgi::GROUP_STEPS) {
+        Run r;
+        while (jb.runs.next(r)) {
+          int kb = r.t0 % jb.KB;  // k-block of a step within its digit pair
+          DigitRuns::Groups groups(r, jb.KB);
+          for (int steps; (steps = groups.next()) > 0;) {
             if (!mbar_wait(accempty(buf), aph[buf] ^ 1, abort_flag)) goto mma_done;
             fence_after();
             const uint32_t dt = tmem_base + buf * TN;
-            const int g1 = g0 + mdgi::GROUP_STEPS < S ? g0 + mdgi::GROUP_STEPS : S;
-            for (int t = g0; t < g1; ++t) {
+            for (int t = 0; t < steps; ++t) {
               if (!mbar_wait(full(st), ph, abort_flag)) goto mma_done;
               fence_after();
               const uint32_t a_addr = smem_base + st * STAGE_BYTES;
@@ -407,10 +453,10 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
               if (!short_block) {
 #pragma unroll
                 for (int kk = 0; kk < TK / 16; ++kk)
-                  mma_bf16_n(dt, da + 2 * kk, db + 2 * kk, idesc, (t > g0 || kk > 0) ? 1u : 0u);
+                  mma_bf16_n(dt, da + 2 * kk, db + 2 * kk, idesc, (t > 0 || kk > 0) ? 1u : 0u);
               } else {
                 for (int kk = 0; kk < jb.ktail; ++kk)
-                  mma_bf16_n(dt, da + 2 * kk, db + 2 * kk, idesc, (t > g0 || kk > 0) ? 1u : 0u);
+                  mma_bf16_n(dt, da + 2 * kk, db + 2 * kk, idesc, (t > 0 || kk > 0) ? 1u : 0u);
               }
               mma_commit(empty(st));
               any = true;
@@ -441,18 +487,17 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
     int buf = 0;
     uint32_t aph[2] = {0, 0};
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-      const TileJob jb = jobs.job(tile);
+      TileJob jb = jobs.job(tile);
       // a 128-column tile is drained by the warps of the first column half
       // alone (128 columns each, as for a 256-column tile); the others only
       // release the accumulator
       const bool active = jb.tn == TN || h == 0;
       const int row = jb.row + 32 * q;
       const int col = jb.col + 128 * h;
-      int chunk = 0;
-      for (int d = 0; d < jb.d0; ++d) chunk += mdgi::diag_chunks(d, jb.s, jb.KB);
-      for (int d = jb.d0; d < jb.d1; ++d) {
-        const int S = mdgi::diag_pairs(d, jb.s) * jb.KB;
-        for (int g0 = 0; g0 < S; g0 += mdgi::GROUP_STEPS) {
+      Run r;
+      while (jb.runs.next(r)) {
+        DigitRuns::Groups groups(r, jb.KB);
+        while (groups.next() > 0) {
           // lane 0 waits; the outcome is broadcast so the warp stays
           // converged for the .sync.aligned TMEM loads
           int ok = 1;
@@ -467,11 +512,8 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
           __syncwarp();
           if (lane == 0) mbar_arrive(accempty(buf));
           buf ^= 1;
-          const int g1 = g0 + mdgi::GROUP_STEPS;
-          if (g1 % mdgi::CHUNK_STEPS == 0 || g1 >= S) {
-            if (active) store_rows(staging, lane, acc, jb.tmC, col, chunk * jb.Mp + row);
-            ++chunk;
-          }
+          if (groups.last() && active)
+            store_rows(staging, lane, acc, jb.tmC, col, r.chunk * jb.Mp + row);
         }
       }
     }
@@ -494,8 +536,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     diag_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
-                        int KB) {
-  tc1_body(SingleJobs{&tmA, &tmB, &tmC, s, D, Mp, Np, KB});
+                        int KB, int cs, int tn, int mt, int nt, int parts) {
+  tc1_body(SingleJobs{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, tn, mt, nt, parts});
 }
 
 // Many problems: a table of GroupedProblem in global memory (tensor maps
@@ -515,17 +557,16 @@ __device__ __forceinline__ const mdgi::GroupedProblem &grouped_find(
 struct GroupedJobs {
   const mdgi::GroupedProblem *probs;
   int count, total;
-  __device__ int tiles() const { return total; }
+  __device__ int units() const { return total; }
   __device__ TileJob job(int u) const {
     const mdgi::GroupedProblem &g = grouped_find(probs, count, u);
     const int lt = u - g.unit_begin, tiles = g.mt * g.nt;
     const int tile = lt % tiles, part = lt / tiles;
-    int d0, d1;
-    part_diagonals(g.s, g.D, part, g.parts, d0, d1);
     return TileJob{reinterpret_cast<const CUtensorMap *>(g.tmA),
                    reinterpret_cast<const CUtensorMap *>(g.tmB),
-                   reinterpret_cast<const CUtensorMap *>(g.tmC), g.s, g.D, g.Mp, g.Np, g.KB,
-                   (tile % g.mt) * TM, (tile / g.mt) * g.tn, g.tn, g.ktail, d0, d1};
+                   reinterpret_cast<const CUtensorMap *>(g.tmC), g.Mp, g.Np, g.KB,
+                   (tile % g.mt) * TM, (tile / g.mt) * g.tn, g.tn, g.ktail,
+                   part_runs(g.s, g.D, g.KB, mdgi::CHUNK_STEPS, part, g.parts)};
   }
 };
 
@@ -651,52 +692,13 @@ __device__ __forceinline__ uint32_t pace_load(int slot, int ncl, uint32_t epoch)
   return (uint32_t)(v >> 32) == epoch ? (uint32_t)v : 0u;
 }
 
-// A run of plane products that goes into one accumulation: product p takes
-// plane a0 + p of A and plane b0 + bstep p of B, KB k-steps each; its first
-// output plane is `chunk`.  cuts: flush groups per plane (sums form).
-struct Run {
-  int a0, b0, products, chunk, cuts;
-};
-
 // One unit of work of the pair kernel over digit planes: a 256 x 256 tile
-// of one problem (rows row0.., columns col0..) and the diagonals [d0, d1) it
-// computes, one run each.  FP32 flushes every GROUP_STEPS k-steps of a run
-// whatever plane they fall in, chunk stores every CHUNK_STEPS.
+// of one problem (rows row0.., columns col0..) and the runs it computes.
 struct PairJob {
-  static constexpr int bstep = -1;
+  using Runs = DigitRuns;
   const CUtensorMap *tmA, *tmB, *tmC;
-  int s, D, Mp, Np, KB, row0, col0, d0, d1;
-
-  struct Runs {
-    int s, KB, d, d1, chunk;
-    __device__ bool next(Run &r) {
-      if (d >= d1) return false;
-      r.a0 = d - (s - 1) > 0 ? d - (s - 1) : 0;
-      r.b0 = d - r.a0;
-      r.products = mdgi::diag_pairs(d, s);
-      r.chunk = chunk;
-      chunk += mdgi::diag_chunks(d, s, KB);
-      ++d;
-      return true;
-    }
-  };
-  // the first chunk's number is wanted by the epilogue alone
-  __device__ Runs runs(bool chunks) const {
-    int chunk = 0;
-    if (chunks)
-      for (int d = 0; d < d0; ++d) chunk += mdgi::diag_chunks(d, s, KB);
-    return Runs{s, KB, d0, d1, chunk};
-  }
-  struct Groups {
-    int pos, steps;
-    __device__ Groups(const Run &r, int KB) : pos(0), steps(r.products * KB) {}
-    __device__ int next() {  // k-steps of the next flush group, 0 at the end
-      const int n = steps - pos < mdgi::GROUP_STEPS ? steps - pos : mdgi::GROUP_STEPS;
-      pos += n;
-      return n;
-    }
-    __device__ bool store() const { return pos % mdgi::CHUNK_STEPS == 0 || pos >= steps; }
-  };
+  int Mp, Np, KB, row0, col0;
+  DigitRuns runs;
 };
 
 // One unit of work over digit and sum planes (cross_sums.cuh): a tile and
@@ -704,54 +706,52 @@ struct PairJob {
 // then the sums of the diagonals from d on, chunk by chunk.  The same plane
 // index on both sides; flush groups never span two planes, because their
 // exactness rests on the norms of windows of single sum planes.
-struct CrossJob {
+struct CrossRuns {
   static constexpr int bstep = 1;
-  const CUtensorMap *tmA, *tmB, *tmC;
-  int Mp, Np, KB, row0, col0;
-  int sq, nsq, d, i, chunk, planes;  // start of the unit's list
-  int plane0, ppc, cuts;             // plane of diagonal d's pair 0 is plane0 + cross_offset(d)
-
-  struct Runs {
-    int sq, nsq, d, i, chunk, planes, plane0, ppc, cuts1, cuts;
-    __device__ bool next(Run &r) {
-      if (planes <= 0) return false;
-      if (sq < nsq) {
-        r = Run{sq, sq, 1, sq, cuts1};
-        ++sq;
-      } else {
-        const int left = mdgi::cross_pairs(d) - i;
-        const int np = left < ppc ? left : ppc;
-        const int t = plane0 + mdgi::cross_offset(d) + i;
-        r = Run{t, t, np, chunk, cuts};
-        ++chunk;
-        i += np;
-        if (np == left) {
-          ++d;
-          i = 0;
-        }
+  int sq, nsq, d, i, chunk, planes;  // where the list goes on, planes left
+  int plane0, ppc, KB;               // plane of diagonal d's pair 0 is plane0 + cross_offset(d)
+  int cuts1, cuts;                   // flush groups per square, per sum
+  __device__ bool next(Run &r) {
+    if (planes <= 0) return false;
+    if (sq < nsq) {
+      r = Run{sq, sq, 0, KB, sq, cuts1};
+      ++sq;
+      --planes;
+    } else {
+      const int left = mdgi::cross_pairs(d) - i;
+      const int np = left < ppc ? left : ppc;
+      const int t = plane0 + mdgi::cross_offset(d) + i;
+      r = Run{t, t, 0, np * KB, chunk, cuts};
+      ++chunk;
+      planes -= np;
+      i += np;
+      if (np == left) {
+        ++d;
+        i = 0;
       }
-      planes -= r.products;
-      return true;
     }
-  };
-  __device__ Runs runs(bool) const {
-    return Runs{sq, nsq, d, i, chunk, planes, plane0, ppc, mdgi::cross_groups(KB), cuts};
+    return true;
   }
   struct Groups {
     int left, KB, cuts, j, at;
-    __device__ Groups(const Run &r, int KB_) : left(r.products), KB(KB_), cuts(r.cuts), j(0), at(0) {}
+    __device__ Groups(const Run &r, int KB_) : left(r.steps), KB(KB_), cuts(r.cuts), j(0), at(0) {}
     __device__ int next() {
       if (left == 0) return 0;
       const int to = ++j * KB / cuts, n = to - at;
       at = to;
-      if (j == cuts) {
-        j = at = 0;
-        --left;
-      }
+      if (j == cuts) j = at = 0;
+      left -= n;
       return n;
     }
-    __device__ bool store() const { return left == 0; }
+    __device__ bool last() const { return left == 0; }
   };
+};
+
+struct CrossJob {
+  using Runs = CrossRuns;
+  const CUtensorMap *tmA, *tmB, *tmC;
+  int Mp, Np, KB, row0, col0;
+  CrossRuns runs;
 };
 
 // A single problem: units are tiles, or parts of tiles (ranges of
@@ -762,20 +762,19 @@ struct CrossJob {
 // them in L2 (raster = 1 walks each column block top to bottom).
 struct PairSingle {
   const CUtensorMap *tmA, *tmB, *tmC;
-  int s, D, Mp, Np, KB;
+  int s, D, Mp, Np, KB, cs;
   int parts, raster;
   __device__ int units() const { return (Mp / 256) * (Np / TN2) * parts; }
   __device__ PairJob job(int u) const {
     const int MB = Mp / 256, NB = Np / TN2, tiles = MB * NB;
     const int tile = u % tiles, part = u / tiles;
-    int d0, d1;
-    part_diagonals(s, D, part, parts, d0, d1);
     const int strip = tile / (MB * raster);
     const int idx = tile - strip * MB * raster;
     const int c0 = strip * raster;
     const int g = NB - c0 < raster ? NB - c0 : raster;
     const int rb = idx / g, cb = c0 + idx - rb * g;
-    return PairJob{tmA, tmB, tmC, s, D, Mp, Np, KB, rb * 256, cb * TN2, d0, d1};
+    return PairJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2,
+                   part_runs(s, D, KB, cs, part, parts)};
   }
 };
 
@@ -790,12 +789,11 @@ struct PairGrouped {
     const mdgi::GroupedProblem &g = grouped_find(probs, count, u);
     const int lt = u - g.unit_begin, tiles = g.mt * g.nt;
     const int tile = lt % tiles, part = lt / tiles;
-    int d0, d1;
-    part_diagonals(g.s, g.D, part, g.parts, d0, d1);
     return PairJob{reinterpret_cast<const CUtensorMap *>(g.tmA),
                    reinterpret_cast<const CUtensorMap *>(g.tmB),
-                   reinterpret_cast<const CUtensorMap *>(g.tmC), g.s, g.D, g.Mp, g.Np, g.KB,
-                   (tile % g.mt) * 256, (tile / g.mt) * TN2, d0, d1};
+                   reinterpret_cast<const CUtensorMap *>(g.tmC), g.Mp, g.Np, g.KB,
+                   (tile % g.mt) * 256, (tile / g.mt) * TN2,
+                   part_runs(g.s, g.D, g.KB, mdgi::CHUNK_STEPS, part, g.parts)};
   }
 };
 
@@ -829,16 +827,17 @@ struct PairCross {
     const int lo = (int)((long long)total * part / parts);
     const int hi = (int)((long long)total * (part + 1) / parts);
     // the runs that start in [lo, hi)
-    CrossJob::Runs it{0, nsq, dlo, 0, D, total, plane0, ppc, 1, 1};
+    const int cuts1 = mdgi::cross_groups(KB);
+    CrossRuns it{0, nsq, dlo, 0, D, total, plane0, ppc, KB, cuts1, cuts()};
     for (int d = 1; d < dlo; ++d) it.chunk += mdgi::cross_chunks(d, ppc);
     Run r;
     while (total - it.planes < lo && it.next(r)) {
     }
-    const CrossJob::Runs first = it;
+    CrossRuns first = it;
     while (total - it.planes < hi && it.next(r)) {
     }
-    return CrossJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2, first.sq, nsq, first.d, first.i,
-                    first.chunk, first.planes - it.planes, plane0, ppc, cuts()};
+    first.planes -= it.planes;
+    return CrossJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2, first};
   }
 };
 
@@ -914,16 +913,15 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       // MMA thread's wait for data runs out, it raises the abort flag and
       // every role leaves with nothing in flight
       for (int u = no_loads ? units : cid; u < units; u += ncl) {
-        const auto jb = jobs.job(u);
+        auto jb = jobs.job(u);
         const int KB = jb.KB;
         const int row = jb.row0 + (int)rank * TM;
         const int col = jb.col0 + (int)rank * BH;
-        auto runs = jb.runs(false);
         Run r;
-        while (runs.next(r)) {
-          const int S = r.products * KB;
-          for (int t = 0; t < S; ++t) {
-            const int q = t / KB, kb = t - q * KB, i = r.a0 + q, j = r.b0 + jb.bstep * q;
+        while (jb.runs.next(r)) {
+          for (int t = r.t0; t < r.t0 + r.steps; ++t) {
+            const int q = t / KB, kb = t - q * KB, i = r.a0 + q;
+            const int j = r.b0 + decltype(jb.runs)::bstep * q;
             if (pacing && steps > *pace_allowed) {
               const unsigned long long t0 = now_ns();
               while (steps > *pace_allowed) {
@@ -963,11 +961,10 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       uint32_t ph = 0, aph[2] = {0, 0};
       bool any = false;
       for (int u = cid; u < units; u += ncl) {
-        const auto jb = jobs.job(u);
-        auto runs = jb.runs(false);
+        auto jb = jobs.job(u);
         Run r;
-        while (runs.next(r)) {
-          typename decltype(jb)::Groups groups(r, jb.KB);
+        while (jb.runs.next(r)) {
+          typename decltype(jb.runs)::Groups groups(r, jb.KB);
           for (int steps; (steps = groups.next()) > 0;) {
             if (!mbar_wait(accempty(buf), aph[buf] ^ 1, abort_flag)) goto mma_done;
             fence_after();
@@ -1043,14 +1040,12 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
     uint32_t aph[2] = {0, 0};
     const uint32_t accempty0[2] = {map_to_rank0(accempty(0)), map_to_rank0(accempty(1))};
     for (int u = cid; u < units; u += ncl) {
-      const auto jb = jobs.job(u);
+      auto jb = jobs.job(u);
       const int row = jb.row0 + (int)rank * TM + 32 * q;
       const int col = jb.col0 + 128 * h;
-      auto runs = jb.runs(true);
       Run r;
-      while (runs.next(r)) {
-        typename decltype(jb)::Groups groups(r, jb.KB);
-        int chunk = r.chunk;
+      while (jb.runs.next(r)) {
+        typename decltype(jb.runs)::Groups groups(r, jb.KB);
         while (groups.next() > 0) {
           int ok = 1;
           if (lane == 0) ok = mbar_wait(accfull(buf), aph[buf], abort_flag) ? 1 : 0;
@@ -1064,10 +1059,7 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(accempty0[buf]);
           buf ^= 1;
-          if (groups.store()) {
-            store_rows(staging, lane, acc, jb.tmC, col, chunk * jb.Mp + row);
-            ++chunk;
-          }
+          if (groups.last()) store_rows(staging, lane, acc, jb.tmC, col, r.chunk * jb.Mp + row);
         }
       }
     }
@@ -1089,8 +1081,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
     diag_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA,
                          const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
-                         int KB, int parts, int raster, int pace, uint32_t epoch, int no_loads) {
-  tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, parts, raster}, pace, epoch, no_loads);
+                         int KB, int cs, int parts, int raster, int pace, uint32_t epoch,
+                         int no_loads) {
+  tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, parts, raster}, pace, epoch,
+           no_loads);
 }
 
 // The diagonal GEMM over digit and sum planes (cross_sums.cuh).  Bound by the
@@ -1171,8 +1165,15 @@ struct PairSchedule {
   uint32_t epoch;
 };
 
-// max_parts: runs of a tile that parts can separate (diagonals).
-PairSchedule pair_schedule(int Mp, int Np, int max_parts, int sms, int parts_opt, int raster_opt,
+// Parts of a problem whose tiles do not fill the workers: a run each where
+// they all fit, else as many as fit (at least `parts`).
+int few_tile_parts(int tiles, int runs, int workers, int parts) {
+  const int fit = workers / tiles;
+  return runs <= fit ? runs : std::max(parts, fit);
+}
+
+// runs: of a tile, what parts can separate.
+PairSchedule pair_schedule(int Mp, int Np, int runs, int sms, int parts_opt, int raster_opt,
                            int pace_opt) {
   PairSchedule sc;
   const int tiles = (Mp / 256) * (Np / TN2);
@@ -1184,7 +1185,7 @@ PairSchedule pair_schedule(int Mp, int Np, int max_parts, int sms, int parts_opt
   const int ncl = sms / 2;
   sc.parts = 1;
   double best = 0.0;
-  for (int u = 1; u <= 8 && u <= max_parts; ++u) {
+  for (int u = 1; u <= 8 && u <= runs; ++u) {
     const long long units = (long long)tiles * u;
     const long long waves = (units + ncl - 1) / ncl;
     const double cost = (double)waves / u * (1.0 + 0.04 * (u - 1));
@@ -1193,6 +1194,7 @@ PairSchedule pair_schedule(int Mp, int Np, int max_parts, int sms, int parts_opt
       sc.parts = u;
     }
   }
+  if ((long long)tiles * sc.parts <= ncl) sc.parts = few_tile_parts(tiles, runs, ncl, sc.parts);
   if (parts_opt > 0) sc.parts = std::min(8, parts_opt);
   // tile order: strips about sqrt(clusters) column blocks wide, so that
   // the tiles in work at one time span few row and column blocks (the
@@ -1255,21 +1257,24 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
   return MDG_SUCCESS;
 }
 
-int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
-                        int ld, long long plane_a, long long plane_b, int *chunks,
-                        long long plane_c, int single, int parts_opt, int raster_opt,
+int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, const void *dA,
+                        const void *dB, int ld, long long plane_a, long long plane_b, int *chunks,
+                        long long plane_c, int cs, int engine, int parts_opt, int raster_opt,
                         cudaStream_t st, int pace_opt) {
   if (Mp % TM || Np % TN || Kp % TK || ld != Kp) return MDG_ERROR_INVALID_SIZE;
   if (plane_a != (long long)Mp * Kp || plane_b != (long long)Np * Kp) return MDG_ERROR_INVALID_SIZE;
   if ((reinterpret_cast<uintptr_t>(dA) | reinterpret_cast<uintptr_t>(dB)) & 15)
     return MDG_ERROR_INVALID_SIZE;
-  // the CTA-pair kernel needs 256-row tiles
-  const bool pair = (Mp % 256 == 0) && !single;
   if (plane_c != (long long)Mp * Np) return MDG_ERROR_INVALID_SIZE;
+  // the CTA-pair kernel needs 256-row tiles
+  const int narrow = engine == 1 ? narrow_tile(m, n) : 0;
+  const bool pair = Mp % 256 == 0 && engine != 2 && !narrow;
+  const int tn = narrow ? narrow : TN;
+  const int runs = total_chunks(s, D, Kp / TK, cs);
   CUtensorMap ma, mb, mc;
-  MDG_TRY(make_out_map(&mc, chunks, Np, (long long)total_chunks(s, D, Kp / TK) * Mp));
+  MDG_TRY(make_out_map(&mc, chunks, Np, (long long)runs * Mp));
   MDG_TRY(make_map(&ma, dA, Kp, (long long)s * Mp, TM));
-  MDG_TRY(make_map(&mb, dB, Kp, (long long)s * Np, pair ? BH : TN));
+  MDG_TRY(make_map(&mb, dB, Kp, (long long)s * Np, pair ? BH : tn));
   int dev = 0, sms = 0;
   MDG_TRY_CUDA(cudaGetDevice(&dev));
   // per-device attribute, set on every launch (no process-wide record that
@@ -1282,13 +1287,18 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, co
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (pair) {
-    const PairSchedule sc = pair_schedule(Mp, Np, D, sms, parts_opt, raster_opt, pace_opt);
+    const PairSchedule sc = pair_schedule(Mp, Np, runs, sms, parts_opt, raster_opt, pace_opt);
     diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
-        ma, mb, mc, s, D, Mp, Np, Kp / TK, sc.parts, sc.raster, sc.pace, sc.epoch, sc.no_loads);
+        ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, sc.parts, sc.raster, sc.pace, sc.epoch,
+        sc.no_loads);
   } else {
-    const int tiles = (Mp / TM) * (Np / TN);
-    const int grid = tiles < sms ? tiles : sms;
-    diag_gemm_tc_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(ma, mb, mc, s, D, Mp, Np, Kp / TK);
+    const int mt = (m + TM - 1) / TM, nt = (n + tn - 1) / tn, tiles = mt * nt;
+    const int parts = parts_opt > 0 ? std::min(8, parts_opt)
+                      : tiles <= sms ? few_tile_parts(tiles, runs, sms, 1)
+                                     : 1;
+    const int grid = (int)std::min<long long>((long long)tiles * parts, sms);
+    diag_gemm_tc_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(ma, mb, mc, s, D, Mp, Np, Kp / TK, cs,
+                                                           tn, mt, nt, parts);
   }
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;

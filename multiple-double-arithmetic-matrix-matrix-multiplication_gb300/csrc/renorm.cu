@@ -20,8 +20,8 @@ constexpr int kTwoColumnDiagonals = 32;
 // Threads run over the rows' groups of V columns, row after row.
 template <int V>
 __global__ void __launch_bounds__(RENORM_THREADS)
-    renorm_kernel(int P, int s, int D, int KB, int planes, int m, int n,
-                  const int *__restrict__ chunks, long long plane_c, int ldcd,
+    renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::ChunkCounts counts,
+                  int m, int n, const int *__restrict__ chunks, long long plane_c, int ldcd,
                   const int *__restrict__ E, const int *__restrict__ F, double *__restrict__ C,
                   int ldc, bool wide) {
   extern __shared__ uint4 smem[];
@@ -29,13 +29,13 @@ __global__ void __launch_bounds__(RENORM_THREADS)
   const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
   const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
   if (r >= m) return;
-  mdgi::renorm_columns<V, false>(P, s, D, KB, planes, n, nullptr, chunks, plane_c, ldcd, E, F, C,
-                                 ldc, r, c0, wide, smem);
+  mdgi::renorm_columns<V, mdgi::kTableChunks>(P, 0, D, 0, planes, n, &counts, chunks, plane_c, ldcd,
+                                              E, F, C, ldc, r, c0, wide, smem);
 }
 
 template <int V>
 __global__ void __launch_bounds__(RENORM_THREADS)
-    cross_renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::CrossChunks cross,
+    cross_renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::ChunkCounts counts,
                         int m, int n, const int *__restrict__ out, long long plane_c, int ldcd,
                         const int *__restrict__ E, const int *__restrict__ F,
                         double *__restrict__ C, int ldc, bool wide) {
@@ -44,8 +44,8 @@ __global__ void __launch_bounds__(RENORM_THREADS)
   const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
   const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
   if (r >= m) return;
-  mdgi::renorm_columns<V, true>(P, 0, D, 0, planes, n, &cross, out, plane_c, ldcd, E, F, C, ldc,
-                                r, c0, wide, smem);
+  mdgi::renorm_columns<V, mdgi::kCrossChunks>(P, 0, D, 0, planes, n, &counts, out, plane_c, ldcd, E,
+                                              F, C, ldc, r, c0, wide, smem);
 }
 
 // Every problem of a batch: block x belongs to the problem whose units hold x.
@@ -59,9 +59,9 @@ __global__ void __launch_bounds__(RENORM_THREADS)
   const long long e = (x - b.out_begin) * (long long)RENORM_THREADS + threadIdx.x;
   const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * 2;
   if (r >= b.m) return;
-  mdgi::renorm_columns<2, false>(b.p, b.s, b.D, b.Kp / 64, b.planes, b.n, nullptr, b.chunks,
-                                 b.plane_c, b.Np, exps + b.offE, exps + b.offF, b.C, b.ldc, r, c0,
-                                 b.wide, smem);
+  mdgi::renorm_columns<2, mdgi::kPlainChunks>(b.p, b.s, b.D, b.Kp / 64, b.planes, b.n, nullptr,
+                                              b.chunks, b.plane_c, b.Np, exps + b.offE,
+                                              exps + b.offF, b.C, b.ldc, r, c0, b.wide, smem);
 }
 
 bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
@@ -77,14 +77,17 @@ unsigned blocks(int m, int n, int V) {
 }
 
 template <int V>
-int launch_direct(int p, int s, int D, int KB, int m, int n, const int *chunks, long long plane_c,
-                  int ldcd, const int *E, const int *F, double *C, int ldc, cudaStream_t st) {
+int launch_direct(int p, int s, int D, int KB, int cs, int m, int n, const int *chunks,
+                  long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
+                  cudaStream_t st) {
+  mdgi::ChunkCounts counts{};
+  int planes = 0;
+  for (int d = 0; d < D; ++d) planes += counts.of[d] = mdgi::diag_chunks(d, s, KB, cs);
   const int smem = mdgi::renorm_smem(D, V, false);
   MDG_TRY_CUDA(cudaFuncSetAttribute(renorm_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     smem));
   renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
-      p, s, D, KB, mdgi::total_chunks(s, D, KB), m, n, chunks, plane_c, ldcd, E, F, C, ldc,
-      aligned16(C));
+      p, D, planes, counts, m, n, chunks, plane_c, ldcd, E, F, C, ldc, aligned16(C));
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }
@@ -92,15 +95,14 @@ int launch_direct(int p, int s, int D, int KB, int m, int n, const int *chunks, 
 template <int V>
 int launch_cross(int p, int D, int KB, int m, int n, const int *out, long long plane_c, int ldcd,
                  const int *E, const int *F, double *C, int ldc, cudaStream_t st) {
-  mdgi::CrossChunks cross{};
-  cross.pairs_per_chunk = mdgi::cross_pairs_per_chunk(KB);
-  for (int d = 1; d < D; ++d)
-    cross.of[d] = (unsigned short)mdgi::cross_chunks(d, cross.pairs_per_chunk);
+  mdgi::ChunkCounts counts{};
+  counts.pairs_per_chunk = mdgi::cross_pairs_per_chunk(KB);
+  for (int d = 1; d < D; ++d) counts.of[d] = mdgi::cross_chunks(d, counts.pairs_per_chunk);
   const int smem = mdgi::renorm_smem(D, V, true);
   MDG_TRY_CUDA(cudaFuncSetAttribute(cross_renorm_kernel<V>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   cross_renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
-      p, D, mdgi::cross_outputs(D, KB), cross, m, n, out, plane_c, ldcd, E, F, C, ldc,
+      p, D, mdgi::cross_outputs(D, KB), counts, m, n, out, plane_c, ldcd, E, F, C, ldc,
       aligned16(C));
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
@@ -110,14 +112,14 @@ int launch_cross(int p, int D, int KB, int m, int n, const int *out, long long p
 
 namespace mdgi {
 
-int launch_renorm(int p, int s, int D, int KB, int m, int n, const int *chunks,
+int launch_renorm(int p, int s, int D, int KB, int cs, int m, int n, const int *chunks,
                   long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
                   cudaStream_t st) {
   if (m == 0 || n == 0) return MDG_SUCCESS;
-  if (!words_for(1, D)) return MDG_ERROR_NOT_SUPPORTED;
+  if (!words_for(1, D) || D > 128) return MDG_ERROR_NOT_SUPPORTED;
   if (two_columns(m, n, chunks, plane_c, ldcd))
-    return launch_direct<2>(p, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
-  return launch_direct<1>(p, s, D, KB, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
+    return launch_direct<2>(p, s, D, KB, cs, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
+  return launch_direct<1>(p, s, D, KB, cs, m, n, chunks, plane_c, ldcd, E, F, C, ldc, st);
 }
 
 int launch_cross_renorm(int p, int D, int KB, int m, int n, const int *out, long long plane_c,

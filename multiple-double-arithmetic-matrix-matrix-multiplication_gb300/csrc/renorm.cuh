@@ -30,11 +30,15 @@ namespace mdgi {
 
 constexpr int RENORM_THREADS = 128;
 
-// Chunks of each diagonal in the cross form, by value to its kernel.
-struct CrossChunks {
-  unsigned short of[128];
-  int pairs_per_chunk;
+// Chunks of each diagonal, by value to a kernel.
+struct ChunkCounts {
+  unsigned of[128];
+  int pairs_per_chunk;  // cross form
 };
+
+// Where renorm_columns has the chunk counts from: chunks of CHUNK_STEPS
+// k-steps (a batch), a table, a table of the cross form.
+enum { kPlainChunks = 0, kTableChunks = 1, kCrossChunks = 2 };
 
 // 64-bit words of W per column: the diagonals', the carry out of them, two
 // of sign (windows of emit_limbs_shared).
@@ -168,9 +172,9 @@ __device__ __forceinline__ void add_at(long long &val, long long &up, long long 
 // is paid once per eight to sixteen loads; in the cross form all D squares go
 // to shared memory first, where the thread turns its own columns into prefix
 // sums.
-template <int V, bool CROSS>
+template <int V, int CHUNKS>
 __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int planes, int n,
-                                               const CrossChunks *cross,
+                                               const ChunkCounts *counts,
                                                const int *__restrict__ chunks, long long plane_c,
                                                int ldcd, const int *__restrict__ E,
                                                const int *__restrict__ F, double *__restrict__ C,
@@ -178,13 +182,14 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
   using I = Ints<V>;
   using Vec = typename I::T;
   constexpr int T = RENORM_THREADS;
+  constexpr bool CROSS = CHUNKS == kCrossChunks;
   const int dwords = (D + 7) / 8;
   // word i of column v at W[(i * V + v) * T]; Q_i at Q[i * T]
   uint64_t *W = reinterpret_cast<uint64_t *>(smem) + threadIdx.x;
   Vec *Q = reinterpret_cast<Vec *>(reinterpret_cast<uint64_t *>(smem) + (dwords + 3) * V * T) +
            threadIdx.x;
   const int *src = chunks + (size_t)r * ldcd + c0;
-  const int ppc = CROSS ? cross->pairs_per_chunk : 0;
+  const int ppc = CROSS ? counts->pairs_per_chunk : 0;
   if constexpr (CROSS) {
     for (int i = 0; i < D; ++i) {
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Q + i * T);
@@ -221,7 +226,7 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
       const int d = D - 1 - (wi * 8 + b);
-      nc[b] = d < 0 ? 0 : CROSS ? cross->of[d] : diag_chunks(d, s, KB);
+      nc[b] = d < 0 ? 0 : CHUNKS == kPlainChunks ? diag_chunks(d, s, KB) : (int)counts->of[d];
       q -= nc[b];
       first[b] = q;
       if (nc[b] > 0) x0[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)q * plane_c));

@@ -128,7 +128,7 @@ __device__ __forceinline__ int64_t exact_int(float x) {
 __global__ void __launch_bounds__(256)
     diag_gemm_v0(int s, int D, int Kp, const __nv_bfloat16 *__restrict__ dA,
                  const __nv_bfloat16 *__restrict__ dB, int ld, long long plane_a,
-                 long long plane_b, int *__restrict__ out, long long plane_c, int ldc) {
+                 long long plane_b, int *__restrict__ out, long long plane_c, int ldc, int cs) {
   __shared__ __align__(16) __nv_bfloat16 As[BM][SK];
   __shared__ __align__(16) __nv_bfloat16 Bs[BN][SK];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(256)
         }
         __syncthreads();
       }
-      const bool group_end = (step % V0_GROUP_STEPS == V0_GROUP_STEPS - 1) || step == S - 1;
-      const bool chunk_end = (step % mdgi::CHUNK_STEPS == mdgi::CHUNK_STEPS - 1) || step == S - 1;
+      const bool chunk_end = step % cs == cs - 1 || step == S - 1;
+      const bool group_end = step % V0_GROUP_STEPS == V0_GROUP_STEPS - 1 || chunk_end;
       if (group_end) {
 #pragma unroll
         for (int a = 0; a < 2; ++a)
@@ -263,7 +263,8 @@ int words_for(int s, int D) {
 }
 
 // sums: sum planes per operand (0: digit pairs alone)
-static SlicePlan layout_slice_plan(int p, int s, int D, int m, int n, int k, int sums) {
+static SlicePlan layout_slice_plan(int p, int s, int D, int m, int n, int k, int sums,
+                                   int cs = CHUNK_STEPS) {
   SlicePlan pl{};
   pl.p = p;
   pl.s = s;
@@ -275,7 +276,8 @@ static SlicePlan layout_slice_plan(int p, int s, int D, int m, int n, int k, int
   pl.Np = (int)align_up(std::max(n, 1), 256);
   pl.Kp = (int)align_up(std::max(k, 1), 64);
   pl.sums = sums;
-  pl.chunks = sums ? cross_outputs(D, pl.Kp / 64) : total_chunks(s, D, pl.Kp / 64);
+  pl.cs = cs;
+  pl.chunks = sums ? cross_outputs(D, pl.Kp / 64) : total_chunks(s, D, pl.Kp / 64, cs);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -300,9 +302,39 @@ SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
   return layout_slice_plan(p, s, D, m, n, k, 0);
 }
 
+int narrow_tile(int m, int n) {
+  const int tn = n <= 128 ? 128 : m <= 128 ? 256 : 0;
+  // a full chip of them asks more operand bytes of L2 than pairs do (tall dd
+  // 16001 x 96 x 3001: 1.84 ms against 1.74)
+  return tn && (long long)ceil_div(m, 128) * ceil_div(n, tn) <= 76 ? tn : 0;
+}
+
+// Measured, chunks of 2032 k-steps and at most 8 parts / this: qd 256^3 107 /
+// 28 us for the GEMM (plan 136 / 61 us a call), dd 64^3 26 / 11 us.
+//
+// k-steps per chunk that let the CTAs of a chip (152, or 76 pairs) share a
+// problem of few tiles: about the steps each can have.  Where a chunk per
+// CTA fits at up to twice that length it is taken, so that none gets two.
+static int chunk_steps(int s, int D, int m, int n, int KB) {
+  const int tn = narrow_tile(m, n);
+  const long long tiles = tn ? (long long)ceil_div(m, 128) * ceil_div(n, tn)
+                             : (long long)ceil_div(m, 256) * ceil_div(n, 256);
+  const int workers = tn ? 152 : 76;
+  long long steps = 0;
+  for (int d = 0; d < D; ++d) steps += (long long)diag_pairs(d, s) * KB;
+  const long long share = (steps * tiles + workers - 1) / workers;
+  if (2 * tiles > workers || share >= CHUNK_STEPS / 2) return CHUNK_STEPS;
+  const int least = std::max(8, (int)(share + 3) / 4 * 4);
+  for (int cs = least; cs <= 2 * least; cs += 4)
+    if (tiles * total_chunks(s, D, KB, cs) <= workers) return cs;
+  return least;
+}
+
 SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k) {
-  const SlicePlan pairs = make_slice_plan(p, s, D, m, n, k);
+  SlicePlan pairs = make_slice_plan(p, s, D, m, n, k);
   const int KB = pairs.Kp / 64;
+  const int cs = chunk_steps(s, D, std::max(m, 1), std::max(n, 1), KB);
+  if (cs != CHUNK_STEPS) pairs = layout_slice_plan(p, s, D, m, n, k, 0, cs);
   if (D < 2 || D > s || KB > CROSS_CHUNK_STEPS || !cross_pays(p, pairs.Mp, pairs.Np, KB))
     return pairs;
   const int all = cross_offset(D), least = cross_pairs(D - 1);
@@ -387,12 +419,12 @@ static DigitSide side_b(const SlicePlan &pl, const double *B, int ldb, const int
 
 int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
                         int ld, long long plane_a, long long plane_b, int *chunks,
-                        long long plane_c, cudaStream_t st) {
+                        long long plane_c, int cs, cudaStream_t st) {
   if (Mp % BM || Np % BN || Kp % 64) return MDG_ERROR_INVALID_SIZE;
   dim3 grid(Np / BN, Mp / BM);
   diag_gemm_v0<<<grid, 256, 0, st>>>(s, D, Kp, reinterpret_cast<const __nv_bfloat16 *>(dA),
                                      reinterpret_cast<const __nv_bfloat16 *>(dB), ld, plane_a,
-                                     plane_b, chunks, plane_c, Np);
+                                     plane_b, chunks, plane_c, Np, cs);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }
@@ -438,14 +470,14 @@ int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, voi
   auto *Cd = reinterpret_cast<int *>(bbase + plb.off_Cd);
   const SlicePlan &pl = plb;
   if (engine != 0) {
-    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, dA, dB, pl.Kp, pla.plane_a,
-                                pl.plane_b, Cd, pl.plane_c, engine == 2 ? 1 : 0, parts, raster, st,
-                                pace));
+    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, rows, pl.n, dA, dB, pl.Kp,
+                                pla.plane_a, pl.plane_b, Cd, pl.plane_c, pl.cs, engine, parts,
+                                raster, st, pace));
   } else {
     MDG_TRY(launch_diag_gemm_v0(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, dA, dB, pl.Kp, pla.plane_a,
-                                pl.plane_b, Cd, pl.plane_c, st));
+                                pl.plane_b, Cd, pl.plane_c, pl.cs, st));
   }
-  return launch_renorm(pl.p, pl.s, pl.D, pl.Kp / 64, rows, pl.n, Cd, pl.plane_c, pl.Np, E, F, C,
+  return launch_renorm(pl.p, pl.s, pl.D, pl.Kp / 64, pl.cs, rows, pl.n, Cd, pl.plane_c, pl.Np, E, F, C,
                        ldc, st);
 }
 
@@ -487,14 +519,14 @@ int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *
                                ldc, st);
   }
   if (engine != 0) {
-    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, dA, dB, pl.Kp, pl.plane_a,
-                                pl.plane_b, Cd, pl.plane_c, engine == 2 ? 1 : 0, parts, raster, st,
-                                pace));
+    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, pl.m, pl.n, dA, dB, pl.Kp,
+                                pl.plane_a, pl.plane_b, Cd, pl.plane_c, pl.cs, engine, parts,
+                                raster, st, pace));
   } else {
     MDG_TRY(launch_diag_gemm_v0(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, dA, dB, pl.Kp, pl.plane_a,
-                                pl.plane_b, Cd, pl.plane_c, st));
+                                pl.plane_b, Cd, pl.plane_c, pl.cs, st));
   }
-  MDG_TRY(launch_renorm(pl.p, pl.s, pl.D, pl.Kp / 64, pl.m, pl.n, Cd, pl.plane_c, pl.Np, E, F,
+  MDG_TRY(launch_renorm(pl.p, pl.s, pl.D, pl.Kp / 64, pl.cs, pl.m, pl.n, Cd, pl.plane_c, pl.Np, E, F,
                         C, ldc, st));
   return MDG_SUCCESS;
 }

@@ -25,12 +25,14 @@ __host__ __device__ inline int diag_pairs(int d, int s) {
   const int lo = d - (s - 1) > 0 ? d - (s - 1) : 0, hi = d < s - 1 ? d : s - 1;
   return hi - lo + 1;
 }
-__host__ __device__ inline int diag_chunks(int d, int s, int KB) {
-  return (diag_pairs(d, s) * KB + CHUNK_STEPS - 1) / CHUNK_STEPS;
+// Small problems cut the diagonals into shorter chunks (`cs` k-steps), so
+// that more CTAs share them.
+__host__ __device__ inline int diag_chunks(int d, int s, int KB, int cs = CHUNK_STEPS) {
+  return (diag_pairs(d, s) * KB + cs - 1) / cs;
 }
-inline int total_chunks(int s, int D, int KB) {
+inline int total_chunks(int s, int D, int KB, int cs = CHUNK_STEPS) {
   int c = 0;
-  for (int d = 0; d < D; ++d) c += diag_chunks(d, s, KB);
+  for (int d = 0; d < D; ++d) c += diag_chunks(d, s, KB, cs);
   return c;
 }
 
@@ -43,14 +45,19 @@ struct SlicePlan {
   // sum planes behind each operand's digit planes (cross_sums.cuh); 0: the
   // diagonal sums come from digit pairs alone.  off_norms: two unsigned.
   int sums;
+  int cs;  // k-steps per chunk (digit pairs)
   size_t off_bits, off_E, off_F, off_norms, off_dA, off_dB, off_Cd, total;
 };
 
 // The plan over digit pairs.
 SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k);
-// The plan over sum planes where that is faster, else make_slice_plan's;
-// never smaller than make_slice_plan's.
+// The plan over sum planes where that is faster; over digit pairs in shorter
+// chunks for small problems; else make_slice_plan's.  Never smaller than
+// make_slice_plan's.
 SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k);
+// Tiles of the single-CTA kernel for small problems of up to 128 rows or
+// columns: 128 rows by tn columns over the valid part (0: CTA pairs).
+int narrow_tile(int m, int n);
 int words_for(int s, int D);
 
 // The FP64-DMMA slice-digit form (digits64.cu): default digits per P
@@ -79,19 +86,20 @@ int launch_digits(int p, int s, const DigitSide &a, const DigitSide &b, unsigned
 // mma.sync engine (Mp % 128, Np % 64, Kp % 64)
 int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
                         int ld, long long plane_a, long long plane_b, int *chunks,
-                        long long plane_c, cudaStream_t st);
-// tcgen05 engine (Mp % 128, Np % 256, Kp % 64, ld == Kp).  single: 1 forces
-// 128 x 256 tiles on one CTA, 0 uses CTA pairs when Mp % 256 == 0.  parts:
-// diagonal ranges per pair tile, 0 = chosen to fill the last wave.  raster:
+                        long long plane_c, int cs, cudaStream_t st);
+// tcgen05 engine (Mp % 128, Np % 256, Kp % 64, ld == Kp; m x n valid).
+// engine: 2 forces 128 x 256 tiles on one CTA, 3 CTA pairs where Mp % 256 ==
+// 0, else pairs or narrow tiles by size.  parts: ranges of a tile's chunks, 0
+// = chosen to fill the chip.  raster:
 // pair tiles run across strips this many 256-column blocks wide (0 = auto).
 // pace: cross-cluster pacing window of the pair kernel in k-steps (0 = the
 // default, or MDG_TC_PACE when set; -1 = off).
-int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
-                        int ld, long long plane_a, long long plane_b, int *chunks,
-                        long long plane_c, int single, int parts, int raster, cudaStream_t st,
-                        int pace = 0);
+int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, const void *dA,
+                        const void *dB, int ld, long long plane_a, long long plane_b, int *chunks,
+                        long long plane_c, int cs, int engine, int parts, int raster,
+                        cudaStream_t st, int pace = 0);
 // Renormalisation of chunk planes (renorm.cu).
-int launch_renorm(int p, int s, int D, int KB, int m, int n, const int *chunks,
+int launch_renorm(int p, int s, int D, int KB, int cs, int m, int n, const int *chunks,
                   long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
                   cudaStream_t st);
 // One problem of a grouped diagonal GEMM: the single-CTA tcgen05 kernel

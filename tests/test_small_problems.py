@@ -1,0 +1,24 @@
+"""The BF16 form on problems of few tiles: chunks cut so that every CTA gets
+a share, narrow tiles for up to 128 rows or columns.  The same bits from the
+automatic choice, the CTA-pair, the single-CTA and the mma.sync engine."""
+import pytest
+
+from conftest import pkg
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,m,n,k", [
+    (2, 1, 1, 1), (2, 64, 64, 64), (4, 128, 128, 65), (4, 129, 128, 300), (4, 128, 129, 1000),
+    (4, 256, 256, 256), (4, 257, 500, 640), (8, 100, 1000, 130), (8, 1000, 100, 77),
+    (16, 130, 130, 129), (2, 16001, 96, 100), (4, 96, 3000, 600), (2, 60, 60, 20000),
+    (4, 512, 512, 200), (8, 700, 300, 900)])
+def test_few_tiles_same_bits(p, m, n, k):
+    import torch
+    api = pkg("api")
+    A = api.generate("normal", p, m, k, 7, -9, 9, scale_rows=True)
+    B = api.generate("uniform", p, k, n, 8)
+    got = api.gemm(A, B)
+    for engine in ("tc", "tc_pair", "mma_sync"):
+        assert torch.equal(got, api.gemm(A, B, engine=engine)), engine
+    assert torch.equal(got, api.gemm(A, B, parts=3))
+    assert api.device_status() == 0
