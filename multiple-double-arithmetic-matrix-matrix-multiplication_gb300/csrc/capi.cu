@@ -306,8 +306,16 @@ static int host_slice_panels_issue(int p, const Opts &o, int m, int n, int k, co
   const int ns = strips > 1 ? (int)align_up((n + strips - 1) / strips, 256) : n;
   SlicePlan pls[kMaxStrips];
   void *ws[kMaxStrips] = {};
+  const int engine = engine_choice(o.engine);
+  // sum planes on CTA pairs, in every strip or none, where their workspaces
+  // are to be had
+  bool sums = engine == 1 || engine == 3;
+  for (int j = 0; j < strips && sums; ++j) {
+    pls[j] = block_slice_plan(p, o.slices, o.diagonals, mp, std::min(ns, n - j * ns), k);
+    sums = pls[j].sums && g_cache.get(3 + j, pls[j].total, &ws[j]) == MDG_SUCCESS;
+  }
   for (int j = 0; j < strips; ++j) {
-    pls[j] = make_slice_plan(p, o.slices, o.diagonals, mp, std::min(ns, n - j * ns), k);
+    if (!sums) pls[j] = make_slice_plan(p, o.slices, o.diagonals, mp, std::min(ns, n - j * ns), k);
     if (pls[j].Mp > 65535 || pls[j].Np > 65535) return MDG_ERROR_NOT_SUPPORTED;
     MDG_TRY(g_cache.get(3 + j, pls[j].total, &ws[j]));
   }
@@ -336,7 +344,6 @@ static int host_slice_panels_issue(int p, const Opts &o, int m, int n, int k, co
   for (int j = 1; j < strips; ++j) MDG_TRY(copy_strip(j));
   MDG_TRY_CUDA(cudaStreamWaitEvent(sc, evB[0], 0));
   MDG_TRY(slice_prepare_b(pls[0], dB, n, ws[0], sc));
-  const int engine = engine_choice(o.engine);
   for (int i = 0; i < panels; ++i) {
     const int r0 = i * mp, rows = std::min(mp, m - r0);
     if (i + 1 < panels) {

@@ -52,14 +52,16 @@ inline int cross_group_end(int dlo, int D, int cap) {
 // buffers (s digit planes of rows x Kp first), and in norms[0] / norms[1]
 // the maxima, over the rows of A / B, the sum planes and the windows of half
 // a flush group, of the sums of squares.
+// One operand alone: the other's rows 0.
 int launch_cross_sums(int s, int dlo, int dhi, int Kp, int rows_a, int rows_b, void *dA, void *dB,
                       long long plane_a, long long plane_b, unsigned *norms, cudaStream_t st);
 
 // The diagonal GEMM over sum planes: the squares (squares = D, or 0 where
 // an earlier launch did them) and the diagonals [dlo, dhi).
 int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_planes, int Mp,
-                           int Np, int Kp, const void *dA, const void *dB, const unsigned *norms,
-                           int *out, int parts, int raster, int pace, cudaStream_t st);
+                           int Np, int Kp, const void *dA, const void *dB, const unsigned *norm_a,
+                           const unsigned *norm_b, int *out, int parts, int raster, int pace,
+                           cudaStream_t st);
 
 // Renormalisation from the cross form's output planes (renorm.cu).
 int launch_cross_renorm(int p, int D, int KB, int m, int n, const int *out, long long plane_c,

@@ -804,15 +804,15 @@ struct PairCross {
   const CUtensorMap *tmA, *tmB, *tmC;
   int D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB;
   int parts, raster;
-  const unsigned *norms;
+  const unsigned *norm_a, *norm_b;
   __device__ int units() const { return (Mp / 256) * (Np / TN2) * parts; }
   // Flush groups per sum plane.  |sum over a group| <= |a| |b| (Cauchy and
-  // Schwarz; every partial sum too) with |a|^2 <= 2 norms[0], |b|^2 <= 2
-  // norms[1] over a whole group (two windows), <= norms[0], norms[1] over
-  // half of one; a quarter holds at most 256 products of 2^16.  FP32 is
-  // exact up to 2^24, so whole groups where 4 norms[0] norms[1] <= 2^48.
+  // Schwarz; every partial sum too) with |a|^2 <= 2 *norm_a, |b|^2 <= 2
+  // *norm_b over a whole group (two windows), <= *norm_a, *norm_b over half
+  // of one; a quarter holds at most 256 products of 2^16.  FP32 is exact up
+  // to 2^24, so whole groups where 4 *norm_a *norm_b <= 2^48.
   __device__ int cuts() const {
-    const unsigned long long n2 = (unsigned long long)norms[0] * norms[1];
+    const unsigned long long n2 = (unsigned long long)*norm_a * *norm_b;
     return mdgi::cross_groups(KB) * (4 * n2 <= 1ull << 48 ? 1 : n2 <= 1ull << 48 ? 2 : 4);
   }
   __device__ CrossJob job(int u) const {
@@ -1099,10 +1099,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                            const __grid_constant__ CUtensorMap tmB,
                            const __grid_constant__ CUtensorMap tmC, int D, int dlo, int dhi,
                            int nsq, int plane0, int ppc, int Mp, int Np, int KB, int parts,
-                           int raster, const unsigned *__restrict__ norms, int pace,
-                           uint32_t epoch, int no_loads) {
+                           int raster, const unsigned *__restrict__ norm_a,
+                           const unsigned *__restrict__ norm_b, int pace, uint32_t epoch,
+                           int no_loads) {
   tc2_body(PairCross{&tmA, &tmB, &tmC, D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB, parts, raster,
-                     norms},
+                     norm_a, norm_b},
            pace, epoch, no_loads);
 }
 
@@ -1234,8 +1235,8 @@ PairSchedule pair_schedule(int Mp, int Np, int runs, int sms, int parts_opt, int
 namespace mdgi {
 
 int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_planes, int Mp,
-                           int Np, int Kp, const void *dA, const void *dB, const unsigned *norms,
-                           int *out, int parts, int raster, int pace, cudaStream_t st) {
+                           int Np, int Kp, const void *dA, const void *dB, const unsigned *norm_a,
+                           const unsigned *norm_b, int *out, int parts, int raster, int pace, cudaStream_t st) {
   if (Mp % 256 || Np % TN2 || Kp % TK) return MDG_ERROR_INVALID_SIZE;
   const int KB = Kp / TK;
   if (KB < 1 || KB > CROSS_CHUNK_STEPS) return MDG_ERROR_INVALID_SIZE;
@@ -1252,7 +1253,7 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
       pair_schedule(Mp, Np, squares + dhi - dlo, sms, parts, raster, pace);
   diag_gemm_cross_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
       ma, mb, mc, D, dlo, dhi, squares, s - cross_offset(dlo), cross_pairs_per_chunk(KB), Mp, Np, KB,
-      sc.parts, sc.raster, norms, sc.pace, sc.epoch, sc.no_loads);
+      sc.parts, sc.raster, norm_a, norm_b, sc.pace, sc.epoch, sc.no_loads);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }

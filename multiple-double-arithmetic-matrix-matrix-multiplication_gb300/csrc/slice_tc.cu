@@ -234,7 +234,10 @@ namespace mdgi {
 // diagonals are done in groups that reuse the buffer).  kCrossMaxBytes:
 // workspace beyond which the digit pairs are used, so that problems which
 // fill the device still fit.
+// kCrossBlockBytes: workspace of a column strip of the host entry, whose
+// sums are all kept for the row panels to come.
 constexpr size_t kCrossSumBytes = 16ull << 30, kCrossMaxBytes = 160ull << 30;
+constexpr size_t kCrossBlockBytes = 32ull << 30;
 
 // Where sum planes beat digit pairs.  They save half the products (time as
 // Mp Np Kp) and cost the writing of the sums (as (Mp + Np) Kp) and a dearer
@@ -429,6 +432,25 @@ int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, co
   return MDG_SUCCESS;
 }
 
+SlicePlan block_slice_plan(int p, int s, int D, int m, int n, int k) {
+  const SlicePlan pairs = make_slice_plan(p, s, D, m, n, k);
+  const int KB = pairs.Kp / 64;
+  if (D < 2 || D > s || KB > CROSS_CHUNK_STEPS || !cross_pays(p, pairs.Mp, pairs.Np, KB))
+    return pairs;
+  const SlicePlan pl = layout_slice_plan(p, s, D, m, n, k, cross_offset(D));
+  return pl.total <= kCrossBlockBytes ? pl : pairs;
+}
+
+// All sums of one side of a block plan, and its norm.
+static int block_sums(const SlicePlan &pl, int rows_a, int rows_b, void *ws, cudaStream_t st) {
+  if (!pl.sums) return MDG_SUCCESS;
+  char *base = reinterpret_cast<char *>(ws);
+  auto *norms = reinterpret_cast<unsigned *>(base + pl.off_norms);
+  MDG_TRY_CUDA(cudaMemsetAsync(norms + (rows_b ? 1 : 0), 0, sizeof(unsigned), st));
+  return launch_cross_sums(pl.s, 1, pl.D, pl.Kp, rows_a, rows_b, base + pl.off_dA,
+                           base + pl.off_dB, pl.plane_a, pl.plane_b, norms, st);
+}
+
 int slice_prepare_b(const SlicePlan &pl, const double *B, int ldb, void *ws, cudaStream_t st) {
   char *base = reinterpret_cast<char *>(ws);
   int *F = reinterpret_cast<int *>(base + pl.off_F);
@@ -437,7 +459,8 @@ int slice_prepare_b(const SlicePlan &pl, const double *B, int ldb, void *ws, cud
   const DigitSide b = side_b(pl, B, ldb, F, base + pl.off_dB);
   DigitSide none = b;
   none.rows = 0;
-  return launch_digits(pl.p, pl.s, none, b, nullptr, st);
+  MDG_TRY(launch_digits(pl.p, pl.s, none, b, nullptr, st));
+  return block_sums(pl, 0, pl.n, ws, st);
 }
 
 int slice_panel_a(const SlicePlan &pl, int rows, const double *A, int lda, void *ws,
@@ -451,7 +474,8 @@ int slice_panel_a(const SlicePlan &pl, int rows, const double *A, int lda, void 
   const DigitSide a = side_a(pl, rows, A, lda, E, base + pl.off_dA);
   DigitSide none = a;
   none.rows = 0;
-  return launch_digits(pl.p, pl.s, a, none, nullptr, st);
+  MDG_TRY(launch_digits(pl.p, pl.s, a, none, nullptr, st));
+  return block_sums(pl, rows, 0, ws, st);
 }
 
 int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, void *wsb, int rows,
@@ -459,7 +483,7 @@ int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, voi
                 int pace) {
   if (rows <= 0) return MDG_SUCCESS;
   if (rows > pla.m || pla.Mp != plb.Mp || pla.Kp != plb.Kp || pla.s != plb.s ||
-      pla.D != plb.D || pla.p != plb.p)
+      pla.D != plb.D || pla.p != plb.p || pla.sums != plb.sums)
     return MDG_ERROR_INVALID_SIZE;
   const char *abase = reinterpret_cast<const char *>(wsa);
   char *bbase = reinterpret_cast<char *>(wsb);
@@ -469,6 +493,14 @@ int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, voi
   const void *dB = bbase + plb.off_dB;
   auto *Cd = reinterpret_cast<int *>(bbase + plb.off_Cd);
   const SlicePlan &pl = plb;
+  if (pl.sums) {
+    const auto *norm_a = reinterpret_cast<const unsigned *>(abase + pla.off_norms);
+    const auto *norm_b = reinterpret_cast<const unsigned *>(bbase + plb.off_norms) + 1;
+    MDG_TRY(launch_diag_gemm_cross(pl.s, pl.D, 1, pl.D, pl.D, pl.sums, pl.Mp, pl.Np, pl.Kp, dA, dB,
+                                   norm_a, norm_b, Cd, parts, raster, pace, st));
+    return launch_cross_renorm(pl.p, pl.D, pl.Kp / 64, rows, pl.n, Cd, pl.plane_c, pl.Np, E, F, C,
+                               ldc, st);
+  }
   if (engine != 0) {
     MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, rows, pl.n, dA, dB, pl.Kp,
                                 pla.plane_a, pl.plane_b, Cd, pl.plane_c, pl.cs, engine, parts,
@@ -513,7 +545,8 @@ int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *
       MDG_TRY(launch_cross_sums(pl.s, lo, hi, pl.Kp, pl.m, pl.n, dA, dB, pl.plane_a, pl.plane_b,
                                 norms, st));
       MDG_TRY(launch_diag_gemm_cross(pl.s, pl.D, lo, hi, lo == 1 ? pl.D : 0, pl.sums, pl.Mp,
-                                     pl.Np, pl.Kp, dA, dB, norms, Cd, parts, raster, pace, st));
+                                     pl.Np, pl.Kp, dA, dB, norms, norms + 1, Cd, parts, raster,
+                                     pace, st));
     }
     return launch_cross_renorm(pl.p, pl.D, pl.Kp / 64, pl.m, pl.n, Cd, pl.plane_c, pl.Np, E, F, C,
                                ldc, st);

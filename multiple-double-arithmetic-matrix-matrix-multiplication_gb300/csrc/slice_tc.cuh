@@ -55,6 +55,10 @@ SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k);
 // chunks for small problems; else make_slice_plan's.  Never smaller than
 // make_slice_plan's.
 SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k);
+// The plan of a row panel by column strip block (slice_block): over sum planes,
+// all of them held, where that is faster and of bounded size, else
+// make_slice_plan's.
+SlicePlan block_slice_plan(int p, int s, int D, int m, int n, int k);
 // Tiles of the single-CTA kernel for small problems of up to 128 rows or
 // columns: 128 rows by tn columns over the valid part (0: CTA pairs).
 int narrow_tile(int m, int n);
