@@ -81,8 +81,9 @@ int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, in
                                  (long long)mdgi::total_chunks(b.s, b.D, b.Kp / 64) * b.Mp));
     g.s = b.s; g.D = b.D; g.Mp = b.Mp; g.Np = b.Np; g.KB = b.Kp / 64;
     g.tn = tn;
-    g.mt = pair ? b.Mp / 256 : (b.m + 127) / 128;
-    g.nt = (b.n + tn - 1) / tn;
+    g.stack = pair ? mdgi::stacked_tiles(b.s, b.D, b.m, b.n, b.Kp / 64) : 0;
+    g.mt = pair && g.stack != 2 ? b.Mp / 256 : (b.m + 127) / 128;
+    g.nt = g.stack == 1 ? (b.n + 127) / 128 : (b.n + tn - 1) / tn;
     g.ktail = (b.k - (g.KB - 1) * 64 + 15) / 16;
     g.parts = 1;
     hg->push_back(g);
@@ -91,7 +92,10 @@ int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, in
   // x tile area
   auto tile_work = [&](const mdgi::GroupedProblem &g) {
     long long pairs = 0;
-    for (int d = 0; d < g.D; ++d) pairs += mdgi::diag_pairs(d, g.s);
+    if (g.stack)
+      for (int d = -(g.D & 1); d < g.D; d += 2) pairs += d + 2;
+    else
+      for (int d = 0; d < g.D; ++d) pairs += mdgi::diag_pairs(d, g.s);
     return pairs * g.KB * (pair ? 4 : g.tn / 128);
   };
   if (split) {
@@ -100,7 +104,7 @@ int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, in
     const long long target =
         std::max(1LL, total / ((long long)std::max(workers, 1) * kSplitUnitsPerWorker));
     for (mdgi::GroupedProblem &g : *hg)
-      g.parts = (int)std::min<long long>(g.D, std::max(1LL, (tile_work(g) + target - 1) / target));
+      g.parts = (int)std::min<long long>(g.stack ? (g.D + 1) / 2 : g.D, std::max(1LL, (tile_work(g) + target - 1) / target));
   }
   // The grouped kernel deals units to CTAs round-robin in table order.
   // Heaviest units first (a quad-double tile carries ~4x the work of a

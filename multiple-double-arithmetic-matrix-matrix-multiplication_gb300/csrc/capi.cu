@@ -720,7 +720,7 @@ int mdg_slice_diagonals(int s, int D, int m, int n, int k, const void *dA, const
   const long long plane_c = (long long)m * n;
   const int eng = engine_choice(0);
   if (eng != 0 && ld == k)
-    return launch_diag_gemm_tc(s, D, m, n, k, m, n, dA, dB, ld, plane_a, plane_b, chunks, plane_c,
+    return launch_diag_gemm_tc(s, D, m, n, k, m, n, k, dA, dB, ld, plane_a, plane_b, chunks, plane_c,
                                CHUNK_STEPS, eng, 0, 0, as_stream(stream));
   return launch_diag_gemm_v0(s, D, m, n, k, dA, dB, ld, plane_a, plane_b, chunks, plane_c,
                              CHUNK_STEPS, as_stream(stream));

@@ -256,21 +256,42 @@ __device__ __forceinline__ void stores_done() {
 }
 
 // A run of plane products that goes into one output plane: `steps` k-steps
-// from step t0 of the products of planes (a0 + p, b0 + bstep p), KB k-steps
-// each, p = 0, 1, ..  cuts: flush groups per plane (sums form).
+// from step t0 of the products of planes (a0 + astep p, b0 + bstep p), KB
+// k-steps each, p = 0, 1, ..  cuts: flush groups per plane (sums form).
 struct Run {
-  int a0, b0, t0, steps, chunk, cuts;
+  int a0, astep, b0, bstep, t0, steps, chunk, cuts;
 };
 
-// Runs over digit planes: the chunks (cs k-steps) of the diagonals.
+// Two diagonals in one 256 x 256 accumulator, for problems that waste less on
+// tiles of 128: the second half of B's rows (kStackN), or of A's (kStackM),
+// is the next digit plane instead of the next 128 columns (rows), so that
+// the halves of the accumulator are diagonals d and d + 1 of a 256 x 128
+// (128 x 256) tile.  A step too many at one end of d is a plane -1, which the
+// TMA fills with zeros.  Pair kernel, D <= s, one chunk per diagonal.  Dd 14
+// digits: 56 steps for the tile of 128 instead of 105 for one of 256 that is
+// half padding; dd 16001 x 96 x 3001 2.50 -> 1.73 ms a call (its GEMM streams
+// A's planes from DRAM, 56 instead of 105 times 97 MB), 64 mixed problems of
+// 32 .. 512 3.15 -> 2.69 ms.
+enum { kStackNone = 0, kStackN = 1, kStackM = 2 };
+
+// Runs over digit planes: the chunks (cs k-steps) of the diagonals; stacked,
+// pairs of diagonals from the top down, an odd first one with d = -1.
 struct DigitRuns {
-  static constexpr int bstep = -1;
-  int s, D, KB, cs, d, c, chunk, left;
+  int s, D, KB, cs, stack, d, c, chunk, left;
   __device__ bool next(Run &r) {
     if (left <= 0 || d >= D) return false;
+    if (stack) {
+      r = stack == kStackN ? Run{0, 1, d, -1, 0, (d + 2) * KB, d, 0}
+                           : Run{d, -1, 0, 1, 0, (d + 2) * KB, d, 0};
+      d += 2;
+      --left;
+      return true;
+    }
     const int S = mdgi::diag_pairs(d, s) * KB;
     r.a0 = d - (s - 1) > 0 ? d - (s - 1) : 0;
     r.b0 = d - r.a0;
+    r.astep = 1;
+    r.bstep = -1;
     r.t0 = c * cs;
     r.steps = S - r.t0 < cs ? S - r.t0 : cs;
     r.chunk = chunk++;
@@ -299,14 +320,19 @@ struct DigitRuns {
 // Part `part` of a tile's runs: run `part` itself where there are as many
 // parts as runs, else the runs that start in the part's 1/parts of the
 // tile's k-steps (none when parts exceeds what the runs allow).
-__device__ __forceinline__ DigitRuns part_runs(int s, int D, int KB, int cs, int part, int parts) {
-  DigitRuns all{s, D, KB, cs, 0, 0, 0, 1 << 30};
+__device__ __forceinline__ DigitRuns part_runs(int s, int D, int KB, int cs, int stack, int part,
+                                               int parts) {
+  DigitRuns all{s, D, KB, cs, stack, stack ? -(D & 1) : 0, 0, 0, 1 << 30};
   if (parts == 1) return all;
   long long steps = 0;
   int runs = 0;
-  for (int d = 0; d < D; ++d) {
-    steps += mdgi::diag_pairs(d, s) * KB;
-    runs += mdgi::diag_chunks(d, s, KB, cs);
+  if (stack) {
+    for (int d = -(D & 1); d < D; d += 2, ++runs) steps += (d + 2) * KB;
+  } else {
+    for (int d = 0; d < D; ++d) {
+      steps += mdgi::diag_pairs(d, s) * KB;
+      runs += mdgi::diag_chunks(d, s, KB, cs);
+    }
   }
   const bool one = parts == runs;
   const long long lo = one ? part : steps * part / parts;
@@ -342,7 +368,7 @@ struct SingleJobs {
   __device__ TileJob job(int u) const {
     const int tiles = mt * nt, tile = u % tiles;
     return TileJob{tmA, tmB, tmC, Mp, Np, KB, (tile % mt) * TM, (tile / mt) * tn, tn, TK / 16,
-                   part_runs(s, D, KB, cs, u / tiles, parts)};
+                   part_runs(s, D, KB, cs, kStackNone, u / tiles, parts)};
   }
 };
 
@@ -405,7 +431,7 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
         Run r;
         while (jb.runs.next(r)) {
           for (int t = r.t0; t < r.t0 + r.steps; ++t) {
-            const int q = t / KB, kb = t - q * KB, i = r.a0 + q, j = r.b0 + DigitRuns::bstep * q;
+            const int q = t / KB, kb = t - q * KB, i = r.a0 + q, j = r.b0 - q;
             if (!mbar_wait(empty(st), ph ^ 1, abort_flag)) goto producer_done;
             mbar_expect_tx(full(st), A_BYTES + jb.tn * TK * 2);
             const uint32_t a_dst = smem_base + st * STAGE_BYTES;
@@ -566,7 +592,7 @@ struct GroupedJobs {
                    reinterpret_cast<const CUtensorMap *>(g.tmB),
                    reinterpret_cast<const CUtensorMap *>(g.tmC), g.Mp, g.Np, g.KB,
                    (tile % g.mt) * TM, (tile / g.mt) * g.tn, g.tn, g.ktail,
-                   part_runs(g.s, g.D, g.KB, mdgi::CHUNK_STEPS, part, g.parts)};
+                   part_runs(g.s, g.D, g.KB, mdgi::CHUNK_STEPS, kStackNone, part, g.parts)};
   }
 };
 
@@ -694,10 +720,10 @@ __device__ __forceinline__ uint32_t pace_load(int slot, int ncl, uint32_t epoch)
 
 // One unit of work of the pair kernel over digit planes: a 256 x 256 tile
 // of one problem (rows row0.., columns col0..) and the runs it computes.
+// ktail: as in TileJob.
 struct PairJob {
-  using Runs = DigitRuns;
   const CUtensorMap *tmA, *tmB, *tmC;
-  int Mp, Np, KB, row0, col0;
+  int Mp, Np, KB, row0, col0, stack, ktail;
   DigitRuns runs;
 };
 
@@ -707,21 +733,20 @@ struct PairJob {
 // index on both sides; flush groups never span two planes, because their
 // exactness rests on the norms of windows of single sum planes.
 struct CrossRuns {
-  static constexpr int bstep = 1;
   int sq, nsq, d, i, chunk, planes;  // where the list goes on, planes left
   int plane0, ppc, KB;               // plane of diagonal d's pair 0 is plane0 + cross_offset(d)
   int cuts1, cuts;                   // flush groups per square, per sum
   __device__ bool next(Run &r) {
     if (planes <= 0) return false;
     if (sq < nsq) {
-      r = Run{sq, sq, 0, KB, sq, cuts1};
+      r = Run{sq, 1, sq, 1, 0, KB, sq, cuts1};
       ++sq;
       --planes;
     } else {
       const int left = mdgi::cross_pairs(d) - i;
       const int np = left < ppc ? left : ppc;
       const int t = plane0 + mdgi::cross_offset(d) + i;
-      r = Run{t, t, 0, np * KB, chunk, cuts};
+      r = Run{t, 1, t, 1, 0, np * KB, chunk, cuts};
       ++chunk;
       planes -= np;
       i += np;
@@ -748,7 +773,7 @@ struct CrossRuns {
 };
 
 struct CrossJob {
-  using Runs = CrossRuns;
+  static constexpr int stack = kStackNone, ktail = TK / 16;
   const CUtensorMap *tmA, *tmB, *tmC;
   int Mp, Np, KB, row0, col0;
   CrossRuns runs;
@@ -762,19 +787,19 @@ struct CrossJob {
 // them in L2 (raster = 1 walks each column block top to bottom).
 struct PairSingle {
   const CUtensorMap *tmA, *tmB, *tmC;
-  int s, D, Mp, Np, KB, cs;
+  int s, D, Mp, Np, KB, cs, stack, ktail, mt, nt;
   int parts, raster;
-  __device__ int units() const { return (Mp / 256) * (Np / TN2) * parts; }
+  __device__ int units() const { return mt * nt * parts; }
   __device__ PairJob job(int u) const {
-    const int MB = Mp / 256, NB = Np / TN2, tiles = MB * NB;
-    const int tile = u % tiles, part = u / tiles;
-    const int strip = tile / (MB * raster);
-    const int idx = tile - strip * MB * raster;
+    const int tiles = mt * nt, tile = u % tiles, part = u / tiles;
+    const int strip = tile / (mt * raster);
+    const int idx = tile - strip * mt * raster;
     const int c0 = strip * raster;
-    const int g = NB - c0 < raster ? NB - c0 : raster;
+    const int g = nt - c0 < raster ? nt - c0 : raster;
     const int rb = idx / g, cb = c0 + idx - rb * g;
-    return PairJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2,
-                   part_runs(s, D, KB, cs, part, parts)};
+    return PairJob{tmA, tmB, tmC, Mp, Np, KB, rb * (stack == kStackM ? 128 : 256),
+                   cb * (stack == kStackN ? 128 : 256), stack, ktail,
+                   part_runs(s, D, KB, cs, stack, part, parts)};
   }
 };
 
@@ -792,8 +817,9 @@ struct PairGrouped {
     return PairJob{reinterpret_cast<const CUtensorMap *>(g.tmA),
                    reinterpret_cast<const CUtensorMap *>(g.tmB),
                    reinterpret_cast<const CUtensorMap *>(g.tmC), g.Mp, g.Np, g.KB,
-                   (tile % g.mt) * 256, (tile / g.mt) * TN2,
-                   part_runs(g.s, g.D, g.KB, mdgi::CHUNK_STEPS, part, g.parts)};
+                   (tile % g.mt) * (g.stack == kStackM ? 128 : 256),
+                   (tile / g.mt) * (g.stack == kStackN ? 128 : 256), g.stack, g.ktail,
+                   part_runs(g.s, g.D, g.KB, mdgi::CHUNK_STEPS, g.stack, part, g.parts)};
   }
 };
 
@@ -915,13 +941,16 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       for (int u = no_loads ? units : cid; u < units; u += ncl) {
         auto jb = jobs.job(u);
         const int KB = jb.KB;
-        const int row = jb.row0 + (int)rank * TM;
-        const int col = jb.col0 + (int)rank * BH;
+        // the odd CTA: the next 128 rows and columns, or the next plane
+        const int next_a = jb.stack == kStackM ? (int)rank : 0;
+        const int next_b = jb.stack == kStackN ? (int)rank : 0;
+        const int row = jb.row0 + ((int)rank - next_a) * TM;
+        const int col = jb.col0 + ((int)rank - next_b) * BH;
         Run r;
         while (jb.runs.next(r)) {
           for (int t = r.t0; t < r.t0 + r.steps; ++t) {
-            const int q = t / KB, kb = t - q * KB, i = r.a0 + q;
-            const int j = r.b0 + decltype(jb.runs)::bstep * q;
+            const int q = t / KB, kb = t - q * KB;
+            const int i = r.a0 + r.astep * q + next_a, j = r.b0 + r.bstep * q + next_b;
             if (pacing && steps > *pace_allowed) {
               const unsigned long long t0 = now_ns();
               while (steps > *pace_allowed) {
@@ -964,6 +993,7 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
         auto jb = jobs.job(u);
         Run r;
         while (jb.runs.next(r)) {
+          int kb = r.t0 % jb.KB;
           typename decltype(jb.runs)::Groups groups(r, jb.KB);
           for (int steps; (steps = groups.next()) > 0;) {
             if (!mbar_wait(accempty(buf), aph[buf] ^ 1, abort_flag)) goto mma_done;
@@ -974,9 +1004,17 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
               fence_after();
               const uint32_t a_addr = smem_base + st * STAGE2_BYTES;
               const uint64_t da = sw128_desc(a_addr), db = sw128_desc(a_addr + A2_BYTES);
+              // the last k-block of a plane: only the MMAs that reach data
+              const bool short_block = kb == jb.KB - 1 && jb.ktail < TK / 16;
+              if (++kb == jb.KB) kb = 0;
+              if (!short_block) {
 #pragma unroll
-              for (int kk = 0; kk < TK / 16; ++kk)
-                mma_bf16_pair(dt, da + 2 * kk, db + 2 * kk, (t > 0 || kk > 0) ? 1u : 0u);
+                for (int kk = 0; kk < TK / 16; ++kk)
+                  mma_bf16_pair(dt, da + 2 * kk, db + 2 * kk, (t > 0 || kk > 0) ? 1u : 0u);
+              } else {
+                for (int kk = 0; kk < jb.ktail; ++kk)
+                  mma_bf16_pair(dt, da + 2 * kk, db + 2 * kk, (t > 0 || kk > 0) ? 1u : 0u);
+              }
               mma_commit_pair(empty(st));
               any = true;
               if (++st == STAGES2) {
@@ -1041,8 +1079,9 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
     const uint32_t accempty0[2] = {map_to_rank0(accempty(0)), map_to_rank0(accempty(1))};
     for (int u = cid; u < units; u += ncl) {
       auto jb = jobs.job(u);
-      const int row = jb.row0 + (int)rank * TM + 32 * q;
-      const int col = jb.col0 + 128 * h;
+      const int next = jb.stack == kStackM ? (int)rank : jb.stack == kStackN ? h : 0;
+      const int row = jb.row0 + (jb.stack == kStackM ? 0 : (int)rank * TM) + 32 * q;
+      const int col = jb.col0 + (jb.stack == kStackN ? 0 : 128 * h);
       Run r;
       while (jb.runs.next(r)) {
         typename decltype(jb.runs)::Groups groups(r, jb.KB);
@@ -1059,7 +1098,9 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(accempty0[buf]);
           buf ^= 1;
-          if (groups.last()) store_rows(staging, lane, acc, jb.tmC, col, r.chunk * jb.Mp + row);
+          // (a diagonal -1 is all zeros)
+          if (groups.last() && r.chunk + next >= 0)
+            store_rows(staging, lane, acc, jb.tmC, col, (r.chunk + next) * jb.Mp + row);
         }
       }
     }
@@ -1081,10 +1122,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
     diag_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA,
                          const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
-                         int KB, int cs, int parts, int raster, int pace, uint32_t epoch,
-                         int no_loads) {
-  tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, parts, raster}, pace, epoch,
-           no_loads);
+                         int KB, int cs, int stack, int ktail, int mt, int nt, int parts,
+                         int raster, int pace, uint32_t epoch, int no_loads) {
+  tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
+           pace, epoch, no_loads);
 }
 
 // The diagonal GEMM over digit and sum planes (cross_sums.cuh).  Bound by the
@@ -1174,10 +1215,10 @@ int few_tile_parts(int tiles, int runs, int workers, int parts) {
 }
 
 // runs: of a tile, what parts can separate.
-PairSchedule pair_schedule(int Mp, int Np, int runs, int sms, int parts_opt, int raster_opt,
+PairSchedule pair_schedule(int mt, int nt, int runs, int sms, int parts_opt, int raster_opt,
                            int pace_opt) {
   PairSchedule sc;
-  const int tiles = (Mp / 256) * (Np / TN2);
+  const int tiles = mt * nt;
   // split tiles into `parts` diagonal ranges when that shrinks the idle
   // part of the last wave of clusters by more than it costs: each extra
   // part makes the work about 4 % slower (fitted to quad-double 4096^3 and
@@ -1200,11 +1241,10 @@ PairSchedule pair_schedule(int Mp, int Np, int runs, int sms, int parts_opt, int
   // tile order: strips about sqrt(clusters) column blocks wide, so that
   // the tiles in work at one time span few row and column blocks (the
   // largest power of two not above sqrt(76) = 8.7 on 152 SMs)
-  const int NB = Np / TN2;
   sc.raster = 1;
   while ((sc.raster * 2) * (sc.raster * 2) <= ncl) sc.raster *= 2;
   if (raster_opt > 0) sc.raster = raster_opt;
-  sc.raster = std::min(NB, sc.raster);
+  sc.raster = std::min(nt, sc.raster);
   const long long units = (long long)tiles * sc.parts;
   sc.clusters = units < ncl ? (int)units : ncl;
   // pacing window in k-steps, 0 = off (MDG_TC_PACE overrides); every
@@ -1250,7 +1290,7 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const PairSchedule sc =
-      pair_schedule(Mp, Np, squares + dhi - dlo, sms, parts, raster, pace);
+      pair_schedule(Mp / 256, Np / TN2, squares + dhi - dlo, sms, parts, raster, pace);
   diag_gemm_cross_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
       ma, mb, mc, D, dlo, dhi, squares, s - cross_offset(dlo), cross_pairs_per_chunk(KB), Mp, Np, KB,
       sc.parts, sc.raster, norm_a, norm_b, sc.pace, sc.epoch, sc.no_loads);
@@ -1258,11 +1298,22 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
   return MDG_SUCCESS;
 }
 
-int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, const void *dA,
+int stacked_tiles(int s, int D, int m, int n, int KB) {
+  if (D > s || (long long)(D + 1) * KB > CHUNK_STEPS) return kStackNone;
+  long long pairs = 0, stacked = 0;
+  for (int d = 0; d < D; ++d) pairs += diag_pairs(d, s);
+  for (int d = -(D & 1); d < D; d += 2) stacked += d + 2;
+  const long long m256 = (m + 255) / 256, n256 = (n + 255) / 256;
+  const long long work[3] = {m256 * n256 * pairs, m256 * ((n + 127) / 128) * stacked,
+                             (m + 127) / 128 * n256 * stacked};
+  return (int)(std::min_element(work, work + 3) - work);
+}
+
+int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int k, const void *dA,
                         const void *dB, int ld, long long plane_a, long long plane_b, int *chunks,
                         long long plane_c, int cs, int engine, int parts_opt, int raster_opt,
                         cudaStream_t st, int pace_opt) {
-  if (Mp % TM || Np % TN || Kp % TK || ld != Kp) return MDG_ERROR_INVALID_SIZE;
+  if (Mp % TM || Np % TN || Kp % TK || ld != Kp || k <= Kp - TK || k > Kp) return MDG_ERROR_INVALID_SIZE;
   if (plane_a != (long long)Mp * Kp || plane_b != (long long)Np * Kp) return MDG_ERROR_INVALID_SIZE;
   if ((reinterpret_cast<uintptr_t>(dA) | reinterpret_cast<uintptr_t>(dB)) & 15)
     return MDG_ERROR_INVALID_SIZE;
@@ -1288,10 +1339,15 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, cons
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (pair) {
-    const PairSchedule sc = pair_schedule(Mp, Np, runs, sms, parts_opt, raster_opt, pace_opt);
+    const int stack =
+        cs == CHUNK_STEPS && engine == 1 ? stacked_tiles(s, D, m, n, Kp / TK) : kStackNone;
+    const int mt = stack == kStackM ? (m + 127) / 128 : Mp / 256;
+    const int nt = stack == kStackN ? (n + 127) / 128 : Np / TN2;
+    const PairSchedule sc = pair_schedule(mt, nt, stack ? (D + 1) / 2 : runs, sms, parts_opt,
+                                          raster_opt, pace_opt);
     diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
-        ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, sc.parts, sc.raster, sc.pace, sc.epoch,
-        sc.no_loads);
+        ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, stack, (k - (Kp - TK) + 15) / 16, mt, nt, sc.parts,
+        sc.raster, sc.pace, sc.epoch, sc.no_loads);
   } else {
     const int mt = (m + TM - 1) / TM, nt = (n + tn - 1) / tn, tiles = mt * nt;
     const int parts = parts_opt > 0 ? std::min(8, parts_opt)

@@ -502,7 +502,7 @@ int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, voi
                                ldc, st);
   }
   if (engine != 0) {
-    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, rows, pl.n, dA, dB, pl.Kp,
+    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, rows, pl.n, pl.k, dA, dB, pl.Kp,
                                 pla.plane_a, pl.plane_b, Cd, pl.plane_c, pl.cs, engine, parts,
                                 raster, st, pace));
   } else {
@@ -552,7 +552,7 @@ int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *
                                ldc, st);
   }
   if (engine != 0) {
-    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, pl.m, pl.n, dA, dB, pl.Kp,
+    MDG_TRY(launch_diag_gemm_tc(pl.s, pl.D, pl.Mp, pl.Np, pl.Kp, pl.m, pl.n, pl.k, dA, dB, pl.Kp,
                                 pl.plane_a, pl.plane_b, Cd, pl.plane_c, pl.cs, engine, parts,
                                 raster, st, pace));
   } else {

@@ -91,14 +91,14 @@ int launch_digits(int p, int s, const DigitSide &a, const DigitSide &b, unsigned
 int launch_diag_gemm_v0(int s, int D, int Mp, int Np, int Kp, const void *dA, const void *dB,
                         int ld, long long plane_a, long long plane_b, int *chunks,
                         long long plane_c, int cs, cudaStream_t st);
-// tcgen05 engine (Mp % 128, Np % 256, Kp % 64, ld == Kp; m x n valid).
+// tcgen05 engine (Mp % 128, Np % 256, Kp % 64, ld == Kp; m x n x k valid).
 // engine: 2 forces 128 x 256 tiles on one CTA, 3 CTA pairs where Mp % 256 ==
 // 0, else pairs or narrow tiles by size.  parts: ranges of a tile's chunks, 0
 // = chosen to fill the chip.  raster:
 // pair tiles run across strips this many 256-column blocks wide (0 = auto).
 // pace: cross-cluster pacing window of the pair kernel in k-steps (0 = the
 // default, or MDG_TC_PACE when set; -1 = off).
-int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, const void *dA,
+int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int k, const void *dA,
                         const void *dB, int ld, long long plane_a, long long plane_b, int *chunks,
                         long long plane_c, int cs, int engine, int parts, int raster,
                         cudaStream_t st, int pace = 0);
@@ -114,14 +114,17 @@ int launch_renorm(int p, int s, int D, int KB, int cs, int m, int n, const int *
 // its mt x nt tiles times `parts` ranges of diagonals (whose digit-pair
 // counts add up to about 1/parts of a tile's pairs each), numbered part
 // after part.  ktail: MMAs of K = 16 that reach data in the last 64-deep
-// k-block (1..4; single-CTA kernel).  Lives in global memory, 64-byte
+// k-block (1..4).  stack: stacked_tiles (pair kernel).  Lives in global memory, 64-byte
 // aligned.
 struct alignas(64) GroupedProblem {
   unsigned char tmA[128];  // CUtensorMap, A planes, box 64 x 128
   unsigned char tmB[128];  // CUtensorMap, B planes, box 64 x tn (pairs: 64 x 128)
   unsigned char tmC[128];  // CUtensorMap, int32 output chunk planes, box 32 x 32
-  int s, D, Mp, Np, KB, unit_begin, tn, mt, nt, ktail, parts;
+  int s, D, Mp, Np, KB, unit_begin, tn, mt, nt, ktail, parts, stack;
 };
+// Tile shape of the pair kernel that pads an m x n problem least: 0 256 x 256,
+// 1 256 x 128, 2 128 x 256 (two diagonals in one accumulator).
+int stacked_tiles(int s, int D, int m, int n, int KB);
 int encode_plane_map(void *map128, const void *base, int Kp, long long rows_total, int box_rows);
 int encode_out_map(void *map128, const void *base, int Np, long long rows_total);
 // The batched plan's entries in the tuning cache (plan.cu), under the

@@ -1,5 +1,6 @@
 """The BF16 form on problems of few tiles: chunks cut so that every CTA gets
-a share, narrow tiles for up to 128 rows or columns.  The same bits from the
+a share, narrow tiles for up to 128 rows or columns, two diagonals in one
+accumulator where that pads less.  The same bits from the
 automatic choice, the CTA-pair, the single-CTA and the mma.sync engine."""
 import pytest
 
@@ -11,7 +12,11 @@ from conftest import pkg
     (2, 1, 1, 1), (2, 64, 64, 64), (4, 128, 128, 65), (4, 129, 128, 300), (4, 128, 129, 1000),
     (4, 256, 256, 256), (4, 257, 500, 640), (8, 100, 1000, 130), (8, 1000, 100, 77),
     (16, 130, 130, 129), (2, 16001, 96, 100), (4, 96, 3000, 600), (2, 60, 60, 20000),
-    (4, 512, 512, 200), (8, 700, 300, 900)])
+    (4, 512, 512, 200), (8, 700, 300, 900),
+    # many tiles of 128 rows or columns: two diagonals per accumulator (even
+    # and odd digit counts, k ending inside a block)
+    (2, 100, 33000, 130), (2, 20000, 300, 70), (8, 20000, 100, 40), (8, 128, 25000, 33),
+    (4, 9000, 384, 200)])
 def test_few_tiles_same_bits(p, m, n, k):
     import torch
     api = pkg("api")
