@@ -44,8 +44,8 @@ using mdgi::SCALE_THREADS;
 // One range: the exponents, at once.  More: maxima by atomics into bits (rows
 // then columns), and exps_kernel after.  Bound by reading A and B once; on
 // small problems one launch instead of two clears, two maxima and two
-// exponent launches (dd 64^3 56 -> 6 us, qd 256^3 64 -> 11 us, qd 8192^3 1.06
-// -> 1.10 ms, 3.9 TB/s).
+// exponent launches (dd 64^3 56 -> 6 us, qd 256^3 64 -> 8 us, qd 8192^3 1.06
+// -> 0.81 ms, 5.3 TB/s).
 __global__ void __launch_bounds__(SCALE_THREADS)
     scale_kernel(int P, int m, int n, int k, const double *__restrict__ A, int lda,
                  const double *__restrict__ B, int ldb, int col_blocks, int cuts,
