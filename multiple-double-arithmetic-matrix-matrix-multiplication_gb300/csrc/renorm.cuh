@@ -168,7 +168,7 @@ __device__ __forceinline__ void add_at(long long &val, long long &up, long long 
 
 // One thread: row r, columns c0 .. c0 + V - 1 (c0 < n) of one problem.
 // planes: chunk planes in all.  The sums of a pass are loaded together, the
-// first two chunks of each of its eight diagonals, so that the DRAM latency
+// first chunks of each of its eight diagonals, so that the DRAM latency
 // is paid once per eight to sixteen loads; in the cross form all D squares go
 // to shared memory first, where the thread turns its own columns into prefix
 // sums.
@@ -183,6 +183,9 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
   using Vec = typename I::T;
   constexpr int T = RENORM_THREADS;
   constexpr bool CROSS = CHUNKS == kCrossChunks;
+  // chunks of a diagonal loaded ahead; four for small outputs (one column),
+  // whose diagonals are cut into more chunks for the GEMM's sake
+  constexpr int kAhead = CHUNKS == kTableChunks && V == 1 ? 4 : 2;
   const int dwords = (D + 7) / 8;
   // word i of column v at W[(i * V + v) * T]; Q_i at Q[i * T]
   uint64_t *W = reinterpret_cast<uint64_t *>(smem) + threadIdx.x;
@@ -221,7 +224,7 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
   int q = planes;  // the chunk planes of the diagonals above the current one start here
 #pragma unroll 1
   for (int wi = 0; wi < dwords; ++wi) {
-    Vec x0[8], x1[8];
+    Vec x0[8], x1[8], x2[kAhead > 2 ? 8 : 1], x3[kAhead > 2 ? 8 : 1];
     int first[8], nc[8];
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
@@ -232,6 +235,12 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
       if (nc[b] > 0) x0[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)q * plane_c));
       if (nc[b] > 1)
         x1[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(q + 1) * plane_c));
+      if constexpr (kAhead > 2) {
+        if (nc[b] > 2)
+          x2[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(q + 2) * plane_c));
+        if (nc[b] > 3)
+          x3[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(q + 3) * plane_c));
+      }
     }
     uint64_t word[V];
 #pragma unroll
@@ -288,18 +297,22 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
             }
           }
         } else {
-          // at most 2^31 2^24 each: the first two chunks of four diagonals
-          // stay below 2^58
+          // at most 2^31 2^24 each: the first four chunks of four diagonals
+          // stay below 2^59
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             val[v] += I::get(x0[b], v) * unit;
             if (nc[b] > 1) val[v] += I::get(x1[b], v) * unit;
+            if constexpr (kAhead > 2) {
+              if (nc[b] > 2) val[v] += I::get(x2[b], v) * unit;
+              if (nc[b] > 3) val[v] += I::get(x3[b], v) * unit;
+            }
           }
-          if (nc[b] > 2) {
+          if (nc[b] > kAhead) {
             long long rest[V];
 #pragma unroll
             for (int v = 0; v < V; ++v) rest[v] = 0;
-            for (int c = 2; c < nc[b]; ++c) {
+            for (int c = kAhead; c < nc[b]; ++c) {
               const Vec x =
                   __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(first[b] + c) * plane_c));
 #pragma unroll
