@@ -31,12 +31,13 @@
 #include "batched_table.cuh"
 
 struct mdg_batch_s {
-  int count = 0, total_units = 0;
+  int count = 0, workers = 0;
   int scale_units = 0, digit_units = 0, renorm_units = 0;
   int max_d = 1;  // most digits (and diagonals) of any problem
   int tiles_policy = MDG_BATCH_TILES_256, split = 1;
   mdgi::BatchProblem *dprobs = nullptr;
   mdgi::GroupedProblem *dgroups = nullptr;
+  int *deal = nullptr;  // starts of the workers' lists, then the lists
   int *exps = nullptr;  // E of all problems then F
   std::vector<mdgi::BatchProblem> hprobs;  // host copy of the table
 };
@@ -66,8 +67,8 @@ int tile_width(int policy, int n) {
 // than once per digit pair.
 constexpr int kSplitUnitsPerWorker = 16;
 
-// The grouped GEMM's table for a tile policy and split mode: B tensor maps
-// with the policy's box, units dealt heaviest first.
+// The grouped GEMM's table for a tile policy and split mode: tensor maps,
+// tiles, parts, and the numbers of each problem's units.
 int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, int workers,
                   std::vector<mdgi::GroupedProblem> *hg, int *total_units) {
   hg->clear();
@@ -106,19 +107,6 @@ int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, in
     for (mdgi::GroupedProblem &g : *hg)
       g.parts = (int)std::min<long long>(g.stack ? (g.D + 1) / 2 : g.D, std::max(1LL, (tile_work(g) + target - 1) / target));
   }
-  // The grouped kernel deals units to CTAs round-robin in table order.
-  // Heaviest units first (a quad-double tile carries ~4x the work of a
-  // double-double one, an octo-double tile ~15x), so that the deal
-  // approximates longest-processing-time-first and the CTAs finish
-  // together; a problem's units stay consecutive.  Only the order changes;
-  // each unit still writes its own problem's chunk planes.
-  auto unit_work = [&](const mdgi::GroupedProblem &g) {
-    return (tile_work(g) + g.parts - 1) / g.parts;
-  };
-  std::stable_sort(hg->begin(), hg->end(),
-                   [&](const mdgi::GroupedProblem &a, const mdgi::GroupedProblem &b) {
-                     return unit_work(a) > unit_work(b);
-                   });
   long long u = 0;
   for (mdgi::GroupedProblem &g : *hg) {
     g.unit_begin = (int)u;
@@ -129,8 +117,10 @@ int grouped_table(const std::vector<BatchProblem> &hp, int policy, int split, in
   return MDG_SUCCESS;
 }
 
+constexpr int kMaxWorkers = 1024;
+
 struct Layout {
-  size_t off_probs, off_groups, off_exps, total;
+  size_t off_probs, off_groups, off_deal, off_exps, total;
   std::vector<size_t> off_dA, off_dB, off_chunks;
 };
 
@@ -145,6 +135,13 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
   };
   L->off_probs = take(sizeof(BatchProblem) * count);
   L->off_groups = take(sizeof(mdgi::GroupedProblem) * count);
+  // the most units a policy can make of the problems
+  long long units = 0;
+  for (int i = 0; i < count; ++i)
+    units += (long long)mdgi::ceil_div(problems[i].m, 128) * mdgi::ceil_div(problems[i].n, 128) *
+             mdg_default_slices(problems[i].p);
+  if (units > (1LL << 30)) return MDG_ERROR_INVALID_SIZE;
+  L->off_deal = take(sizeof(int) * ((size_t)kMaxWorkers + 1 + units));
   int rows = 0, cols = 0;
   for (int i = 0; i < count; ++i) {
     rows += std::max(problems[i].m, 1);
@@ -257,14 +254,20 @@ int apply_tiles(mdg_batch_s *h, int policy, int split, cudaStream_t st) {
   int dev = 0, sms = 0;
   MDG_TRY_CUDA(cudaGetDevice(&dev));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int all = std::min(policy == MDG_BATCH_TILES_PAIR ? sms / 2 : sms, kMaxWorkers);
   std::vector<mdgi::GroupedProblem> hg;
+  std::vector<int> starts, order;
   int units = 0;
-  MDG_TRY(grouped_table(h->hprobs, policy, split,
-                        policy == MDG_BATCH_TILES_PAIR ? sms / 2 : sms, &hg, &units));
+  MDG_TRY(grouped_table(h->hprobs, policy, split, all, &hg, &units));
+  const int workers = std::min(units, all);
+  MDG_TRY(mdgi::deal_units(hg, workers, &starts, &order));
+  starts.insert(starts.end(), order.begin(), order.end());
+  MDG_TRY_CUDA(cudaMemcpyAsync(h->deal, starts.data(), sizeof(int) * starts.size(),
+                               cudaMemcpyHostToDevice, st));
   MDG_TRY_CUDA(cudaMemcpyAsync(h->dgroups, hg.data(), sizeof(mdgi::GroupedProblem) * h->count,
                                cudaMemcpyHostToDevice, st));
   MDG_TRY_CUDA(cudaStreamSynchronize(st));
-  h->total_units = units;
+  h->workers = workers;
   h->tiles_policy = policy;
   h->split = split;
   return MDG_SUCCESS;
@@ -301,6 +304,7 @@ int mdg_batch_create(const mdg_problem *problems, int count, void *workspace,
   }
   h->dprobs = reinterpret_cast<BatchProblem *>(ws + L.off_probs);
   h->dgroups = reinterpret_cast<mdgi::GroupedProblem *>(ws + L.off_groups);
+  h->deal = reinterpret_cast<int *>(ws + L.off_deal);
   h->exps = reinterpret_cast<int *>(ws + L.off_exps);
   cudaStream_t s = mdgi::as_stream(stream);
   // zero digit planes: the digit kernel writes only the valid rows and
@@ -340,7 +344,8 @@ int mdg_batch_run(mdg_batch_s *h, void *stream) {
   cudaStream_t st = mdgi::as_stream(stream);
   MDG_TRY(mdgi::launch_batch_scale(h->dprobs, h->count, h->scale_units, h->exps, st));
   MDG_TRY(mdgi::launch_batch_digits(h->dprobs, h->count, h->digit_units, h->max_d, h->exps, st));
-  MDG_TRY(mdgi::launch_diag_gemm_grouped(h->dgroups, h->count, h->total_units,
+  MDG_TRY(mdgi::launch_diag_gemm_grouped(h->dgroups, h->count, h->workers, h->deal,
+                                         h->deal + h->workers + 1,
                                          h->tiles_policy == MDG_BATCH_TILES_PAIR, st));
   MDG_TRY(mdgi::launch_batch_renorm(h->dprobs, h->count, h->renorm_units, h->max_d, h->exps, st));
   return MDG_SUCCESS;

@@ -26,6 +26,10 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <functional>
+#include <queue>
+#include <utility>
+#include <vector>
 
 #include "common.cuh"
 #include "cross_sums.cuh"
@@ -278,7 +282,7 @@ enum { kStackNone = 0, kStackN = 1, kStackM = 2 };
 // pairs of diagonals from the top down, an odd first one with d = -1.
 struct DigitRuns {
   int s, D, KB, cs, stack, d, c, chunk, left;
-  __device__ bool next(Run &r) {
+  __host__ __device__ bool next(Run &r) {
     if (left <= 0 || d >= D) return false;
     if (stack) {
       r = stack == kStackN ? Run{0, 1, d, -1, 0, (d + 2) * KB, d, 0}
@@ -320,7 +324,7 @@ struct DigitRuns {
 // Part `part` of a tile's runs: run `part` itself where there are as many
 // parts as runs, else the runs that start in the part's 1/parts of the
 // tile's k-steps (none when parts exceeds what the runs allow).
-__device__ __forceinline__ DigitRuns part_runs(int s, int D, int KB, int cs, int stack, int part,
+__host__ __device__ __forceinline__ DigitRuns part_runs(int s, int D, int KB, int cs, int stack, int part,
                                                int parts) {
   DigitRuns all{s, D, KB, cs, stack, stack ? -(D & 1) : 0, 0, 0, 1 << 30};
   if (parts == 1) return all;
@@ -360,11 +364,18 @@ struct TileJob {
   DigitRuns runs;
 };
 
+// Workers (CTAs or clusters) take the units of a single problem in turn.
+struct DealtInTurn {
+  __device__ int first(int worker, int) const { return worker; }
+  __device__ int step(int workers) const { return workers; }
+  __device__ int unit(int i) const { return i; }
+};
+
 // A single problem cut into mt x nt tiles of 128 x tn, each into parts.
-struct SingleJobs {
+struct SingleJobs : DealtInTurn {
   const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, cs, tn, mt, nt, parts;
-  __device__ int units() const { return mt * nt * parts; }
+  __device__ int last(int) const { return mt * nt * parts; }
   __device__ TileJob job(int u) const {
     const int tiles = mt * nt, tile = u % tiles;
     return TileJob{tmA, tmB, tmC, Mp, Np, KB, (tile % mt) * TM, (tile / mt) * tn, tn, TK / 16,
@@ -415,7 +426,8 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
   fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  const int tiles = jobs.units();
+  const int worker = blockIdx.x, first = jobs.first(worker, gridDim.x);
+  const int last = jobs.last(worker), step = jobs.step(gridDim.x);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -425,18 +437,18 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
       // per stage: a copy was issued (bit of `issued`), parity of its phase
       // (bit of `last_par`); bit masks so that they stay in registers
       uint32_t issued = 0, last_par = 0;
-      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        TileJob jb = jobs.job(tile);
+      for (int i = first; i < last; i += step) {
+        TileJob jb = jobs.job(jobs.unit(i));
         const int KB = jb.KB;
         Run r;
         while (jb.runs.next(r)) {
           for (int t = r.t0; t < r.t0 + r.steps; ++t) {
-            const int q = t / KB, kb = t - q * KB, i = r.a0 + q, j = r.b0 - q;
+            const int q = t / KB, kb = t - q * KB, pa = r.a0 + q, pb = r.b0 - q;
             if (!mbar_wait(empty(st), ph ^ 1, abort_flag)) goto producer_done;
             mbar_expect_tx(full(st), A_BYTES + jb.tn * TK * 2);
             const uint32_t a_dst = smem_base + st * STAGE_BYTES;
-            tma_load_2d(a_dst, jb.tmA, kb * TK, i * jb.Mp + jb.row, full(st));
-            tma_load_2d(a_dst + A_BYTES, jb.tmB, kb * TK, j * jb.Np + jb.col, full(st));
+            tma_load_2d(a_dst, jb.tmA, kb * TK, pa * jb.Mp + jb.row, full(st));
+            tma_load_2d(a_dst + A_BYTES, jb.tmB, kb * TK, pb * jb.Np + jb.col, full(st));
             last_par = (last_par & ~(1u << st)) | (ph << st);
             issued |= 1u << st;
             if (++st == STAGES) {
@@ -457,8 +469,8 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
       int st = 0, buf = 0;
       uint32_t ph = 0, aph[2] = {0, 0};
       bool any = false;
-      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        TileJob jb = jobs.job(tile);
+      for (int i = first; i < last; i += step) {
+        TileJob jb = jobs.job(jobs.unit(i));
         const uint32_t idesc = (IDESC & ~(0x3Fu << 17)) | ((uint32_t)(jb.tn >> 3) << 17);
         Run r;
         while (jb.runs.next(r)) {
@@ -512,8 +524,8 @@ __device__ __forceinline__ void tc1_body(const Jobs &jobs) {
     for (int j = 0; j < 128; ++j) acc[j] = 0;
     int buf = 0;
     uint32_t aph[2] = {0, 0};
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-      TileJob jb = jobs.job(tile);
+    for (int i = first; i < last; i += step) {
+      TileJob jb = jobs.job(jobs.unit(i));
       // a 128-column tile is drained by the warps of the first column half
       // alone (128 columns each, as for a 256-column tile); the others only
       // release the accumulator
@@ -563,7 +575,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
                         int KB, int cs, int tn, int mt, int nt, int parts) {
-  tc1_body(SingleJobs{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, tn, mt, nt, parts});
+  tc1_body(SingleJobs{{}, &tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, tn, mt, nt, parts});
 }
 
 // Many problems: a table of GroupedProblem in global memory (tensor maps
@@ -580,10 +592,18 @@ __device__ __forceinline__ const mdgi::GroupedProblem &grouped_find(
   return probs[lo];
 }
 
-struct GroupedJobs {
+// Units dealt by the host: worker w takes order[starts[w]] .. .
+struct DealtByHost {
+  const int *starts, *order;
+  __device__ int first(int worker, int) const { return starts[worker]; }
+  __device__ int last(int worker) const { return starts[worker + 1]; }
+  __device__ int step(int) const { return 1; }
+  __device__ int unit(int i) const { return order[i]; }
+};
+
+struct GroupedJobs : DealtByHost {
   const mdgi::GroupedProblem *probs;
-  int count, total;
-  __device__ int units() const { return total; }
+  int count;
   __device__ TileJob job(int u) const {
     const mdgi::GroupedProblem &g = grouped_find(probs, count, u);
     const int lt = u - g.unit_begin, tiles = g.mt * g.nt;
@@ -598,8 +618,8 @@ struct GroupedJobs {
 
 __global__ void __launch_bounds__(THREADS, 1)
     diag_gemm_tc_grouped_kernel(const mdgi::GroupedProblem *__restrict__ probs, int count,
-                                int total) {
-  tc1_body(GroupedJobs{probs, count, total});
+                                const int *__restrict__ starts, const int *__restrict__ order) {
+  tc1_body(GroupedJobs{{starts, order}, probs, count});
 }
 
 // ------------------------------------------------------------------------
@@ -785,11 +805,11 @@ struct CrossJob {
 // of `raster` column blocks, then down the rows, so that the clusters busy at
 // the same time read few distinct A row blocks and B column blocks and share
 // them in L2 (raster = 1 walks each column block top to bottom).
-struct PairSingle {
+struct PairSingle : DealtInTurn {
   const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, cs, stack, ktail, mt, nt;
   int parts, raster;
-  __device__ int units() const { return mt * nt * parts; }
+  __device__ int last(int) const { return mt * nt * parts; }
   __device__ PairJob job(int u) const {
     const int tiles = mt * nt, tile = u % tiles, part = u / tiles;
     const int strip = tile / (mt * raster);
@@ -806,10 +826,9 @@ struct PairSingle {
 // Many problems (GroupedProblem table in global memory, tensor maps with
 // 128-row boxes for A and B, Mp a multiple of 256): units are 256 x 256
 // tiles times diagonal ranges, numbered as for the single-CTA kernel.
-struct PairGrouped {
+struct PairGrouped : DealtByHost {
   const mdgi::GroupedProblem *probs;
-  int count, total;
-  __device__ int units() const { return total; }
+  int count;
   __device__ PairJob job(int u) const {
     const mdgi::GroupedProblem &g = grouped_find(probs, count, u);
     const int lt = u - g.unit_begin, tiles = g.mt * g.nt;
@@ -826,12 +845,12 @@ struct PairGrouped {
 // A single problem over digit and sum planes: units are tiles, or parts of
 // tiles whose lists hold about 1/parts of its products each (cut between
 // output planes), in the order of PairSingle's.
-struct PairCross {
+struct PairCross : DealtInTurn {
   const CUtensorMap *tmA, *tmB, *tmC;
   int D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB;
   int parts, raster;
   const unsigned *norm_a, *norm_b;
-  __device__ int units() const { return (Mp / 256) * (Np / TN2) * parts; }
+  __device__ int last(int) const { return (Mp / 256) * (Np / TN2) * parts; }
   // Flush groups per sum plane.  |sum over a group| <= |a| |b| (Cauchy and
   // Schwarz; every partial sum too) with |a|^2 <= 2 *norm_a, |b|^2 <= 2
   // *norm_b over a whole group (two windows), <= *norm_a, *norm_b over half
@@ -922,8 +941,8 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
   fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  const int units = jobs.units();
   const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
+  const int first = jobs.first(cid, ncl), last = jobs.last(cid), step = jobs.step(ncl);
   const bool pacer = leader && pace > 0 && ncl <= PACE_SLOTS;
   if (warp == 0) {
     if (lane == 0) {
@@ -938,8 +957,8 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       // no_loads (self-test of the bounded waits): issue no copy, so the
       // MMA thread's wait for data runs out, it raises the abort flag and
       // every role leaves with nothing in flight
-      for (int u = no_loads ? units : cid; u < units; u += ncl) {
-        auto jb = jobs.job(u);
+      for (int n = no_loads ? last : first; n < last; n += step) {
+        auto jb = jobs.job(jobs.unit(n));
         const int KB = jb.KB;
         // the odd CTA: the next 128 rows and columns, or the next plane
         const int next_a = jb.stack == kStackM ? (int)rank : 0;
@@ -989,8 +1008,8 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
       int st = 0, buf = 0;
       uint32_t ph = 0, aph[2] = {0, 0};
       bool any = false;
-      for (int u = cid; u < units; u += ncl) {
-        auto jb = jobs.job(u);
+      for (int n = first; n < last; n += step) {
+        auto jb = jobs.job(jobs.unit(n));
         Run r;
         while (jb.runs.next(r)) {
           int kb = r.t0 % jb.KB;
@@ -1077,8 +1096,8 @@ __device__ __forceinline__ void tc2_body(const Jobs &jobs, int pace, uint32_t ep
     int buf = 0;
     uint32_t aph[2] = {0, 0};
     const uint32_t accempty0[2] = {map_to_rank0(accempty(0)), map_to_rank0(accempty(1))};
-    for (int u = cid; u < units; u += ncl) {
-      auto jb = jobs.job(u);
+    for (int n = first; n < last; n += step) {
+      auto jb = jobs.job(jobs.unit(n));
       const int next = jb.stack == kStackM ? (int)rank : jb.stack == kStackN ? h : 0;
       const int row = jb.row0 + (jb.stack == kStackM ? 0 : (int)rank * TM) + 32 * q;
       const int col = jb.col0 + (jb.stack == kStackN ? 0 : 128 * h);
@@ -1124,7 +1143,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                          const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
                          int KB, int cs, int stack, int ktail, int mt, int nt, int parts,
                          int raster, int pace, uint32_t epoch, int no_loads) {
-  tc2_body(PairSingle{&tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
+  tc2_body(PairSingle{{}, &tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
            pace, epoch, no_loads);
 }
 
@@ -1143,7 +1162,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                            int raster, const unsigned *__restrict__ norm_a,
                            const unsigned *__restrict__ norm_b, int pace, uint32_t epoch,
                            int no_loads) {
-  tc2_body(PairCross{&tmA, &tmB, &tmC, D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB, parts, raster,
+  tc2_body(PairCross{{}, &tmA, &tmB, &tmC, D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB, parts, raster,
                      norm_a, norm_b},
            pace, epoch, no_loads);
 }
@@ -1152,8 +1171,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
 // on different problems).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
     diag_gemm_tc2_grouped_kernel(const mdgi::GroupedProblem *__restrict__ probs, int count,
-                                 int total) {
-  tc2_body(PairGrouped{probs, count, total}, 0, 0, 0);
+                                 const int *__restrict__ starts, const int *__restrict__ order) {
+  tc2_body(PairGrouped{{starts, order}, probs, count}, 0, 0, 0);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -1369,25 +1388,62 @@ int encode_out_map(void *map128, const void *base, int Np, long long rows_total)
   return make_out_map(reinterpret_cast<CUtensorMap *>(map128), base, Np, rows_total);
 }
 
-int launch_diag_gemm_grouped(const GroupedProblem *dev_probs, int count, int total_units,
-                             int pair, cudaStream_t st) {
-  if (total_units == 0) return MDG_SUCCESS;
-  int dev = 0, sms = 0;
-  MDG_TRY_CUDA(cudaGetDevice(&dev));
-  MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+// The units of a table (numbered as the kernels number them) over the
+// workers: the dearest first, each to the worker with the least so far.  A
+// unit's cost in k-steps: its own, about 6 per run for the drain and the
+// store, about 10 to fill and empty the pipeline.  Dealt in turn, one worker's
+// share could be a third above the mean (64 mixed problems of 32 .. 512: 2.67
+// -> 2.40 ms a call).
+int deal_units(const std::vector<GroupedProblem> &probs, int workers, std::vector<int> *starts,
+               std::vector<int> *order) {
+  struct Unit {
+    long long cost;
+    int id;
+  };
+  std::vector<Unit> units;
+  for (const GroupedProblem &g : probs)
+    for (int part = 0; part < g.parts; ++part) {
+      DigitRuns runs = part_runs(g.s, g.D, g.KB, CHUNK_STEPS, g.stack, part, g.parts);
+      long long cost = 10;
+      for (Run r; runs.next(r);) cost += r.steps + 6;
+      for (int tile = 0; tile < g.mt * g.nt; ++tile)
+        units.push_back(Unit{cost * (g.tn == 128 && !g.stack ? 2 : 4),
+                             g.unit_begin + part * g.mt * g.nt + tile});
+    }
+  std::stable_sort(units.begin(), units.end(),
+                   [](const Unit &a, const Unit &b) { return a.cost > b.cost; });
+  typedef std::pair<long long, int> Load;
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+  for (int w = 0; w < workers; ++w) least.push(Load(0, w));
+  std::vector<std::vector<int>> of(workers);
+  for (const Unit &u : units) {
+    const Load l = least.top();
+    least.pop();
+    of[l.second].push_back(u.id);
+    least.push(Load(l.first + u.cost, l.second));
+  }
+  starts->assign(1, 0);
+  order->clear();
+  for (const auto &list : of) {
+    order->insert(order->end(), list.begin(), list.end());
+    starts->push_back((int)order->size());
+  }
+  return MDG_SUCCESS;
+}
+
+int launch_diag_gemm_grouped(const GroupedProblem *dev_probs, int count, int workers,
+                             const int *dev_starts, const int *dev_order, int pair,
+                             cudaStream_t st) {
   if (pair) {
     MDG_TRY_CUDA(cudaFuncSetAttribute(diag_gemm_tc2_grouped_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
-    const int ncl = sms / 2;
-    const int clusters = total_units < ncl ? total_units : ncl;
-    diag_gemm_tc2_grouped_kernel<<<2 * clusters, THREADS2, SMEM2_BYTES, st>>>(dev_probs, count,
-                                                                            total_units);
+    diag_gemm_tc2_grouped_kernel<<<2 * workers, THREADS2, SMEM2_BYTES, st>>>(
+        dev_probs, count, dev_starts, dev_order);
   } else {
     MDG_TRY_CUDA(cudaFuncSetAttribute(diag_gemm_tc_grouped_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    const int grid = total_units < sms ? total_units : sms;
-    diag_gemm_tc_grouped_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(dev_probs, count,
-                                                                   total_units);
+    diag_gemm_tc_grouped_kernel<<<workers, THREADS, SMEM_BYTES, st>>>(dev_probs, count, dev_starts,
+                                                                     dev_order);
   }
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;

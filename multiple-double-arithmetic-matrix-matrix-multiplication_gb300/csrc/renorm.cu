@@ -17,9 +17,12 @@ using mdgi::RENORM_THREADS;
 constexpr long long kTwoColumnEntries = 1 << 19;
 constexpr int kTwoColumnDiagonals = 32;
 
-// Threads run over the rows' groups of V columns, row after row.
+// Threads run over the rows' groups of V columns, row after row.  (Blocks per
+// SM: with two columns the registers otherwise leave 5, and the kernel waits
+// for its loads: dd 16001 x 96 60 -> 48 us with 7, qd 8192 x 8192, cross form,
+// 6.97 -> 6.30 ms with 6, 64 mixed problems 375 -> 325 us with 7.)
 template <int V>
-__global__ void __launch_bounds__(RENORM_THREADS)
+__global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 7 : 1)
     renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::ChunkCounts counts,
                   int m, int n, const int *__restrict__ chunks, long long plane_c, int ldcd,
                   const int *__restrict__ E, const int *__restrict__ F, double *__restrict__ C,
@@ -34,7 +37,7 @@ __global__ void __launch_bounds__(RENORM_THREADS)
 }
 
 template <int V>
-__global__ void __launch_bounds__(RENORM_THREADS)
+__global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 6 : 1)
     cross_renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::ChunkCounts counts,
                         int m, int n, const int *__restrict__ out, long long plane_c, int ldcd,
                         const int *__restrict__ E, const int *__restrict__ F,
@@ -49,7 +52,7 @@ __global__ void __launch_bounds__(RENORM_THREADS)
 }
 
 // Every problem of a batch: block x belongs to the problem whose units hold x.
-__global__ void __launch_bounds__(RENORM_THREADS)
+__global__ void __launch_bounds__(RENORM_THREADS, 7)
     batch_renorm_kernel(const mdgi::BatchProblem *__restrict__ pr, int count,
                         const int *__restrict__ exps) {
   extern __shared__ uint4 smem[];

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <string>
+#include <vector>
 
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -133,9 +134,14 @@ int encode_out_map(void *map128, const void *base, int Np, long long rows_total)
 // policy), and a new record.
 void tune_lookup_batch(const std::string &key, int *policy, int *split);
 void tune_record_batch(const std::string &key, int policy, int split, double ms);
+// The units of the table over the workers (CTAs, or CTA pairs): worker w takes
+// order[starts[w]] .. order[starts[w + 1] - 1].
+int deal_units(const std::vector<GroupedProblem> &probs, int workers, std::vector<int> *starts,
+               std::vector<int> *order);
 // pair: the CTA-pair kernel (Mp of every problem a multiple of 256).
-int launch_diag_gemm_grouped(const GroupedProblem *dev_probs, int count, int total_units,
-                             int pair, cudaStream_t st);
+int launch_diag_gemm_grouped(const GroupedProblem *dev_probs, int count, int workers,
+                             const int *dev_starts, const int *dev_order, int pair,
+                             cudaStream_t st);
 
 // Waits for the device; MDG_ERROR_TIMEOUT if a bounded wait of the tcgen05
 // engine gave up since the last call (the flag is then cleared).
