@@ -190,6 +190,7 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
       b.dB = reinterpret_cast<__nv_bfloat16 *>(ws + L->off_dB[i]);
       b.chunks = reinterpret_cast<int *>(ws + L->off_chunks[i]);
       b.planes = nch;
+      b.top = mdgi::renorm_top(D, mdgi::diag_chunks(D - 1, s, Kp / 64));
       b.wide = reinterpret_cast<uintptr_t>(q.C) % 16 == 0;
       b.plane_a = (long long)Mp * Kp;
       b.plane_b = (long long)Np * Kp;

@@ -23,7 +23,7 @@ struct BatchProblem {
   int offE, offF;  // exponents of A's rows at offE, of B's columns at offF
   __nv_bfloat16 *dA, *dB;
   int *chunks;
-  int planes, wide;  // chunk planes in all; C is 16-byte aligned
+  int planes, top, wide;  // chunk planes in all; renorm_top; C is 16-byte aligned
   long long plane_a, plane_b, plane_c;
   int scale_begin, scale_b_off;  // first scale unit; units of A's rows
   int dig_begin, dig_b_off;      // first digit unit; units of A's digit rows

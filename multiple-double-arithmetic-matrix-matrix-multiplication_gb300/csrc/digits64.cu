@@ -153,13 +153,13 @@ __global__ void __launch_bounds__(128)
 
 // C[r][c] = RN_P(W * 2^(E[r] + F[c] - 2 (DB - 1) - DB (D - 1))), W built
 // from the top diagonal down: W = W 2^DB + C_d.
-// W is built in registers and rounded from shared memory (emit_limbs_shared).
+// W is built in registers and rounded from shared memory (emit_limbs).
 template <int NW>
 __global__ void __launch_bounds__(128)
     renorm64_kernel(int P, int D, int m, int n, const long long *__restrict__ Cd,
                     const int *__restrict__ E, const int *__restrict__ F, double *__restrict__ C,
                     int ldc, bool wide) {
-  __shared__ uint64_t words[(NW + 2) * 128];
+  __shared__ uint32_t pieces[(2 * NW + 2) * 128];
   const int r = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
   if (c >= n || r >= m) return;
   uint64_t w[NW];
@@ -173,17 +173,17 @@ __global__ void __launch_bounds__(128)
     mdgi::wide_add_shifted<NW>(w, src[(size_t)d * m * n], 0);
   }
   const int scale = E[r] + F[c] - 2 * (DB - 1) - DB * (D - 1);
-  uint64_t *out = words + threadIdx.x;
+  uint32_t *out = pieces + threadIdx.x;
   int lsb = 64 * NW;
 #pragma unroll
   for (int i = NW - 1; i >= 0; --i) {
-    out[i * 128] = w[i];
+    out[2 * i * 128] = (uint32_t)w[i];
+    out[(2 * i + 1) * 128] = (uint32_t)(w[i] >> 32);
     if (w[i]) lsb = 64 * i + __ffsll((long long)w[i]) - 1;
   }
   const uint64_t sign = (uint64_t)((int64_t)w[NW - 1] >> 63);
-  out[NW * 128] = out[(NW + 1) * 128] = sign;
-  mdgi::emit_limbs_shared(P, out, 128, 64 * NW, lsb, sign, scale, C + ((size_t)r * ldc + c) * P,
-                          wide);
+  out[2 * NW * 128] = out[(2 * NW + 1) * 128] = (uint32_t)sign;
+  mdgi::emit_limbs<128>(P, out, 64 * NW, lsb, sign, scale, C + ((size_t)r * ldc + c) * P, wide);
 }
 
 template <int NW>

@@ -23,7 +23,7 @@ constexpr int kTwoColumnDiagonals = 32;
 // 6.97 -> 6.30 ms with 6, 64 mixed problems 375 -> 325 us with 7.)
 template <int V>
 __global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 7 : 1)
-    renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::ChunkCounts counts,
+    renorm_kernel(int P, int D, int planes, int top, const __grid_constant__ mdgi::ChunkCounts counts,
                   int m, int n, const int *__restrict__ chunks, long long plane_c, int ldcd,
                   const int *__restrict__ E, const int *__restrict__ F, double *__restrict__ C,
                   int ldc, bool wide) {
@@ -32,13 +32,13 @@ __global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 7 : 1)
   const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
   const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
   if (r >= m) return;
-  mdgi::renorm_columns<V, mdgi::kTableChunks>(P, 0, D, 0, planes, n, &counts, chunks, plane_c, ldcd,
+  mdgi::renorm_columns<V, mdgi::kTableChunks>(P, 0, D, 0, planes, top, n, &counts, chunks, plane_c, ldcd,
                                               E, F, C, ldc, r, c0, wide, smem);
 }
 
 template <int V>
 __global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 6 : 1)
-    cross_renorm_kernel(int P, int D, int planes, const __grid_constant__ mdgi::ChunkCounts counts,
+    cross_renorm_kernel(int P, int D, int planes, int top, const __grid_constant__ mdgi::ChunkCounts counts,
                         int m, int n, const int *__restrict__ out, long long plane_c, int ldcd,
                         const int *__restrict__ E, const int *__restrict__ F,
                         double *__restrict__ C, int ldc, bool wide) {
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 6 : 1)
   const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
   const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
   if (r >= m) return;
-  mdgi::renorm_columns<V, mdgi::kCrossChunks>(P, 0, D, 0, planes, n, &counts, out, plane_c, ldcd, E,
+  mdgi::renorm_columns<V, mdgi::kCrossChunks>(P, 0, D, 0, planes, top, n, &counts, out, plane_c, ldcd, E,
                                               F, C, ldc, r, c0, wide, smem);
 }
 
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(RENORM_THREADS, 7)
   const long long e = (x - b.out_begin) * (long long)RENORM_THREADS + threadIdx.x;
   const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * 2;
   if (r >= b.m) return;
-  mdgi::renorm_columns<2, mdgi::kPlainChunks>(b.p, b.s, b.D, b.Kp / 64, b.planes, b.n, nullptr,
+  mdgi::renorm_columns<2, mdgi::kPlainChunks>(b.p, b.s, b.D, b.Kp / 64, b.planes, b.top, b.n, nullptr,
                                               b.chunks, b.plane_c, b.Np, exps + b.offE,
                                               exps + b.offF, b.C, b.ldc, r, c0, b.wide, smem);
 }
@@ -84,13 +84,18 @@ int launch_direct(int p, int s, int D, int KB, int cs, int m, int n, const int *
                   long long plane_c, int ldcd, const int *E, const int *F, double *C, int ldc,
                   cudaStream_t st) {
   mdgi::ChunkCounts counts{};
-  int planes = 0;
-  for (int d = 0; d < D; ++d) planes += counts.of[d] = mdgi::diag_chunks(d, s, KB, cs);
+  int planes = 0, most = 1;
+  for (int d = 0; d < D; ++d) {
+    const int nc = mdgi::diag_chunks(d, s, KB, cs);
+    counts.of[d] = nc;
+    planes += nc;
+    most = std::max(most, nc);
+  }
   const int smem = mdgi::renorm_smem(D, V, false);
   MDG_TRY_CUDA(cudaFuncSetAttribute(renorm_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     smem));
   renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
-      p, D, planes, counts, m, n, chunks, plane_c, ldcd, E, F, C, ldc, aligned16(C));
+      p, D, planes, mdgi::renorm_top(D, most), counts, m, n, chunks, plane_c, ldcd, E, F, C, ldc, aligned16(C));
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }
@@ -100,12 +105,16 @@ int launch_cross(int p, int D, int KB, int m, int n, const int *out, long long p
                  const int *E, const int *F, double *C, int ldc, cudaStream_t st) {
   mdgi::ChunkCounts counts{};
   counts.pairs_per_chunk = mdgi::cross_pairs_per_chunk(KB);
-  for (int d = 1; d < D; ++d) counts.of[d] = mdgi::cross_chunks(d, counts.pairs_per_chunk);
+  int most = 0;
+  for (int d = 1; d < D; ++d) {
+    counts.of[d] = mdgi::cross_chunks(d, counts.pairs_per_chunk);
+    most = std::max(most, (int)counts.of[d]);
+  }
   const int smem = mdgi::renorm_smem(D, V, true);
   MDG_TRY_CUDA(cudaFuncSetAttribute(cross_renorm_kernel<V>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   cross_renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
-      p, D, mdgi::cross_outputs(D, KB), counts, m, n, out, plane_c, ldcd, E, F, C, ldc,
+      p, D, mdgi::cross_outputs(D, KB), mdgi::renorm_top(D, most + 1), counts, m, n, out, plane_c, ldcd, E, F, C, ldc,
       aligned16(C));
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;

@@ -2,8 +2,8 @@
 // kernels (renorm.cu) and the batched one (batched_stages.cuh).
 //
 // W = sum_d C_d 256^(D-1-d), C_d the sum of diagonal d's chunk planes, is
-// built from the least significant diagonal up, eight diagonals (one 64-bit
-// word) per pass, and rounded to P limbs.  W lives in shared memory and the
+// built from the least significant diagonal up, eight diagonals (two 32-bit
+// pieces) per pass, and rounded to P limbs.  W lives in shared memory and the
 // passes are a loop: with W in registers every word position had to be
 // unrolled, and the code outgrew the instruction cache (registers / shared
 // memory: dd 64 x 64 29 / 8 us, qd 256 x 256 49 / 14 us, dd 16001 x 96 142 /
@@ -11,6 +11,9 @@
 // limb count and the width run-time numbers, so one kernel serves every P
 // and one launch a whole batch (four launches before; 64 mixed problems of
 // 32 .. 512: 3.84 -> 3.42 ms a call).
+// Cutting limbs from 32-bit pieces with funnel shifts, from a bound on W's
+// top bit down, instead of from 64-bit words: qd 1024^2, cross form, 90 -> 83
+// us, od 2048^2 775 -> 693, hd 1024^2 583 -> 553, dd 16001 x 96 48 -> 42 us.
 //
 // In the cross form (cross_sums.cuh) the planes are the squares P_i and the
 // chunks S of products of sums: a chunk holds the pairs i in [i0, i1) of
@@ -40,13 +43,22 @@ struct ChunkCounts {
 // k-steps (a batch), a table, a table of the cross form.
 enum { kPlainChunks = 0, kTableChunks = 1, kCrossChunks = 2 };
 
-// 64-bit words of W per column: the diagonals', the carry out of them, two
-// of sign (windows of emit_limbs_shared).
-__host__ __device__ inline int renorm_words(int D) { return (D + 7) / 8 + 3; }
+// 32-bit pieces of W per column: the diagonals' (eight diagonals make two),
+// the carry out of them (two), two of sign.
+__host__ __device__ inline int renorm_pieces(int D) { return 2 * ((D + 7) / 8) + 4; }
 
 // Shared memory of a block: W, and in the cross form the prefix sums.
 __host__ __device__ inline int renorm_smem(int D, int V, bool cross) {
-  return RENORM_THREADS * V * (8 * renorm_words(D) + (cross ? 4 * (D + 1) : 0));
+  return RENORM_THREADS * V * 4 * (renorm_pieces(D) + (cross ? D + 1 : 0));
+}
+
+// A bit position from which W is all sign: a diagonal is the sum of at most
+// `terms` int32, and the diagonals' weights add up to less than 256/255 of the
+// first one's.
+inline int renorm_top(int D, int terms) {
+  int bits = 0;
+  while ((1 << bits) < terms) ++bits;
+  return 8 * (D - 1) + 33 + bits;
 }
 
 // V adjacent int32.
@@ -65,87 +77,78 @@ struct Ints<2> {
   static __device__ __forceinline__ T put(const int (&x)[2]) { return make_int2(x[0], x[1]); }
 };
 
-// The P limbs of W 2^scale from W's words (word i at w[i * stride]): limb l
-// is the residual R_l = W - (limbs 0..l-1), rounded to nearest-even to 53
-// bits.  W itself is never modified: after a limb rounded at bit sh, the
-// residual is W's bits below sh with every bit from sh up equal to f, where
-// f is all ones if that limb was rounded up and zero otherwise (rounding up
-// leaves a negative remainder, rounding down a non-negative one, and |R|
-// is below 2^sh either way).  So each limb needs: the highest bit of R
-// that differs from f (its magnitude), a 64-bit window of R at that bit,
-// and whether any bit of W lies below the rounding position (the sticky
-// bit, from W's lowest set bit lsb).  The search looks at a 128-bit window
-// of R ending at the current cut h and moves down 64 bits at a time while
-// the window's upper half carries nothing but f.  wide: out is 16-byte
-// aligned and limbs leave in pairs.
-__device__ __forceinline__ void emit_limbs_shared(int P, const uint64_t *w, int stride, int h,
-                                                  int lsb, uint64_t f, int scale, double *out,
-                                                  bool wide) {
+// 64 bits of W (piece i at w[i * STRIDE]) from bit pos.
+template <int STRIDE>
+__device__ __forceinline__ uint64_t bits64(const uint32_t *w, int pos) {
+  const uint32_t *p = w + (pos >> 5) * STRIDE;
+  const int r = pos & 31;
+  const uint32_t a = p[0], b = p[STRIDE], c = p[2 * STRIDE];
+  return (uint64_t)__funnelshift_r(b, c, r) << 32 | __funnelshift_r(a, b, r);
+}
+
+// The P limbs of W 2^scale: limb l is the residual R_l = W - (limbs 0..l-1),
+// rounded to nearest-even to 53 bits.  W itself is never modified: after a
+// limb rounded at bit sh, the residual is W's bits below sh with every bit
+// from sh up equal to f, where f is all ones if that limb was rounded up and
+// zero otherwise (rounding up leaves a negative remainder, rounding down a
+// non-negative one, and |R| is below 2^sh either way).  So each limb needs:
+// the highest bit t of R that differs from f (its magnitude), found 64 bits
+// at a time from the cut h down, mostly at once; the 54 bits from t down,
+// with f above; and whether any bit of W lies below them (the sticky bit,
+// from W's lowest set bit lsb).  Bits of W from h up are f at the start.
+// wide: out is 16-byte aligned and limbs leave in pairs.
+template <int STRIDE>
+__device__ __forceinline__ void emit_limbs(int P, const uint32_t *w, int h, int lsb, uint64_t f,
+                                           int scale, double *out, bool wide) {
   double even = 0.0;
 #pragma unroll 1
   for (int l = 0; l < P; ++l) {
     double val = 0.0;
     if (f != 0 || lsb < h) {  // else R = 0
-      int b0, t;
-      uint64_t lo, hi;
-      for (;;) {  // h drops by 64 per pass
-        b0 = h > 128 ? h - 128 : 0;
-        const uint64_t *p = w + (b0 >> 6) * stride;
-        const int r = b0 & 63;
-        const uint64_t w0 = p[0], w1 = p[stride], w2 = p[2 * stride];
-        lo = r ? ((w0 >> r) | (w1 << (64 - r))) : w0;
-        hi = r ? ((w1 >> r) | (w2 << (64 - r))) : w1;
-        const int cut = h - b0;  // 0..128: window bits from cut up are f
-        if (cut < 64) {
-          const uint64_t keep = cut ? ((1ull << cut) - 1) : 0ull;
-          lo = (lo & keep) | (f & ~keep);
-          hi = f;
-        } else if (cut < 128) {
-          const uint64_t keep = cut > 64 ? ((1ull << (cut - 64)) - 1) : 0ull;
-          hi = (hi & keep) | (f & ~keep);
-        }
-        const uint64_t xh = hi ^ f, xl = lo ^ f;
-        if (xh) {
-          t = b0 + 127 - __clzll((long long)xh);
+      int t;
+      for (;;) {
+        const int b = h > 64 ? h - 64 : 0;
+        uint64_t x = bits64<STRIDE>(w, b) ^ f;
+        if (h < 64) x &= (1ull << h) - 1;
+        if (x) {
+          t = b + 63 - __clzll((long long)x);
           break;
         }
-        if (b0 == 0) {
-          t = xl ? 63 - __clzll((long long)xl) : -1;  // -1: R = -1
+        if (b == 0) {
+          t = -1;  // R = -1
           break;
         }
-        h = b0 + 64;
+        h = b;
       }
-      // rounding position sh; x = bits [sh - 1, sh + 63) of R: the round bit,
-      // then m = floor(R / 2^sh), |m| <= 2^53 (sh = 0: R itself, b0 = 0)
+      // rounding position sh; m = floor(R / 2^sh), |m| <= 2^53
       const int sh = t > 52 ? t - 52 : 0;
-      uint64_t x;
-      if (sh == 0) {
-        x = lo << 1;
+      int64_t m;
+      bool up = false;
+      if (sh > 0) {
+        const uint64_t y = bits64<STRIDE>(w, sh - 1);
+        const int64_t x = (int64_t)((y & ((1ull << 54) - 1)) | f << 54);
+        m = x >> 1;
+        up = (x & 1) && (lsb < sh - 1 || (m & 1));
       } else {
-        const int o = sh - 1 - b0;  // 0..127
-        if (o < 64)
-          x = o ? ((lo >> o) | (hi << (64 - o))) : lo;
-        else
-          x = o > 64 ? ((hi >> (o - 64)) | (f << (128 - o))) : hi;
+        const uint64_t keep = (2ull << t) - 1;  // t = -1: none
+        m = (int64_t)((bits64<STRIDE>(w, 0) & (t < 0 ? 0ull : keep)) | (f & ~(t < 0 ? 0ull : keep)));
       }
-      const int64_t m = (int64_t)x >> 1;
-      const bool up = sh > 0 && (x & 1ull) && (lsb < sh - 1 || (m & 1));
-      const int64_t mr = up ? m + 1 : m;
+      if (up) ++m;
       f = up ? ~0ull : 0ull;
       h = sh;
-      // mr 2^(sh + scale) as a double; with the top bit at 52 (or 53) and a
-      // normal exponent it is assembled from its fields by integer
-      // instructions, otherwise converted and scaled in FP64
-      const bool neg = mr < 0;
-      const uint64_t mm = neg ? (uint64_t)(-mr) : (uint64_t)mr;
-      const bool carry = mm >> 53;
-      const uint64_t frac = carry ? (mm >> 1) : mm;
-      const int be = sh + scale + 52 + (carry ? 1 : 0) + 1023;
-      if ((frac >> 52) == 1 && be >= 1 && be <= 2046)
-        val = __longlong_as_double((long long)(((uint64_t)be << 52) | (frac & ((1ull << 52) - 1))));
-      else
+      // m 2^(sh + scale): with its top bit at 52, or 53 after rounding up,
+      // and a normal exponent the bits are put together as integers (the
+      // leading bit, and a carry into bit 53, add to the exponent field)
+      const bool neg = m < 0;
+      const uint64_t mm = neg ? (uint64_t)(-m) : (uint64_t)m;
+      const int be = sh + scale + 52 + 1023;
+      if (mm >> 52 && be >= 1 && be <= 2045) {
+        const int hi = (int)(mm >> 32) + ((be - 1) << 20);
+        val = __hiloint2double(neg ? hi | (int)0x80000000 : hi, (int)mm);
+      } else {
         val = ldexp((double)mm, sh + scale);
-      if (neg) val = -val;
+        if (neg) val = -val;
+      }
     }
     if (!wide)
       out[l] = val;
@@ -167,13 +170,14 @@ __device__ __forceinline__ void add_at(long long &val, long long &up, long long 
 }
 
 // One thread: row r, columns c0 .. c0 + V - 1 (c0 < n) of one problem.
-// planes: chunk planes in all.  The sums of a pass are loaded together, the
+// planes: chunk planes in all.  top: renorm_top.  The sums of a pass are loaded together, the
 // first chunks of each of its eight diagonals, so that the DRAM latency
 // is paid once per eight to sixteen loads; in the cross form all D squares go
 // to shared memory first, where the thread turns its own columns into prefix
 // sums.
 template <int V, int CHUNKS>
-__device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int planes, int n,
+__device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int planes, int top,
+                                               int n,
                                                const ChunkCounts *counts,
                                                const int *__restrict__ chunks, long long plane_c,
                                                int ldcd, const int *__restrict__ E,
@@ -187,9 +191,9 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
   // whose diagonals are cut into more chunks for the GEMM's sake
   constexpr int kAhead = CHUNKS == kTableChunks && V == 1 ? 4 : 2;
   const int dwords = (D + 7) / 8;
-  // word i of column v at W[(i * V + v) * T]; Q_i at Q[i * T]
-  uint64_t *W = reinterpret_cast<uint64_t *>(smem) + threadIdx.x;
-  Vec *Q = reinterpret_cast<Vec *>(reinterpret_cast<uint64_t *>(smem) + (dwords + 3) * V * T) +
+  // piece i of column v at W[(i * V + v) * T]; Q_i at Q[i * T]
+  uint32_t *W = reinterpret_cast<uint32_t *>(smem) + threadIdx.x;
+  Vec *Q = reinterpret_cast<Vec *>(reinterpret_cast<uint32_t *>(smem) + (2 * dwords + 4) * V * T) +
            threadIdx.x;
   const int *src = chunks + (size_t)r * ldcd + c0;
   const int ppc = CROSS ? counts->pairs_per_chunk : 0;
@@ -242,7 +246,6 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
           x3[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(q + 3) * plane_c));
       }
     }
-    uint64_t word[V];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       long long val[V], up[V];
@@ -325,33 +328,31 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
       }
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        const uint64_t bits = (uint32_t)val[v];
-        word[v] = half ? (word[v] | bits << 32) : bits;
+        const uint32_t bits = (uint32_t)val[v];
+        W[((2 * wi + half) * V + v) * T] = bits;
+        if (bits && lsb[v] == 1 << 20) lsb[v] = 64 * wi + 32 * half + __ffs((int)bits) - 1;
         carry[v] = (val[v] >> 32) + up[v];
       }
-    }
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      W[(wi * V + v) * T] = word[v];
-      if (word[v] && lsb[v] == 1 << 20) lsb[v] = 64 * wi + __ffsll((long long)word[v]) - 1;
     }
   }
   const int scale = E[r] - 14 - 8 * (D - 1);
 #pragma unroll
   for (int v = 0; v < V; ++v) {
-    const uint64_t f = (uint64_t)(carry[v] >> 63);
-    W[(dwords * V + v) * T] = (uint64_t)carry[v];
-    W[((dwords + 1) * V + v) * T] = f;
-    W[((dwords + 2) * V + v) * T] = f;
+    uint32_t *above = W + (2 * dwords * V + v) * T;
+    const uint32_t f = (uint32_t)(carry[v] >> 63);
+    above[0] = (uint32_t)carry[v];
+    above[V * T] = (uint32_t)(carry[v] >> 32);
+    above[2 * V * T] = f;
+    above[3 * V * T] = f;
     if (carry[v] && lsb[v] == 1 << 20) lsb[v] = 64 * dwords + __ffsll(carry[v]) - 1;
   }
 #pragma unroll 1
   for (int v = 0; v < V; ++v) {
     if (c0 + v >= n) break;
     const int low = V == 2 && v ? lsb[V - 1] : lsb[0];
-    const long long top = V == 2 && v ? carry[V - 1] : carry[0];
-    emit_limbs_shared(P, W + v * T, V * T, 64 * (dwords + 1), low, (uint64_t)(top >> 63),
-                      scale + F[c0 + v], C + ((size_t)r * ldc + c0 + v) * P, wide);
+    const long long over = V == 2 && v ? carry[V - 1] : carry[0];
+    emit_limbs<V * T>(P, W + v * T, top, low, (uint64_t)(over >> 63), scale + F[c0 + v],
+                      C + ((size_t)r * ldc + c0 + v) * P, wide);
   }
 }
 
