@@ -240,6 +240,23 @@ static size_t least_workspace_bytes(int form, int p, int m, int n, int k, const 
   return make_slice_plan(p, o.slices, o.diagonals, m, n, k).total;
 }
 
+int slice_gemm(int p, int m, int n, int k, const double *A, int lda, int trans_a, const double *B,
+               int ldb, int trans_b, double *C, int ldc, const mdg_options *opt, void *workspace,
+               size_t workspace_bytes_, void *stream) {
+  Opts o;
+  MDG_TRY(resolve_opts(MDG_FORM_SLICE_BF16, p, opt, &o));
+  // the sum-plane form where it pays, on CTA pairs, in a workspace that
+  // holds it; otherwise the digit pairs
+  const int engine = engine_choice(o.engine);
+  SlicePlan pl = best_slice_plan(p, o.slices, o.diagonals, m, n, k);
+  if ((pl.sums && (engine == 0 || engine == 2)) || workspace_bytes_ < pl.total)
+    pl = make_slice_plan(p, o.slices, o.diagonals, m, n, k);
+  if (!workspace || workspace_bytes_ < pl.total) return MDG_ERROR_WORKSPACE;
+  if (pl.Mp > 65535 || pl.Np > 65535) return MDG_ERROR_NOT_SUPPORTED;
+  return run_slice_gemm(pl, A, lda, B, ldb, C, ldc, workspace, engine, o.parts, o.raster,
+                        as_stream(stream), o.pace, trans_a, trans_b);
+}
+
 }  // namespace mdgi
 
 using namespace mdgi;
@@ -450,18 +467,9 @@ int mdg_gemm(int form, int p, int m, int n, int k, const double *A, int lda, con
     NvtxRange range("mdg plain");
     return launch_plain_gemm(p, m, n, k, A, lda, B, ldb, C, ldc, st);
   }
-  if (form == MDG_FORM_SLICE_BF16) {
-    // the sum-plane form where it pays, on CTA pairs, in a workspace that
-    // holds it; otherwise the digit pairs
-    const int engine = engine_choice(o.engine);
-    SlicePlan pl = best_slice_plan(p, o.slices, o.diagonals, m, n, k);
-    if (pl.sums && (engine == 0 || engine == 2 || workspace_bytes_ < pl.total))
-      pl = make_slice_plan(p, o.slices, o.diagonals, m, n, k);
-    if (!workspace || workspace_bytes_ < pl.total) return MDG_ERROR_WORKSPACE;
-    if (pl.Mp > 65535 || pl.Np > 65535) return MDG_ERROR_NOT_SUPPORTED;
-    return run_slice_gemm(pl, A, lda, B, ldb, C, ldc, workspace, engine, o.parts, o.raster, st,
-                          o.pace);
-  }
+  if (form == MDG_FORM_SLICE_BF16)
+    return slice_gemm(p, m, n, k, A, lda, 0, B, ldb, 0, C, ldc, opt, workspace, workspace_bytes_,
+                      stream);
   const size_t need = workspace_bytes(form, p, m, n, k, o);
   if (!workspace || workspace_bytes_ < need) return MDG_ERROR_WORKSPACE;
   if (form == MDG_FORM_FP64_SPLIT)

@@ -40,36 +40,48 @@ using mdgi::SCALE_ROWS;
 using mdgi::SCALE_THREADS;
 
 // ------------------------------------------------------------ exponents --
-// Column blocks of B, then row blocks of A, each cut into `cuts` ranges of k.
-// One range: the exponents, at once.  More: maxima by atomics into bits (rows
-// then columns), and exps_kernel after.  Bound by reading A and B once; on
-// small problems one launch instead of two clears, two maxima and two
-// exponent launches (dd 64^3 56 -> 6 us, qd 256^3 64 -> 8 us, qd 8192^3 1.06
-// -> 0.81 ms, 5.3 TB/s).
+// One operand of the scale stage: the exponents of `count` rows of X (count x
+// k), or, trans, of `count` columns (k x count).
+struct ScaleSide {
+  const double *X;
+  int ld, trans, count;
+  int *E;
+};
+
+// Blocks of 8 rows or columns of the first side, then of the second, each cut
+// into `cuts` ranges of k.  One range: the exponents, at once.  More: maxima
+// by atomics into bits (first side, then second), and exps_kernel after.  Bound
+// by reading A and B once; on small problems one launch instead of two
+// clears, two maxima and two exponent launches (dd 64^3 56 -> 6 us, qd 256^3
+// 64 -> 8 us, qd 8192^3 1.06 -> 0.81 ms, 5.3 TB/s).
 __global__ void __launch_bounds__(SCALE_THREADS)
-    scale_kernel(int P, int m, int n, int k, const double *__restrict__ A, int lda,
-                 const double *__restrict__ B, int ldb, int col_blocks, int cuts,
-                 int *__restrict__ E, int *__restrict__ F, unsigned long long *bits) {
-  const int blk = blockIdx.x / cuts, cut = blockIdx.x - blk * cuts;
+    scale_kernel(int P, int k, const ScaleSide a, const ScaleSide b, int blocks_a, int cuts,
+                 unsigned long long *bits) {
+  static_assert(SCALE_ROWS == SCALE_COLS, "a block takes as many rows as columns");
+  int blk = blockIdx.x / cuts;
+  const int cut = blockIdx.x - blk * cuts;
   const int k0 = (int)((long long)k * cut / cuts), k1 = (int)((long long)k * (cut + 1) / cuts);
-  if (blk < col_blocks) {
-    const int c = blk * SCALE_COLS + (int)threadIdx.x;
-    const unsigned long long mx = mdgi::col_max(P, B, ldb, blk * SCALE_COLS, n, k0, k1);
-    if (threadIdx.x >= SCALE_COLS || c >= n) return;
-    if (cuts == 1)
-      F[c] = mdgi::scale_exp(__longlong_as_double((long long)mx));
-    else
-      atomicMax(bits + m + c, mx);
+  const bool second = blk >= blocks_a;
+  const ScaleSide &d = second ? b : a;
+  if (second) blk -= blocks_a;
+  int i;  // this thread's row or column, where it holds the maximum
+  unsigned long long mx;
+  bool holds;
+  if (d.trans) {
+    i = blk * SCALE_COLS + (int)threadIdx.x;
+    mx = mdgi::col_max(P, d.X, d.ld, blk * SCALE_COLS, d.count, k0, k1);
+    holds = threadIdx.x < SCALE_COLS && i < d.count;
   } else {
-    const int r = (blk - col_blocks) * SCALE_ROWS + (int)(threadIdx.x >> 5);
-    if (r >= m) return;
-    const unsigned long long mx = mdgi::row_max(P, A, lda, r, k0, k1);
-    if (threadIdx.x & 31) return;
-    if (cuts == 1)
-      E[r] = mdgi::scale_exp(__longlong_as_double((long long)mx));
-    else
-      atomicMax(bits + r, mx);
+    i = blk * SCALE_ROWS + (int)(threadIdx.x >> 5);
+    if (i >= d.count) return;
+    mx = mdgi::row_max(P, d.X, d.ld, i, k0, k1);
+    holds = (threadIdx.x & 31) == 0;
   }
+  if (!holds) return;
+  if (cuts == 1)
+    d.E[i] = mdgi::scale_exp(__longlong_as_double((long long)mx));
+  else
+    atomicMax(bits + (second ? a.count : 0) + i, mx);
 }
 
 __global__ void exps_kernel(int m, int n, const unsigned long long *__restrict__ bits,
@@ -351,22 +363,26 @@ SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k) {
 
 int launch_scale_exponents(int p, int m, int n, int k, const double *A, int lda,
                            const double *B, int ldb, unsigned long long *bits, int *E, int *F,
-                           cudaStream_t st) {
-  if (m <= 0 && n <= 0) return MDG_SUCCESS;
-  const int col_blocks = ceil_div(std::max(n, 0), SCALE_COLS);
-  const long long blocks = (long long)col_blocks + ceil_div(std::max(m, 0), SCALE_ROWS);
+                           cudaStream_t st, int trans_a, int trans_b) {
+  m = std::max(m, 0);
+  n = std::max(n, 0);
+  if (m == 0 && n == 0) return MDG_SUCCESS;
+  // B first: its few columns of a tall problem take longest
+  const ScaleSide b{B, ldb, !trans_b, n, F}, a{A, lda, trans_a, m, E};
+  const int blocks_b = ceil_div(n, SCALE_COLS);
+  const long long blocks = (long long)blocks_b + ceil_div(m, SCALE_ROWS);
   // a thread takes k / 32 entries one after another: ranges of k where that
   // is long and the blocks leave SMs idle (four 256-thread blocks fill one
   // of 152)
-  const int cuts = (int)std::min<long long>(
-      std::max<long long>(1, 608 / std::max<long long>(blocks, 1)), std::max(1, k / 1024));
+  const int cuts = (int)std::min<long long>(std::max<long long>(1, 608 / blocks),
+                                            std::max(1, k / 1024));
   if (cuts > 1)
     MDG_TRY_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned long long) * ((size_t)m + n), st));
-  scale_kernel<<<(unsigned)(blocks * cuts), SCALE_THREADS, 0, st>>>(p, m, n, k, A, lda, B, ldb,
-                                                                    col_blocks, cuts, E, F, bits);
+  scale_kernel<<<(unsigned)(blocks * cuts), SCALE_THREADS, 0, st>>>(p, k, b, a, blocks_b, cuts,
+                                                                    bits);
   MDG_TRY_LAUNCH();
   if (cuts > 1) {
-    exps_kernel<<<ceil_div((long long)m + n, 256), 256, 0, st>>>(m, n, bits, E, F);
+    exps_kernel<<<ceil_div((long long)m + n, 256), 256, 0, st>>>(n, m, bits, F, E);
     MDG_TRY_LAUNCH();
   }
   return MDG_SUCCESS;
@@ -409,14 +425,14 @@ static unsigned long long *plan_bits(const SlicePlan &pl, void *ws) {
 }
 
 static DigitSide side_a(const SlicePlan &pl, int rows, const double *A, int lda, const int *E,
-                        void *planes) {
-  return DigitSide{A, E, reinterpret_cast<__nv_bfloat16 *>(planes), lda, 0, rows, pl.k, pl.Kp,
+                        void *planes, int trans = 0) {
+  return DigitSide{A, E, reinterpret_cast<__nv_bfloat16 *>(planes), lda, trans, rows, pl.k, pl.Kp,
                    pl.Kp, pl.plane_a};
 }
 
 static DigitSide side_b(const SlicePlan &pl, const double *B, int ldb, const int *F,
-                        void *planes) {
-  return DigitSide{B, F, reinterpret_cast<__nv_bfloat16 *>(planes), ldb, 1, pl.n, pl.k, pl.Kp,
+                        void *planes, int trans = 0) {
+  return DigitSide{B, F, reinterpret_cast<__nv_bfloat16 *>(planes), ldb, !trans, pl.n, pl.k, pl.Kp,
                    pl.Kp, pl.plane_b};
 }
 
@@ -521,7 +537,7 @@ int slice_panel(const SlicePlan &pl, int rows, const double *A, int lda, double 
 
 int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *B, int ldb,
                    double *C, int ldc, void *ws, int engine, int parts, int raster,
-                   cudaStream_t st, int pace) {
+                   cudaStream_t st, int pace, int trans_a, int trans_b) {
   char *base = reinterpret_cast<char *>(ws);
   int *E = reinterpret_cast<int *>(base + pl.off_E);
   int *F = reinterpret_cast<int *>(base + pl.off_F);
@@ -533,9 +549,9 @@ int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *
   {
     NvtxRange r("split: scale exponents and digits");
     MDG_TRY(launch_scale_exponents(pl.p, pl.m, pl.n, pl.k, A, lda, B, ldb, plan_bits(pl, ws), E,
-                                   F, st));
-    MDG_TRY(launch_digits(pl.p, pl.s, side_a(pl, pl.m, A, lda, E, dA), side_b(pl, B, ldb, F, dB),
-                          norms, st));
+                                   F, st, trans_a, trans_b));
+    MDG_TRY(launch_digits(pl.p, pl.s, side_a(pl, pl.m, A, lda, E, dA, trans_a),
+                          side_b(pl, B, ldb, F, dB, trans_b), norms, st));
   }
   NvtxRange r2("diagonal GEMM and renormalisation");
   if (pl.sums) {

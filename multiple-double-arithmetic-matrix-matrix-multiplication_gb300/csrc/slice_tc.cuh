@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include "mdgemm.h"
+
 namespace mdgi {
 
 // The diagonal sums are written as int32 "chunk" planes: the products of
@@ -77,11 +79,11 @@ Digits64Plan make_digits64_plan(int p, int s, int D, int m, int n, int k);
 int run_digits64_gemm(const Digits64Plan &pl, const double *A, int lda, const double *B, int ldb,
                       double *C, int ldc, void *ws, cudaStream_t st);
 
-// Scale exponents of A's rows (m of them) and B's columns (n); bits: m + n
-// words of scratch.
+// Scale exponents of op(A)'s rows (m of them) and op(B)'s columns (n); bits:
+// m + n words of scratch.  trans_a: A is k x m; trans_b: B is n x k.
 int launch_scale_exponents(int p, int m, int n, int k, const double *A, int lda,
                            const double *B, int ldb, unsigned long long *bits, int *E, int *F,
-                           cudaStream_t st);
+                           cudaStream_t st, int trans_a = 0, int trans_b = 0);
 // Digit planes of two operands (slice_stages.cuh; rows = 0: none), and zeros
 // into norms[0], norms[1] where given.
 struct DigitSide;
@@ -151,7 +153,14 @@ int tc_device_status();
 // 3 = tcgen05 CTA pairs
 int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *B, int ldb,
                    double *C, int ldc, void *ws, int engine, int parts, int raster,
-                   cudaStream_t st, int pace = 0);
+                   cudaStream_t st, int pace = 0, int trans_a = 0, int trans_b = 0);
+
+// mdg_gemm of the BF16 form on checked arguments, m, n, k > 0, with operands
+// that may be given transposed (A k x m, B n x k): the digit planes are
+// formed from either layout.
+int slice_gemm(int p, int m, int n, int k, const double *A, int lda, int trans_a, const double *B,
+               int ldb, int trans_b, double *C, int ldc, const mdg_options *opt, void *workspace,
+               size_t workspace_bytes, void *stream);
 
 // run_slice_gemm in two parts, for callers that split A into row panels
 // (the pipelined host path): slice_prepare_b computes the column exponents

@@ -14,9 +14,8 @@ from conftest import pkg
 
 def test_workspace_holds_the_pairs_and_the_rule_is_on_sizes():
     api, L = pkg("api"), pkg("_lib").lib()
-    for p, m, n, k, sums in [(4, 1024, 1024, 1024, True), (4, 64, 64, 64, False),
-                             (4, 1024, 1024, 256, False), (2, 16001, 96, 3001, False),
-                             (8, 2048, 2048, 2048, True), (16, 1024, 1024, 512, True),
+    for p, m, n, k, sums in [(4, 1024, 1024, 1024, True), (2, 16001, 96, 3001, False),
+                             (4, 4096, 4096, 256, False), (8, 2048, 2048, 2048, True), (16, 1024, 1024, 512, True),
                              (4, 1024, 1024, 70000, False), (4, 65536, 65536, 8192, False)]:
         full = api.workspace_size("slice_bf16", p, m, n, k)
         least = L.mdg_gemm_least_workspace_size(2, p, m, n, k, None)
