@@ -175,8 +175,10 @@ int plan_batch(const mdg_problem *problems, int count, Layout *L, mdg_batch_s *h
     // digits: valid rows and k-positions only (the padding is cleared once,
     // by mdg_batch_create)
     const long long kpairs = (q.k + 1) / 2;
-    const long long digit_a = mdgi::ceil_div(q.m * kpairs, mdgi::DIGIT_THREADS);
-    const long long digit_b = mdgi::ceil_div(q.n * kpairs, mdgi::DIGIT_THREADS);
+    const long long digit_a = 
+        mdgi::ceil_div(mdgi::digit_threads(q.p, 0, q.m, (int)kpairs), mdgi::DIGIT_THREADS);
+    const long long digit_b = 
+        mdgi::ceil_div(mdgi::digit_threads(q.p, 1, q.n, (int)kpairs), mdgi::DIGIT_THREADS);
     if (digit_u + digit_a + digit_b > (1LL << 30)) return MDG_ERROR_INVALID_SIZE;
     const long long out_u = mdgi::ceil_div((long long)q.m * ((q.n + 1) / 2), mdgi::RENORM_THREADS);
     if (renorm_u + out_u > (1LL << 30)) return MDG_ERROR_INVALID_SIZE;

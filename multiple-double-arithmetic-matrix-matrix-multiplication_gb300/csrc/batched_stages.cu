@@ -45,11 +45,11 @@ __global__ void __launch_bounds__(DIGIT_THREADS)
              : mdgi::DigitSide{b.A, exps + b.offE, b.dA, b.lda, 0, b.m, b.k, b.Kp, b.Kp, b.plane_a};
   const int groups = (b.k + 1) / 2;
   const long long e = lu * (long long)DIGIT_THREADS + threadIdx.x;
-  const int row = (int)(e / groups);
+  int row, group;
+  mdgi::digit_place(b.p, d.trans, e, groups, row, group);
   if (row >= d.rows) return;
-  const int pc = (int)(e - (long long)row * groups) * 2;
   const bool wide = reinterpret_cast<uintptr_t>(d.X) % 16 == 0;
-  mdgi::digits_group<2, 2>(b.p, b.s, d, row, pc, wide, smem);
+  mdgi::digits_group<2, 2>(b.p, b.s, d, row, group * 2, wide, smem);
 }
 
 }  // namespace

@@ -142,6 +142,32 @@ struct DigitSide {
   long long plane_stride;
 };
 
+// Digit rows that neighbouring threads take together: in a transposed operand
+// the entries of one k lie side by side along the rows, up to four of them in
+// a 128-byte line, which a row per 128 threads fetched for each of them.  (A
+// warp then stores 32 bytes of each row of a plane: eight rows, for P = 2,
+// would be half sectors.)  Both operands: qd 1024^3 53 -> 45 us, qd 8192^3
+// 3.06 -> 2.6 ms, od 2048^3 393 -> 353 us.
+__host__ __device__ inline int digit_row_shift(int P, int trans) {
+  return !trans || P == 16 ? 0 : P == 8 ? 1 : 2;  // log2 of their number
+}
+
+// Threads of a side whose rows take `groups` groups of k-positions each, and
+// the row and group of thread e.
+__host__ __device__ inline long long digit_threads(int P, int trans, int rows, int groups) {
+  const int shift = digit_row_shift(P, trans);
+  return (((long long)rows + (1 << shift) - 1) >> shift << shift) * groups;
+}
+__device__ __forceinline__ void digit_place(int P, int trans, long long e, int groups, int &row,
+                                            int &group) {
+  const int shift = digit_row_shift(P, trans);
+  const long long v = e >> shift;
+  // (a 64-bit division is a hundred instructions)
+  const int band = v >> 32 ? (int)(v / groups) : (int)((uint32_t)v / (uint32_t)groups);
+  row = (band << shift) + ((int)e & ((1 << shift) - 1));
+  group = (int)(v - (long long)band * groups);
+}
+
 // One thread: the digits of V adjacent entries (row, pc0 ..) of one side.
 //
 // V = sum_l floor(a_l 2^(S-E)) is collected in 32-bit pieces, one signed

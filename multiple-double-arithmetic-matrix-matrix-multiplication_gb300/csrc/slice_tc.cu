@@ -97,21 +97,20 @@ __global__ void exps_kernel(int m, int n, const unsigned long long *__restrict__
 
 // --------------------------------------------------------------- digits --
 // Both operands in one launch; threads run over the sides' groups of V
-// k-positions, row after row, so plane stores are coalesced for A and B
-// alike.  norms: two counters of a later stage, cleared on the way.
+// k-positions (digit_place), so plane stores are coalesced for A and B alike.  norms: two counters of a later stage, cleared on the way.
 template <int V, int PL>
 __global__ void __launch_bounds__(DIGIT_THREADS)
-    digits_kernel(int P, int s, const DigitSide a, const DigitSide b, bool wide, unsigned *norms) {
+    digits_kernel(int P, int s, const DigitSide a, const DigitSide b, long long of_a, bool wide,
+                  unsigned *norms) {
   extern __shared__ uint4 smem[];
   const long long e = blockIdx.x * (long long)DIGIT_THREADS + threadIdx.x;
   if (norms && e < 2) norms[e] = 0;
   const int groups = a.cols_pad / V;
-  const long long of_a = (long long)a.rows * groups;
   const DigitSide &d = e < of_a ? a : b;
-  const long long i = e < of_a ? e : e - of_a;
-  const int row = (int)(i / groups);
+  int row, group;
+  mdgi::digit_place(P, d.trans, e < of_a ? e : e - of_a, groups, row, group);
   if (row >= d.rows) return;
-  mdgi::digits_group<V, PL>(P, s, d, row, (int)(i - (long long)row * groups) * V, wide, smem);
+  mdgi::digits_group<V, PL>(P, s, d, row, group * V, wide, smem);
 }
 
 // ---------------------------------------------------- diagonal GEMM v0 --
@@ -394,9 +393,10 @@ static int launch_digits_v(int p, int s, const DigitSide &a, const DigitSide &b,
   const int smem = digit_smem(s, V);
   MDG_TRY_CUDA(cudaFuncSetAttribute(digits_kernel<V, PL>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const long long groups = (long long)(a.rows + b.rows) * (a.cols_pad / V);
+  const long long of_a = digit_threads(p, a.trans, a.rows, a.cols_pad / V);
+  const long long threads = of_a + digit_threads(p, b.trans, b.rows, a.cols_pad / V);
   digits_kernel<V, PL>
-      <<<ceil_div(groups, DIGIT_THREADS), DIGIT_THREADS, smem, st>>>(p, s, a, b, wide, norms);
+      <<<ceil_div(threads, DIGIT_THREADS), DIGIT_THREADS, smem, st>>>(p, s, a, b, of_a, wide, norms);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }
