@@ -62,6 +62,24 @@ DIAG_TRAFFIC_BYTES = {"qd8192_normal": 473.09e9, "qd4096_normal": 73.51e9}
 DEFAULT_SLICES = {2: 14, 4: 28, 8: 55, 16: 110}
 
 
+def slice_launches(s, m, n, k, sums):
+    """Kernels of one BF16-form GEMM: scale, digits, diagonal GEMM and
+    renormalisation; in the sum-plane form (sums) a launch for the sums and
+    one for the GEMM per group of diagonals whose sums fit 16 GiB."""
+    if not sums:
+        return 4
+    up = lambda x, a: -(-x // a) * a
+    cap = (16 << 30) // (2 * up(k, 64) * (up(m, 256) + up(n, 256)))
+    cap = max(cap, s // 2)
+    groups, lo = 0, 1
+    while lo < s:
+        hi = lo
+        while hi < s and (hi + 1) ** 2 // 4 - lo * lo // 4 <= cap:
+            hi += 1
+        groups, lo = groups + 1, hi
+    return 3 + 2 * groups
+
+
 def digit_pairs(s, D):
     """Digit pairs (i, j), i + j = d < D, of s digits per operand."""
     return sum(min(d, s - 1) - max(0, d - (s - 1)) + 1 for d in range(D))
@@ -326,8 +344,9 @@ def batched_tile_work(probs, slices, policy="256"):
     P: useful (2 m n k per digit pair of the s diagonals kept) and as the
     grouped kernel pads it: single-CTA tiles pad rows to 128, columns to the
     tile width of the policy and k to 16 (the last 64-deep block issues only
-    the MMAs that reach data); CTA-pair tiles pad rows and columns to 256
-    and k to 64."""
+    the MMAs that reach data); CTA-pair tiles pad rows and columns to 256, or
+    one of them to 128 with two diagonals per accumulator (one step more per
+    pair of diagonals), whichever is less, and k to 16."""
     def pairs(s):
         return sum(min(d, s - 1) - max(0, d - (s - 1)) + 1 for d in range(s))
     up = lambda x, a: -(-x // a) * a
@@ -342,7 +361,11 @@ def batched_tile_work(probs, slices, policy="256"):
         q = pairs(slices[P])
         useful += 2.0 * m * n * k * q
         if policy == "pair":
-            padded += 2.0 * up(m, 256) * up(n, 256) * up(k, 64) * q
+            s = slices[P]
+            two = sum(d + 2 for d in range(-(s & 1), s, 2))
+            padded += 2.0 * up(k, 16) * min(up(m, 256) * up(n, 256) * q,
+                                            up(m, 256) * 2 * up(n, 128) * two,
+                                            2 * up(m, 128) * up(n, 256) * two)
         else:
             padded += 2.0 * up(m, 128) * width(n) * up(k, 16) * q
     return useful, padded
@@ -410,9 +433,8 @@ def bench_batched(api, inputs, stream):
             "slice_graph_gflops": flops / t_graph / 1e9, "slice_graph_ms": t_graph * 1e3,
             "per_p": per_p,
             # kernels per plan run: exponents of all rows and columns, digits
-            # of all operands, the grouped diagonal GEMM, and one
-            # renormalisation per limb count present
-            "slice_launches_per_batch": 3 + len({pr[0] for pr in probs}),
+            # of all operands, the grouped diagonal GEMM, the renormalisation
+            "slice_launches_per_batch": 4,
             "tile_policy": policy,
             "split": plan.split,
             "plain_loop_gflops": flops / t_loop / 1e9, "plain_loop_ms": t_loop * 1e3,
@@ -420,7 +442,7 @@ def bench_batched(api, inputs, stream):
             "slice_equals_single_problem": bool(same),
             "diag_bf16_tflop": {"useful": useful / 1e12, "padded": padded / 1e12,
                                 "useful_frac": useful / padded,
-                                "tiles": ("256 x 256 (CTA pairs, rows padded to 256)"
+                                "tiles": ("256 x 256, 256 x 128 or 128 x 256 (CTA pairs)"
                                           if policy == "pair" else
                                           f"128 x {policy} columns (single CTA)")
                                          + " under the tuned policy, k padded to 16"}}
@@ -629,6 +651,8 @@ def main():
     dC = torch.empty((m, n, P), dtype=torch.float64, device="cuda")
     need = api.workspace_size("slice_bf16", P, m, n, k)
     ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    # products of sum planes (s squares and s^2 / 4 sums) or digit pairs
+    sums = (need - L.mdg_gemm_least_workspace_size(2, P, m, n, k, None)) > 2 * s * (m + n) * k
 
     def step():
         api.gemm(dA, dB, "slice_bf16", out=dC, workspace=ws)
@@ -794,15 +818,21 @@ def main():
                                                / bf16_burst) if clk.get("sm_mhz") else None,
                          "clock_note": "frac_at_max_clock scales the achieved rate by "
                                        "sm_max_mhz / the median SM clock sampled over the "
-                                       "timed steps (the kernel is 95 % of a step)",
+                                       "timed steps",
                          "traffic": DIAG_TRAFFIC_BYTES.get(args.workload),
                          "traffic_note": "DRAM bytes per launch, one-pass ncu capture of this "
                                          "workload (null where none was taken)",
-                         "kernel": "diag_gemm", "kernel_ms": t_diag * 1e3,
+                         "kernel": "diag_gemm over digit pairs, timed alone",
+                         "kernel_ms": t_diag * 1e3,
                          "algorithmic_tflop_per_launch": tflop,
+                         # what a timed step multiplies on the tensor cores
+                         "step_form": "sum planes" if sums else "digit pairs",
+                         "step_plane_products": s + s * s // 4 if sums else pairs,
+                         "step_tflops": tflop / pairs * (s + s * s // 4 if sums else pairs)
+                         / t_step,
                          "peak_kind": f"{peak_kind} bf16 burst (frac_sustained: against "
                                       "the sustained figure)"},
-            "gpu_launches": 8 * args.steps,
+            "gpu_launches": slice_launches(s, m, n, k, sums) * args.steps,
             "clocks": clk,
             "error_bits": {"slice_bf16": [round(x, 1) for x in bits["slice_bf16"]],
                            "sample": f"{len(rows)}x{len(cols)} entries, exact integer product",
