@@ -344,9 +344,8 @@ def batched_tile_work(probs, slices, policy="256"):
     P: useful (2 m n k per digit pair of the s diagonals kept) and as the
     grouped kernel pads it: single-CTA tiles pad rows to 128, columns to the
     tile width of the policy and k to 16 (the last 64-deep block issues only
-    the MMAs that reach data); CTA-pair tiles pad rows and columns to 256, or
-    one of them to 128 with two diagonals per accumulator (one step more per
-    pair of diagonals), whichever is less, and k to 16."""
+    the MMAs that reach data); CTA-pair tiles pad rows and columns to 256
+    and k to 64."""
     def pairs(s):
         return sum(min(d, s - 1) - max(0, d - (s - 1)) + 1 for d in range(s))
     up = lambda x, a: -(-x // a) * a
@@ -361,11 +360,7 @@ def batched_tile_work(probs, slices, policy="256"):
         q = pairs(slices[P])
         useful += 2.0 * m * n * k * q
         if policy == "pair":
-            s = slices[P]
-            two = sum(d + 2 for d in range(-(s & 1), s, 2))
-            padded += 2.0 * up(k, 16) * min(up(m, 256) * up(n, 256) * q,
-                                            up(m, 256) * 2 * up(n, 128) * two,
-                                            2 * up(m, 128) * up(n, 256) * two)
+            padded += 2.0 * up(m, 256) * up(n, 256) * up(k, 64) * q
         else:
             padded += 2.0 * up(m, 128) * width(n) * up(k, 16) * q
     return useful, padded
@@ -442,7 +437,9 @@ def bench_batched(api, inputs, stream):
             "slice_equals_single_problem": bool(same),
             "diag_bf16_tflop": {"useful": useful / 1e12, "padded": padded / 1e12,
                                 "useful_frac": useful / padded,
-                                "tiles": ("256 x 256, 256 x 128 or 128 x 256 (CTA pairs)"
+                                "tiles": ("256 x 256 (CTA pairs; problems that 256 x 128 or "
+                                          "128 x 256 tiles pad less take those, so padded is "
+                                          "an upper bound)"
                                           if policy == "pair" else
                                           f"128 x {policy} columns (single CTA)")
                                          + " under the tuned policy, k padded to 16"}}

@@ -1389,11 +1389,13 @@ int encode_out_map(void *map128, const void *base, int Np, long long rows_total)
 }
 
 // The units of a table (numbered as the kernels number them) over the
-// workers: the dearest first, each to the worker with the least so far.  A
+// workers, in the table's order, each to the worker with the least so far.  A
 // unit's cost in k-steps: its own, about 6 per run for the drain and the
-// store, about 10 to fill and empty the pipeline.  Dealt in turn, one worker's
-// share could be a third above the mean (64 mixed problems of 32 .. 512: 2.67
-// -> 2.40 ms a call).
+// store, about 10 to fill and empty the pipeline.  The table's order, dear
+// problems first and a problem's units in a row, keeps the workers on few
+// problems at a time.  ms a call, units in turn / dearest unit first / in the
+// table's order: 64 mixed problems of 32 .. 512 2.67 / 2.30 / 2.12, 256 of
+// them - / 9.5 / 8.6, their octo-double ones on 128 x 256 tiles - / 11.6 / 7.5.
 int deal_units(const std::vector<GroupedProblem> &probs, int workers, std::vector<int> *starts,
                std::vector<int> *order) {
   struct Unit {
@@ -1410,8 +1412,6 @@ int deal_units(const std::vector<GroupedProblem> &probs, int workers, std::vecto
         units.push_back(Unit{cost * (g.tn == 128 && !g.stack ? 2 : 4),
                              g.unit_begin + part * g.mt * g.nt + tile});
     }
-  std::stable_sort(units.begin(), units.end(),
-                   [](const Unit &a, const Unit &b) { return a.cost > b.cost; });
   typedef std::pair<long long, int> Load;
   std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
   for (int w = 0; w < workers; ++w) least.push(Load(0, w));
