@@ -133,7 +133,9 @@ int mdg_gemm(int form, int p, int m, int n, int k, const double *A, int lda,
  * form on the transposed operands, then the addition; with k = 0 C is
  * cleared (or kept, when accumulating).  Extends the reference's square,
  * overwrite-only call (TCcuda.h:66).  Workspace: mdg_gemm_ex_workspace_size
- * (the inner GEMM's plus transposed copies and the product when needed). */
+ * (the inner GEMM's, plus the product when accumulating and, in the forms other
+ * than BF16, transposed copies; the BF16 form reads a transposed operand in
+ * place). */
 size_t mdg_gemm_ex_workspace_size(int form, int trans_a, int trans_b, int accumulate,
                                   int p, int m, int n, int k, const mdg_options *opt);
 int mdg_gemm_ex(int form, int trans_a, int trans_b, int accumulate, int p, int m, int n,
@@ -173,7 +175,7 @@ void mdg_host_free(void *ptr);
  * it synchronises `stream`.  mdg_batch_run only launches kernels (one for
  * the exponents of every row and column, one for the digits of every
  * operand, one grouped tcgen05 diagonal GEMM over the tiles of every
- * problem, and one renormalisation per limb count present) and may be
+ * problem, and one renormalisation of every C) and may be
  * captured into a CUDA graph; each C equals the single-problem mdg_gemm
  * result bit for bit.  No counterpart in the reference. */
 typedef struct mdg_batch_s *mdg_batch;
@@ -221,7 +223,7 @@ int mdg_batch_tune(mdg_batch batch, void *stream);
  * integrations that forbid allocation after start-up.  No counterpart in
  * the reference.  The scratch is a fixed array of mdg_static_scratch_bytes()
  * (64 MiB) inside the library, held on every GPU that loads it; a problem
- * whose BF16 workspace (mdg_gemm_workspace_size) is larger gets
+ * whose least BF16 workspace (mdg_gemm_least_workspace_size) is larger gets
  * MDG_ERROR_TOO_LARGE (e.g. quad-double fits up to 512^3, octo-double up to
  * 256^3).  The first call in a CUDA context (the device's primary context,
  * or one the caller made current) looks up the array's device address and

@@ -17,11 +17,14 @@
 // before any stream capture.  A context created later (after
 // cudaDeviceReset, or a driver-API context the caller makes current) has its
 // own id and gets its own lookup.  All calls share the array and it keeps
-// the previous call's contents: every region the pipeline reads is written
-// first (the row / column maxima are cleared, digit planes are written in
-// full including padding, every chunk plane is written by the diagonal
-// GEMM), and calls that overlap on the GPU race on the array, so a caller
-// must order them (one stream, or events).
+// the previous call's contents: everything that reaches C is written first
+// (the row / column maxima are cleared where ranges of k share them, the
+// digits of every row and column are written with their padding in k, every
+// chunk plane is written by the diagonal GEMM).  Rows of the digit planes
+// beyond m and n keep old contents; they reach only rows and columns of the
+// chunk planes beyond m and n, which nothing reads.  Calls that overlap on
+// the GPU race on the array, so a caller must order them (one stream, or
+// events).
 #include <cuda.h>
 
 #include <mutex>

@@ -1,5 +1,5 @@
 // Renormalisation of diagonal sums to P limbs, shared by the single-problem
-// kernels (renorm.cu) and the batched one (batched_stages.cuh).
+// and batched kernels (renorm.cu).
 //
 // W = sum_d C_d 256^(D-1-d), C_d the sum of diagonal d's chunk planes, is
 // built from the least significant diagonal up, eight diagonals (two 32-bit
