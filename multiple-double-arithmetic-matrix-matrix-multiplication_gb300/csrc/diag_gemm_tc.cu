@@ -799,17 +799,32 @@ struct CrossJob {
   CrossRuns runs;
 };
 
+// The units of one problem as the host deals them (deal_single): cluster w takes
+// order[starts[w]] .. order[starts[w + 1] - 1].  Travels as a kernel argument.
+constexpr int kDealtUnits = 1024, kDealtWorkers = 80;
+struct UnitDeal {
+  unsigned short starts[kDealtWorkers + 1], order[kDealtUnits];
+};
+
 // A single problem: units are tiles, or parts of tiles (ranges of
 // diagonals whose digit-pair counts add up to about 1/parts of the tile's
 // work), taken in strips of `raster` column blocks: tiles run across a strip
 // of `raster` column blocks, then down the rows, so that the clusters busy at
 // the same time read few distinct A row blocks and B column blocks and share
 // them in L2 (raster = 1 walks each column block top to bottom).
-struct PairSingle : DealtInTurn {
+// deal: the units as the host deals them, else (null) the clusters take them in
+// turn.
+struct PairSingle {
+  const UnitDeal *deal;
   const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, cs, stack, ktail, mt, nt;
   int parts, raster;
-  __device__ int last(int) const { return mt * nt * parts; }
+  __device__ int first(int worker, int) const { return deal ? deal->starts[worker] : worker; }
+  __device__ int last(int worker) const {
+    return deal ? deal->starts[worker + 1] : mt * nt * parts;
+  }
+  __device__ int step(int workers) const { return deal ? 1 : workers; }
+  __device__ int unit(int i) const { return deal ? deal->order[i] : i; }
   __device__ PairJob job(int u) const {
     const int tiles = mt * nt, tile = u % tiles, part = u / tiles;
     const int strip = tile / (mt * raster);
@@ -1142,8 +1157,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                          const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmC, int s, int D, int Mp, int Np,
                          int KB, int cs, int stack, int ktail, int mt, int nt, int parts,
-                         int raster, int pace, uint32_t epoch, int no_loads) {
-  tc2_body(PairSingle{{}, &tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
+                         int raster, int pace, uint32_t epoch, int no_loads, int dealt,
+                         const __grid_constant__ UnitDeal deal) {
+  tc2_body(PairSingle{dealt ? &deal : nullptr, &tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
            pace, epoch, no_loads);
 }
 
@@ -1231,6 +1247,82 @@ struct PairSchedule {
 int few_tile_parts(int tiles, int runs, int workers, int parts) {
   const int fit = workers / tiles;
   return runs <= fit ? runs : std::max(parts, fit);
+}
+
+// Dealing of units of work to workers (clusters or CTAs) by cost.
+struct Unit {
+  long long cost;
+  int id;
+};
+
+// A unit's cost in k-steps: its own, about 6 per run for the drain and the
+// store, about 10 to fill and empty the pipeline.
+long long unit_cost(DigitRuns runs) {
+  long long cost = 10;
+  for (Run r; runs.next(r);) cost += r.steps + 6;
+  return cost;
+}
+
+// Each unit, in the order given, to the worker with the least so far; the
+// largest sum.
+long long deal_in_order(const std::vector<Unit> &units, int workers, std::vector<int> *starts,
+                        std::vector<int> *order) {
+  typedef std::pair<long long, int> Load;
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+  for (int w = 0; w < workers; ++w) least.push(Load(0, w));
+  std::vector<std::vector<int>> of(workers);
+  long long most = 0;
+  for (const Unit &u : units) {
+    const Load l = least.top();
+    least.pop();
+    of[l.second].push_back(u.id);
+    least.push(Load(l.first + u.cost, l.second));
+    most = std::max(most, l.first + u.cost);
+  }
+  starts->assign(1, 0);
+  order->clear();
+  for (const auto &list : of) {
+    order->insert(order->end(), list.begin(), list.end());
+    starts->push_back((int)order->size());
+  }
+  return most;
+}
+
+// The units (tile, run) of a single problem, the longest runs first, dealt,
+// where that ends sooner than sc's parts taken in turn.  Clusters at work
+// then have runs of about equal length and one problem's planes, so no pacing.
+// us a call, in turn / a tile's runs in a row / the longest runs first: dd
+// 16001 x 96 x 3001 1666 / 1584 / 1600, od 3000 x 64 x 1000 1106 / 1100 / 991,
+// dd 4000 x 64 x 300 102 / 102 / 89, qd 2000 x 300 x 450 316 / 317 / 282, dd
+// 3000 x 1000 x 500 375 / 376 / 344, qd 700 x 300 x 200 125 / 116 / 96.
+bool deal_single(int tiles, const DigitRuns &all, int runs, int ncl, PairSchedule *sc,
+                 UnitDeal *deal) {
+  const long long all_units = (long long)tiles * runs;
+  if (ncl > kDealtWorkers || all_units > kDealtUnits) return false;
+  if (sc->parts == runs && all_units <= ncl) return false;  // a unit each already
+  std::vector<long long> in_turn(ncl, 0);
+  for (int part = 0; part < sc->parts; ++part) {
+    const long long cost =
+        unit_cost(part_runs(all.s, all.D, all.KB, all.cs, all.stack, part, sc->parts));
+    for (int t = 0; t < tiles; ++t) in_turn[(part * tiles + t) % ncl] += cost;
+  }
+  std::vector<Unit> units;
+  DigitRuns it = all;
+  Run r;
+  for (int part = 0; part < runs && it.next(r); ++part)
+    for (int t = 0; t < tiles; ++t) units.push_back(Unit{r.steps + 16, part * tiles + t});
+  std::stable_sort(units.begin(), units.end(),
+                   [](const Unit &a, const Unit &b) { return a.cost > b.cost; });
+  std::vector<int> starts, order;
+  if (deal_in_order(units, ncl, &starts, &order) >=
+      *std::max_element(in_turn.begin(), in_turn.end()))
+    return false;
+  std::copy(starts.begin(), starts.end(), deal->starts);
+  std::copy(order.begin(), order.end(), deal->order);
+  sc->parts = runs;
+  sc->clusters = std::min(ncl, tiles * runs);
+  sc->pace = 0;
+  return true;
 }
 
 // runs: of a tile, what parts can separate.
@@ -1338,7 +1430,7 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
     return MDG_ERROR_INVALID_SIZE;
   if (plane_c != (long long)Mp * Np) return MDG_ERROR_INVALID_SIZE;
   // the CTA-pair kernel needs 256-row tiles
-  const int narrow = engine == 1 ? narrow_tile(m, n) : 0;
+  const int narrow = engine == 1 ? narrow_tile(s, D, m, n, Kp / TK) : 0;
   const bool pair = Mp % 256 == 0 && engine != 2 && !narrow;
   const int tn = narrow ? narrow : TN;
   const int runs = total_chunks(s, D, Kp / TK, cs);
@@ -1362,11 +1454,16 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
         cs == CHUNK_STEPS && engine == 1 ? stacked_tiles(s, D, m, n, Kp / TK) : kStackNone;
     const int mt = stack == kStackM ? (m + 127) / 128 : Mp / 256;
     const int nt = stack == kStackN ? (n + 127) / 128 : Np / TN2;
-    const PairSchedule sc = pair_schedule(mt, nt, stack ? (D + 1) / 2 : runs, sms, parts_opt,
-                                          raster_opt, pace_opt);
+    const int separable = stack ? (D + 1) / 2 : runs;
+    PairSchedule sc = pair_schedule(mt, nt, separable, sms, parts_opt, raster_opt, pace_opt);
+    UnitDeal deal = {};
+    // a schedule that the caller asks for is kept
+    const bool dealt = parts_opt <= 0 && pace_opt <= 0 &&
+                       deal_single(mt * nt, part_runs(s, D, Kp / TK, cs, stack, 0, 1), separable,
+                                   sms / 2, &sc, &deal);
     diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
         ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, stack, (k - (Kp - TK) + 15) / 16, mt, nt, sc.parts,
-        sc.raster, sc.pace, sc.epoch, sc.no_loads);
+        sc.raster, sc.pace, sc.epoch, sc.no_loads, dealt, deal);
   } else {
     const int mt = (m + TM - 1) / TM, nt = (n + tn - 1) / tn, tiles = mt * nt;
     const int parts = parts_opt > 0 ? std::min(8, parts_opt)
@@ -1398,36 +1495,15 @@ int encode_out_map(void *map128, const void *base, int Np, long long rows_total)
 // them - / 9.5 / 8.6, their octo-double ones on 128 x 256 tiles - / 11.6 / 7.5.
 int deal_units(const std::vector<GroupedProblem> &probs, int workers, std::vector<int> *starts,
                std::vector<int> *order) {
-  struct Unit {
-    long long cost;
-    int id;
-  };
   std::vector<Unit> units;
   for (const GroupedProblem &g : probs)
     for (int part = 0; part < g.parts; ++part) {
-      DigitRuns runs = part_runs(g.s, g.D, g.KB, CHUNK_STEPS, g.stack, part, g.parts);
-      long long cost = 10;
-      for (Run r; runs.next(r);) cost += r.steps + 6;
+      const long long cost = unit_cost(part_runs(g.s, g.D, g.KB, CHUNK_STEPS, g.stack, part, g.parts));
       for (int tile = 0; tile < g.mt * g.nt; ++tile)
         units.push_back(Unit{cost * (g.tn == 128 && !g.stack ? 2 : 4),
                              g.unit_begin + part * g.mt * g.nt + tile});
     }
-  typedef std::pair<long long, int> Load;
-  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
-  for (int w = 0; w < workers; ++w) least.push(Load(0, w));
-  std::vector<std::vector<int>> of(workers);
-  for (const Unit &u : units) {
-    const Load l = least.top();
-    least.pop();
-    of[l.second].push_back(u.id);
-    least.push(Load(l.first + u.cost, l.second));
-  }
-  starts->assign(1, 0);
-  order->clear();
-  for (const auto &list : of) {
-    order->insert(order->end(), list.begin(), list.end());
-    starts->push_back((int)order->size());
-  }
+  deal_in_order(units, workers, starts, order);
   return MDG_SUCCESS;
 }
 

@@ -316,11 +316,39 @@ SlicePlan make_slice_plan(int p, int s, int D, int m, int n, int k) {
   return layout_slice_plan(p, s, D, m, n, k, 0);
 }
 
-int narrow_tile(int m, int n) {
+// What the diagonal GEMM takes on a problem of few tiles, in us: k-steps of the
+// busiest worker.  A k-step of 32 KiB of operands a CTA takes 0.43 us where
+// all 152 SMs ask L2 for them (11 TB/s), 48 KiB 0.62, and 0.27 by itself; 16
+// k-steps go to the ends of a run.  Estimated / measured whole calls,
+// short chunks against two diagonals an accumulator: qd 2000 x 100 x 500 154 -
+// 86 / 218 - 160 us, 100 x 2000 x 500 116 - 86 / 190 - 158, 500 x 64 x 500 44 -
+// 65 / 88 - 117, od 300 x 128 x 700 150 - 168 / 247 - 269, 3000 x 64 x 1000
+// 1680 - 880 / 1899 - 977, dd 300 x 300 x 2000 83 - 125 / 159 - 204.
+static double chunked_us(int s, int D, int KB, long long tiles, int tn) {
+  long long steps = 0;
+  for (int d = 0; d < D; ++d) steps += (long long)diag_pairs(d, s) * KB;
+  const double share = (double)steps * tiles / (tn ? 152 : 76) + 16.0;
+  return share * (tn == 256 ? 0.62 : 0.43);
+}
+
+static double stacked_us(int s, int D, int m, int n, int KB) {
+  const int stack = stacked_tiles(s, D, m, n, KB);
+  if (!stack) return 1e30;
+  const long long tiles = stack == 1 ? (long long)ceil_div(m, 256) * ceil_div(n, 128)
+                                     : (long long)ceil_div(m, 128) * ceil_div(n, 256);
+  long long steps = 0;
+  for (int d = -(D & 1); d < D; d += 2) steps += (long long)(d + 2) * KB + 16;
+  return std::max(0.43 * (double)steps * tiles / 76, 0.27 * ((D + 1.0) * KB + 16.0));
+}
+
+int narrow_tile(int s, int D, int m, int n, int KB) {
   const int tn = n <= 128 ? 128 : m <= 128 ? 256 : 0;
+  if (!tn) return 0;
+  const long long tiles = (long long)ceil_div(m, 128) * ceil_div(n, tn);
   // a full chip of them asks more operand bytes of L2 than pairs do (tall dd
   // 16001 x 96 x 3001: 1.84 ms against 1.74)
-  return tn && (long long)ceil_div(m, 128) * ceil_div(n, tn) <= 76 ? tn : 0;
+  if (tiles > 76 || stacked_us(s, D, m, n, KB) < chunked_us(s, D, KB, tiles, tn)) return 0;
+  return tn;
 }
 
 // Measured, chunks of 2032 k-steps and at most 8 parts / this: qd 256^3 107 /
@@ -330,14 +358,16 @@ int narrow_tile(int m, int n) {
 // problem of few tiles: about the steps each can have.  Where a chunk per
 // CTA fits at up to twice that length it is taken, so that none gets two.
 static int chunk_steps(int s, int D, int m, int n, int KB) {
-  const int tn = narrow_tile(m, n);
+  const int tn = narrow_tile(s, D, m, n, KB);
   const long long tiles = tn ? (long long)ceil_div(m, 128) * ceil_div(n, tn)
                              : (long long)ceil_div(m, 256) * ceil_div(n, 256);
   const int workers = tn ? 152 : 76;
   long long steps = 0;
   for (int d = 0; d < D; ++d) steps += (long long)diag_pairs(d, s) * KB;
   const long long share = (steps * tiles + workers - 1) / workers;
-  if (2 * tiles > workers || share >= CHUNK_STEPS / 2) return CHUNK_STEPS;
+  if (2 * tiles > workers || share >= CHUNK_STEPS / 2 ||
+      stacked_us(s, D, m, n, KB) < chunked_us(s, D, KB, tiles, tn))
+    return CHUNK_STEPS;
   const int least = std::max(8, (int)(share + 3) / 4 * 4);
   for (int cs = least; cs <= 2 * least; cs += 4)
     if (tiles * total_chunks(s, D, KB, cs) <= workers) return cs;

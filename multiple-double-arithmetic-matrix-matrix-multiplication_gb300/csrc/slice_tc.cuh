@@ -64,7 +64,7 @@ SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k);
 SlicePlan block_slice_plan(int p, int s, int D, int m, int n, int k);
 // Tiles of the single-CTA kernel for small problems of up to 128 rows or
 // columns: 128 rows by tn columns over the valid part (0: CTA pairs).
-int narrow_tile(int m, int n);
+int narrow_tile(int s, int D, int m, int n, int KB);
 int words_for(int s, int D);
 
 // The FP64-DMMA slice-digit form (digits64.cu): default digits per P

@@ -27,3 +27,22 @@ def test_few_tiles_same_bits(p, m, n, k):
         assert torch.equal(got, api.gemm(A, B, engine=engine)), engine
     assert torch.equal(got, api.gemm(A, B, parts=3))
     assert api.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,m,n,k", [
+    # digit pairs over a few tiles, a run of diagonals a unit: stacked on either
+    # side (odd and even digit counts), unstacked, as many units as fit the
+    # argument (2, 37000, 64: 145 x 7 = 1015) and one tile row more (1022), one
+    # more again (1029: in turn)
+    (8, 3000, 64, 100), (16, 100, 1000, 90), (4, 2000, 300, 450), (2, 900, 900, 300),
+    (16, 500, 500, 70), (2, 37000, 64, 70), (2, 37200, 100, 40), (2, 37500, 64, 40)])
+def test_dealt_units_same_bits(p, m, n, k):
+    import torch
+    api = pkg("api")
+    A = api.generate("uniform", p, m, k, 17, -9, 9, scale_rows=True)
+    B = api.generate("normal", p, k, n, 18)
+    got = api.gemm(A, B)
+    assert torch.equal(got, api.gemm(A, B, parts=1))
+    assert torch.equal(got, api.gemm(A, B, engine="tc"))
+    assert api.device_status() == 0
