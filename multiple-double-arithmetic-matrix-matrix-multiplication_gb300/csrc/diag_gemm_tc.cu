@@ -756,7 +756,7 @@ struct CrossRuns {
   int sq, nsq, d, i, chunk, planes;  // where the list goes on, planes left
   int plane0, ppc, KB;               // plane of diagonal d's pair 0 is plane0 + cross_offset(d)
   int cuts1, cuts;                   // flush groups per square, per sum
-  __device__ bool next(Run &r) {
+  __host__ __device__ bool next(Run &r) {
     if (planes <= 0) return false;
     if (sq < nsq) {
       r = Run{sq, 1, sq, 1, 0, KB, sq, cuts1};
@@ -792,6 +792,26 @@ struct CrossRuns {
   };
 };
 
+// Part `part` of a tile's list over the squares (nsq of them) and the diagonals
+// [dlo, dhi): the runs that start in the part's 1/parts of its products.
+__host__ __device__ __forceinline__ CrossRuns cross_part(int D, int dlo, int dhi, int nsq,
+                                                         int plane0, int ppc, int KB, int cuts,
+                                                         int part, int parts) {
+  const int total = nsq + mdgi::cross_offset(dhi) - mdgi::cross_offset(dlo);
+  const int lo = (int)((long long)total * part / parts);
+  const int hi = (int)((long long)total * (part + 1) / parts);
+  CrossRuns it{0, nsq, dlo, 0, D, total, plane0, ppc, KB, mdgi::cross_groups(KB), cuts};
+  for (int d = 1; d < dlo; ++d) it.chunk += mdgi::cross_chunks(d, ppc);
+  Run r;
+  while (total - it.planes < lo && it.next(r)) {
+  }
+  CrossRuns first = it;
+  while (total - it.planes < hi && it.next(r)) {
+  }
+  first.planes -= it.planes;
+  return first;
+}
+
 struct CrossJob {
   static constexpr int stack = kStackNone, ktail = TK / 16;
   const CUtensorMap *tmA, *tmB, *tmC;
@@ -806,25 +826,26 @@ struct UnitDeal {
   unsigned short starts[kDealtWorkers + 1], order[kDealtUnits];
 };
 
+// Units of a single problem: as dealt, or (null) in turn.
+struct MaybeDealt {
+  const UnitDeal *deal;
+  __device__ int first(int worker, int) const { return deal ? deal->starts[worker] : worker; }
+  __device__ int end(int worker, int units) const { return deal ? deal->starts[worker + 1] : units; }
+  __device__ int step(int workers) const { return deal ? 1 : workers; }
+  __device__ int unit(int i) const { return deal ? deal->order[i] : i; }
+};
+
 // A single problem: units are tiles, or parts of tiles (ranges of
 // diagonals whose digit-pair counts add up to about 1/parts of the tile's
 // work), taken in strips of `raster` column blocks: tiles run across a strip
 // of `raster` column blocks, then down the rows, so that the clusters busy at
 // the same time read few distinct A row blocks and B column blocks and share
 // them in L2 (raster = 1 walks each column block top to bottom).
-// deal: the units as the host deals them, else (null) the clusters take them in
-// turn.
-struct PairSingle {
-  const UnitDeal *deal;
+struct PairSingle : MaybeDealt {
   const CUtensorMap *tmA, *tmB, *tmC;
   int s, D, Mp, Np, KB, cs, stack, ktail, mt, nt;
   int parts, raster;
-  __device__ int first(int worker, int) const { return deal ? deal->starts[worker] : worker; }
-  __device__ int last(int worker) const {
-    return deal ? deal->starts[worker + 1] : mt * nt * parts;
-  }
-  __device__ int step(int workers) const { return deal ? 1 : workers; }
-  __device__ int unit(int i) const { return deal ? deal->order[i] : i; }
+  __device__ int last(int worker) const { return end(worker, mt * nt * parts); }
   __device__ PairJob job(int u) const {
     const int tiles = mt * nt, tile = u % tiles, part = u / tiles;
     const int strip = tile / (mt * raster);
@@ -860,12 +881,14 @@ struct PairGrouped : DealtByHost {
 // A single problem over digit and sum planes: units are tiles, or parts of
 // tiles whose lists hold about 1/parts of its products each (cut between
 // output planes), in the order of PairSingle's.
-struct PairCross : DealtInTurn {
+struct PairCross : MaybeDealt {
   const CUtensorMap *tmA, *tmB, *tmC;
   int D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB;
   int parts, raster;
   const unsigned *norm_a, *norm_b;
-  __device__ int last(int) const { return (Mp / 256) * (Np / TN2) * parts; }
+  __device__ int last(int worker) const {
+    return end(worker, (Mp / 256) * (Np / TN2) * parts);
+  }
   // Flush groups per sum plane.  |sum over a group| <= |a| |b| (Cauchy and
   // Schwarz; every partial sum too) with |a|^2 <= 2 *norm_a, |b|^2 <= 2
   // *norm_b over a whole group (two windows), <= *norm_a, *norm_b over half
@@ -883,21 +906,8 @@ struct PairCross : DealtInTurn {
     const int c0 = strip * raster;
     const int g = NB - c0 < raster ? NB - c0 : raster;
     const int rb = idx / g, cb = c0 + idx - rb * g;
-    const int total = nsq + mdgi::cross_offset(dhi) - mdgi::cross_offset(dlo);
-    const int lo = (int)((long long)total * part / parts);
-    const int hi = (int)((long long)total * (part + 1) / parts);
-    // the runs that start in [lo, hi)
-    const int cuts1 = mdgi::cross_groups(KB);
-    CrossRuns it{0, nsq, dlo, 0, D, total, plane0, ppc, KB, cuts1, cuts()};
-    for (int d = 1; d < dlo; ++d) it.chunk += mdgi::cross_chunks(d, ppc);
-    Run r;
-    while (total - it.planes < lo && it.next(r)) {
-    }
-    CrossRuns first = it;
-    while (total - it.planes < hi && it.next(r)) {
-    }
-    first.planes -= it.planes;
-    return CrossJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2, first};
+    return CrossJob{tmA, tmB, tmC, Mp, Np, KB, rb * 256, cb * TN2,
+                    cross_part(D, dlo, dhi, nsq, plane0, ppc, KB, cuts(), part, parts)};
   }
 };
 
@@ -1159,7 +1169,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                          int KB, int cs, int stack, int ktail, int mt, int nt, int parts,
                          int raster, int pace, uint32_t epoch, int no_loads, int dealt,
                          const __grid_constant__ UnitDeal deal) {
-  tc2_body(PairSingle{dealt ? &deal : nullptr, &tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
+  tc2_body(PairSingle{{dealt ? &deal : nullptr}, &tmA, &tmB, &tmC, s, D, Mp, Np, KB, cs, stack, ktail, mt, nt, parts, raster},
            pace, epoch, no_loads);
 }
 
@@ -1177,8 +1187,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
                            int nsq, int plane0, int ppc, int Mp, int Np, int KB, int parts,
                            int raster, const unsigned *__restrict__ norm_a,
                            const unsigned *__restrict__ norm_b, int pace, uint32_t epoch,
-                           int no_loads) {
-  tc2_body(PairCross{{}, &tmA, &tmB, &tmC, D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB, parts, raster,
+                           int no_loads, int dealt, const __grid_constant__ UnitDeal deal) {
+  tc2_body(PairCross{{dealt ? &deal : nullptr}, &tmA, &tmB, &tmC, D, dlo, dhi, nsq, plane0, ppc, Mp, Np, KB, parts, raster,
                      norm_a, norm_b},
            pace, epoch, no_loads);
 }
@@ -1257,7 +1267,8 @@ struct Unit {
 
 // A unit's cost in k-steps: its own, about 6 per run for the drain and the
 // store, about 10 to fill and empty the pipeline.
-long long unit_cost(DigitRuns runs) {
+template <class Runs>
+long long unit_cost(Runs runs) {
   long long cost = 10;
   for (Run r; runs.next(r);) cost += r.steps + 6;
   return cost;
@@ -1288,29 +1299,41 @@ long long deal_in_order(const std::vector<Unit> &units, int workers, std::vector
   return most;
 }
 
-// The units (tile, run) of a single problem, the longest runs first, dealt,
-// where that ends sooner than sc's parts taken in turn.  Clusters at work
-// then have runs of about equal length and one problem's planes, so no pacing.
-// us a call, in turn / a tile's runs in a row / the longest runs first: dd
-// 16001 x 96 x 3001 1666 / 1584 / 1600, od 3000 x 64 x 1000 1106 / 1100 / 991,
-// dd 4000 x 64 x 300 102 / 102 / 89, qd 2000 x 300 x 450 316 / 317 / 282, dd
-// 3000 x 1000 x 500 375 / 376 / 344, qd 700 x 300 x 200 125 / 116 / 96.
-bool deal_single(int tiles, const DigitRuns &all, int runs, int ncl, PairSchedule *sc,
+// The units (tile, part) of a single problem, the dearest first, dealt, where
+// that ends sooner than sc's parts taken in turn.  Clusters at work then have
+// units of about equal length and few planes between them, so no pacing.
+// us a call over digit pairs, in turn / a tile's runs in a row / the longest
+// runs first: dd 16001 x 96 x 3001 1666 / 1584 / 1600, od 3000 x 64 x 1000 1106
+// / 1100 / 991, dd 4000 x 64 x 300 102 / 102 / 89, qd 2000 x 300 x 450 316 / 317
+// / 282, dd 3000 x 1000 x 500 375 / 376 / 344, qd 700 x 300 x 200 125 / 116 / 96.
+// Over sum planes, in turn / 24 / 32 / 48 / 64 parts dealt: qd 1024^3 658 / 637 /
+// 627 / 624 / 625 (64 of 76 clusters at work / all), 1000 x 777 x 1531 884 / 844
+// / 843 / 831 / 833, od 1024^3 2060 / 1990 / 2000 / 1960 / 1954, hd 1024 x 1024 x
+// 512 4584 / 4520 / 4368 / 4448 / 4480, qd 2048^3 (16 parts) 3620 / 3400.  But a
+// product of more than about 3 ms runs at the power cap, where the idle clusters'
+// share of the power drives the others, and the worse sharing of planes costs:
+// od 2048^3 12.3 / 12.7 ms, qd 3000 x 2500 x 3000 8.95 / 9.2, od 1500^3 5.5 / 5.7,
+// hd 2048 x 2048 x 512 14.37 / 14.39: in turn beyond kCrossDealSteps k-steps a
+// cluster (qd 2048^3 6036, od 1500^3 9219).
+constexpr int kCrossDealParts = 48;
+constexpr long long kCrossDealSteps = 7000;
+
+// cost(part, parts): of a unit, 0 where it has no runs; fine: the parts to deal.
+template <class Cost>
+bool deal_single(int tiles, int fine, const Cost &cost, int ncl, PairSchedule *sc,
                  UnitDeal *deal) {
-  const long long all_units = (long long)tiles * runs;
+  const long long all_units = (long long)tiles * fine;
   if (ncl > kDealtWorkers || all_units > kDealtUnits) return false;
-  if (sc->parts == runs && all_units <= ncl) return false;  // a unit each already
+  if (sc->parts == fine && all_units <= ncl) return false;  // a unit each already
   std::vector<long long> in_turn(ncl, 0);
   for (int part = 0; part < sc->parts; ++part) {
-    const long long cost =
-        unit_cost(part_runs(all.s, all.D, all.KB, all.cs, all.stack, part, sc->parts));
-    for (int t = 0; t < tiles; ++t) in_turn[(part * tiles + t) % ncl] += cost;
+    const long long c = cost(part, sc->parts);
+    for (int t = 0; t < tiles; ++t) in_turn[(part * tiles + t) % ncl] += c;
   }
   std::vector<Unit> units;
-  DigitRuns it = all;
-  Run r;
-  for (int part = 0; part < runs && it.next(r); ++part)
-    for (int t = 0; t < tiles; ++t) units.push_back(Unit{r.steps + 16, part * tiles + t});
+  for (int part = 0; part < fine; ++part)
+    if (const long long c = cost(part, fine))
+      for (int t = 0; t < tiles; ++t) units.push_back(Unit{c, part * tiles + t});
   std::stable_sort(units.begin(), units.end(),
                    [](const Unit &a, const Unit &b) { return a.cost > b.cost; });
   std::vector<int> starts, order;
@@ -1319,8 +1342,8 @@ bool deal_single(int tiles, const DigitRuns &all, int runs, int ncl, PairSchedul
     return false;
   std::copy(starts.begin(), starts.end(), deal->starts);
   std::copy(order.begin(), order.end(), deal->order);
-  sc->parts = runs;
-  sc->clusters = std::min(ncl, tiles * runs);
+  sc->parts = fine;
+  sc->clusters = (int)std::min<long long>(ncl, (long long)units.size());
   sc->pace = 0;
   return true;
 }
@@ -1400,11 +1423,25 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
   MDG_TRY_CUDA(cudaFuncSetAttribute(diag_gemm_cross_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const PairSchedule sc =
-      pair_schedule(Mp / 256, Np / TN2, squares + dhi - dlo, sms, parts, raster, pace);
+  const int tiles = (Mp / 256) * (Np / TN2), plane0 = s - cross_offset(dlo);
+  const int ppc = cross_pairs_per_chunk(KB);
+  PairSchedule sc = pair_schedule(Mp / 256, Np / TN2, squares + dhi - dlo, sms, parts, raster, pace);
+  UnitDeal deal = {};
+  bool dealt = false;
+  const int products = squares + cross_offset(dhi) - cross_offset(dlo);
+  if (parts <= 0 && pace <= 0 &&
+      (long long)tiles * products * KB <= kCrossDealSteps * (sms / 2)) {
+    auto cost = [&](int part, int of) -> long long {
+      const CrossRuns r =
+          cross_part(D, dlo, dhi, squares, plane0, ppc, KB, cross_groups(KB), part, of);
+      return r.planes > 0 ? unit_cost(r) : 0;
+    };
+    const int fine = std::min(products, std::min(kCrossDealParts, kDealtUnits / tiles));
+    dealt = fine > 0 && deal_single(tiles, fine, cost, sms / 2, &sc, &deal);
+  }
   diag_gemm_cross_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
-      ma, mb, mc, D, dlo, dhi, squares, s - cross_offset(dlo), cross_pairs_per_chunk(KB), Mp, Np, KB,
-      sc.parts, sc.raster, norm_a, norm_b, sc.pace, sc.epoch, sc.no_loads);
+      ma, mb, mc, D, dlo, dhi, squares, plane0, ppc, Mp, Np, KB, sc.parts, sc.raster, norm_a, norm_b,
+      sc.pace, sc.epoch, sc.no_loads, dealt, deal);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;
 }
@@ -1457,10 +1494,12 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
     const int separable = stack ? (D + 1) / 2 : runs;
     PairSchedule sc = pair_schedule(mt, nt, separable, sms, parts_opt, raster_opt, pace_opt);
     UnitDeal deal = {};
+    auto cost = [&](int part, int parts) {
+      return unit_cost(part_runs(s, D, Kp / TK, cs, stack, part, parts));
+    };
     // a schedule that the caller asks for is kept
     const bool dealt = parts_opt <= 0 && pace_opt <= 0 &&
-                       deal_single(mt * nt, part_runs(s, D, Kp / TK, cs, stack, 0, 1), separable,
-                                   sms / 2, &sc, &deal);
+                       deal_single(mt * nt, separable, cost, sms / 2, &sc, &deal);
     diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
         ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, stack, (k - (Kp - TK) + 15) / 16, mt, nt, sc.parts,
         sc.raster, sc.pace, sc.epoch, sc.no_loads, dealt, deal);

@@ -88,3 +88,21 @@ def test_smaller_workspace_gives_the_same_bits():
     assert L.mdg_gemm(*args, least, st) == 0
     assert torch.equal(C, ref)
     assert L.mdg_gemm(*args, least - 1, st) == 5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,m,n,k", [
+    # units dealt to the clusters: more clusters than tiles, chunks of several
+    # planes and of one, tiles at the argument's limit; the last beyond the
+    # sizes that are dealt
+    (4, 1000, 777, 1531), (16, 900, 1000, 530), (2, 1500, 1300, 16000), (2, 3000, 3000, 1024),
+    (8, 1500, 1500, 1100)])
+def test_dealt_sums_same_bits(p, m, n, k):
+    import torch
+    api = pkg("api")
+    A = api.generate("normal", p, m, k, 21, -9, 9, scale_rows=True)
+    B = api.generate("uniform", p, k, n, 22)
+    got = api.gemm(A, B)
+    assert torch.equal(got, api.gemm(A, B, parts=1))
+    assert torch.equal(got, api.gemm(A, B, engine="tc"))
+    assert api.device_status() == 0
