@@ -8,7 +8,6 @@
 
 namespace {
 
-constexpr int WINDOW_VECS = 64;  // 16-byte vectors of a window: 8 k-steps of 64 BF16
 constexpr int SUM_WARPS = 8;
 
 // a + b of two BF16 pairs, exact for integers of magnitude <= 128 each
@@ -31,8 +30,11 @@ __device__ __forceinline__ float add_squares(uint32_t z, float acc) {
 // Writing bounds it: 2 bytes out per sum against 2 digits in per D / 2 sums.
 // qd 8192^3: 52.6 GB of sums in 11.6 ms (4.5 TB/s); qd 1024^3: 0.82 GB in
 // 140 us, 6.2 TB/s of DRAM traffic.
+// Digit rows lie `stride` vectors apart, the longest window's: with 64 for every
+// size the 110 digits of a hexa-double row let two blocks on an SM (hd 1024 x 1024
+// x 512 1272 us, 1022 now).
 __global__ void __launch_bounds__(32 * SUM_WARPS)
-    cross_sums_kernel(int s, int plo, int phi, int digits, int KB, int windows, int rows_a,
+    cross_sums_kernel(int s, int plo, int phi, int digits, int KB, int windows, int stride, int rows_a,
                       __nv_bfloat16 *dA, __nv_bfloat16 *dB, long long plane_a, long long plane_b,
                       unsigned *norms) {
   extern __shared__ uint4 digit_rows[];
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(32 * SUM_WARPS)
 
   for (int i = warp; i < digits; i += SUM_WARPS)
     for (int v = lane; v < nv; v += 32) {
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(digit_rows + i * WINDOW_VECS + v);
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(digit_rows + i * stride + v);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
                    "l"(base + i * plane + v)
                    : "memory");
@@ -61,7 +63,7 @@ __global__ void __launch_bounds__(32 * SUM_WARPS)
     // a square, so the rounded root has the right integer part)
     const int d = (int)sqrtf((float)(4 * q + 3));
     const int i = q - mdgi::cross_offset(d), j = d - i;
-    const uint4 *xi = digit_rows + i * WINDOW_VECS, *xj = digit_rows + j * WINDOW_VECS;
+    const uint4 *xi = digit_rows + i * stride, *xj = digit_rows + j * stride;
     uint4 *out = base + (s + q - plo) * plane;
     float sq = 0.0f;  // at most 16 squares of 2^16 a lane: exact
     for (int v = lane; v < nv; v += 32) {
@@ -92,11 +94,13 @@ namespace mdgi {
 int launch_cross_sums(int s, int dlo, int dhi, int Kp, int rows_a, int rows_b, void *dA, void *dB,
                       long long plane_a, long long plane_b, unsigned *norms, cudaStream_t st) {
   const int KB = Kp / 64, windows = 2 * cross_groups(KB);
-  const int smem = dhi * WINDOW_VECS * 16;
+  // 16-byte vectors of the longest window (at most 8 k-steps of 64 BF16)
+  const int stride = (KB + windows - 1) / windows * 8;
+  const int smem = dhi * stride * 16;
   MDG_TRY_CUDA(cudaFuncSetAttribute(cross_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     smem));
   cross_sums_kernel<<<dim3(rows_a + rows_b, windows), 32 * SUM_WARPS, smem, st>>>(
-      s, cross_offset(dlo), cross_offset(dhi), dhi, KB, windows, rows_a,
+      s, cross_offset(dlo), cross_offset(dhi), dhi, KB, windows, stride, rows_a,
       reinterpret_cast<__nv_bfloat16 *>(dA), reinterpret_cast<__nv_bfloat16 *>(dB), plane_a,
       plane_b, norms);
   MDG_TRY_LAUNCH();

@@ -1176,7 +1176,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS2, 1)
 // The diagonal GEMM over digit and sum planes (cross_sums.cuh).  Bound by the
 // tensor cores as the kernel above, at 224 instead of 406 products of planes
 // for quad-double: qd 8192^3 146 instead of 268 ms (1684 TFLOP/s done), od
-// 2048^3 8.5 instead of 16.4 ms, qd 1024^3 353 instead of 607 us.  Flush
+// 2048^3 8.5 instead of 16.4 ms, qd 1024^3 312 instead of 607 us.  Flush
 // groups of 16, 8 and 4 k-steps (whole, halves, quarters) cost 17.0, 17.9
 // and 27.7 ms on the same quad-double 4096 x 4096 x 2048 digit pairs: reading
 // the accumulators back takes about 4000 cycles, 4 k-steps of products 2048.
@@ -1525,9 +1525,8 @@ int encode_out_map(void *map128, const void *base, int Np, long long rows_total)
 }
 
 // The units of a table (numbered as the kernels number them) over the
-// workers, in the table's order, each to the worker with the least so far.  A
-// unit's cost in k-steps: its own, about 6 per run for the drain and the
-// store, about 10 to fill and empty the pipeline.  The table's order, dear
+// workers, in the table's order, each to the worker with the least so far.  The
+// table's order, dear
 // problems first and a problem's units in a row, keeps the workers on few
 // problems at a time.  ms a call, units in turn / dearest unit first / in the
 // table's order: 64 mixed problems of 32 .. 512 2.67 / 2.30 / 2.12, 256 of
