@@ -13,7 +13,11 @@ using mdgi::RENORM_THREADS;
 // doubles the threads and leaves more blocks their shared memory.  Two / one:
 // dd 16001 x 96 58 / 68 us, qd 8192 x 8192 (cross form) 6.8 / 7.6 ms, qd 1024
 // x 1024 92 / 92 us; with the prefix sums of 55 and 110 diagonals od 2048 x
-// 2048 1275 / 833, hd 1024 x 1024 1120 / 630 us.
+// 2048 1275 / 833, hd 1024 x 1024 1120 / 630 us.  Beyond 32 diagonals the kernel
+// that keeps no prefix sums, where each diagonal is one chunk: od 2048 x 2048
+// one column with prefix sums 690, without 691, two columns 593 us; hd 1024 x
+// 1024 549, 324, 296; but qd 2048 x 2048 308 (two columns), 350, 313, dd 3000 x
+// 3000 293, 459, 417.
 constexpr long long kTwoColumnEntries = 1 << 19;
 constexpr int kTwoColumnDiagonals = 32;
 
@@ -49,6 +53,23 @@ __global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 6 : 1)
   if (r >= m) return;
   mdgi::renorm_columns<V, mdgi::kCrossChunks>(P, 0, D, 0, planes, top, n, &counts, out, plane_c, ldcd, E,
                                               F, C, ldc, r, c0, wide, smem);
+}
+
+// The same where no diagonal has more than one chunk, without prefix sums in
+// shared memory: those of 110 diagonals left 12 warps on an SM.
+template <int V>
+__global__ void __launch_bounds__(RENORM_THREADS, V == 2 ? 5 : 8)
+    whole_renorm_kernel(int P, int D, int planes, int top, const __grid_constant__ mdgi::ChunkCounts counts,
+                        int m, int n, const int *__restrict__ out, long long plane_c, int ldcd,
+                        const int *__restrict__ E, const int *__restrict__ F,
+                        double *__restrict__ C, int ldc, bool wide) {
+  extern __shared__ uint4 smem[];
+  const int groups = (n + V - 1) / V;
+  const long long e = blockIdx.x * (long long)RENORM_THREADS + threadIdx.x;
+  const int r = (int)(e / groups), c0 = (int)(e - (long long)r * groups) * V;
+  if (r >= m) return;
+  mdgi::renorm_columns<V, mdgi::kCrossWhole>(P, 0, D, 0, planes, top, n, &counts, out, plane_c, ldcd, E,
+                                             F, C, ldc, r, c0, wide, smem);
 }
 
 // Every problem of a batch: block x belongs to the problem whose units hold x.
@@ -110,10 +131,11 @@ int launch_cross(int p, int D, int KB, int m, int n, const int *out, long long p
     counts.of[d] = mdgi::cross_chunks(d, counts.pairs_per_chunk);
     most = std::max(most, (int)counts.of[d]);
   }
-  const int smem = mdgi::renorm_smem(D, V, true);
-  MDG_TRY_CUDA(cudaFuncSetAttribute(cross_renorm_kernel<V>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  cross_renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
+  const bool whole = most <= 1 && D > kTwoColumnDiagonals;
+  const int smem = mdgi::renorm_smem(D, V, !whole);
+  const auto kernel = whole ? whole_renorm_kernel<V> : cross_renorm_kernel<V>;
+  MDG_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kernel<<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
       p, D, mdgi::cross_outputs(D, KB), mdgi::renorm_top(D, most + 1), counts, m, n, out, plane_c, ldcd, E, F, C, ldc,
       aligned16(C));
   MDG_TRY_LAUNCH();
@@ -139,7 +161,9 @@ int launch_cross_renorm(int p, int D, int KB, int m, int n, const int *out, long
                         cudaStream_t st) {
   if (m == 0 || n == 0) return MDG_SUCCESS;
   if (!words_for(1, D) || KB > CROSS_CHUNK_STEPS) return MDG_ERROR_NOT_SUPPORTED;
-  if (D <= kTwoColumnDiagonals && two_columns(m, n, out, plane_c, ldcd))
+  // 'whole', beyond kTwoColumnDiagonals: the last diagonal's pairs fit a chunk
+  const bool two = D <= kTwoColumnDiagonals || cross_pairs(D - 1) <= cross_pairs_per_chunk(KB);
+  if (two && two_columns(m, n, out, plane_c, ldcd))
     return launch_cross<2>(p, D, KB, m, n, out, plane_c, ldcd, E, F, C, ldc, st);
   return launch_cross<1>(p, D, KB, m, n, out, plane_c, ldcd, E, F, C, ldc, st);
 }

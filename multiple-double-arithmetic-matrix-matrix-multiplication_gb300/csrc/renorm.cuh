@@ -21,7 +21,10 @@
 //   sum over the chunk of A_i B_j + A_j B_i
 //     = S - sum_{i0 <= i < i1} P_i - sum_{d-i1 < j <= d-i0} P_j   (mod 2^32),
 // two differences of prefix sums Q_i = P_0 + .. + P_{i-1}; diagonal d has
-// its chunks, and P_{d/2} for even d.
+// its chunks, and P_{d/2} for even d.  Where a chunk holds all pairs of its
+// diagonal ("whole") that is S - Q_{d+1}, plus P_{d/2} for even d: Q_D is summed
+// first and reduced by P_d after diagonal d, at the price of loading the squares
+// again, which L2 then holds.
 #pragma once
 
 #include <stdint.h>
@@ -40,8 +43,9 @@ struct ChunkCounts {
 };
 
 // Where renorm_columns has the chunk counts from: chunks of CHUNK_STEPS
-// k-steps (a batch), a table, a table of the cross form.
-enum { kPlainChunks = 0, kTableChunks = 1, kCrossChunks = 2 };
+// k-steps (a batch), a table, a table of the cross form, one with at most one
+// chunk a diagonal.
+enum { kPlainChunks = 0, kTableChunks = 1, kCrossChunks = 2, kCrossWhole = 3 };
 
 // 32-bit pieces of W per column: the diagonals' (eight diagonals make two),
 // the carry out of them (two), two of sign.
@@ -186,7 +190,7 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
   using I = Ints<V>;
   using Vec = typename I::T;
   constexpr int T = RENORM_THREADS;
-  constexpr bool CROSS = CHUNKS == kCrossChunks;
+  constexpr bool CROSS = CHUNKS == kCrossChunks, WHOLE = CHUNKS == kCrossWhole;
   // chunks of a diagonal loaded ahead; four for small outputs (one column),
   // whose diagonals are cut into more chunks for the GEMM's sake
   constexpr int kAhead = CHUNKS == kTableChunks && V == 1 ? 4 : 2;
@@ -218,6 +222,18 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
     Q[D * T] = I::put(run);
   }
 
+  unsigned all[V];  // WHOLE: P_0 + .. + P_d of the diagonal at hand
+#pragma unroll
+  for (int v = 0; v < V; ++v) all[v] = 0;
+  if constexpr (WHOLE) {
+#pragma unroll 8
+    for (int i = 0; i < D; ++i) {
+      const Vec x = __ldcg(reinterpret_cast<const Vec *>(src + (size_t)i * plane_c));
+#pragma unroll
+      for (int v = 0; v < V; ++v) all[v] += (unsigned)I::get(x, v);
+    }
+  }
+
   long long carry[V];
   int lsb[V];
 #pragma unroll
@@ -229,6 +245,7 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
 #pragma unroll 1
   for (int wi = 0; wi < dwords; ++wi) {
     Vec x0[8], x1[8], x2[kAhead > 2 ? 8 : 1], x3[kAhead > 2 ? 8 : 1];
+    Vec p[WHOLE ? 8 : 1], mid[WHOLE ? 4 : 1];  // P_d; P_{d/2} of every other d
     int first[8], nc[8];
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
@@ -237,7 +254,11 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
       q -= nc[b];
       first[b] = q;
       if (nc[b] > 0) x0[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)q * plane_c));
-      if (nc[b] > 1)
+      if constexpr (WHOLE) {
+        if (d >= 0) p[b] = __ldcg(reinterpret_cast<const Vec *>(src + (size_t)d * plane_c));
+        if (d >= 0 && !(d & 1))
+          mid[b >> 1] = __ldcg(reinterpret_cast<const Vec *>(src + (size_t)(d / 2) * plane_c));
+      } else if (nc[b] > 1)
         x1[b] = __ldcs(reinterpret_cast<const Vec *>(src + (size_t)(q + 1) * plane_c));
       if constexpr (kAhead > 2) {
         if (nc[b] > 2)
@@ -259,7 +280,17 @@ __device__ __forceinline__ void renorm_columns(int P, int s, int D, int KB, int 
         const int b = 4 * half + j, d = D - 1 - (wi * 8 + b);
         if (d < 0) continue;
         const long long unit = 1ll << (8 * j);
-        if constexpr (CROSS) {
+        if constexpr (WHOLE) {
+          const bool even = !(d & 1);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const int square = even ? I::get(mid[b >> 1], v) : 0;
+            const unsigned sums = nc[b] ? (unsigned)I::get(x0[b], v) : 0u;
+            val[v] += square * unit;
+            val[v] += (int)(sums - all[v] + (unsigned)square) * unit;
+            all[v] -= (unsigned)I::get(p[b], v);
+          }
+        } else if constexpr (CROSS) {
           const bool even = !(d & 1);
           int square[V];  // P_{d/2}
           if (even) {

@@ -106,3 +106,19 @@ def test_dealt_sums_same_bits(p, m, n, k):
     assert torch.equal(got, api.gemm(A, B, parts=1))
     assert torch.equal(got, api.gemm(A, B, engine="tc"))
     assert api.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,m,n,k,kw", [
+    # the renormalisation without prefix sums: 33 diagonals and more, one chunk a
+    # diagonal; one and two columns a thread, odd columns; the k from which the
+    # longest diagonals have two chunks (28 pairs of 36 and 37 k-blocks)
+    (4, 1000, 777, 1024, {"slices": 33, "diagonals": 33}),
+    (8, 600, 611, 1024, {}), (8, 800, 777, 64 * 36, {}), (8, 800, 777, 64 * 37, {}),
+    (16, 600, 700, 700, {}), (16, 800, 801, 513, {})])
+def test_renorm_of_whole_diagonals(p, m, n, k, kw):
+    import torch
+    api = pkg("api")
+    A = api.generate("normal", p, m, k, 31, -9, 9, scale_rows=True)
+    B = api.generate("uniform", p, k, n, 32)
+    assert torch.equal(api.gemm(A, B, **kw), api.gemm(A, B, engine="tc", **kw))
