@@ -56,6 +56,18 @@ bool alloc_over_limit(size_t bytes);
     if (mdg_s_ != MDG_SUCCESS) return mdg_s_; \
   } while (0)
 
+namespace mdgi {
+// Lets blocks of `kernel` have up to `most` bytes of dynamic shared memory.
+// The limit belongs to the kernel, not to a launch: all host threads share it,
+// and one that lowers it to its own call's size has another's launch refused.
+// So `most` is the same at every call, what the largest accepted call needs.
+template <class Kernel>
+int allow_smem(Kernel kernel, int most) {
+  MDG_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  return MDG_SUCCESS;
+}
+}  // namespace mdgi
+
 // Internal launchers (one translation unit each); all return mdg_status.
 namespace mdgi {
 int launch_plain_gemm(int p, int m, int n, int k, const double *A, int lda, const double *B,

@@ -5,10 +5,13 @@
 
 #include "common.cuh"
 #include "cross_sums.cuh"
+#include "slice_tc.cuh"
 
 namespace {
 
 constexpr int SUM_WARPS = 8;
+// 16-byte vectors of a digit row's window: at most 8 k-steps of 64 BF16
+constexpr int MAX_WINDOW = 64;
 
 // a + b of two BF16 pairs, exact for integers of magnitude <= 128 each
 __device__ __forceinline__ uint32_t add_pair(uint32_t a, uint32_t b) {
@@ -94,11 +97,10 @@ namespace mdgi {
 int launch_cross_sums(int s, int dlo, int dhi, int Kp, int rows_a, int rows_b, void *dA, void *dB,
                       long long plane_a, long long plane_b, unsigned *norms, cudaStream_t st) {
   const int KB = Kp / 64, windows = 2 * cross_groups(KB);
-  // 16-byte vectors of the longest window (at most 8 k-steps of 64 BF16)
+  // vectors of the longest window
   const int stride = (KB + windows - 1) / windows * 8;
   const int smem = dhi * stride * 16;
-  MDG_TRY_CUDA(cudaFuncSetAttribute(cross_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    smem));
+  MDG_TRY(allow_smem(cross_sums_kernel, MAX_DIAGONALS * MAX_WINDOW * 16));
   cross_sums_kernel<<<dim3(rows_a + rows_b, windows), 32 * SUM_WARPS, smem, st>>>(
       s, cross_offset(dlo), cross_offset(dhi), dhi, KB, windows, stride, rows_a,
       reinterpret_cast<__nv_bfloat16 *>(dA), reinterpret_cast<__nv_bfloat16 *>(dB), plane_a,

@@ -159,9 +159,9 @@ int launch_plain_gemm(int p, int m, int n, int k, const double *A, int lda, cons
 int launch_plain_batched(const mdg_problem *dev_problems, int count, int max_p,
                          const int *dev_tile_starts, int total_tiles, cudaStream_t st) {
   if (total_tiles == 0) return MDG_SUCCESS;
-  const size_t smem = 2 * T * T * (size_t)max_p * sizeof(double);
-  MDG_TRY_CUDA(cudaFuncSetAttribute(plain_batched_kernel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr size_t entry = 2 * T * T * sizeof(double);
+  const size_t smem = entry * max_p;
+  MDG_TRY(allow_smem(plain_batched_kernel, (int)entry * 16));
   int dev = 0, sms = 0, per_sm = 0;
   MDG_TRY_CUDA(cudaGetDevice(&dev));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -65,7 +65,10 @@ SlicePlan block_slice_plan(int p, int s, int D, int m, int n, int k);
 // Tiles of the single-CTA kernel for small problems of up to 128 rows or
 // columns: 128 rows by tn columns over the valid part (0: CTA pairs).
 int narrow_tile(int s, int D, int m, int n, int KB);
+// 64-bit words for s digits and D diagonals, 0 where they are too many: no call
+// comes with more than MAX_SLICES and MAX_DIAGONALS.
 int words_for(int s, int D);
+constexpr int MAX_SLICES = 119, MAX_DIAGONALS = 112;
 
 // The FP64-DMMA slice-digit form (digits64.cu): default digits per P
 // (19-bit), integer words, workspace layout and the whole GEMM.

@@ -1,0 +1,63 @@
+"""What the library asks of the CUDA runtime, on a runtime made for the purpose
+(tests/cpp/fake_cudart.cpp): no GPU, no kernel runs."""
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT, pkg
+
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    lib = pkg("_lib").LIB_PATH
+    if not os.path.exists(lib):
+        pkg("build").build()
+    out = str(tmp_path_factory.mktemp("fake") / "fake_cudart")
+    libdir = os.path.dirname(lib)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-rdynamic", "-I", os.path.join(ROOT, "include"),
+                    "-I", os.path.join(CUDA, "include"),
+                    os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), "-L", libdir,
+                    "-lmdgemm", "-Wl,-rpath," + libdir, "-Wl,--allow-shlib-undefined", "-o", out],
+                   check=True, capture_output=True)
+
+    def run(*words, **env):
+        r = subprocess.run([out] + [str(w) for w in words], capture_output=True, text=True,
+                           timeout=120, env={**os.environ, **env})
+        assert r.returncode == 0, r.stderr[-2000:]
+        return [line.split() for line in r.stdout.splitlines()]
+
+    return run
+
+
+def _statuses(lines):
+    return [int(line[2]) for line in lines if line[0] == "status"]
+
+
+def test_a_kernels_shared_memory_limit_is_the_same_at_every_call(fake):
+    """The limit belongs to the kernel and all host threads share it: one that
+    set its own call's size would have the launches of others refused."""
+    words = []
+    for p in (2, 4, 8, 16):
+        for shape in ((64, 64, 64), (256, 100, 90), (1024, 1024, 512), (600, 700, 1024),
+                      (3000, 64, 100), (900, 900, 20000)):
+            words += ["gemm", 2, p, *shape]
+        words += ["batch", p, 64, 96, 65, "batched", 0, p, 10, 20, 30, "gemm", 3, p, 50, 60, 70,
+                  "gemm", 0, p, 50, 60, 70]
+    words += ["digits", 119, 112, "gemm", 2, 16, 64, 64, 64, "gemm", 2, 16, 1024, 1024, 1024]
+    words += ["gemm", 2, 16, 1024, 1024, 20000]
+    lines = fake(*words)
+    assert set(_statuses(lines)) == {0}
+    limits, launches = {}, {}
+    for line in lines:
+        if line[0] == "limit":
+            limits.setdefault(line[1], set()).add(int(line[2]))
+        elif line[0] == "launch":
+            launches[line[1]] = max(launches.get(line[1], 0), int(line[2]))
+    assert len(limits) >= 15
+    assert {k: v for k, v in limits.items() if len(v) > 1} == {}
+    for kernel, smem in launches.items():
+        assert smem <= max(limits.get(kernel, {48 * 1024})), kernel
+    assert max(max(v) for v in limits.values()) <= 227 * 1024
