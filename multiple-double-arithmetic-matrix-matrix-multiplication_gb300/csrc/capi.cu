@@ -106,10 +106,7 @@ struct DeviceCache {
       ptr[slot] = nullptr;
       cap[slot] = 0;
       cudaError_t e = cudaMalloc(&ptr[slot], bytes);
-      if (e != cudaSuccess) {
-        set_cuda_error(e);
-        return MDG_ERROR_ALLOCATION;
-      }
+      if (e != cudaSuccess) return allocation_failed(e);
       cap[slot] = bytes;
     }
     *out = ptr[slot];
@@ -522,9 +519,8 @@ int mdg_host_alloc(size_t bytes, void **out) {
   if (alloc_over_limit(bytes)) return MDG_ERROR_ALLOCATION;
   cudaError_t e = cudaHostAlloc(out, bytes ? bytes : 1, cudaHostAllocPortable);
   if (e != cudaSuccess) {
-    set_cuda_error(e);
     *out = nullptr;
-    return MDG_ERROR_ALLOCATION;
+    return allocation_failed(e);
   }
   return MDG_SUCCESS;
 }

@@ -66,6 +66,15 @@ int allow_smem(Kernel kernel, int most) {
   MDG_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   return MDG_SUCCESS;
 }
+
+// An allocation that failed with e: its text is kept and the thread's last error
+// cleared, which the check after the next launch would otherwise take for the
+// launch's own.
+inline int allocation_failed(cudaError_t e) {
+  set_cuda_error(e);
+  cudaGetLastError();
+  return MDG_ERROR_ALLOCATION;
+}
 }  // namespace mdgi
 
 // Internal launchers (one translation unit each); all return mdg_status.

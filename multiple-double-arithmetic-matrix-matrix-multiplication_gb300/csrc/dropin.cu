@@ -29,7 +29,11 @@ namespace {
 struct DevBuf {
   double *p = nullptr;
   explicit DevBuf(size_t n) {
-    if (n && cudaMalloc(&p, n * sizeof(double)) != cudaSuccess) p = nullptr;
+    const cudaError_t e = n ? cudaMalloc(&p, n * sizeof(double)) : cudaSuccess;
+    if (e != cudaSuccess) {
+      mdgi::allocation_failed(e);
+      p = nullptr;
+    }
   }
   ~DevBuf() {
     if (p) cudaFree(p);

@@ -199,14 +199,11 @@ int mdg_plan_create(int form, int p, int m, int n, int k, const mdg_options *opt
   if (st == MDG_SUCCESS && bytes) {
     cudaError_t e = cudaMalloc(&h->ws, bytes);
     if (e == cudaErrorMemoryAllocation && least < bytes) {
-      cudaGetLastError();  // handled: the smaller workspace gives the same bits
+      mdgi::allocation_failed(e);  // handled: the smaller workspace gives the same bits
       bytes = least;
       e = cudaMalloc(&h->ws, bytes);
     }
-    if (e != cudaSuccess) {
-      mdgi::set_cuda_error(e);
-      st = MDG_ERROR_ALLOCATION;
-    }
+    if (e != cudaSuccess) st = mdgi::allocation_failed(e);
     h->bytes = bytes;
   }
   if (st != MDG_SUCCESS) {

@@ -61,3 +61,21 @@ def test_a_kernels_shared_memory_limit_is_the_same_at_every_call(fake):
     for kernel, smem in launches.items():
         assert smem <= max(limits.get(kernel, {48 * 1024})), kernel
     assert max(max(v) for v in limits.values()) <= 227 * 1024
+
+
+@pytest.mark.parametrize("p,m,n,k,operands", [
+    (4, 1024, 1024, 1024, 3 << 25),      # one workspace, 1.1 GiB with the sum planes
+    (2, 2048, 256, 300, 0),              # row panels: nothing to fall back to
+])
+def test_host_entry_after_an_allocation_that_failed(fake, p, m, n, k, operands):
+    """A workspace with sum planes that the device has no room for: the call
+    runs over digit pairs, and the failed allocation's error is not taken for
+    that of a launch.  Without room for those either, the call says so and the
+    next one that fits succeeds."""
+    least = pkg("_lib").lib().mdg_gemm_least_workspace_size(2, p, m, n, k, None)
+    if operands:
+        lines = fake("capacity", operands + least, "host", p, m, n, k)
+        assert ["oom"] in [line[:1] for line in lines] and _statuses(lines) == [0]
+    lines = fake("capacity", 24 << 20, "host", p, m, n, k, "host", 2, 32, 32, 32, "plan", p, m, n, k,
+                 "gemm", 2, 2, 32, 32, 32)
+    assert _statuses(lines) == [9, 0, 9, 0]  # 9: allocation failed
