@@ -83,12 +83,16 @@ struct DeviceCache {
       if (!ev) MDG_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     return MDG_SUCCESS;
   }
-  void release_locked() {
-    for (int i = 0; i < 3 + kMaxStrips; ++i) {
+  // frees the buffers of `slot` and of the slots after it
+  void drop(int slot) {
+    for (int i = slot; i < 3 + kMaxStrips; ++i) {
       if (ptr[i]) cudaFree(ptr[i]);
       ptr[i] = nullptr;
       cap[i] = 0;
     }
+  }
+  void release_locked() {
+    drop(0);
     for (auto &st : streams) {
       if (st) cudaStreamDestroy(st);
       st = nullptr;
@@ -98,6 +102,8 @@ struct DeviceCache {
       ev = nullptr;
     }
   }
+  // A call takes its slots in order: where memory is short, the ones after
+  // `slot` hold what earlier calls left and are given back first.
   int get(int slot, size_t bytes, void **out) {
     if (bytes == 0) bytes = 256;
     if (alloc_over_limit(bytes)) return MDG_ERROR_ALLOCATION;
@@ -106,7 +112,15 @@ struct DeviceCache {
       ptr[slot] = nullptr;
       cap[slot] = 0;
       cudaError_t e = cudaMalloc(&ptr[slot], bytes);
-      if (e != cudaSuccess) return allocation_failed(e);
+      if (e != cudaSuccess) {
+        allocation_failed(e);
+        drop(slot);
+        e = cudaMalloc(&ptr[slot], bytes);
+      }
+      if (e != cudaSuccess) {
+        ptr[slot] = nullptr;
+        return allocation_failed(e);
+      }
       cap[slot] = bytes;
     }
     *out = ptr[slot];
@@ -326,8 +340,13 @@ static int host_slice_panels_issue(int p, const Opts &o, int m, int n, int k, co
   bool sums = engine == 1 || engine == 3;
   for (int j = 0; j < strips && sums; ++j) {
     pls[j] = block_slice_plan(p, o.slices, o.diagonals, mp, std::min(ns, n - j * ns), k);
-    sums = pls[j].sums && g_cache.get(3 + j, pls[j].total, &ws[j]) == MDG_SUCCESS;
+    sums = pls[j].sums != 0;
   }
+  for (int j = 0; j < strips && sums; ++j)
+    if (g_cache.get(3 + j, pls[j].total, &ws[j]) != MDG_SUCCESS) {
+      g_cache.drop(3);  // the pairs of all strips may fit in what the first ones got
+      sums = false;
+    }
   for (int j = 0; j < strips; ++j) {
     if (!sums) pls[j] = make_slice_plan(p, o.slices, o.diagonals, mp, std::min(ns, n - j * ns), k);
     if (pls[j].Mp > 65535 || pls[j].Np > 65535) return MDG_ERROR_NOT_SUPPORTED;

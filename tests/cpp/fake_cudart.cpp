@@ -144,7 +144,7 @@ cudaError_t cudaFuncSetAttribute(const void *fun, enum cudaFuncAttribute, int va
 }
 
 cudaError_t cudaMalloc(void **p, size_t bytes) {
-  if (bytes > capacity - in_use) {
+  if (in_use + bytes > capacity) {
     std::printf("oom %zu\n", bytes);
     *p = nullptr;
     return last_error = cudaErrorMemoryAllocation;

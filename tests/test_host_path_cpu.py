@@ -79,3 +79,20 @@ def test_host_entry_after_an_allocation_that_failed(fake, p, m, n, k, operands):
     lines = fake("capacity", 24 << 20, "host", p, m, n, k, "host", 2, 32, 32, 32, "plan", p, m, n, k,
                  "gemm", 2, 2, 32, 32, 32)
     assert _statuses(lines) == [9, 0, 9, 0]  # 9: allocation failed
+
+
+def test_host_entry_gives_back_memory_that_it_does_not_use(fake):
+    """Two column strips.  Room for one strip's sum planes but not for two:
+    both strips run over digit pairs, in the room the first one had.  And a
+    call that finds the device filled by an earlier call's workspaces."""
+    p, m, n, k = 2, 2048, 4096, 1024
+    operands = 8 * p * (m * k + k * n + m * n)
+    sums = [int(line[1]) for line in fake("host", p, m, n, k) if line[0] == "malloc"][3:]
+    pairs = pkg("_lib").lib().mdg_gemm_least_workspace_size(2, p, 1024, 2048, k, None)
+    assert len(sums) == 2 and sums[0] + pairs > sums[0] + (16 << 20) > 2 * pairs
+    room = operands + sums[0] + (16 << 20)
+    lines = fake("capacity", room, "host", p, m, n, k)
+    assert _statuses(lines) == [0]
+    assert [int(line[1]) for line in lines if line[0] == "malloc"][-2:] == [pairs, pairs]
+    lines = fake("host", p, m, n, k, "capacity", room + (1 << 20), "host", p, m, n + 8, k)
+    assert _statuses(lines) == [0, 0]
