@@ -329,10 +329,12 @@ int mdg_renorm_diagonals(int p, int s, int D, int k, int m, int n,
  * schedule it runs with.  mdg_plan_tune times the schedules that give the
  * same bits (BF16 form: CTA pairs with diagonal ranges per tile auto / 1 /
  * 2 / 4, tile strips 4 or 16 column blocks wide, pacing windows 32 or 128
- * k-steps or none, and the single-CTA engine) on the caller's operands, keeps the
+ * k-steps or none, the single-CTA engine, and the automatic engine where it has
+ * tiles of its own) on the caller's operands, keeps the
  * fastest, and records it in the library's tuning cache under the device
  * (GPU name and driver version) and the shape class (form, P, digits,
- * padded m, n, k); plans created later for the same class start from the
+ * padded m, n, k, and the automatic tiles where they follow the valid m and n);
+ * plans created later for the same class start from the
  * cached schedule.  Other forms have nothing to tune.  The cache persists
  * as a JSON file through mdg_tune_cache_save / mdg_tune_cache_load. */
 typedef struct mdg_plan_s *mdg_plan;

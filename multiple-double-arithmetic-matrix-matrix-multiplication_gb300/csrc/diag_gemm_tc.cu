@@ -1467,9 +1467,9 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
     return MDG_ERROR_INVALID_SIZE;
   if (plane_c != (long long)Mp * Np) return MDG_ERROR_INVALID_SIZE;
   // the CTA-pair kernel needs 256-row tiles
-  const int narrow = engine == 1 ? narrow_tile(s, D, m, n, Kp / TK) : 0;
-  const bool pair = Mp % 256 == 0 && engine != 2 && !narrow;
-  const int tn = narrow ? narrow : TN;
+  const AutoTiles own = engine == 1 ? auto_tiles(s, D, m, n, Kp / TK, cs) : AutoTiles{};
+  const bool pair = Mp % 256 == 0 && engine != 2 && !own.narrow;
+  const int tn = own.narrow ? own.narrow : TN;
   const int runs = total_chunks(s, D, Kp / TK, cs);
   CUtensorMap ma, mb, mc;
   MDG_TRY(make_out_map(&mc, chunks, Np, (long long)runs * Mp));
@@ -1487,8 +1487,7 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (pair) {
-    const int stack =
-        cs == CHUNK_STEPS && engine == 1 ? stacked_tiles(s, D, m, n, Kp / TK) : kStackNone;
+    const int stack = own.stack;
     const int mt = stack == kStackM ? (m + 127) / 128 : Mp / 256;
     const int nt = stack == kStackN ? (n + 127) / 128 : Np / TN2;
     const int separable = stack ? (D + 1) / 2 : runs;

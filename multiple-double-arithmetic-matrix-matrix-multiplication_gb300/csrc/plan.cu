@@ -5,16 +5,19 @@
 // the BF16 slice-digit form, mdg_plan_tune times the schedules that return
 // the same bits (the CTA-pair engine with 0 = auto, 1, 2 or 4 diagonal ranges
 // per tile, tile strips 4 or 16 column blocks wide, pacing windows of 32 and
-// 128 k-steps or none, and the single-CTA engine) on the caller's own
-// operands and keeps
+// 128 k-steps or none, the single-CTA engine, and the automatic choice where
+// that has tiles of its own) on the caller's own operands and keeps
 // the fastest.  Choices live in a process-wide cache keyed by device ("<GPU
 // name>|<driver version>") and shape class ("<form> <P> <s> <D> <Mp> <Np>
-// <Kp>", the padded sizes the kernels see); mdg_tune_cache_save / _load keep
+// <Kp>", the padded sizes the kernels see; where the automatic tiles follow the
+// valid sizes too, " narrow <columns>" or " stack <side>" and m and n in units
+// of 128 behind them); mdg_tune_cache_save / _load keep
 // it as a small JSON file.  Slice and diagonal counts change the rounding, so
 // they stay the caller's options and are part of the key, not tuned.  The
 // batched plan (batched.cu) records its tile policy and split mode here
 // too, under "batch <count> <hash of the problem shapes>".
 #include <cctype>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -46,6 +49,15 @@ int device_key(std::string *out) {
   return MDG_SUCCESS;
 }
 
+// The automatic engine's own tiles for a problem that runs in `bytes` of
+// workspace.
+mdgi::AutoTiles own_tiles(int p, int s, int D, int m, int n, int k, size_t bytes) {
+  if (m == 0 || n == 0 || k == 0) return mdgi::AutoTiles{};
+  mdgi::SlicePlan pl = mdgi::best_slice_plan(p, s, D, m, n, k);
+  if (bytes < pl.total) pl = mdgi::make_slice_plan(p, s, D, m, n, k);
+  return pl.sums ? mdgi::AutoTiles{} : mdgi::auto_tiles(s, D, m, n, pl.Kp / 64, pl.cs);
+}
+
 std::string shape_key(int form, int p, int m, int n, int k, const mdg_options *opt) {
   const int s = (opt && opt->slices) ? opt->slices
                 : form == MDG_FORM_FP64_DIGITS ? mdg_default_fp64_digits(p)
@@ -53,7 +65,14 @@ std::string shape_key(int form, int p, int m, int n, int k, const mdg_options *o
   const int D = (opt && opt->diagonals) ? opt->diagonals : s;
   const mdgi::SlicePlan pl = mdgi::make_slice_plan(p, s, D, m, n, k);
   char buf[160];
-  std::snprintf(buf, sizeof(buf), "%d %d %d %d %d %d %d", form, p, s, D, pl.Mp, pl.Np, pl.Kp);
+  int len = std::snprintf(buf, sizeof(buf), "%d %d %d %d %d %d %d", form, p, s, D, pl.Mp, pl.Np, pl.Kp);
+  // a 256 x 256 class holds problems that waste less on other tiles and ones that
+  // do not (n = 96 and n = 256)
+  const mdgi::AutoTiles own =
+      form == MDG_FORM_SLICE_BF16 ? own_tiles(p, s, D, m, n, k, SIZE_MAX) : mdgi::AutoTiles{};
+  if (own.narrow || own.stack)
+    std::snprintf(buf + len, sizeof(buf) - len, " %s %d %d %d", own.narrow ? "narrow" : "stack",
+                  own.narrow ? own.narrow : own.stack, (m + 127) / 128, (n + 127) / 128);
   return buf;
 }
 
@@ -234,10 +253,17 @@ int mdg_plan_tune(mdg_plan plan, const double *A, int lda, const double *B, int 
   mdgi::NvtxRange range("mdg plan tune");
   // schedules with the same bits: CTA pairs (engine 2) with parts auto / 1 /
   // 2 / 4, tile strips of 4 and 16 column blocks, pacing windows 32, 128 and
-  // off, and single CTAs (engine 1): {engine, parts, raster, pace}
-  const int cand[10][4] = {{2, 0, 0, 0},  {2, 1, 0, 0},   {2, 2, 0, 0},  {2, 4, 0, 0},
+  // off, single CTAs (engine 1), and the automatic choice (0) where it is none
+  // of these: {engine, parts, raster, pace}.  A forced engine has no narrow tiles
+  // and no stacked diagonals (us: dd 16001 x 96 x 3001 2292 forced, 1594
+  // automatic; od 8000 x 100 x 2000 9628 and 4711).
+  const int cand[11][4] = {{2, 0, 0, 0},  {2, 1, 0, 0},   {2, 2, 0, 0},  {2, 4, 0, 0},
                            {2, 0, 4, 0},  {2, 0, 16, 0},  {2, 0, 0, 32}, {2, 0, 0, 128},
-                           {2, 0, 0, -1}, {1, 0, 0, 0}};
+                           {2, 0, 0, -1}, {1, 0, 0, 0},   {0, 0, 0, 0}};
+  const int s = plan->opt.slices ? plan->opt.slices : mdg_default_slices(plan->p);
+  const mdgi::AutoTiles own = own_tiles(plan->p, s, plan->opt.diagonals ? plan->opt.diagonals : s,
+                                        plan->m, plan->n, plan->k, plan->bytes);
+  const int choices = own.narrow || own.stack ? 11 : 10;
   cudaStream_t st = mdgi::as_stream(stream);
   cudaEvent_t e0, e1;
   MDG_TRY_CUDA(cudaEventCreate(&e0));
@@ -245,7 +271,8 @@ int mdg_plan_tune(mdg_plan plan, const double *A, int lda, const double *B, int 
   mdg_options best = plan->opt;
   float best_ms = 0.0f;
   int status = MDG_SUCCESS;
-  for (const auto &c : cand) {
+  for (int i = 0; i < choices; ++i) {
+    const int *c = cand[i];
     mdg_options o = plan->opt;
     o.engine = c[0];
     o.parts = c[1];

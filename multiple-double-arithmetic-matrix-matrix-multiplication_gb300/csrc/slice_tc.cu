@@ -351,6 +351,11 @@ int narrow_tile(int s, int D, int m, int n, int KB) {
   return tn;
 }
 
+AutoTiles auto_tiles(int s, int D, int m, int n, int KB, int cs) {
+  const int narrow = narrow_tile(s, D, m, n, KB);
+  return AutoTiles{narrow, !narrow && cs == CHUNK_STEPS ? stacked_tiles(s, D, m, n, KB) : 0};
+}
+
 // Measured, chunks of 2032 k-steps and at most 8 parts / this: qd 256^3 107 /
 // 28 us for the GEMM (plan 136 / 61 us a call), dd 64^3 26 / 11 us.
 //

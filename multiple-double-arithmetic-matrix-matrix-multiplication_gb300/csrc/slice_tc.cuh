@@ -65,6 +65,13 @@ SlicePlan block_slice_plan(int p, int s, int D, int m, int n, int k);
 // Tiles of the single-CTA kernel for small problems of up to 128 rows or
 // columns: 128 rows by tn columns over the valid part (0: CTA pairs).
 int narrow_tile(int s, int D, int m, int n, int KB);
+// What engine 1 makes of a plan over digit pairs beyond 256 x 256 tiles: narrow
+// tiles, or two diagonals an accumulator (stacked_tiles; chunks of CHUNK_STEPS).
+// The forced engines have neither.
+struct AutoTiles {
+  int narrow, stack;
+};
+AutoTiles auto_tiles(int s, int D, int m, int n, int KB, int cs);
 // 64-bit words for s digits and D diagonals, 0 where they are too many: no call
 // comes with more than MAX_SLICES and MAX_DIAGONALS.
 int words_for(int s, int D);

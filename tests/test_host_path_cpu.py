@@ -96,3 +96,37 @@ def test_host_entry_gives_back_memory_that_it_does_not_use(fake):
     assert [int(line[1]) for line in lines if line[0] == "malloc"][-2:] == [pairs, pairs]
     lines = fake("host", p, m, n, k, "capacity", room + (1 << 20), "host", p, m, n + 8, k)
     assert _statuses(lines) == [0, 0]
+
+
+def _schedules(lines):
+    return [tuple(int(v) for v in line[3:]) for line in lines if line[0] == "status"
+            and line[1] in ("plan", "tune")]
+
+
+@pytest.mark.parametrize("p,m,n,k,wide_m,wide_n", [
+    (2, 16001, 96, 3001, 16001, 256),   # two diagonals an accumulator
+    (8, 100, 20000, 100, 256, 20000),
+    (4, 100, 100, 500, 256, 256),       # tiles of 128 columns
+])
+def test_tuning_can_keep_the_automatic_tiles(fake, tmp_path, p, m, n, k, wide_m, wide_n):
+    """The runtime times tiles that only the automatic engine has as the fastest:
+    a tuned plan keeps them, later plans of the shape too, and records of the
+    padded sizes (older files, wider problems) do not apply to it."""
+    import json
+    own, wide = (p, m, n, k), (p, wide_m, wide_n, k)
+    out = tmp_path / "tune.json"
+    lines = fake("tune", *own, "plan", *own, "plan", *wide, "save", out)
+    assert _schedules(lines) == [(0, 0, 0, 0)] * 3
+    key = list(json.loads(out.read_text())["fake|1"])
+    assert len(key) == 1
+    old = tmp_path / "old.json"
+    padded = " ".join(key[0].split()[:7])
+    assert padded != key[0]
+    old.write_text(json.dumps({"fake|1": {padded: {"engine": 1, "parts": 2, "raster": 0,
+                                                   "pace": 0, "ms": 1.0}}}))
+    assert _schedules(fake("load", old, "plan", *own, "plan", *wide)) == [(0,) * 4, (1, 2, 0, 0)]
+
+
+def test_tuning_of_ordinary_shapes_picks_an_engine(fake):
+    lines = fake("tune", 4, 1024, 768, 512, "plan", 4, 1000, 700, 500)
+    assert _schedules(lines) == [(2, 0, 0, 0)] * 2
