@@ -1247,8 +1247,11 @@ int make_out_map(CUtensorMap *m, const void *base, int Np, long long rows_total)
 }
 
 // How one launch of a pair kernel runs: work units, tile order, pacing.
+// as_asked: the parts or a pacing window are the caller's (or MDG_TC_PACE's), so
+// the units are taken in turn.
 struct PairSchedule {
   int clusters, parts, raster, pace, no_loads;
+  bool as_asked;
   uint32_t epoch;
 };
 
@@ -1389,9 +1392,11 @@ PairSchedule pair_schedule(int mt, int nt, int runs, int sms, int parts_opt, int
   // drift to correct there and only costs (qd 1024^3: 7 % slower paced), so
   // the default turns it off; an explicit window still applies.
   sc.pace = units <= ncl ? 0 : kDefaultPace;
-  if (const char *e = std::getenv("MDG_TC_PACE")) sc.pace = std::max(0, std::atoi(e));
+  const char *e = std::getenv("MDG_TC_PACE");
+  if (pace_opt == 0 && e) pace_opt = std::atoi(e) > 0 ? std::atoi(e) : -1;
   if (pace_opt > 0) sc.pace = pace_opt;
   if (pace_opt < 0) sc.pace = 0;
+  sc.as_asked = parts_opt > 0 || pace_opt > 0;
   static std::atomic<uint32_t> epochs{0};
   sc.epoch = ++epochs;
   if (sc.epoch == 0) sc.epoch = ++epochs;
@@ -1429,7 +1434,7 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
   UnitDeal deal = {};
   bool dealt = false;
   const int products = squares + cross_offset(dhi) - cross_offset(dlo);
-  if (parts <= 0 && pace <= 0 &&
+  if (!sc.as_asked &&
       (long long)tiles * products * KB <= kCrossDealSteps * (sms / 2)) {
     auto cost = [&](int part, int of) -> long long {
       const CrossRuns r =
@@ -1496,8 +1501,7 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
     auto cost = [&](int part, int parts) {
       return unit_cost(part_runs(s, D, Kp / TK, cs, stack, part, parts));
     };
-    // a schedule that the caller asks for is kept
-    const bool dealt = parts_opt <= 0 && pace_opt <= 0 &&
+    const bool dealt = !sc.as_asked &&
                        deal_single(mt * nt, separable, cost, sms / 2, &sc, &deal);
     diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
         ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, stack, (k - (Kp - TK) + 15) / 16, mt, nt, sc.parts,

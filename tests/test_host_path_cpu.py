@@ -130,3 +130,19 @@ def test_tuning_can_keep_the_automatic_tiles(fake, tmp_path, p, m, n, k, wide_m,
 def test_tuning_of_ordinary_shapes_picks_an_engine(fake):
     lines = fake("tune", 4, 1024, 768, 512, "plan", 4, 1000, 700, 500)
     assert _schedules(lines) == [(2, 0, 0, 0)] * 2
+
+
+@pytest.mark.parametrize("shape", [(4, 1024, 1024, 1024), (2, 16001, 96, 3001)])
+def test_pacing_window_of_the_environment(fake, shape):
+    """MDG_TC_PACE sets the window on the launches whose units would otherwise be
+    dealt by cost, as mdg_options.pace does; 0 and no value leave them dealt."""
+    def schedules(**env):
+        lines = [line[3:] for line in fake("gemm", 2, *shape, **env)
+                 if line[0] == "launch" and line[1].startswith("diag_gemm")]
+        return [dict(word.split("=") for word in line) for line in lines]
+
+    for env in ({}, {"MDG_TC_PACE": "0"}):
+        for s in schedules(**env):
+            assert (s["pace"], s["dealt"]) == ("0", "1"), env
+    for s in schedules(MDG_TC_PACE="96"):
+        assert (s["pace"], s["dealt"]) == ("96", "0")
