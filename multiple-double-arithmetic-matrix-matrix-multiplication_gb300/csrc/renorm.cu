@@ -18,7 +18,14 @@ using mdgi::RENORM_THREADS;
 // one column with prefix sums 690, without 691, two columns 593 us; hd 1024 x
 // 1024 549, 324, 296; but qd 2048 x 2048 308 (two columns), 350, 313, dd 3000 x
 // 3000 293, 459, 417.
-constexpr long long kTwoColumnEntries = 1 << 19;
+//
+// From 2^17 entries on.  The kernel alone, one / two: dd 14 diagonals 512 x 512
+// 18.5 / 10.4, 256 x 512 11.1 / 8.3 us; qd 28 of them 512 x 512 31.9 / 18.4, 256 x
+// 512 18.5 / 12.4, 256 x 256 12.1 / 10.3.  But problems below cut their diagonals
+// into short chunks, which one column loads four at a time: whole calls qd 256^3
+// 57.4 / 59.4, 128^3 49.3 / 53.2, od 128^3 63.7 / 69.8, qd 400^3 122 / 110, 700 x
+// 700 x 256 172 / 142, hd 500 x 500 x 70 425 / 378.
+constexpr long long kTwoColumnEntries = 1 << 17;
 constexpr int kTwoColumnDiagonals = 32;
 
 // Threads run over the rows' groups of V columns, row after row.  (Blocks per

@@ -14,6 +14,7 @@
 //   tune P M N K             the same with mdg_plan_tune before
 //   batch P M N K            mdg_batch_create and mdg_batch_run of one problem
 //   batched FORM P M N K     mdg_gemm_batched of one problem
+//   renorm P M N K           mdg_renorm_diagonals, default digits
 //   save PATH / load PATH    the tuning cache
 // and prints, a line each:
 //   limit KERNEL BYTES       cudaFuncAttributeMaxDynamicSharedMemorySize
@@ -274,6 +275,11 @@ int main(int argc, char **argv) {
         if (status == 0 && cmd == "tune") status = mdg_plan_tune(plan, dev, k, dev, n, dev_out, n, nullptr);
         if (status == 0) mdg_plan_schedule(plan, &o);
         mdg_plan_destroy(plan);
+      } else if (cmd == "renorm") {
+        const int s = mdg_default_slices(p);
+        const int *in = reinterpret_cast<const int *>(dev);
+        status = mdg_renorm_diagonals(p, s, s, k, m, n, in, (long long)m * n, n, in, in, dev_out, n,
+                                      nullptr);
       } else if (cmd == "batch") {
         const mdg_problem q{p, m, n, k, dev, dev, dev_out, k, n, n};
         mdg_batch batch = nullptr;

@@ -146,3 +146,12 @@ def test_pacing_window_of_the_environment(fake, shape):
             assert (s["pace"], s["dealt"]) == ("0", "1"), env
     for s in schedules(MDG_TC_PACE="96"):
         assert (s["pace"], s["dealt"]) == ("96", "0")
+
+
+@pytest.mark.parametrize("m,n,columns", [(512, 512, 2), (256, 512, 2), (255, 512, 1),
+                                         (512, 513, 1), (700, 900, 2)])
+def test_renormalisation_takes_two_columns_a_thread(fake, m, n, columns):
+    """From 2^17 entries on, where rows of the chunk planes are aligned for it."""
+    for p in (2, 4, 8):
+        names = [line[1] for line in fake("renorm", p, m, n, 500) if line[0] == "launch"]
+        assert names == [f"renorm_kernelILi{columns}EEE"]

@@ -39,3 +39,11 @@ def test_renorm_word_edges(orc, p, D, k):
                                        (8, 55, 524, 1002, 64)])
 def test_renorm_two_columns(orc, p, D, m, n, k):
     _check(orc, p, D, k, m, n, D)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,D,m,n,k", [(4, 28, 256, 512, 5000), (4, 28, 255, 514, 5000),
+                                       (2, 14, 361, 364, 64), (8, 55, 257, 511, 300)])
+def test_renorm_where_two_columns_begin(orc, p, D, m, n, k):
+    """Around 2^17 entries, odd rows of planes among them."""
+    _check(orc, p, D, k, m, n, D + 1)
