@@ -893,10 +893,11 @@ struct PairCross : MaybeDealt {
   // Schwarz; every partial sum too) with |a|^2 <= 2 *norm_a, |b|^2 <= 2
   // *norm_b over a whole group (two windows), <= *norm_a, *norm_b over half
   // of one; a quarter holds at most 256 products of 2^16.  FP32 is exact up
-  // to 2^24, so whole groups where 4 *norm_a *norm_b <= 2^48.
+  // to 2^24, so whole groups where 4 *norm_a *norm_b <= 2^48.  (Rows of non-finite
+  // entries can have any norm; n2 cannot wrap, 4 n2 could.)
   __device__ int cuts() const {
     const unsigned long long n2 = (unsigned long long)*norm_a * *norm_b;
-    return mdgi::cross_groups(KB) * (4 * n2 <= 1ull << 48 ? 1 : n2 <= 1ull << 48 ? 2 : 4);
+    return mdgi::cross_groups(KB) * (n2 <= 1ull << 46 ? 1 : n2 <= 1ull << 48 ? 2 : 4);
   }
   __device__ CrossJob job(int u) const {
     const int MB = Mp / 256, NB = Np / TN2, tiles = MB * NB;

@@ -122,3 +122,36 @@ def test_renorm_of_whole_diagonals(p, m, n, k, kw):
     A = api.generate("normal", p, m, k, 31, -9, 9, scale_rows=True)
     B = api.generate("uniform", p, k, n, 32)
     assert torch.equal(api.gemm(A, B, **kw), api.gemm(A, B, engine="tc", **kw))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("even,odd,infinite", [(-70, -71, False), (-128, -127, False),
+                                               (-128, -127, True)])
+def test_flush_interval_of_uneven_digits(even, odd, infinite):
+    """Products of sums of about 141^2 and 255^2 that differ from k to k, so that
+    1024 of them lose bits in FP32.  infinite: besides, a row of A and a column of
+    B with an infinity and digits beyond 128; the norms of their sums, 2^31 each,
+    must not make the interval of the others longer (4 x 2^62 is 0 modulo 2^64)."""
+    import torch
+    api = pkg("api")
+    p, n, r, c = 4, 1024, 5, 7
+    digits = [-70] + [odd if i & 1 else even for i in range(1, api.default_slices(p))]
+    one, two = (torch.from_numpy(_constant(api, p, n, n, x)).cuda()
+                for x in (digits, [d + (i & 1) for i, d in enumerate(digits)]))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A, B = (torch.where(torch.rand((n, n, 1), generator=g, device="cuda") < 0.5, one, two)
+            for _ in range(2))
+    if infinite:
+        A[r] = 0
+        A[r, 0, 0] = float("inf")
+        e = int(api.scale_exponents(A, B)[0][r])
+        A[r, 1:3, 0] = 2.0 ** (8 + e)  # leading digit 2^15, twice in a window
+        B[:, c] = A[r]
+        d = api.slice_digits(A, api.scale_exponents(A, B)[0], len(digits))[:, r].float()
+        assert d[0, 1:3].tolist() == [2.0 ** 15] * 2 and float(d.abs().sum()) == 2.0 ** 16
+    got, want = api.gemm(A, B), api.gemm(A, B, engine="tc")
+    if infinite:
+        for x in (got, want):
+            x[r] = 0
+            x[:, c] = 0
+    assert torch.equal(got, want)
