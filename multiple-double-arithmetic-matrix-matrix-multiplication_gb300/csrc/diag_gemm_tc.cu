@@ -1269,13 +1269,34 @@ struct Unit {
   int id;
 };
 
-// A unit's cost in k-steps: its own, about 6 per run for the drain and the
-// store, about 10 to fill and empty the pipeline.
-template <class Runs>
-long long unit_cost(Runs runs) {
-  long long cost = 10;
-  for (Run r; runs.next(r);) cost += r.steps + 6;
+// The costs in k-steps of the `parts` parts that `all` is cut into: a part's own
+// steps, about 6 per run for the drain and the store, about 10 to fill and empty
+// the pipeline.  A run of size(run) belongs to the part whose 1/parts of `total`
+// it starts in, as part_runs and cross_part cut; all in one walk, since a walk a
+// part cost the host more than the rest of a call (hd 256^3 147 us a call).
+// runs: how many each part has.
+template <class Runs, class Size>
+std::vector<long long> part_costs(Runs all, long long total, int parts, const Size &size,
+                                  std::vector<int> *runs = nullptr) {
+  std::vector<long long> cost(parts, 10);
+  if (runs) runs->assign(parts, 0);
+  long long at = 0;
+  for (Run r; all.next(r); at += size(r)) {
+    const int part = (int)(((at + 1) * parts - 1) / total);
+    cost[part] += r.steps + 6;
+    if (runs) ++(*runs)[part];
+  }
   return cost;
+}
+
+// The same over digit planes (part_runs).
+std::vector<long long> digit_part_costs(int s, int D, int KB, int cs, int stack, int parts) {
+  const DigitRuns all = part_runs(s, D, KB, cs, stack, 0, 1);
+  long long steps = 0, runs = 0;
+  DigitRuns it = all;
+  for (Run r; it.next(r); ++runs) steps += r.steps;
+  if (parts == runs) return part_costs(all, runs, parts, [](const Run &) { return 1; });
+  return part_costs(all, steps, parts, [](const Run &r) { return r.steps; });
 }
 
 // Each unit, in the order given, to the worker with the least so far; the
@@ -1285,21 +1306,21 @@ long long deal_in_order(const std::vector<Unit> &units, int workers, std::vector
   typedef std::pair<long long, int> Load;
   std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
   for (int w = 0; w < workers; ++w) least.push(Load(0, w));
-  std::vector<std::vector<int>> of(workers);
+  std::vector<int> of(units.size());  // the unit's worker
+  starts->assign(workers + 1, 0);
   long long most = 0;
-  for (const Unit &u : units) {
+  for (size_t i = 0; i < units.size(); ++i) {
     const Load l = least.top();
     least.pop();
-    of[l.second].push_back(u.id);
-    least.push(Load(l.first + u.cost, l.second));
-    most = std::max(most, l.first + u.cost);
+    of[i] = l.second;
+    ++(*starts)[l.second + 1];
+    least.push(Load(l.first + units[i].cost, l.second));
+    most = std::max(most, l.first + units[i].cost);
   }
-  starts->assign(1, 0);
-  order->clear();
-  for (const auto &list : of) {
-    order->insert(order->end(), list.begin(), list.end());
-    starts->push_back((int)order->size());
-  }
+  for (int w = 0; w < workers; ++w) (*starts)[w + 1] += (*starts)[w];
+  std::vector<int> next(starts->begin(), starts->end() - 1);
+  order->resize(units.size());
+  for (size_t i = 0; i < units.size(); ++i) (*order)[next[of[i]]++] = units[i].id;
   return most;
 }
 
@@ -1322,24 +1343,26 @@ long long deal_in_order(const std::vector<Unit> &units, int workers, std::vector
 constexpr int kCrossDealParts = 48;
 constexpr long long kCrossDealSteps = 7000;
 
-// cost(part, parts): of a unit, 0 where it has no runs; fine: the parts to deal.
-template <class Cost>
-bool deal_single(int tiles, int fine, const Cost &cost, int ncl, PairSchedule *sc,
+// costs(parts): of a tile's parts, 0 for one that has no runs; fine: the parts to
+// deal.
+template <class Costs>
+bool deal_single(int tiles, int fine, const Costs &costs, int ncl, PairSchedule *sc,
                  UnitDeal *deal) {
   const long long all_units = (long long)tiles * fine;
   if (ncl > kDealtWorkers || all_units > kDealtUnits) return false;
   if (sc->parts == fine && all_units <= ncl) return false;  // a unit each already
   std::vector<long long> in_turn(ncl, 0);
-  for (int part = 0; part < sc->parts; ++part) {
-    const long long c = cost(part, sc->parts);
-    for (int t = 0; t < tiles; ++t) in_turn[(part * tiles + t) % ncl] += c;
-  }
-  std::vector<Unit> units;
+  const std::vector<long long> coarse = costs(sc->parts), cost = costs(fine);
+  for (int part = 0; part < sc->parts; ++part)
+    for (int t = 0; t < tiles; ++t) in_turn[(part * tiles + t) % ncl] += coarse[part];
+  std::vector<int> parts;
   for (int part = 0; part < fine; ++part)
-    if (const long long c = cost(part, fine))
-      for (int t = 0; t < tiles; ++t) units.push_back(Unit{c, part * tiles + t});
-  std::stable_sort(units.begin(), units.end(),
-                   [](const Unit &a, const Unit &b) { return a.cost > b.cost; });
+    if (cost[part]) parts.push_back(part);
+  std::stable_sort(parts.begin(), parts.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+  std::vector<Unit> units;
+  units.reserve(parts.size() * tiles);
+  for (int part : parts)
+    for (int t = 0; t < tiles; ++t) units.push_back(Unit{cost[part], part * tiles + t});
   std::vector<int> starts, order;
   if (deal_in_order(units, ncl, &starts, &order) >=
       *std::max_element(in_turn.begin(), in_turn.end()))
@@ -1437,13 +1460,17 @@ int launch_diag_gemm_cross(int s, int D, int dlo, int dhi, int squares, int sum_
   const int products = squares + cross_offset(dhi) - cross_offset(dlo);
   if (!sc.as_asked &&
       (long long)tiles * products * KB <= kCrossDealSteps * (sms / 2)) {
-    auto cost = [&](int part, int of) -> long long {
-      const CrossRuns r =
-          cross_part(D, dlo, dhi, squares, plane0, ppc, KB, cross_groups(KB), part, of);
-      return r.planes > 0 ? unit_cost(r) : 0;
+    auto costs = [&](int of) {
+      std::vector<int> runs;
+      std::vector<long long> cost = part_costs(
+          cross_part(D, dlo, dhi, squares, plane0, ppc, KB, cross_groups(KB), 0, 1), products, of,
+          [KB](const Run &r) { return r.steps / KB; }, &runs);
+      for (int part = 0; part < of; ++part)
+        if (!runs[part]) cost[part] = 0;
+      return cost;
     };
     const int fine = std::min(products, std::min(kCrossDealParts, kDealtUnits / tiles));
-    dealt = fine > 0 && deal_single(tiles, fine, cost, sms / 2, &sc, &deal);
+    dealt = fine > 0 && deal_single(tiles, fine, costs, sms / 2, &sc, &deal);
   }
   diag_gemm_cross_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
       ma, mb, mc, D, dlo, dhi, squares, plane0, ppc, Mp, Np, KB, sc.parts, sc.raster, norm_a, norm_b,
@@ -1499,11 +1526,9 @@ int launch_diag_gemm_tc(int s, int D, int Mp, int Np, int Kp, int m, int n, int 
     const int separable = stack ? (D + 1) / 2 : runs;
     PairSchedule sc = pair_schedule(mt, nt, separable, sms, parts_opt, raster_opt, pace_opt);
     UnitDeal deal = {};
-    auto cost = [&](int part, int parts) {
-      return unit_cost(part_runs(s, D, Kp / TK, cs, stack, part, parts));
-    };
+    auto costs = [&](int parts) { return digit_part_costs(s, D, Kp / TK, cs, stack, parts); };
     const bool dealt = !sc.as_asked &&
-                       deal_single(mt * nt, separable, cost, sms / 2, &sc, &deal);
+                       deal_single(mt * nt, separable, costs, sms / 2, &sc, &deal);
     diag_gemm_tc2_kernel<<<2 * sc.clusters, THREADS2, SMEM2_BYTES, st>>>(
         ma, mb, mc, s, D, Mp, Np, Kp / TK, cs, stack, (k - (Kp - TK) + 15) / 16, mt, nt, sc.parts,
         sc.raster, sc.pace, sc.epoch, sc.no_loads, dealt, deal);
@@ -1538,13 +1563,14 @@ int encode_out_map(void *map128, const void *base, int Np, long long rows_total)
 int deal_units(const std::vector<GroupedProblem> &probs, int workers, std::vector<int> *starts,
                std::vector<int> *order) {
   std::vector<Unit> units;
-  for (const GroupedProblem &g : probs)
-    for (int part = 0; part < g.parts; ++part) {
-      const long long cost = unit_cost(part_runs(g.s, g.D, g.KB, CHUNK_STEPS, g.stack, part, g.parts));
+  for (const GroupedProblem &g : probs) {
+    const std::vector<long long> cost =
+        digit_part_costs(g.s, g.D, g.KB, CHUNK_STEPS, g.stack, g.parts);
+    for (int part = 0; part < g.parts; ++part)
       for (int tile = 0; tile < g.mt * g.nt; ++tile)
-        units.push_back(Unit{cost * (g.tn == 128 && !g.stack ? 2 : 4),
+        units.push_back(Unit{cost[part] * (g.tn == 128 && !g.stack ? 2 : 4),
                              g.unit_begin + part * g.mt * g.nt + tile});
-    }
+  }
   deal_in_order(units, workers, starts, order);
   return MDG_SUCCESS;
 }

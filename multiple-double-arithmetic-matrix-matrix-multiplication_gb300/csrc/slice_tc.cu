@@ -374,9 +374,16 @@ static int chunk_steps(int s, int D, int m, int n, int KB) {
       stacked_us(s, D, m, n, KB) < chunked_us(s, D, KB, tiles, tn))
     return CHUNK_STEPS;
   const int least = std::max(8, (int)(share + 3) / 4 * 4);
-  for (int cs = least; cs <= 2 * least; cs += 4)
-    if (tiles * total_chunks(s, D, KB, cs) <= workers) return cs;
-  return least;
+  // (longer chunks are never more)
+  int lo = 0, hi = least / 4 + 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (tiles * total_chunks(s, D, KB, least + 4 * mid) <= workers)
+      hi = mid;
+    else
+      lo = mid + 1;
+  }
+  return lo <= least / 4 ? least + 4 * lo : least;
 }
 
 SlicePlan best_slice_plan(int p, int s, int D, int m, int n, int k) {

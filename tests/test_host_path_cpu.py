@@ -155,3 +155,43 @@ def test_renormalisation_takes_two_columns_a_thread(fake, m, n, columns):
     for p in (2, 4, 8):
         names = [line[1] for line in fake("renorm", p, m, n, 500) if line[0] == "launch"]
         assert names == [f"renorm_kernelILi{columns}EEE"]
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 256, 256), (500, 500, 70)])
+def test_host_time_of_a_dealt_call(fake, m, n, k):
+    """The host deals the units of a hexa-double problem of few tiles in a walk
+    over its runs (a few times the cost of one that is not dealt), not in a walk
+    a part (eight and more times)."""
+    import time
+
+    def seconds(calls, *shape):
+        best = 1e9
+        for _ in range(5):
+            t = time.perf_counter()
+            fake(*(["gemm", 2, 16, *shape] * calls))
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    plain, dealt = (seconds(1501, *s) - seconds(1, *s) for s in ((64, 64, 64), (m, n, k)))
+    assert dealt < 4.5 * plain, (dealt, plain)
+
+
+def test_the_smaller_workspace_is_asked_for_when_memory_is_short(monkeypatch):
+    """api.gemm's workspace: what the call can do without is worked out only after
+    an allocation failed."""
+    import torch
+    api = pkg("api")
+    ws, got = api._workspace(4096, lambda: pytest.fail("memory was there"), "cpu")
+    assert (ws.numel(), got) == (4096, 4096)
+    empty = torch.empty
+
+    def short(n, **kw):
+        if n > 3000:
+            raise torch.OutOfMemoryError("short")
+        return empty(n, **kw)
+
+    monkeypatch.setattr(api.torch, "empty", short)
+    ws, got = api._workspace(4096, lambda: 1096, "cpu")
+    assert (ws.numel(), got) == (3000, 3000)
+    with pytest.raises(torch.OutOfMemoryError):
+        api._workspace(4096, lambda: 0, "cpu")
