@@ -191,10 +191,12 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[32]) {
 }
 
 // The accumulator holds integer-valued floats with |x| <= 2^24; the
-// conversion to int32 is exact.
+// conversion to int32 is exact.  Sums of sum planes' products are taken modulo
+// 2^32 (cross_sums.cuh), so without sign.
 __device__ __forceinline__ void add_exact(int *acc, const uint32_t (&r)[32]) {
 #pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] += __float2int_rn(__uint_as_float(r[j]));
+  for (int j = 0; j < 32; ++j)
+    acc[j] = (int)((uint32_t)acc[j] + (uint32_t)__float2int_rn(__uint_as_float(r[j])));
 }
 
 // Adds 128 accumulator columns (starting at taddr) into acc: four 32-column
