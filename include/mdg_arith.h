@@ -69,9 +69,11 @@ static inline bool is_zero(double x) { return x == 0.0; }
 /* s + err == a + b exactly for any a, b.  Host: Knuth's six operations.
  * Device: Dekker's three on the operands in order; b - (s - a) is exact where
  * the exponent of a is not below that of b, which the high words decide.
- * The error is the same number; the two cases in which Knuth's operations
+ * The error is the same number; two cases in which Knuth's operations
  * return something else are restored: an error of -0 (b = -0) is +0 there,
- * and NaN where s overflows or is not finite. */
+ * and NaN where s overflows or is not finite.  A third is not: where s is finite
+ * but s - a overflows, next to the largest double (a = -3 2^970, b = DBL_MAX),
+ * theirs is NaN and this one the error. */
 MDG_HD double two_sum(double a, double b, double *err) {
   double s = a + b;
 #if defined(__CUDA_ARCH__)

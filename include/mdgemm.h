@@ -120,7 +120,9 @@ size_t mdg_gemm_least_workspace_size(int form, int p, int m, int n, int k,
 
 /* C = A * B, all device pointers, asynchronous on `stream`.
  * Replaces matmulTCnt (TCcuda.cu:248, form PLAIN) and the split GEMM of
- * TCtest.cu:48-114 (form FP64_SPLIT); any m, n, k >= 0. */
+ * TCtest.cu:48-114 (form FP64_SPLIT); any m, n, k >= 0.  The digit forms are for
+ * finite entries: a row of A or a column of B with an infinity or a NaN leaves its
+ * row or column of C unspecified, and no other. */
 int mdg_gemm(int form, int p, int m, int n, int k, const double *A, int lda,
              const double *B, int ldb, double *C, int ldc,
              const mdg_options *opt, void *workspace, size_t workspace_bytes,
@@ -231,7 +233,7 @@ int mdg_batch_tune(mdg_batch batch, void *stream);
  * or one the caller made current) looks up the array's device address and
  * should come before any stream capture; a context created later, e.g.
  * after cudaDeviceReset, gets its own lookup.  Calls share the array and it
- * keeps the last call's contents (each call writes every region it reads):
+ * keeps the last call's contents (what reaches C is written by each call):
  * calls that overlap on the GPU race, so order them on one stream. */
 size_t mdg_static_scratch_bytes(void);
 int mdg_gemm_slice_static(int p, int m, int n, int k, const double *A, int lda,

@@ -133,14 +133,7 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
          ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(IDESC), "r"(acc));
-}
-
-// The same with a run-time instruction descriptor (tile width per job).
+// idesc: IDESC with the tile width of the job.
 __device__ __forceinline__ void mma_bf16_n(uint32_t d_tmem, uint64_t a, uint64_t b,
                                            uint32_t idesc, uint32_t acc) {
   asm volatile(

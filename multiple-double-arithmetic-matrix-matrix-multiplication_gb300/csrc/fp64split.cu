@@ -40,11 +40,13 @@ struct ConvStrides {
 // the SM alone in 540, so the two operand loads of a DMMA need no reuse; what
 // counts is that every SM quarter gets an equal share to the end.  Diagonal i
 // costs i / 4 + 1 chunks a k: so the tiles are the smallest, the dear
-// diagonals come first, and kDynamicSmem holds back all but 17 blocks per
+// diagonals come first, and kDynamicSmem holds back all but 16 blocks per
 // SM, so that an SM takes its next block as it finishes one.  With 64 x 32
 // tiles of four warps, all resident at once: qd 251 x 300 x 277 8.98 -> 6.49
 // ms a call, qd 100^3 1.02 -> 0.42, dd 64^3 0.35 -> 0.08, qd 512^3 41.1 ->
-// 39.9 (1.02 of the DGEMM rate for the chunks done).
+// 39.9 (1.02 of the DGEMM rate for the chunks done).  On slice planes, whose
+// loads touch a sector each: 16 planes of 251 x 300 x 277 8.86 -> 6.34 ms, 512^3
+// 41.8 -> 39.5, 12 of 300 x 100 x 900 10.3 -> 5.1.
 constexpr int kDynamicSmem = 13000;
 
 __global__ void __launch_bounds__(32)

@@ -1,5 +1,6 @@
-// Fixed-width two's complement integers in registers, used by the digit
-// split and by the renormalisation of the slice-digit form.  Word 0 is the
+// Fixed-width two's complement integers in registers, used by the digit split and
+// the diagonal sums of the FP64 digit form (digits64.cu); the exact significand
+// and the scale exponent of both digit forms.  Word 0 is the
 // least significant.  Every loop is unrolled over the compile-time width so
 // that the words stay in registers; positions that vary at run time are
 // handled with predicated selects instead of indexed accesses.

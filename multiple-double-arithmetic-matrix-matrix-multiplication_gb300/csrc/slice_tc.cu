@@ -570,12 +570,6 @@ int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, voi
                        ldc, st);
 }
 
-int slice_panel(const SlicePlan &pl, int rows, const double *A, int lda, double *C, int ldc,
-                void *ws, int engine, int parts, int raster, cudaStream_t st, int pace) {
-  MDG_TRY(slice_panel_a(pl, rows, A, lda, ws, st));
-  return slice_block(pl, ws, pl, ws, rows, C, ldc, engine, parts, raster, st, pace);
-}
-
 int run_slice_gemm(const SlicePlan &pl, const double *A, int lda, const double *B, int ldb,
                    double *C, int ldc, void *ws, int engine, int parts, int raster,
                    cudaStream_t st, int pace, int trans_a, int trans_b) {

@@ -172,21 +172,14 @@ int slice_gemm(int p, int m, int n, int k, const double *A, int lda, int trans_a
                int ldb, int trans_b, double *C, int ldc, const mdg_options *opt, void *workspace,
                size_t workspace_bytes, void *stream);
 
-// run_slice_gemm in two parts, for callers that split A into row panels
-// (the pipelined host path): slice_prepare_b computes the column exponents
-// and digits of B once; slice_panel then computes rows (<= pl.m) rows of C
-// from the matching rows of A.  Every row of C depends only on its row of A
-// and on all of B, so panels give the bits of one run_slice_gemm.
+// run_slice_gemm in parts, for the host entry, which splits A into row panels and
+// B into column strips (each with its own plan and workspace): slice_prepare_b
+// computes a strip's exponents, digits and sums once, slice_panel_a those of
+// rows (<= pl.m) rows of A into wsa, slice_block then those rows of C against the
+// strip of plb / wsb (plans of equal m, k, s, D).  A row of C depends only on its
+// row of A and a column only on its column of B, so blocks give the bits of one
+// run_slice_gemm.
 int slice_prepare_b(const SlicePlan &pl, const double *B, int ldb, void *ws, cudaStream_t st);
-int slice_panel(const SlicePlan &pl, int rows, const double *A, int lda, double *C, int ldc,
-                void *ws, int engine, int parts, int raster, cudaStream_t st, int pace = 0);
-// slice_panel in two parts, for callers that also split B into column
-// strips (each with its own plan and workspace, prepared by
-// slice_prepare_b): slice_panel_a computes the exponents and digits of
-// rows (<= pla.m) rows of A into wsa; slice_block then computes those rows
-// of C against the strip of plb / wsb (plans of equal m, k, s, D).  Every
-// column of C depends only on its column of B, so blocks give the bits of
-// one run_slice_gemm.
 int slice_panel_a(const SlicePlan &pl, int rows, const double *A, int lda, void *ws,
                   cudaStream_t st);
 int slice_block(const SlicePlan &pla, const void *wsa, const SlicePlan &plb, void *wsb, int rows,
