@@ -148,8 +148,9 @@ int mdg_gemm_ex(int form, int trans_a, int trans_b, int accumulate, int p, int m
                 size_t workspace_bytes, void *stream);
 
 /* C = A * B with HOST buffers: copies in, computes, copies out, waits.
- * Device memory comes from a cache owned by the library (freed by
- * mdg_release_cache).  This is the call the std::vector wrappers make. */
+ * Device memory comes from a cache owned by the library, which keeps it (A, B, C,
+ * and in the BF16 form up to 32 GiB of workspace for each of up to two column
+ * strips) until mdg_release_cache or until a later call needs the room.  This is the call the std::vector wrappers make. */
 int mdg_gemm_host(int form, int p, int m, int n, int k, const double *A,
                   const double *B, double *C, const mdg_options *opt);
 
