@@ -67,7 +67,7 @@ int launch_batch_digits(const BatchProblem *pr, int count, int units, int max_s,
                         cudaStream_t st) {
   if (units == 0) return MDG_SUCCESS;
   const int smem = digit_smem(max_s, 2);
-  MDG_TRY(allow_smem(batch_digits_kernel, digit_smem(MAX_SLICES, 2)));
+  MDG_TRY(allow_smem(batch_digits_kernel, smem, digit_smem(MAX_SLICES, 2)));
   batch_digits_kernel<<<units, DIGIT_THREADS, smem, st>>>(pr, count, exps);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;

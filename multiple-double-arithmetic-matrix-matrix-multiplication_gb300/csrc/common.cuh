@@ -57,12 +57,15 @@ bool alloc_over_limit(size_t bytes);
   } while (0)
 
 namespace mdgi {
-// Lets blocks of `kernel` have up to `most` bytes of dynamic shared memory.
-// The limit belongs to the kernel, not to a launch: all host threads share it,
-// and one that lowers it to its own call's size has another's launch refused.
-// So `most` is the same at every call, what the largest accepted call needs.
+// Lets blocks of `kernel` have `bytes` of dynamic shared memory, of at most `most`
+// at any call.  Up to 48 KiB need nothing.  Beyond, the limit that is set belongs
+// to the kernel, not to a launch: all host threads share it, and one that set its
+// own call's size would have another's launch refused.  So it is always `most`.
+// (Setting it costs the host about a microsecond; the limit of other calls is never
+// lowered, so blocks of up to 48 KiB can go without.)
 template <class Kernel>
-int allow_smem(Kernel kernel, int most) {
+int allow_smem(Kernel kernel, int bytes, int most) {
+  if (bytes <= 48 * 1024) return MDG_SUCCESS;
   MDG_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   return MDG_SUCCESS;
 }

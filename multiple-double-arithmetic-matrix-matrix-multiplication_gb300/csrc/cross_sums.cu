@@ -100,7 +100,7 @@ int launch_cross_sums(int s, int dlo, int dhi, int Kp, int rows_a, int rows_b, v
   // vectors of the longest window
   const int stride = (KB + windows - 1) / windows * 8;
   const int smem = dhi * stride * 16;
-  MDG_TRY(allow_smem(cross_sums_kernel, MAX_DIAGONALS * MAX_WINDOW * 16));
+  MDG_TRY(allow_smem(cross_sums_kernel, smem, MAX_DIAGONALS * MAX_WINDOW * 16));
   cross_sums_kernel<<<dim3(rows_a + rows_b, windows), 32 * SUM_WARPS, smem, st>>>(
       s, cross_offset(dlo), cross_offset(dhi), dhi, KB, windows, stride, rows_a,
       reinterpret_cast<__nv_bfloat16 *>(dA), reinterpret_cast<__nv_bfloat16 *>(dB), plane_a,

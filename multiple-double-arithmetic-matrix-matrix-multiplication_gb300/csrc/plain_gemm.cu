@@ -161,7 +161,7 @@ int launch_plain_batched(const mdg_problem *dev_problems, int count, int max_p,
   if (total_tiles == 0) return MDG_SUCCESS;
   constexpr size_t entry = 2 * T * T * sizeof(double);
   const size_t smem = entry * max_p;
-  MDG_TRY(allow_smem(plain_batched_kernel, (int)entry * 16));
+  MDG_TRY(allow_smem(plain_batched_kernel, (int)smem, (int)entry * 16));
   int dev = 0, sms = 0, per_sm = 0;
   MDG_TRY_CUDA(cudaGetDevice(&dev));
   MDG_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

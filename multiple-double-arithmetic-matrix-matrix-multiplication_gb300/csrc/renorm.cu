@@ -120,7 +120,7 @@ int launch_direct(int p, int s, int D, int KB, int cs, int m, int n, const int *
     most = std::max(most, nc);
   }
   const int smem = mdgi::renorm_smem(D, V, false);
-  MDG_TRY(mdgi::allow_smem(renorm_kernel<V>, mdgi::renorm_smem(mdgi::MAX_DIAGONALS, V, false)));
+  MDG_TRY(mdgi::allow_smem(renorm_kernel<V>, smem, mdgi::renorm_smem(mdgi::MAX_DIAGONALS, V, false)));
   renorm_kernel<V><<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
       p, D, planes, mdgi::renorm_top(D, most), counts, m, n, chunks, plane_c, ldcd, E, F, C, ldc, aligned16(C));
   MDG_TRY_LAUNCH();
@@ -140,7 +140,7 @@ int launch_cross(int p, int D, int KB, int m, int n, const int *out, long long p
   const bool whole = most <= 1 && D > kTwoColumnDiagonals;
   const int smem = mdgi::renorm_smem(D, V, !whole);
   const auto kernel = whole ? whole_renorm_kernel<V> : cross_renorm_kernel<V>;
-  MDG_TRY(mdgi::allow_smem(kernel, mdgi::renorm_smem(mdgi::MAX_DIAGONALS, V, !whole)));
+  MDG_TRY(mdgi::allow_smem(kernel, smem, mdgi::renorm_smem(mdgi::MAX_DIAGONALS, V, !whole)));
   kernel<<<blocks(m, n, V), RENORM_THREADS, smem, st>>>(
       p, D, mdgi::cross_outputs(D, KB), mdgi::renorm_top(D, most + 1), counts, m, n, out, plane_c, ldcd, E, F, C, ldc,
       aligned16(C));
@@ -178,7 +178,7 @@ int launch_batch_renorm(const BatchProblem *pr, int count, int units, int max_d,
                         cudaStream_t st) {
   if (units == 0) return MDG_SUCCESS;
   const int smem = renorm_smem(max_d, 2, false);
-  MDG_TRY(allow_smem(batch_renorm_kernel, renorm_smem(MAX_DIAGONALS, 2, false)));
+  MDG_TRY(allow_smem(batch_renorm_kernel, smem, renorm_smem(MAX_DIAGONALS, 2, false)));
   batch_renorm_kernel<<<units, RENORM_THREADS, smem, st>>>(pr, count, exps);
   MDG_TRY_LAUNCH();
   return MDG_SUCCESS;

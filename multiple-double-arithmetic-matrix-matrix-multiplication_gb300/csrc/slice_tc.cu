@@ -438,7 +438,7 @@ template <int V, int PL>
 static int launch_digits_v(int p, int s, const DigitSide &a, const DigitSide &b, bool wide,
                            unsigned *norms, cudaStream_t st) {
   const int smem = digit_smem(s, V);
-  MDG_TRY(allow_smem(digits_kernel<V, PL>, digit_smem(MAX_SLICES, V)));
+  MDG_TRY(allow_smem(digits_kernel<V, PL>, smem, digit_smem(MAX_SLICES, V)));
   const long long of_a = digit_threads(p, a.trans, a.rows, a.cols_pad / V);
   const long long threads = of_a + digit_threads(p, b.trans, b.rows, a.cols_pad / V);
   digits_kernel<V, PL>
