@@ -58,14 +58,14 @@ bool alloc_over_limit(size_t bytes);
 
 namespace mdgi {
 // Lets blocks of `kernel` have `bytes` of dynamic shared memory, of at most `most`
-// at any call.  Up to 48 KiB need nothing.  Beyond, the limit that is set belongs
-// to the kernel, not to a launch: all host threads share it, and one that set its
-// own call's size would have another's launch refused.  So it is always `most`.
-// (Setting it costs the host about a microsecond; the limit of other calls is never
-// lowered, so blocks of up to 48 KiB can go without.)
+// at any call.  Up to 48 KiB, of which static memory takes a little, need nothing.
+// Beyond, the limit that is set belongs to the kernel, not to a launch: all host
+// threads share it, and one that set its own call's size would have another's
+// launch refused.  So it is always `most`.  (Setting it costs the host about a
+// microsecond; no call lowers it, so small blocks can go without.)
 template <class Kernel>
 int allow_smem(Kernel kernel, int bytes, int most) {
-  if (bytes <= 48 * 1024) return MDG_SUCCESS;
+  if (bytes <= 47 * 1024) return MDG_SUCCESS;
   MDG_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   return MDG_SUCCESS;
 }

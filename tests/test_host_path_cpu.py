@@ -48,6 +48,8 @@ def test_a_kernels_shared_memory_limit_is_the_same_at_every_call(fake):
                   "gemm", 0, p, 50, 60, 70]
     words += ["digits", 119, 112, "gemm", 2, 16, 64, 64, 64, "gemm", 2, 16, 1024, 1024, 1024]
     words += ["gemm", 2, 16, 1024, 1024, 20000]
+    # 48 rows of 1 KiB in the sums kernel: the default limit without static memory
+    words += ["digits", 48, 48, "gemm", 2, 4, 1024, 1024, 1024]
     lines = fake(*words)
     assert set(_statuses(lines)) == {0}
     limits, launches = {}, {}
@@ -56,10 +58,12 @@ def test_a_kernels_shared_memory_limit_is_the_same_at_every_call(fake):
             limits.setdefault(line[1], set()).add(int(line[2]))
         elif line[0] == "launch":
             launches[line[1]] = max(launches.get(line[1], 0), int(line[2]))
+            assert int(line[2]) <= 47 * 1024 or previous[:2] == ["limit", line[1]]
+        previous = line
     assert len(limits) >= 8 and len(launches) >= 20
     assert {k: v for k, v in limits.items() if len(v) > 1} == {}
     for kernel, smem in launches.items():
-        assert smem <= max(limits.get(kernel, {48 * 1024})), kernel
+        assert smem <= max(limits.get(kernel, {47 * 1024})), kernel
     assert max(max(v) for v in limits.values()) <= 227 * 1024
 
 

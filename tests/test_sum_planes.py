@@ -155,3 +155,15 @@ def test_flush_interval_of_uneven_digits(even, odd, infinite):
             x[r] = 0
             x[:, c] = 0
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("digits", [47, 48, 49])
+def test_digit_rows_around_the_default_shared_memory_limit(digits):
+    """48 digit rows of 1 KiB and a few bytes of static memory are more than a
+    block gets unasked."""
+    import torch
+    api = pkg("api")
+    A, B = api.generate("uniform", 4, 800, 1024, 61), api.generate("normal", 4, 1024, 800, 62)
+    kw = {"slices": digits, "diagonals": digits}
+    assert torch.equal(api.gemm(A, B, **kw), api.gemm(A, B, engine="tc", **kw))
