@@ -202,7 +202,9 @@ enum {
   MDG_BATCH_TILES_PAIR = 3
 };
 /* Re-deals the plan's tiles under `policy` (uploads the tile table and
- * synchronises `stream`; not during a capture).  mdg_batch_tiles returns
+ * synchronises `stream`; not during a capture).  CTA pairs are another kernel: a
+ * graph that captured mdg_batch_run must be captured again when the policy changes
+ * to or from MDG_BATCH_TILES_PAIR, by mdg_batch_tune too.  mdg_batch_tiles returns
  * the policy in use; a new plan starts with the policy recorded by
  * mdg_batch_tune for its problem shapes, else MDG_BATCH_TILES_256. */
 int mdg_batch_set_tiles(mdg_batch batch, int policy, void *stream);

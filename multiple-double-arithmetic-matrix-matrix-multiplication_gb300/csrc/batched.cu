@@ -37,7 +37,7 @@ struct mdg_batch_s {
   int tiles_policy = MDG_BATCH_TILES_256, split = 1;
   mdgi::BatchProblem *dprobs = nullptr;
   mdgi::GroupedProblem *dgroups = nullptr;
-  int *deal = nullptr;  // starts of the workers' lists, then the lists
+  int *deal = nullptr;  // starts of the workers' lists, the lists at kMaxWorkers + 1
   int *exps = nullptr;  // E of all problems then F
   std::vector<mdgi::BatchProblem> hprobs;  // host copy of the table
 };
@@ -270,15 +270,17 @@ int apply_tiles(mdg_batch_s *h, int policy, int split, cudaStream_t st) {
   std::vector<int> starts, order;
   int units = 0;
   MDG_TRY(grouped_table(h->hprobs, policy, split, all, &hg, &units));
-  const int workers = std::min(units, all);
-  MDG_TRY(mdgi::deal_units(hg, workers, &starts, &order));
+  // as many workers and the lists in the same place whatever the number of units:
+  // a launch that a graph captured before finds the present ones
+  MDG_TRY(mdgi::deal_units(hg, all, &starts, &order));
+  starts.resize(kMaxWorkers + 1, units);
   starts.insert(starts.end(), order.begin(), order.end());
   MDG_TRY_CUDA(cudaMemcpyAsync(h->deal, starts.data(), sizeof(int) * starts.size(),
                                cudaMemcpyHostToDevice, st));
   MDG_TRY_CUDA(cudaMemcpyAsync(h->dgroups, hg.data(), sizeof(mdgi::GroupedProblem) * h->count,
                                cudaMemcpyHostToDevice, st));
   MDG_TRY_CUDA(cudaStreamSynchronize(st));
-  h->workers = workers;
+  h->workers = all;
   h->tiles_policy = policy;
   h->split = split;
   return MDG_SUCCESS;
@@ -356,7 +358,7 @@ int mdg_batch_run(mdg_batch_s *h, void *stream) {
   MDG_TRY(mdgi::launch_batch_scale(h->dprobs, h->count, h->scale_units, h->exps, st));
   MDG_TRY(mdgi::launch_batch_digits(h->dprobs, h->count, h->digit_units, h->max_d, h->exps, st));
   MDG_TRY(mdgi::launch_diag_gemm_grouped(h->dgroups, h->count, h->workers, h->deal,
-                                         h->deal + h->workers + 1,
+                                         h->deal + kMaxWorkers + 1,
                                          h->tiles_policy == MDG_BATCH_TILES_PAIR, st));
   MDG_TRY(mdgi::launch_batch_renorm(h->dprobs, h->count, h->renorm_units, h->max_d, h->exps, st));
   return MDG_SUCCESS;

@@ -12,7 +12,9 @@
 //   host P M N K             mdg_gemm_host, BF16 form
 //   plan P M N K             mdg_plan_create, its schedule, mdg_plan_destroy
 //   tune P M N K             the same with mdg_plan_tune before
-//   batch P M N K            mdg_batch_create and mdg_batch_run of one problem
+//   batch P M N K            mdg_batch_create and mdg_batch_run of one problem, then
+//                            with the split mode off: what the first run's launch of
+//                            the grouped GEMM, replayed, finds in the second's tables
 //   batched FORM P M N K     mdg_gemm_batched of one problem
 //   renorm P M N K           mdg_renorm_diagonals, default digits
 //   save PATH / load PATH    the tuning cache
@@ -20,6 +22,7 @@
 //   limit KERNEL BYTES       cudaFuncAttributeMaxDynamicSharedMemorySize
 //   launch KERNEL SMEM [stack=S] [pace=P dealt=D]
 //   malloc BYTES / oom BYTES / free BYTES
+//   replay UNIT ..           the units that the replayed launch takes, in order
 //   status COMMAND STATUS [engine parts raster pace]
 #include <cuda.h>
 #include <cuda_runtime_api.h>
@@ -66,6 +69,30 @@ std::string plain_name(const std::string &mangled) {
   std::string name = mangled.substr(i, len), rest = mangled.substr(i + len);
   if (!rest.empty() && rest[0] == 'I') name += rest.substr(0, rest.find('v'));
   return name;
+}
+
+// The grouped GEMM's launches, and the words last copied to the device.
+struct Grouped {
+  unsigned workers;
+  const int *starts, *order;
+};
+std::vector<Grouped> grouped;
+std::map<uintptr_t, int> device_words;
+bool recording = false;  // (during batch commands)
+
+// The units that a launch's workers find there; -1: no such word was written.
+std::vector<int> units_of(const Grouped &g) {
+  auto word = [](const int *p) {
+    const auto it = device_words.find((uintptr_t)p);
+    return it == device_words.end() ? -1 : it->second;
+  };
+  std::vector<int> units;
+  for (unsigned w = 0; w < g.workers; ++w) {
+    const int first = word(g.starts + w), last = word(g.starts + w + 1);
+    if (first < 0 || last < 0 || last - first > 1 << 20) return {-1};
+    for (int i = first; i < last; ++i) units.push_back(word(g.order + i));
+  }
+  return units;
 }
 
 template <class T>
@@ -122,7 +149,7 @@ cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *fun) {
   *k = reinterpret_cast<cudaKernel_t>(const_cast<void *>(fun));
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t kernel, dim3, dim3, void **args, size_t smem,
+cudaError_t __cudaLaunchKernel(cudaKernel_t kernel, dim3 grid, dim3, void **args, size_t smem,
                                cudaStream_t) {
   const std::string name = kernels()[kernel];
   std::printf("launch %s %zu", name.c_str(), smem);
@@ -135,6 +162,8 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t kernel, dim3, dim3, void **args, siz
   } else if (name == "diag_gemm_cross_kernel") {
     std::printf(" pace=%d dealt=%d", arg<int>(args, 16), arg<int>(args, 19));
   }
+  if (name.find("grouped") != std::string::npos)
+    grouped.push_back(Grouped{grid.x, arg<const int *>(args, 2), arg<const int *>(args, 3)});
   std::printf("\n");
   return cudaSuccess;
 }
@@ -218,7 +247,11 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *, const void *, size_t, enum cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t bytes, enum cudaMemcpyKind kind,
+                            cudaStream_t) {
+  if (recording && kind == cudaMemcpyHostToDevice)
+    for (size_t i = 0; i + 4 <= bytes; i += 4)
+      std::memcpy(&device_words[(uintptr_t)to + i], (const char *)from + i, 4);
   return cudaSuccess;
 }
 cudaError_t cudaMemcpy2DAsync(void *, size_t, const void *, size_t, size_t, size_t,
@@ -283,8 +316,16 @@ int main(int argc, char **argv) {
       } else if (cmd == "batch") {
         const mdg_problem q{p, m, n, k, dev, dev, dev_out, k, n, n};
         mdg_batch batch = nullptr;
+        recording = true;
         status = mdg_batch_create(&q, 1, dev_out, mdg_batch_workspace_size(&q, 1), nullptr, &batch);
         if (status == 0) status = mdg_batch_run(batch, nullptr);
+        if (status == 0) status = mdg_batch_set_split(batch, 0, nullptr);
+        if (status == 0) {
+          std::printf("replay");
+          for (int u : units_of(grouped.back())) std::printf(" %d", u);
+          std::printf("\n");
+        }
+        recording = false;
         mdg_batch_destroy(batch);
       } else {
         std::fprintf(stderr, "unknown command %s\n", cmd.c_str());

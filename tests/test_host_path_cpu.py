@@ -199,3 +199,13 @@ def test_the_smaller_workspace_is_asked_for_when_memory_is_short(monkeypatch):
     assert (ws.numel(), got) == (3000, 3000)
     with pytest.raises(torch.OutOfMemoryError):
         api._workspace(4096, lambda: 0, "cpu")
+
+
+@pytest.mark.parametrize("p,m,n,k", [(2, 40, 40, 40), (8, 500, 300, 200), (16, 2000, 1500, 100)])
+def test_a_captured_batch_finds_its_units_after_the_split_mode_changed(fake, p, m, n, k):
+    """A graph captured with heavy tiles split, replayed after mdg_batch_set_split(0):
+    the launch it holds takes each of the new table's units (tiles) once."""
+    lines = fake("batch", p, m, n, k)
+    assert _statuses(lines) == [0]
+    units = [int(u) for line in lines if line[0] == "replay" for u in line[1:]]
+    assert sorted(units) == list(range(-(-m // 128) * -(-n // 256)))
