@@ -89,9 +89,12 @@ def workspace_size(form, p, m, n, k, **kw):
     return lib().mdg_gemm_workspace_size(FORMS[form], p, m, n, k, ctypes.byref(_opts(**kw)))
 
 
-def _workspace(need, spare, device):
-    """`need` bytes on the device, or, where they are not to be had, need -
-    spare(): the BF16 form gives the same bits without its sum planes."""
+def _workspace(need, spare, device, given=None):
+    """The caller's workspace where it holds need - spare() bytes (the BF16 form
+    gives the same bits without its sum planes), else `need` bytes on the
+    device, or need - spare() where those are not to be had; and its size."""
+    if given is not None and (given.numel() >= need or given.numel() >= need - spare()):
+        return given, min(given.numel(), need)
     try:
         return torch.empty(need, dtype=torch.uint8, device=device), need
     except torch.OutOfMemoryError:
@@ -118,8 +121,9 @@ def gemm(A, B, form="slice_bf16", out=None, workspace=None, stream=None, **kw):
     C = out if out is not None else torch.empty((m, n, p), dtype=torch.float64, device=A.device)
     opt = _opts(**kw)
     need = lib().mdg_gemm_workspace_size(FORMS[form], p, m, n, k, ctypes.byref(opt))
-    if need and (workspace is None or workspace.numel() < need):
-        workspace, need = _workspace(need, lambda: _spare(form, p, m, n, k, opt), A.device)
+    if need:
+        workspace, need = _workspace(need, lambda: _spare(form, p, m, n, k, opt), A.device,
+                                     workspace)
     check(lib().mdg_gemm(FORMS[form], p, m, n, k, _ptr(A), max(k, 1), _ptr(B), max(n, 1),
                          _ptr(C), max(n, 1), ctypes.byref(opt), _ptr(workspace) if need else None,
                          need, _stream(stream)), "mdg_gemm")
@@ -157,8 +161,9 @@ def gemm_ex(A, B, form="slice_bf16", trans_a=False, trans_b=False, C=None, accum
     f = FORMS[form]
     need = lib().mdg_gemm_ex_workspace_size(f, int(trans_a), int(trans_b), int(accumulate), p, m,
                                             n, k, ctypes.byref(opt))
-    if need and (workspace is None or workspace.numel() < need):
-        workspace, need = _workspace(need, lambda: _spare(form, p, m, n, k, opt), A.device)
+    if need:
+        workspace, need = _workspace(need, lambda: _spare(form, p, m, n, k, opt), A.device,
+                                     workspace)
     check(lib().mdg_gemm_ex(f, int(trans_a), int(trans_b), int(accumulate), p, m, n, k,
                             _ptr(A), _ld(A, p), _ptr(B), _ld(B, p), _ptr(C), _ld(C, p),
                             ctypes.byref(opt), _ptr(workspace) if need else None, need,

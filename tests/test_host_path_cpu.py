@@ -209,3 +209,34 @@ def test_a_captured_batch_finds_its_units_after_the_split_mode_changed(fake, p, 
     assert _statuses(lines) == [0]
     units = [int(u) for line in lines if line[0] == "replay" for u in line[1:]]
     assert sorted(units) == list(range(-(-m // 128) * -(-n // 256)))
+
+
+def test_a_callers_workspace_without_room_for_sum_planes_is_used():
+    """One made for the digit pairs, as mdg_gemm takes it; a smaller one is not."""
+    import torch
+    api = pkg("api")
+    for size, used in ((8000, 4096), (4096, 4096), (3500, 3500), (3000, 3000)):
+        given = torch.empty(size, dtype=torch.uint8)
+        ws, got = api._workspace(4096, lambda: 1096, "cpu", given)
+        assert ws is given and got == used
+    given = torch.empty(2999, dtype=torch.uint8)
+    ws, got = api._workspace(4096, lambda: 1096, "cpu", given)
+    assert ws is not given and ws.numel() == got == 4096
+
+
+@pytest.mark.gpu
+def test_gemm_in_a_callers_workspace_for_digit_pairs():
+    import torch
+    api, L = pkg("api"), pkg("_lib").lib()
+    p, n = 4, 1024
+    A, B = api.generate("uniform", p, n, n, 1), api.generate("uniform", p, n, n, 2)
+    ref = api.gemm(A, B)
+    ws = torch.empty(L.mdg_gemm_least_workspace_size(2, p, n, n, n, None), dtype=torch.uint8,
+                     device="cuda")
+    out = torch.empty_like(ref)
+    free = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    api.gemm(A, B, out=out, workspace=ws)
+    assert torch.cuda.max_memory_allocated() == free and torch.equal(out, ref)
+    ex = api.gemm_ex(A, B.transpose(0, 1).contiguous(), trans_b=True, C=out, workspace=ws)
+    assert torch.equal(ex, ref)
